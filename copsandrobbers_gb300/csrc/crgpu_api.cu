@@ -88,6 +88,8 @@ struct cr_solver {
     uint32_t* d_nbr = nullptr;
     uint32_t* d_iso = nullptr;
     uint32_t* d_rhop = nullptr;
+    uint16_t* d_ell = nullptr;        // hop lists of the last column's tile form
+    uint32_t* d_ell_off = nullptr;
     uint8_t* d_cover = nullptr;   // first-pass neighbour-slot masks (p = 1, max degree <= 32)
     int cover_w = 0, npad = 0;
     ColMeta* d_meta = nullptr;
@@ -294,7 +296,7 @@ static void free_v1(cr_solver* s) {
     void* ptrs[] = {s->d_rp, s->d_col, s->d_binom, s->d_configs, s->d_hop, s->d_table,
                     s->d_marked, s->d_front, s->d_fflag, s->d_meta, s->d_counters, s->d_err,
                     s->d_heads, s->d_trans, s->d_cand, s->d_cbits, s->d_list, s->d_clist, s->d_sync,
-                    s->d_rrp, s->d_rcol, s->d_nbr, s->d_iso, s->d_rhop, s->d_cover,
+                    s->d_rrp, s->d_rcol, s->d_nbr, s->d_iso, s->d_rhop, s->d_cover, s->d_ell, s->d_ell_off,
                     s->d_crp, s->d_ccol, s->d_ciso, s->d_h1};
     for (void* q : ptrs) s->ctx->cache.put(q);   // the context keeps large blocks for reuse
     s->d_rp = nullptr; s->d_col = nullptr; s->d_binom = nullptr; s->d_configs = nullptr;
@@ -303,7 +305,7 @@ static void free_v1(cr_solver* s) {
     s->d_heads = nullptr; s->d_trans = nullptr; s->d_cand = nullptr; s->d_cbits = nullptr;
     s->d_list = nullptr; s->d_clist = nullptr; s->d_sync = nullptr;
     s->d_rrp = nullptr; s->d_rcol = nullptr; s->d_nbr = nullptr; s->d_iso = nullptr; s->d_rhop = nullptr;
-    s->d_cover = nullptr;
+    s->d_cover = nullptr; s->d_ell = nullptr; s->d_ell_off = nullptr;
     s->d_crp = nullptr; s->d_ccol = nullptr; s->d_ciso = nullptr; s->d_h1 = nullptr;
     if (s->h_pinned) cudaFreeHost(s->h_pinned);
     s->h_pinned = nullptr;
@@ -325,6 +327,8 @@ static V1Dev dev_view(const cr_solver* s) {
     d.g.nbr = s->d_nbr;
     d.g.isolated = s->d_iso;
     d.g.rhop = s->d_rhop;
+    d.g.ell = s->d_ell;
+    d.g.ell_off = s->d_ell_off;
     d.g.maxdeg = s->maxdeg;
     d.g.cover = s->d_cover;
     d.g.cover_w = s->cover_w;
@@ -409,6 +413,27 @@ static int alloc_v1(cr_solver* s) {
                 rhop[(size_t)u * s->rwp + (r >> 5)] |= 1u << (r & 31);
     CR_CUDA(ctx, cudaMalloc(&s->d_rhop, rhop.size() * 4));
     CR_CUDA(ctx, cudaMemcpyAsync(s->d_rhop, rhop.data(), rhop.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    // hop(r) as padded lists, 32 vertices side by side (the last column's tile form)
+    std::vector<uint32_t> ell_off(s->rw + 1, 0);
+    std::vector<uint16_t> ell;
+    for (int w = 0; w < s->rw; ++w) {
+        size_t longest = 0;
+        std::vector<uint16_t> of[32];
+        for (int j = 0; j < 32 && w * 32 + j < s->n; ++j) {
+            const uint32_t* h = hop.data() + (size_t)(w * 32 + j) * s->rwp;
+            for (int u = 0; u < s->n; ++u)
+                if ((h[u >> 5] >> (u & 31)) & 1u) of[j].push_back((uint16_t)u);
+            longest = std::max(longest, of[j].size());
+        }
+        for (size_t e = 0; e < longest; ++e)
+            for (int j = 0; j < 32; ++j) ell.push_back(e < of[j].size() ? of[j][e] : (uint16_t)(s->rw * 32));
+        ell_off[w + 1] = (uint32_t)(ell.size() / 32);
+    }
+    if (ell.empty()) ell.push_back(0);
+    CR_CUDA(ctx, cudaMalloc(&s->d_ell, ell.size() * 2));
+    CR_CUDA(ctx, cudaMalloc(&s->d_ell_off, ell_off.size() * 4));
+    CR_CUDA(ctx, cudaMemcpyAsync(s->d_ell, ell.data(), ell.size() * 2, cudaMemcpyHostToDevice, ctx->stream));
+    CR_CUDA(ctx, cudaMemcpyAsync(s->d_ell_off, ell_off.data(), ell_off.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
     // the cops' out-neighbour masks (capture-seed closed form) and their in-neighbour CSR
     // (push mode), both of the cops' move graph
     const std::vector<uint32_t>& crp = s->h_crp;

@@ -83,7 +83,7 @@ __host__ __device__ inline uint64_t binom_dev(int64_t n, int64_t k) {
 
 // Byte offsets of one (n, k, p) solve inside a slot.
 struct JobLayout {
-    size_t binom, configs, nbr, iso, hop, rhop, cover, table, marked, front, h1, list, clist, fflag, cand,
+    size_t binom, configs, nbr, iso, hop, rhop, ell, ell_off, cover, table, marked, front, h1, list, clist, fflag, cand,
         cbits, sync, meta, counters, err, total;
 };
 
@@ -103,6 +103,9 @@ __host__ __device__ inline JobLayout job_layout(int n, int k, int p, int S) {
     L.iso = take((size_t)rwp * 4);
     L.hop = take((size_t)n * rwp * 4);
     L.rhop = take((size_t)n * rwp * 4);
+    // neighbour lists of the last column's tile form: 32 side by side, each up to n long
+    L.ell = take((size_t)((n + 31) / 32) * 32 * n * 2);
+    L.ell_off = take((size_t)((n + 31) / 32 + 1) * 4);
     // uncovered-slot masks of the fused first pass (p = 1), up to 4 bytes per mask
     L.cover = take(p == 1 ? 2 * (size_t)n * ((n + 7) & ~7) * 4 : 0);
     L.table = take(C * (size_t)n * cols);
@@ -184,6 +187,33 @@ __device__ void build_cover(V1Dev& d, uint8_t* cov, int maxdeg) {
     __syncthreads();
 }
 
+// The padded neighbour lists of the last column's tile form (d.g.ell): row word w's 32 lists
+// take as many rows as the longest of them.  The block has a warp for every word (n <= 128).
+__device__ void build_ell(V1Dev& d, uint16_t* ell, uint32_t* off) {
+    const int n = d.g.n, rw = d.g.rw, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = warp * 32 + lane;
+    uint32_t e0 = 0, deg = 0;
+    if (r < n) {
+        e0 = d.g.row_ptr[r];
+        deg = d.g.row_ptr[r + 1] - e0;
+    }
+    const uint32_t longest = __reduce_max_sync(0xFFFFFFFFu, deg);
+    if (warp < rw && lane == 0) off[warp + 1] = longest;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        off[0] = 0;
+        for (int w = 0; w < rw; ++w) off[w + 1] += off[w];
+    }
+    __syncthreads();
+    if (warp < rw) {
+        uint16_t* at = ell + (size_t)off[warp] * 32 + lane;
+        for (uint32_t e = 0; e < longest; ++e) at[e * 32] = e < deg ? d.g.col[e0 + e] : (uint16_t)(rw * 32);
+    }
+    d.g.ell = ell;
+    d.g.ell_off = off;
+    __syncthreads();
+}
+
 // Column col's row list from its flag plane, by the whole block (after the fused first pass).
 __device__ void block_list_compact(const V1Dev& d, int col) {
     const uint8_t* f = d.fflag + (size_t)col * d.C;
@@ -260,7 +290,7 @@ __device__ int solve_job(const BatchDev& b, unsigned char* slot, int gi, int jr,
     const int maxdeg = b.maxdeg[gi];
     const bool fused = P1 && maxdeg <= 32;
     // ---- buildAuxGraph: zeroed planes, rank table, neighbour masks, configurations
-    block_fill(slot + L.nbr, 0, L.cover - L.nbr);
+    block_fill(slot + L.nbr, 0, L.ell - L.nbr);
     if (!fused) {
         block_fill(slot + L.marked, 0, L.front - L.marked);
         block_fill(d.table, kUnmarked, C * (size_t)n * cols);
@@ -302,6 +332,7 @@ __device__ int solve_job(const BatchDev& b, unsigned char* slot, int gi, int jr,
         }
     }
     __syncthreads();
+    if (P1) build_ell(d, reinterpret_cast<uint16_t*>(slot + L.ell), reinterpret_cast<uint32_t*>(slot + L.ell_off));
     if (!P1) {
         for (int r = threadIdx.x; r < n; r += blockDim.x) {
             uint32_t cur[kBatchMaxN / 32], nxt[kBatchMaxN / 32];
@@ -383,7 +414,7 @@ __device__ int solve_job(const BatchDev& b, unsigned char* slot, int gi, int jr,
             } else if (col < cols - 1) {
                 direct_body<G>(d, col, nx, 0, 1);
             } else {
-                and_body<P1, G>(d, col, 0, 1);
+                last_column_body<P1, G>(d, col, 0, 1);
             }
             __syncthreads();
         }
@@ -502,7 +533,8 @@ size_t batch_smem(int threads, int max_n) {
         const size_t push = (size_t)warps * S * rwp;
         const size_t pull = cop + rank_table_words(kBatchMaxK, n);
         const size_t pair = (size_t)pair_smem_words(n);
-        best = std::max(best, std::max(std::max(pull, pair), std::max(andb, push)) * 4);
+        const size_t tile = (size_t)warps * and_tile_quads((n + 31) / 32) * 4;
+        best = std::max(best, std::max(std::max(std::max(pull, pair), tile), std::max(andb, push)) * 4);
     }
     return best;
 }

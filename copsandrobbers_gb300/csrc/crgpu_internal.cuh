@@ -76,6 +76,11 @@ struct DevGraph {
     const uint8_t* cover;
     int cover_w;
     int npad;
+    // hop(r) of every vertex as padded lists for the last column's tile form: the lists of the 32
+    // vertices of row word w take rows ell_off[w] .. ell_off[w + 1] of 32 entries, lane r & 31's
+    // entries down its column, padded with rw * 32.  Null = the tile form is not used.
+    const uint16_t* ell = nullptr;
+    const uint32_t* ell_off = nullptr;
     int nnz = -1;             // row_ptr[n] when the host knows it (sizes shared-memory staging)
     // The cops' move graph when it differs from the robber's (row_ptr / col above), i.e. under
     // the stay-allowed rules; null = the same graph.  rrow_ptr / rcol and nbr always describe

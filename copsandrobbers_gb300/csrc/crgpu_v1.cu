@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(256) k_direct(V1Dev d, int col, int nx) {
 // that this latency-bound body needs more)
 template <bool P1, int G>
 __global__ void __launch_bounds__(256, 4) k_and(V1Dev d, int col) {
-    and_body<P1, G>(d, col, blockIdx.x, gridDim.x);
+    last_column_body<P1, G>(d, col, blockIdx.x, gridDim.x);
 }
 // The last column inside the device-side pass loop, with the loop's bookkeeping in its last
 // block: the pass's count joins the history, the loop goes on while the pass found something
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(256, 4) k_and(V1Dev d, int col) {
 template <bool P1, int G>
 __global__ void __launch_bounds__(256, 4) k_and_end(V1Dev d, int col, LoopCtl c) {
     if (c.fused_prep1) prep_clear_cand(d, blockIdx.x, gridDim.x);   // this column's prep, the rest
-    and_body<P1, G>(d, col, blockIdx.x, gridDim.x);
+    last_column_body<P1, G>(d, col, blockIdx.x, gridDim.x);
     __syncthreads();
     if (threadIdx.x == 0 && grid_last_block(d, gridDim.x)) {
         const int i = *c.idx;
@@ -166,6 +166,8 @@ size_t and_smem_bytes(int S, int rwp, int n) {
     (void)n;
     return (size_t)8 * (32 / group_lanes(rwp)) * and_group_words(S, rwp) * sizeof(uint32_t);
 }
+// Eight warps of the last column's tile form.
+static size_t and_tile_smem_bytes(int rw) { return (size_t)8 * and_tile_quads(rw) * 16; }
 
 static int pull_words(int S, int rwp) {
     int w = S * rwp, p = 2;
@@ -243,6 +245,8 @@ size_t and_stage_words(int n, int rwp, int nnz) {
 
 template <bool P1, int G>
 static void launch_and_g(const V1Dev& d, int col, int grid, size_t sm, cudaStream_t st, const LoopCtl* loop) {
+    const void* kern = loop ? (const void*)k_and_end<P1, G> : (const void*)k_and<P1, G>;
+    if (sm > 40 * 1024) raise_smem_limit(kern, sm);   // (the kernel has static shared memory too)
     if (loop) k_and_end<P1, G><<<grid, 256, sm, st>>>(d, col, *loop);
     else k_and<P1, G><<<grid, 256, sm, st>>>(d, col);
 }
@@ -259,6 +263,7 @@ static void launch_and_p(const V1Dev& d0, int col, int grid, cudaStream_t st, co
             sm += words * 4;
         }
     }
+    if (d.g.ell) sm = std::max(sm, and_tile_smem_bytes(d.g.rw));
     switch (group_lanes(d.g.rwp)) {
         case 4: launch_and_g<P1, 4>(d, col, grid, sm, st, loop); break;
         case 8: launch_and_g<P1, 8>(d, col, grid, sm, st, loop); break;

@@ -419,7 +419,7 @@ __host__ __device__ inline int init_pass1_smem_words(int n, int rwp) { return 25
 
 template <int K, int W, bool FULL>
 __device__ CR_BODY_INLINE void init_pass1_single(const V1Dev& d, unsigned wk, unsigned nwk) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // FULL: n = 256 exactly, so every lane owns 8 robbers and every row word has a lane
     const int n = FULL ? 256 : d.g.n, rw = FULL ? 8 : d.g.rw, rwp = FULL ? 8 : d.g.rwp;
@@ -996,7 +996,7 @@ __device__ __forceinline__ void group_or(uint32_t (&acc)[NWP], int gl, uint32_t*
 // words, and the group reduces them by halving.
 template <int K, int NWP, int G>
 __device__ CR_BODY_INLINE void cop_pull_body(const V1Dev& d, int col, int nx, unsigned wk, unsigned nwk) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     constexpr int CPW = 32 / G;
     constexpr int U = 4;  // successor tuples in flight per lane
     const int warp = threadIdx.x >> 5;
@@ -1188,7 +1188,7 @@ __host__ __device__ inline int pair_chunk_words(int n, int S, int rwp) {
 __host__ __device__ inline int pair_smem_words(int n) { return rank_table_words(3, n) + kPairStageWords; }
 
 __device__ CR_BODY_INLINE void pair_h1_body(const V1Dev& d, int nx, unsigned wk, unsigned nwk) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     __shared__ uint32_t s_xy[32];
     constexpr int K = 3;
     const int n = d.g.n, rwp = d.g.rwp, S = d.S;
@@ -1285,7 +1285,7 @@ __device__ CR_BODY_INLINE void pair_h1_body(const V1Dev& d, int nx, unsigned wk,
 // Stage 2: a lane group per configuration, its lanes over the deg^2 pairs (x, y).
 template <int NWP, int G>
 __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, unsigned wk, unsigned nwk) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     constexpr int K = 3;
     constexpr int CPW = 32 / G;
     const int warp = threadIdx.x >> 5;
@@ -1372,7 +1372,7 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
 // successor is visited.  All seed values are 0: one slot.
 template <int K, int G>
 __device__ CR_BODY_INLINE void cop_seed_body(const V1Dev& d, int col, int nx, unsigned wk, unsigned nwk) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     constexpr int CPW = 32 / G;
     const int warp = threadIdx.x >> 5;
     const Lanes<G> L(threadIdx.x & 31);
@@ -1421,7 +1421,7 @@ __device__ CR_BODY_INLINE void cop_seed_body(const V1Dev& d, int col, int nx, un
 // list atomic per warp and round.  Each entry's flag is cleared as it is taken.
 template <int K>
 __device__ CR_BODY_INLINE void cop_push_body(const V1Dev& d, int col, int nx, unsigned wk, unsigned nwk) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n = d.g.n, rwp = d.g.rwp, S = d.S;
     const ColMeta mi = d.meta[nx];
@@ -1508,7 +1508,7 @@ __device__ CR_BODY_INLINE void cop_push_body(const V1Dev& d, int col, int nx, un
 // zeroing each row right after reading it here cost six times the reads).
 template <int G>
 __device__ CR_BODY_INLINE void cop_apply_body(const V1Dev& d, int col, int nx, unsigned wk, unsigned nwk) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     constexpr int CPW = 32 / G;
     const int warp = threadIdx.x >> 5;
     const Lanes<G> L(threadIdx.x & 31);
@@ -1545,7 +1545,7 @@ __device__ CR_BODY_INLINE void cop_apply_body(const V1Dev& d, int col, int nx, u
 // over column nx's row list (each entry's flag cleared as it is taken).
 template <int G>
 __device__ CR_BODY_INLINE void direct_body(const V1Dev& d, int col, int nx, unsigned wk, unsigned nwk) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     constexpr int CPW = 32 / G;
     const int warp = threadIdx.x >> 5;
     const Lanes<G> L(threadIdx.x & 31);
@@ -1604,7 +1604,7 @@ __device__ CR_BODY_INLINE void direct_body(const V1Dev& d, int col, int nx, unsi
 // unmarked; an r with empty hop(r) has value 1.
 template <bool P1, int G>
 __device__ CR_BODY_INLINE void and_body(const V1Dev& d, int col, unsigned wk, unsigned nwk) {
-    extern __shared__ uint32_t sm[];
+    extern __shared__ __align__(16) uint32_t sm[];
     constexpr int CPW = 32 / G;
     const int warp = threadIdx.x >> 5;
     const Lanes<G> L(threadIdx.x & 31);
@@ -1905,6 +1905,253 @@ __device__ CR_BODY_INLINE void and_body(const V1Dev& d, int col, unsigned wk, un
         }
     }
     t.flush(d, col, L.lane);
+}
+
+// The table bytes of one row word's new marks, a lane per robber: n1 / n0 = the marks of the
+// higher and the lower value, at = the byte of the word's first robber.  The warp's stores fall
+// in one stretch of 32 * cols bytes, where a loop over one lane's bits is a transaction per byte.
+__device__ __forceinline__ void store_word(uint8_t* at, uint32_t n1, uint32_t n0, int v1, int v0, int cols, int lane) {
+    if (((n1 | n0) >> lane) & 1u) at[lane * cols] = (uint8_t)(1 | (((n1 >> lane) & 1u ? v1 : v0) << 1));
+}
+
+// Whether a warp writes its new marks word by word (store_word) or each lane the bits of its own
+// words, from the lane's marks and non-empty words.  By words costs about 15 instructions and a
+// transaction and a half per word; by lanes about 10 instructions per mark of the fullest lane and
+// a scattered transaction per mark, the transactions being the SM's and the instructions a
+// quarter's: by words where 8 words < 5 fullest + 2 marks.  (At n = 128 the two meet near two marks
+// per word: 80 against 90 us for a last column of 1.8 marks per word, 181 against 101 us at 3.8.)
+__device__ __forceinline__ bool by_words(int marks, int words) {
+    return 8 * __reduce_add_sync(FULL_MASK, words) <
+           5 * __reduce_max_sync(FULL_MASK, marks) + 2 * __reduce_add_sync(FULL_MASK, marks);
+}
+
+// 32 x 32 bit transpose across a warp: lane i holds row i and gets column i back (bit j of lane i
+// becomes bit i of lane j).  Each of the five steps swaps one bit of the lane index with the same
+// bit of the bit index: one shuffle, one rotate, one select.
+__device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
+    uint32_t keep = 0x0000FFFFu;
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        const uint32_t y = __shfl_xor_sync(FULL_MASK, x, s);
+        const bool up = (lane & s) != 0;
+        const uint32_t r = __funnelshift_l(y, y, up ? 32 - s : s);
+        const uint32_t k = up ? ~keep : keep;
+        x = (x & k) | (r & ~k);
+        keep ^= keep << (s >> 1);
+    }
+    return x;
+}
+
+// Shared-memory quads (16 bytes) of one warp of the tile form: an entry per vertex, the neutral
+// entry, and two words per (row word, lane).
+__host__ __device__ inline int and_tile_quads(int rw) { return rw * 48 + 1; }
+
+// Last column over long row lists, fresh form (see and_body): a warp takes 32 listed rows and
+// turns its words of column 0's marks and of the fresh marks of the (at most two) value slots
+// from one word per (row, 32 robbers) into one word per (vertex, 32 rows).  A lane then owns a
+// robber r and decides it for all 32 rows at once: over v in hop(r), the AND of v's marked words
+// says in which rows r is complete, the OR of v's fresh words of a slot in which rows it meets a
+// fresh mark of that slot.  hop(r) comes from the ELL lists (d.g.ell), padded with the neutral
+// entry (all marked, nothing fresh), so a warp walks the 32 lists of a word in step.  The results
+// are turned back to row words, masked with the open states and written by the row's lane.
+// Bound: issue and shared-memory wavefronts, about 25 warp instructions per row at n = 128 where
+// the row-by-row form takes several hundred (its bit loops diverge over the rows of a warp), and
+// in the densest passes the table bytes.  Last columns of a whole solve: G(n, p) n = 128 1016 us
+// row by row, 531 us in tiles; Delaunay n = 199 9.0 and 3.5 ms; n = 389 195 and 70 ms.
+__device__ CR_BODY_INLINE void and_tile_body(const V1Dev& d, int col, unsigned wk, unsigned nwk) {
+    extern __shared__ __align__(16) uint32_t sm[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = d.g.n, rw = d.g.rw, rwp = d.g.rwp, S = d.S, cols = d.cols;
+    const ColMeta mi = d.meta[0];
+    const int out_base = d.meta[col].base;
+    const int slo = mi.lo - mi.base, shi = mi.hi - mi.base;
+    const bool two = shi > slo;
+    // values of the two slots, and their output slots; values >= 127 stay unmarked
+    const int v1 = mi.hi + 1, v0 = mi.lo + 1;
+    const int so1 = v1 - out_base, so0 = v0 - out_base;
+    const uint32_t keep1 = v1 < kMaxRound ? FULL_MASK : 0u, keep0 = two && v0 < kMaxRound ? FULL_MASK : 0u;
+    uint4* sx = reinterpret_cast<uint4*>(sm) + warp * and_tile_quads(rw);
+    uint32_t* sn1 = reinterpret_cast<uint32_t*>(sx + rw * 32 + 1) + lane;
+    uint32_t* sn0 = sn1 + rw * 32;
+    const uint16_t* CR_RESTRICT ell = d.g.ell + lane;
+    const uint32_t* CR_RESTRICT ell_off = d.g.ell_off;
+    const RowList rl(d, 0, mi);
+    const bool vec4 = (rwp & 3) == 0;
+    if (lane == 0) sx[rw * 32] = make_uint4(FULL_MASK, 0u, 0u, 0u);
+    Tally t;
+    const uint32_t tiles = (rl.n + 31) / 32, step = nwk * (blockDim.x >> 5);
+    for (uint32_t tile = wk * (blockDim.x >> 5) + warp; tile < tiles; tile += step) {
+        const uint32_t li = tile * 32 + lane;
+        const bool valid = li < rl.n;
+        const uint32_t cid = valid ? rl.id(li) : 0u;
+        if (valid) d.fflag[cid] = 0;
+        const uint32_t* m0 = d.marked + (size_t)cid * rwp;
+        const uint32_t* f1 = d.front + ((size_t)cid * S + shi) * rwp;
+        const uint32_t* f0 = d.front + ((size_t)cid * S + slo) * rwp;
+        __syncwarp();
+        for (int w0 = 0; w0 < rw; w0 += 4) {
+            uint4 a = make_uint4(0u, 0u, 0u, 0u), h = a, l = a;
+            if (valid) {
+                if (vec4) {
+                    a = *reinterpret_cast<const uint4*>(m0 + w0);
+                    h = *reinterpret_cast<const uint4*>(f1 + w0);
+                    if (two) l = *reinterpret_cast<const uint4*>(f0 + w0);
+                } else {   // rows of one or two words
+                    a.x = m0[0]; h.x = f1[0];
+                    if (rw > 1) { a.y = m0[1]; h.y = f1[1]; }
+                    if (two) {
+                        l.x = f0[0];
+                        if (rw > 1) l.y = f0[1];
+                    }
+                }
+            }
+            const uint32_t av[4] = {a.x, a.y, a.z, a.w}, hv[4] = {h.x, h.y, h.z, h.w}, lv[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (w0 + j >= rw) break;
+                uint4 e;
+                e.x = warp_transpose(av[j], lane);
+                e.y = warp_transpose(hv[j], lane);
+                e.z = two ? warp_transpose(lv[j], lane) : 0u;
+                e.w = 0u;
+                sx[(w0 + j) * 32 + lane] = e;
+            }
+        }
+        __syncwarp();
+        bool found = false;
+        for (int w = 0; w < rw; ++w) {
+            uint32_t all = FULL_MASK, t1 = 0u, t0 = 0u;
+            const uint32_t e1 = CR_LDG(&ell_off[w + 1]);
+#pragma unroll 4
+            for (uint32_t e = CR_LDG(&ell_off[w]); e < e1; ++e) {
+                const uint4 x = sx[CR_LDG(&ell[e * 32])];
+                all &= x.x;
+                t1 |= x.y;
+                t0 |= x.z;
+            }
+            uint32_t n1 = all & t1 & keep1, n0 = all & t0 & ~t1 & keep0;
+            if (__any_sync(FULL_MASK, (n1 | n0) != 0u)) {
+                found = true;
+                n1 = warp_transpose(n1, lane);
+                if (two) n0 = warp_transpose(n0, lane);
+            }
+            sn1[w * 32] = n1;
+            sn0[w * 32] = n0;
+        }
+        if (!found) continue;
+        // the row's lane again: mask with the open states
+        uint32_t* mrow = d.marked + ((size_t)col * d.C + cid) * rwp;
+        uint32_t any1 = 0u, any0 = 0u;
+        int marks = 0, words = 0;
+        if (valid) {
+            for (int w = 0; w < rw; ++w) {
+                const uint32_t mc = mrow[w], n1 = sn1[w * 32] & ~mc, n0 = sn0[w * 32] & ~mc;
+                sn1[w * 32] = n1;
+                sn0[w * 32] = n0;
+                any1 |= n1;
+                any0 |= n0;
+                if (n1 | n0) {
+                    mrow[w] = mc | n1 | n0;
+                    marks += __popc(n1 | n0);
+                    ++words;
+                }
+            }
+        }
+        t.cnt += marks;
+        const bool newrow = (any1 | any0) != 0u;
+        if (newrow) {
+            if (any1) {
+                t.lo = min(t.lo, v1);
+                t.hi = max(t.hi, v1);
+                if (so1 < 0 || so1 >= S) t.err |= kErrSlot;
+            }
+            if (any0) {
+                t.lo = min(t.lo, v0);
+                t.hi = max(t.hi, v0);
+                if (so0 < 0 || so0 >= S) t.err |= kErrSlot;
+            }
+            uint32_t* frow = d.front + ((size_t)col * d.C + cid) * S * rwp;
+            for (int so = 0; so < S; ++so) {
+                const uint32_t* src = so == so1 ? sn1 : (two && so == so0 ? sn0 : nullptr);
+                if (vec4) {
+                    for (int w = 0; w < rwp; w += 4) {
+                        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                        if (src) {
+                            x.x = src[w * 32];
+                            if (w + 1 < rw) x.y = src[(w + 1) * 32];
+                            if (w + 2 < rw) x.z = src[(w + 2) * 32];
+                            if (w + 3 < rw) x.w = src[(w + 3) * 32];
+                        }
+                        *reinterpret_cast<uint4*>(frow + so * rwp + w) = x;
+                    }
+                } else {
+                    for (int w = 0; w < rwp; ++w) frow[so * rwp + w] = src && w < rw ? src[w * 32] : 0u;
+                }
+            }
+            d.fflag[(size_t)col * d.C + cid] = 1;
+            t.rows++;
+        }
+        if (by_words(marks, words)) {
+            __syncwarp();
+            for (int w = 0; w < rw; ++w) {
+                const uint32_t* row1 = sn1 - lane + w * 32;
+                unsigned rows = __ballot_sync(FULL_MASK, valid && (sn1[w * 32] | sn0[w * 32]) != 0u);
+                while (rows) {
+                    const int i = __ffs(rows) - 1;
+                    rows &= rows - 1;
+                    const uint32_t id = __shfl_sync(FULL_MASK, cid, i);
+                    store_word(d.table + ((size_t)id * n + w * 32) * cols + col, row1[i], row1[rw * 32 + i], v1, v0, cols, lane);
+                }
+            }
+            __syncwarp();
+        } else if (newrow) {
+            uint8_t* trow = d.table + (size_t)cid * n * cols + col;
+            for (int w = 0; w < rw; ++w) {
+                const uint32_t n1 = sn1[w * 32];
+                uint32_t b = n1 | sn0[w * 32];
+                while (b) {
+                    const int j = __ffs(b) - 1;
+                    b &= b - 1;
+                    trow[(size_t)(w * 32 + j) * cols] = (uint8_t)(1 | (((n1 >> j) & 1u ? v1 : v0) << 1));
+                }
+            }
+        }
+        // list the tile's new rows: one atomic per tile
+        const unsigned nb = __ballot_sync(FULL_MASK, newrow);
+        if (nb) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&d.meta[col].len, __popc(nb));
+            at = __shfl_sync(FULL_MASK, at, 0);
+            if (newrow) d.list[(size_t)col * d.C + at + __popc(nb & ((1u << lane) - 1u))] = cid;
+        }
+    }
+    t.flush(d, col, lane);
+}
+
+// The tile form takes the fresh form's columns (see and_body) whose new marks span at most two
+// values, on graphs where every robber can move, when the row list gives at least half of the
+// launch's warps a tile: a shorter list leaves most warps idle for a tile's whole latency, where
+// the row form spreads it over all of them.
+__device__ __forceinline__ bool and_takes_tiles(const V1Dev& d, const ColMeta& mi, unsigned nwk) {
+    const int slo = mi.lo - mi.base, shi = mi.hi - mi.base;
+    if (!d.g.ell || !d.fresh_last || mi.hi < mi.lo || mi.old_hi > mi.lo || slo < 0 || shi >= d.S || shi > slo + 1)
+        return false;
+    const unsigned long long rows = mi.len < 0 ? d.C : (unsigned)mi.len;
+    if (rows < 16ull * nwk * (blockDim.x >> 5)) return false;
+    for (int w = 0; w < d.g.rw; ++w)
+        if (CR_LDG(&d.g.isolated[w])) return false;
+    return true;
+}
+
+template <bool P1, int G>
+__device__ CR_BODY_INLINE void last_column_body(const V1Dev& d, int col, unsigned wk, unsigned nwk) {
+    const ColMeta mi = d.meta[0];
+    if (and_takes_tiles(d, mi, nwk)) {
+        if (wk == 0 && threadIdx.x == 0) d.meta[0].clean = 1;   // every listed flag is cleared
+        and_tile_body(d, col, wk, nwk);
+    } else {
+        and_body<P1, G>(d, col, wk, nwk);
+    }
 }
 
 // findFinalResult (k_cops_visibility.cpp:301-331): over the configurations whose column-0 row
