@@ -35,7 +35,7 @@ void launch_popcount(const uint32_t* plane, size_t words, unsigned long long* ou
 int max_cop_blocks_per_sm(int k, int rwp, int S);
 bool pull_supported(int S, int rwp);
 int cop_launches(int direct);
-int cop_launches_k(int direct, int k, bool sep);
+int cop_launches_k(int direct, bool sep);
 size_t cop_smem_bytes(int S, int rwp);
 size_t and_smem_bytes(int S, int rwp, int n);
 void launch_unrank(const uint32_t* B, int n, int k, uint32_t C, uint16_t* out, int grid, cudaStream_t st);
@@ -78,11 +78,11 @@ struct cr_solver {
     uint32_t* d_front = nullptr;
     uint8_t* d_fflag = nullptr;
     uint32_t* d_cand = nullptr;
-    uint32_t* d_h1 = nullptr;   // k = 3: H1 rows of the separable dense cop turn
+    uint32_t* d_h1 = nullptr;   // k = 2, 3, 4: head rows of the separable dense cop turn
     uint32_t* d_cbits = nullptr;      // push-mode candidate bitmap
     uint32_t* d_list = nullptr;       // [cols][C] row lists of the frontiers
     uint32_t* d_clist = nullptr;      // [C] push-mode candidate list
-    unsigned* d_sync = nullptr;       // [2] prep's block count, candidate count
+    unsigned* d_sync = nullptr;       // [kSyncWords] prep's block count, candidate count, units
     uint32_t* d_rrp = nullptr;
     uint16_t* d_rcol = nullptr;
     uint32_t* d_nbr = nullptr;
@@ -247,12 +247,24 @@ int cr_graph_parse(const char* text, size_t len, int32_t* n_out, uint32_t* row_p
 
 static int slots_for(int n) { (void)n; return 2; }
 
-// H1 rows of the separable dense cop turn (k = 3): every pair {x <= y} times every vertex,
-// one frontier row each; about 3/8 of the table's bytes.  0 when the turn keeps the
-// tuple-gathering form.
+// Head rows of the separable dense cop turn (k = 2, 3, 4): every multiset of k - 1 vertices times
+// every vertex, one frontier row each; about k/8 of a p = 1 table's bytes.  0 when the turn keeps
+// the tuple-gathering form (k = 1, or more than two value slots).
 static uint64_t h1_bytes(int n, int k, int S, int rwp) {
-    if (k != 3 || !pull_supported(S, rwp)) return 0;
-    return (uint64_t)n * (n + 1) / 2 * n * S * rwp * 4;
+    if (k < 2 || S != 2 || !pull_supported(S, rwp)) return 0;
+    return binom_u64((int64_t)n + k - 2, k - 1) * n * S * rwp * 4;
+}
+
+// The head rows of a solver.  k = 2 and 4 do without them (in the tuple-gathering form) where
+// the device has no room.
+static cudaError_t alloc_h1(cr_solver* s) {
+    const uint64_t hb = h1_bytes(s->n, s->k, s->S, s->rwp);
+    if (!hb) return cudaSuccess;
+    const cudaError_t e = s->ctx->cache.get((void**)&s->d_h1, hb);
+    if (e != cudaErrorMemoryAllocation || s->k == 3) return e;
+    cudaGetLastError();
+    s->d_h1 = nullptr;
+    return cudaSuccess;
 }
 
 static void layout(int n, int k, int p, int rules, int S, uint64_t* C, int* cols, int* rw, int* rwp) {
@@ -274,8 +286,8 @@ uint64_t cr_solver_footprint(int32_t n, int32_t k, int32_t p, int32_t rules) {
     b += (uint64_t)cols * C * rwp * 4;                   // marked
     b += (uint64_t)cols * C * S * rwp * 4;               // frontiers
     b += C * S * rwp * 4 + cand_bits_bytes(C) + C * 4;   // push-mode candidate rows, bitmap, list
-    b += (uint64_t)cols * C * 4 + 2 * sizeof(unsigned);  // frontier row lists, prep/list counters
-    b += h1_bytes(n, k, S, rwp);                         // separable dense cop turn (k = 3)
+    b += (uint64_t)cols * C * 4 + kSyncWords * sizeof(unsigned);  // frontier row lists, prep/list counters
+    b += h1_bytes(n, k, S, rwp);                         // separable dense cop turn
     b += (uint64_t)cols * C;                             // flags
     b += C * (uint64_t)k * 2;                            // configs
     b += (uint64_t)n * rwp * 4 * 3 + (uint64_t)k * (n + 1) * 4 + (1u << 16);
@@ -351,7 +363,7 @@ static V1Dev dev_view(const cr_solver* s) {
     d.cand = s->d_cand;
     d.h1 = s->d_h1;
     d.cbits = s->d_cbits;
-    // forms switched off: no pair rows (the tuple pull), a push ratio that always or never
+    // forms switched off: no head rows (the tuple pull), a push ratio that always or never
     // pushes, the last column's general form
     if (!(s->forms & CR_FORM_SEPARABLE)) d.h1 = nullptr;
     if (!(s->forms & CR_FORM_PULL)) d.push_ratio = 0u;
@@ -398,10 +410,10 @@ static int alloc_v1(cr_solver* s) {
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_cbits, cand_bits_bytes(C)));
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_list, (size_t)s->cols * C * 4));
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_clist, C * 4));
-    CR_CUDA(ctx, cudaMalloc(&s->d_sync, 2 * sizeof(unsigned)));
+    CR_CUDA(ctx, cudaMalloc(&s->d_sync, kSyncWords * sizeof(unsigned)));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_cand, 0, C * s->S * s->rwp * 4, ctx->stream));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_cbits, 0, cand_bits_bytes(C), ctx->stream));
-    if (const uint64_t hb = h1_bytes(s->n, s->k, s->S, s->rwp)) CR_CUDA(ctx, ctx->cache.get((void**)&s->d_h1, hb));
+    CR_CUDA(ctx, alloc_h1(s));
     CR_CUDA(ctx, cudaMalloc(&s->d_hop, (size_t)s->n * s->rwp * 4));
     std::vector<uint32_t> hop = hop_masks(s);
     CR_CUDA(ctx, cudaMemcpyAsync(s->d_hop, hop.data(), hop.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
@@ -675,7 +687,7 @@ static int v1_init(cr_solver* s, uint64_t* caps) {
     // producer appends to column 0's
     meta[0] = ColMeta{0, 0, 0, 1, (int)std::min<uint64_t>(C, INT32_MAX), 0, -1, 0};
     meta[1] = ColMeta{0, 0, 0, 0, (int)std::min<uint64_t>(C, INT32_MAX), 1, -1, 0};
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_sync, 0, 2 * sizeof(unsigned), st));
+    CR_CUDA(ctx, cudaMemsetAsync(s->d_sync, 0, kSyncWords * sizeof(unsigned), st));
     CR_CUDA(ctx, cudaMemcpyAsync(s->d_meta, meta.data(), sizeof(ColMeta) * s->cols, cudaMemcpyHostToDevice, st));
     V1Dev d = dev_view(s);
     launch_init(d, s->grid_small, st);
@@ -704,7 +716,7 @@ static int v1_init_pass1_enqueue(cr_solver* s, bool defer_list = false) {
     // flags after the kernel, by k_list_compact or (defer_list) by the pass loop's entry
     ColMeta meta[2] = {ColMeta{0, 0, 0, 0, (int)std::min<uint64_t>(s->C, INT32_MAX), 0, -1, 1},
                        ColMeta{1, kEmptyLo, -1, 0, 0, 0, 0, 0, 0, defer_list ? 1 : 0}};
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_sync, 0, 2 * sizeof(unsigned), st));
+    CR_CUDA(ctx, cudaMemsetAsync(s->d_sync, 0, kSyncWords * sizeof(unsigned), st));
     CR_CUDA(ctx, cudaMemcpyAsync(s->d_meta, meta, sizeof(meta), cudaMemcpyHostToDevice, st));
     V1Dev d = dev_view(s);
     CR_CUDA(ctx, cudaEventRecord(s->evc0, st));
@@ -806,7 +818,7 @@ static int v1_pass(cr_solver* s, uint64_t* found) {
     CR_CUDA(ctx, cudaStreamSynchronize(st));
     int per_pass = s->cols;  // prep kernels
     for (int col = 0; col < s->cols; ++col)
-        per_pass += col % 2 == 0 ? cop_launches_k(0, s->k, s->d_h1 != nullptr && (s->forms & CR_FORM_SEPARABLE)) : (col < s->cols - 1 ? cop_launches(1) : 1);
+        per_pass += col % 2 == 0 ? cop_launches_k(0, s->d_h1 != nullptr && (s->forms & CR_FORM_SEPARABLE)) : (col < s->cols - 1 ? cop_launches(1) : 1);
     s->stats.kernel_launches += per_pass;
     *found = s->h_pinned[0];
     return CR_OK;
@@ -865,7 +877,7 @@ static int grow_slots_and_replay(cr_solver* s) {
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_cand, (size_t)s->C * s->S * s->rwp * 4));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_cand, 0, (size_t)s->C * s->S * s->rwp * 4, ctx->stream));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_cbits, 0, cand_bits_bytes(s->C), ctx->stream));
-    if (const uint64_t hb = h1_bytes(s->n, s->k, s->S, s->rwp)) CR_CUDA(ctx, ctx->cache.get((void**)&s->d_h1, hb));
+    CR_CUDA(ctx, alloc_h1(s));
     const int per_sm = max_cop_blocks_per_sm(s->k, s->rwp, s->S);
     s->grid_cop = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 7) / 8, (uint64_t)ctx->num_sms * per_sm));
     uint64_t caps;
@@ -1018,7 +1030,7 @@ static int v1_run_on_device(cr_solver* s) {
     // column's in the cop turn and the last column
     int per_pass = s->cols == 2 ? 0 : s->cols - 1;
     for (int col = 0; col < s->cols; ++col)
-        per_pass += col % 2 == 0 ? cop_launches_k(0, s->k, s->d_h1 != nullptr && (s->forms & CR_FORM_SEPARABLE)) : (col < s->cols - 1 ? cop_launches(1) : 1);
+        per_pass += col % 2 == 0 ? cop_launches_k(0, s->d_h1 != nullptr && (s->forms & CR_FORM_SEPARABLE)) : (col < s->cols - 1 ? cop_launches(1) : 1);
     s->stats.kernel_launches += (int64_t)per_pass * loop_passes + 1;   // and the loop's entry
     if (bits & kErrRank) return fail(ctx, CR_ERR_INTERNAL, "successor rank out of range");
     if (bits & kErrSlot) {

@@ -111,16 +111,16 @@ __host__ __device__ inline JobLayout job_layout(int n, int k, int p, int S) {
     L.table = take(C * (size_t)n * cols);
     L.marked = take((size_t)cols * C * rwp * 4);
     L.front = take((size_t)cols * C * S * rwp * 4);
-    // k = 3: rows of the separable dense cop turn (written before they are read each pass,
-    // so they sit outside the regions the block zeroes)
-    L.h1 = take(k == 3 ? (size_t)n * (n + 1) / 2 * n * S * rwp * 4 : 0);
+    // k = 2, 3: head rows of the separable dense cop turn (written before they are read each
+    // pass, so they sit outside the regions the block zeroes)
+    L.h1 = take(k >= 2 ? (size_t)binom_dev((int64_t)n + k - 2, k - 1) * n * S * rwp * 4 : 0);
     // frontier row lists and the push-mode candidate list (written before they are read)
     L.list = take((size_t)cols * C * 4);
     L.clist = take(C * 4);
     L.fflag = take((size_t)cols * C);
     L.cand = take(C * S * rwp * 4);
     L.cbits = take(cand_bits_bytes(C));
-    L.sync = take(2 * sizeof(unsigned));
+    L.sync = take(kSyncWords * sizeof(unsigned));
     L.meta = take(sizeof(ColMeta) * cols);
     L.counters = take(4 * sizeof(unsigned long long));
     L.err = take(sizeof(unsigned));
@@ -264,7 +264,7 @@ __device__ int solve_job(const BatchDev& b, unsigned char* slot, int gi, int jr,
     d.front = reinterpret_cast<uint32_t*>(slot + L.front);
     d.fflag = slot + L.fflag;
     d.cand = reinterpret_cast<uint32_t*>(slot + L.cand);
-    d.h1 = K == 3 ? reinterpret_cast<uint32_t*>(slot + L.h1) : nullptr;
+    d.h1 = K >= 2 ? reinterpret_cast<uint32_t*>(slot + L.h1) : nullptr;
     d.cbits = reinterpret_cast<uint32_t*>(slot + L.cbits);
     d.list = reinterpret_cast<uint32_t*>(slot + L.list);
     d.clist = reinterpret_cast<uint32_t*>(slot + L.clist);
@@ -400,12 +400,14 @@ __device__ int solve_job(const BatchDev& b, unsigned char* slot, int gi, int jr,
             if (col % 2 == 0) {
                 cop_seed_body<K, G>(d, col, nx, 0, 1);
                 __syncthreads();
-                cop_pull_body<K, NWP, G>(d, col, nx, 0, 1);
-                __syncthreads();
-                if (K == 3) {
-                    pair_h1_body(d, nx, 0, 1);
+                if constexpr (K == 1) {
+                    cop_pull_body<K, NWP, G>(d, col, nx, 0, 1);
                     __syncthreads();
-                    sep_pull_body<NWP, G>(d, col, nx, 0, 1);
+                }
+                if constexpr (K >= 2) {
+                    head_rows_body<K, RWP>(d, nx, 0, 1);
+                    __syncthreads();
+                    sep_pull_body<K, RWP>(d, col, nx, 0, 1);
                     __syncthreads();
                 }
                 cop_push_body<K>(d, col, nx, 0, 1);
@@ -532,9 +534,9 @@ size_t batch_smem(int threads, int max_n) {
         const size_t andb = (size_t)warps * CPW * and_group_words(S, rwp);
         const size_t push = (size_t)warps * S * rwp;
         const size_t pull = cop + rank_table_words(kBatchMaxK, n);
-        const size_t pair = (size_t)pair_smem_words(n);
+        const size_t head = (size_t)head_smem_words(threads, kBatchMaxK, n, rwp);
         const size_t tile = (size_t)warps * and_tile_quads((n + 31) / 32) * 4;
-        best = std::max(best, std::max(std::max(std::max(pull, pair), tile), std::max(andb, push)) * 4);
+        best = std::max(best, std::max(std::max(std::max(pull, head), tile), std::max(andb, push)) * 4);
     }
     return best;
 }

@@ -34,6 +34,8 @@ constexpr unsigned kErrBudget = 4u;  // a bounded device loop ran out
 // (scatter with atomic ORs); a denser one is pulled by every configuration (gather).
 constexpr int kPushRatio = 16;
 
+constexpr int kSyncWords = 3;   // counters of V1Dev::sync
+
 // Range and base of the value slots of one column's frontier.
 struct ColMeta {
     int base;    // value of slot 0
@@ -113,13 +115,16 @@ struct V1Dev {
     uint32_t* front;
     uint8_t* fflag;
     uint32_t* cand;           // [C][S][rwp]: push-mode OR of successor frontier rows
-    // k = 3 dense cop turns: H1 rows [P][n][S][rwp], P = n(n+1)/2 pairs {x <= y}; H1[{x,y}][c]
-    // = OR over z in N(c) of the frontier row of sort(x, y, z).  Null = the tuple-gathering pull.
+    // Dense cop turns of k = 2, 3, 4 in separable form: rows [heads][n][S][rwp], a head being a
+    // multiset of k - 1 vertices; row [h][c] = OR over z in N(c) of the frontier row of sort(h, z).
+    // Null = the tuple-gathering pull.
     uint32_t* h1 = nullptr;
     uint32_t* cbits;          // [ceil(C / 32)]: bit C set = cand row C non-empty
     uint32_t* list;           // [cols][C]: the row lists of the columns' frontiers
     uint32_t* clist;          // [C]: ids of the non-empty cand rows (sync[1] of them)
-    unsigned* sync;           // [2]: blocks done with the current prep, cand rows listed
+    // [kSyncWords]: blocks done with the current prep, cand rows listed, units of the separable
+    // turn handed out
+    unsigned* sync;
     ColMeta* meta;            // [cols]
     unsigned long long* pass_new;
     unsigned int* err;

@@ -111,7 +111,7 @@ Layout plan(int n, size_t nnz, int k, int cols, uint64_t C, int rwp, int S) {
     L.cbits = take(cand_bits_bytes(C));
     L.list = take((size_t)cols * C * 4);
     L.clist = take(C * 4);
-    L.sync = take(2 * sizeof(unsigned));
+    L.sync = take(kSyncWords * sizeof(unsigned));
     L.meta = take(sizeof(ColMeta) * cols);
     L.counters = take(4 * sizeof(unsigned long long));
     L.err = take(sizeof(unsigned));

@@ -26,12 +26,13 @@
 // The cop turn runs in one of these forms, chosen on the device from the frontier's row count:
 //   seed          the capture seeds of column 1 before pass 1, in closed form: the OR of the
 //                 seed rows over T(C) is the union of the cops' neighbourhoods;
-//   pull (dense)  every configuration ORs the frontier rows of its successors (k_cop_pull), or
-//                 for k = 3 in separable form through pair rows (pair_h1 + sep_pull);
+//   pull (dense)  every configuration ORs the frontier rows of its successors: for k = 2, 3, 4
+//                 in separable form through head rows (head_rows + sep_pull), else one by one
+//                 (k_cop_pull);
 //   push (sparse) every row of the frontier's list is ORed into the candidate rows of its
 //                 predecessors with atomics, then only those rows are marked (push + apply).
 // k_cop_a and k_cop_b carry the seed, push, apply and separable bodies (each body returns at
-// once unless its form applies), so a cop turn is two launches for k = 3 and three otherwise.
+// once unless its form applies), so a cop turn is two launches with head rows and three without.
 #include "crgpu_internal.cuh"
 
 #include <algorithm>
@@ -69,19 +70,19 @@ __global__ void __launch_bounds__(256) k_cop_pull(V1Dev d, int col, int nx) {
 }
 // The other cop-turn forms share two launches, each body returning at once unless its form
 // applies (the form is chosen on the device from the input frontier):
-//   k_cop_a  the capture-seed form, the push scatter, or (k = 3) the separable turn's pair rows;
-//   k_cop_b  the separable turn's configurations (k = 3) or the push form's marking.
-// The tuple-gathering pull (k != 3, or no pair rows) keeps its own launch: it wants up to 127
+//   k_cop_a  the capture-seed form, the push scatter, or the separable turn's head rows;
+//   k_cop_b  the separable turn's configurations or the push form's marking.
+// The tuple-gathering pull (k = 1, or no head rows) keeps its own launch: it wants up to 127
 // registers, the bodies here at most 64 (80 with 32-word rows), being latency-bound.
 template <int K, int NWP, int G>
 __global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_a(V1Dev d, int col, int nx) {
     cop_seed_body<K, G>(d, col, nx, blockIdx.x, gridDim.x);
     cop_push_body<K>(d, col, nx, blockIdx.x, gridDim.x);
-    if constexpr (K == 3) pair_h1_body(d, nx, blockIdx.x, gridDim.x);
+    if constexpr (K >= 2) head_rows_body<K, NWP / 2>(d, nx, blockIdx.x, gridDim.x);
 }
 template <int K, int NWP, int G>
 __global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_b(V1Dev d, int col, int nx) {
-    if constexpr (K == 3) sep_pull_body<NWP, G>(d, col, nx, blockIdx.x, gridDim.x);
+    if constexpr (K >= 2) sep_pull_body<K, NWP / 2>(d, col, nx, blockIdx.x, gridDim.x);
     cop_apply_body<G>(d, col, nx, blockIdx.x, gridDim.x);
 }
 // k_cop_b inside the device-side pass loop of a p = 1 solve, followed by the last column's prep
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_b(V1Dev d, int c
 // and in the last block the column's state reset.  The candidate rows wait for the last column.
 template <int K, int NWP, int G>
 __global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_b_end(V1Dev d, int col, int nx) {
-    if constexpr (K == 3) sep_pull_body<NWP, G>(d, col, nx, blockIdx.x, gridDim.x);
+    if constexpr (K >= 2) sep_pull_body<K, NWP / 2>(d, col, nx, blockIdx.x, gridDim.x);
     cop_apply_body<G>(d, col, nx, blockIdx.x, gridDim.x);
     prep_clear_flags(d, nx, blockIdx.x, gridDim.x);
     __syncthreads();
@@ -181,9 +182,10 @@ template <int K, int NWP, int G>
 static void launch_cop_ng(const V1Dev& d, int col, int nx, int grid, cudaStream_t st, bool end) {
     const size_t sm = cop_smem_bytes(d.S, d.g.rwp);
     const size_t smr = sm + (size_t)rank_table_words(K, d.g.n) * 4;
-    const size_t sma = K == 3 ? std::max(smr, (size_t)pair_smem_words(d.g.n) * 4) : smr;
+    const size_t sma = d.h1 ? std::max(smr, (size_t)head_smem_words(256, K, d.g.n, d.g.rwp) * 4) : smr;
+    if (sma > 40 * 1024) raise_smem_limit((const void*)k_cop_a<K, NWP, G>, sma);   // (plus the static part)
     k_cop_a<K, NWP, G><<<grid, 256, sma, st>>>(d, col, nx);
-    if (!(K == 3 && d.h1)) k_cop_pull<K, NWP, G><<<grid, 256, smr, st>>>(d, col, nx);
+    if (!d.h1) k_cop_pull<K, NWP, G><<<grid, 256, smr, st>>>(d, col, nx);
     if (end) k_cop_b_end<K, NWP, G><<<grid, 256, sm, st>>>(d, col, nx);
     else k_cop_b<K, NWP, G><<<grid, 256, sm, st>>>(d, col, nx);
 }
@@ -235,7 +237,7 @@ void launch_cop(const V1Dev& d, int col, int nx, int direct, int grid, cudaStrea
 }
 
 int cop_launches(int direct) { return direct ? 1 : 3; }
-int cop_launches_k(int direct, int k, bool sep) { return direct ? 1 : (k == 3 && sep ? 2 : 3); }
+int cop_launches_k(int direct, bool sep) { return direct ? 1 : (sep ? 2 : 3); }
 
 // Shared-memory words the last-column body stages the graph in: transposed hop rows, row
 // pointers and neighbour lists.

@@ -48,9 +48,6 @@ __host__ __device__ inline int and_group_words(int S, int rwp) { return 3 * rwp 
 // Words of shared memory the pull body stages the rank table in (16-byte multiple).
 __host__ __device__ inline int rank_table_words(int k, int n) { return (k * (n + 1) + 3) & ~3; }
 
-// Words of shared memory the separable turn's pair rows stage frontier rows in (16 KB).
-constexpr int kPairStageWords = 4096;
-
 __device__ __forceinline__ bool frontier_sparse(const V1Dev& d, const ColMeta& m) {
     return (unsigned long long)m.rows * d.push_ratio < d.C;
 }
@@ -200,7 +197,10 @@ __device__ CR_BODY_INLINE void prep_reset(const V1Dev& d, int col, int nx) {
     }
     mo->seed = 0;
     if (col == 0) *d.pass_new = 0ull;
-    if (col % 2 == 0) d.sync[1] = 0u;                // the push form's candidate list
+    if (col % 2 == 0) {
+        d.sync[1] = 0u;                              // the push form's candidate list
+        d.sync[2] = 0u;                              // the separable turn's units
+    }
     if (col == d.cols - 1) d.meta[0].append = 0;   // column 0's seeded frontier is consumed
 }
 
@@ -1006,7 +1006,7 @@ __device__ CR_BODY_INLINE void cop_pull_body(const V1Dev& d, int col, int nx, un
     const ColMeta mi = d.meta[nx];
     if (mi.hi < mi.lo) return;                              // empty frontier: nothing changes
     if (mi.seed || frontier_sparse(d, mi)) return;       // the seed or push form handles it
-    if (K == 3 && d.h1) return;                             // the separable form handles it
+    if (d.h1) return;                                       // the separable form handles it
     const int base_in = mi.base;
     const int s_used = min(mi.hi - base_in + 1, S);
     const int nwords = s_used * rwp;
@@ -1150,221 +1150,456 @@ __device__ CR_BODY_INLINE void cop_pull_body(const V1Dev& d, int col, int nx, un
     t.flush(d, col, L.lane);
 }
 
-// Pair index of the multiset {x <= y} among all pairs in lexicographic order, and its inverse.
-__device__ __forceinline__ uint32_t pair_index(int x, int y, int n) {
-    return (uint32_t)(x * (2 * n - x + 1) / 2 + (y - x));
+// The table bytes of one row word's new marks, a lane per robber: n1 / n0 = the marks of the
+// higher and the lower value, at = the byte of the word's first robber.  The warp's stores fall
+// in one stretch of 32 * cols bytes, where a loop over one lane's bits is a transaction per byte.
+__device__ __forceinline__ void store_word(uint8_t* at, uint32_t n1, uint32_t n0, int v1, int v0, int cols, int lane) {
+    if (((n1 | n0) >> lane) & 1u) at[lane * cols] = (uint8_t)(1 | (((n1 >> lane) & 1u ? v1 : v0) << 1));
 }
-__device__ __forceinline__ void pair_of(uint32_t q, int n, int& x, int& y) {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if ((uint32_t)(mid * (2 * n - mid + 1) / 2) <= q) lo = mid;
-        else hi = mid - 1;
+
+// Whether a warp writes its new marks word by word (store_word) or each lane the bits of its own
+// words, from the lane's marks and non-empty words.  By words costs about 15 instructions and a
+// transaction and a half per word; by lanes about 10 instructions per mark of the fullest lane and
+// a scattered transaction per mark, the transactions being the SM's and the instructions a
+// quarter's: by words where 8 words < 5 fullest + 2 marks.  (At n = 128 the two meet near two marks
+// per word: 80 against 90 us for a last column of 1.8 marks per word, 181 against 101 us at 3.8.)
+__device__ __forceinline__ bool by_words(int marks, int words) {
+    return 8 * __reduce_add_sync(FULL_MASK, words) <
+           5 * __reduce_max_sync(FULL_MASK, marks) + 2 * __reduce_add_sync(FULL_MASK, marks);
+}
+
+// Heads: sorted multisets h[0] <= .. <= h[M-1] of M = k - 1 vertices, numbered in colexicographic
+// order (by the largest vertex first), so the heads below a bound on their largest vertex are the
+// first heads_below<M>(bound) ones, whatever n is.
+template <int M>
+__host__ __device__ __forceinline__ uint32_t heads_below(uint32_t x) {
+    return M == 1 ? x : (M == 2 ? x * (x + 1) / 2 : x * (x + 1) * (x + 2) / 6);   // n <= 512: 32 bits
+}
+template <int M>
+__device__ __forceinline__ uint32_t head_index(const int (&h)[M]) {
+    uint32_t q = (uint32_t)h[0];
+    if (M > 1) q += heads_below<2>(h[M > 1 ? 1 : 0]);
+    if (M > 2) q += heads_below<3>(h[M > 2 ? 2 : 0]);
+    return q;
+}
+template <int M>
+__device__ __forceinline__ void head_of(uint32_t q, int (&h)[M]) {
+    if (M > 2) {
+        int z = (int)cbrtf(6.0f * (float)q);   // within one of the answer; made exact below
+        while (heads_below<3>(z) > q) --z;
+        while (heads_below<3>(z + 1) <= q) ++z;
+        q -= heads_below<3>(z);
+        h[M - 1] = z;
     }
-    x = lo;
-    y = lo + (int)(q - (uint32_t)(lo * (2 * n - lo + 1) / 2));
+    if (M > 1) {
+        int y = (int)((sqrtf(8.0f * (float)q + 1.0f) - 1.0f) * 0.5f);
+        while (y > 0 && heads_below<2>(y) > q) --y;
+        while (heads_below<2>(y + 1) <= q) ++y;
+        q -= heads_below<2>(y);
+        h[M > 1 ? 1 : 0] = y;
+    }
+    h[0] = (int)q;
 }
 
-// Dense cop turn for k = 3 in separable form.  The OR over T(C) of the frontier rows F[C'],
-// C' = sort(x, y, z) with x in N(c1), y in N(c2), z in N(c3), splits into two stages:
-//   H1[{x, y}][c] = OR over z in N(c) of F[sort(x, y, z)]             (pair_h1_body)
-//   acc(C)        = OR over x in N(c1), y in N(c2) of H1[{x, y}][c3]  (sep_pull_body)
-// so a configuration reads deg^2 rows of H1 (consecutive configurations read consecutive
-// rows) instead of ranking and gathering deg^3 successor tuples.  OR is exact, so the marks
-// are the pull's.
-// Stage 1: a block per pair {x, y}.  Its n frontier rows F[sort(x, y, z)], z = 0 .. n-1, are
-// staged in shared memory (one rank and one row load per z; a row whose flag is clear counts
-// as empty), then every H1 row of the pair is the OR of the staged rows of N(c): the ranks
-// are taken once per (pair, z), not per (pair, c, z in N(c)), and the pair's n output rows are
-// written as one contiguous stretch.  A block takes as many consecutive pairs per round as
-// give each of its threads a unit of work (one pair for 256 threads at n = 128, four for the
-// batch kernel's 1024); rows wider than the staging area go one pair at a time in word chunks.
-__host__ __device__ inline int pair_chunk_words(int n, int S, int rwp) {
-    const int budget = kPairStageWords / n;
-    const int w = S * rwp;
-    if (w <= budget) return w;
-    return (rwp & 3) == 0 ? (budget & ~3) : budget;
-}
-__host__ __device__ inline int pair_smem_words(int n) { return rank_table_words(3, n) + kPairStageWords; }
+// Dense cop turn for k = 2, 3, 4 in separable form.  The OR over T(C) of the frontier rows F[C'],
+// C' = sort(x_1 .. x_k) with x_i in N(c_i), splits into two stages:
+//   H1[h][c] = OR over z in N(c) of F[sort(h, z)], h a head           (head_rows_body)
+//   acc(C)   = OR over x_i in N(c_i), i < k, of H1[{x_i}][c_k]        (sep_pull_body)
+// so a configuration reads deg^(k-1) rows of H1, consecutive configurations consecutive rows,
+// instead of ranking and gathering deg^k successor tuples.  OR is exact, so the marks are the
+// pull's.
+// A lane's NW words of a row.
+template <int NW>
+struct Words {
+    uint32_t w[NW];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int i = 0; i < NW; ++i) w[i] = 0u;
+    }
+    __device__ __forceinline__ void orr(const Words& o) {
+#pragma unroll
+        for (int i = 0; i < NW; ++i) w[i] |= o.w[i];
+    }
+    __device__ __forceinline__ uint32_t any() const {
+        uint32_t x = 0u;
+#pragma unroll
+        for (int i = 0; i < NW; ++i) x |= w[i];
+        return x;
+    }
+    __device__ __forceinline__ void load(const uint32_t* p) {
+        if (NW == 4) {
+            const uint4 v = *reinterpret_cast<const uint4*>(p);
+            w[0] = v.x; w[NW > 1 ? 1 : 0] = v.y; w[NW > 2 ? 2 : 0] = v.z; w[NW > 3 ? 3 : 0] = v.w;
+        } else if (NW == 2) {
+            const uint2 v = *reinterpret_cast<const uint2*>(p);
+            w[0] = v.x; w[NW > 1 ? 1 : 0] = v.y;
+        } else {
+            w[0] = p[0];
+        }
+    }
+    __device__ __forceinline__ void ldg(const uint32_t* p) {
+        if (NW == 4) {
+            const uint4 v = CR_LDG(reinterpret_cast<const uint4*>(p));
+            w[0] = v.x; w[NW > 1 ? 1 : 0] = v.y; w[NW > 2 ? 2 : 0] = v.z; w[NW > 3 ? 3 : 0] = v.w;
+        } else if (NW == 2) {
+            const uint2 v = CR_LDG(reinterpret_cast<const uint2*>(p));
+            w[0] = v.x; w[NW > 1 ? 1 : 0] = v.y;
+        } else {
+            w[0] = CR_LDG(p);
+        }
+    }
+    __device__ __forceinline__ void store(uint32_t* p) const {
+        if (NW == 4) *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[NW > 1 ? 1 : 0], w[NW > 2 ? 2 : 0], w[NW > 3 ? 3 : 0]);
+        else if (NW == 2) *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[NW > 1 ? 1 : 0]);
+        else p[0] = w[0];
+    }
+};
 
-__device__ CR_BODY_INLINE void pair_h1_body(const V1Dev& d, int nx, unsigned wk, unsigned nwk) {
+// Stage 1: a block takes a few heads per round (as many as give each of its threads a row).  The
+// n frontier rows F[sort(h, z)] of each head are staged in shared memory (a row whose flag is
+// clear counts as empty), then every H1 row of the head is the OR of the staged rows of N(c), and
+// the head's rows are written as one contiguous stretch.  A thread handles NW words of a row in
+// both value slots.  Inserting z at position i of a head splits the rank into a constant of
+// (head, i) and a term of (i, z), so a row's rank is one table entry and one add.
+// Bound: issue and shared-memory reads; both planes stay in L2 up to n of about 128.  Per launch:
+// G(n, p) n = 128 42 us with a rank per unit, 35 us so; Delaunay n = 389 4.9 and 3.4 ms.
+__host__ __device__ constexpr int lane_words(int RW) { return RW < 4 ? RW : 4; }
+__host__ __device__ constexpr int row_lanes(int RW) { return RW <= 4 ? 1 : (RW <= 8 ? 2 : 4); }
+// Heads per round of a block, and the body's words of shared memory.
+__host__ __device__ inline int heads_per_round(int threads, int n, int rwp) {
+    const int lq = rwp <= 4 ? 1 : (rwp <= 8 ? 2 : 4);
+    const int h = threads / lq / n;
+    return h < 1 ? 1 : (h > 32 ? 32 : h);
+}
+__host__ __device__ inline int head_smem_words(int threads, int k, int n, int rwp) {
+    return rank_table_words(k, n) + heads_per_round(threads, n, rwp) * n * 2 * rwp;
+}
+
+template <int K, int RW>
+__device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned wk, unsigned nwk) {
     extern __shared__ __align__(16) uint32_t sm[];
-    __shared__ uint32_t s_xy[32];
-    constexpr int K = 3;
-    const int n = d.g.n, rwp = d.g.rwp, S = d.S;
+    constexpr int M = K - 1, NW = lane_words(RW), LQ = row_lanes(RW);
+    __shared__ uint16_t s_head[32][M];
+    __shared__ uint32_t s_rank[32][K];
+    const int n = d.g.n, rwp = d.g.rwp, np1 = n + 1;
     const ColMeta mi = d.meta[nx];
     if (!d.h1 || mi.hi < mi.lo || mi.seed || frontier_sparse(d, mi)) return;
-    const int s_used = min(mi.hi - mi.base + 1, S);
-    const int nwords = s_used * rwp;
-    const int np1 = n + 1;
-    uint32_t* sB = sm;
+    const bool two = mi.hi > mi.base;          // the second value slot is in use
+    uint32_t* sD = sm;                         // [K][n + 1]: the rank's term of (position, z)
     uint32_t* stage = sm + rank_table_words(K, n);
-    for (int i = threadIdx.x; i < K * np1; i += blockDim.x) sB[i] = CR_LDG(&d.binom[i]);
-    const uint32_t* CR_RESTRICT fin = d.front + (size_t)nx * d.C * S * rwp;
+    for (int i = threadIdx.x; i < K * np1; i += blockDim.x) {
+        const uint32_t next = i + np1 < K * np1 ? CR_LDG(&d.binom[i + np1]) : 0u;
+        sD[i] = next - CR_LDG(&d.binom[i]);
+    }
+    const uint32_t* CR_RESTRICT fin = d.front + (size_t)nx * d.C * 2 * rwp;
     const uint8_t* CR_RESTRICT fflag_in = d.fflag + (size_t)nx * d.C;
     const uint32_t* CR_RESTRICT rp = cop_rows(d.g);
     const uint16_t* CR_RESTRICT adj = cop_cols(d.g);
-    const bool vec4 = (rwp & 3) == 0;
-    const int U = vec4 ? 4 : 1;
-    const int wc = pair_chunk_words(n, S, rwp);
-    const size_t rstride = (size_t)S * rwp;
-    const uint32_t P = (uint32_t)(n * (n + 1) / 2);
-    // pairs per round: enough units for every thread of the block when a row is staged whole
-    int PR = 1;
-    if (wc >= nwords) {
-        PR = (int)blockDim.x / (n * (nwords / U));
-        PR = max(1, min(PR, min(32, kPairStageWords / (n * wc))));
-    }
+    const uint32_t rs = 2u * rwp;              // words of a row (S = 2 slots wherever H1 exists)
+    const int w0 = ((int)threadIdx.x % LQ) * NW, first = (int)threadIdx.x / LQ, per_it = (int)blockDim.x / LQ;
+    const bool mine = w0 < rwp;                // rows of 12 words: the last of 4 lanes has none
+    const uint32_t P = heads_below<M>(n);
+    const int PR = heads_per_round(blockDim.x, n, rwp);
     unsigned err = 0;
     for (uint32_t q0 = wk * PR; q0 < P; q0 += nwk * PR) {
         const int np = (int)min((uint32_t)PR, P - q0);
         if ((int)threadIdx.x < np) {
-            int x, y;
-            pair_of(q0 + threadIdx.x, n, x, y);
-            s_xy[threadIdx.x] = (uint32_t)x | ((uint32_t)y << 16);
+            int h[M];
+            head_of<M>(q0 + threadIdx.x, h);
+            // position i: sum over j < i of B[j][h_{j-1}] - B[j][h_j], then B[i][h_{i-1}], then
+            // -B[i+1][h_i], then sum over j > i of B[j+1][h_{j-1}] - B[j+1][h_j]
+#pragma unroll
+            for (int i = 0; i < K; ++i) {
+                uint32_t r = CR_LDG(&d.binom[i * np1 + (i ? h[i ? i - 1 : 0] : 0)]);
+#pragma unroll
+                for (int j = 0; j < M; ++j) {
+                    if (j < i) r += CR_LDG(&d.binom[j * np1 + (j ? h[j ? j - 1 : 0] : 0)]) - CR_LDG(&d.binom[j * np1 + h[j]]);
+                    else if (j == i) r -= CR_LDG(&d.binom[(j + 1) * np1 + h[j]]);
+                    else r += CR_LDG(&d.binom[(j + 1) * np1 + h[j - 1 < 0 ? 0 : j - 1]]) - CR_LDG(&d.binom[(j + 1) * np1 + h[j]]);
+                }
+                s_rank[threadIdx.x][i] = r;
+            }
+#pragma unroll
+            for (int i = 0; i < M; ++i) s_head[threadIdx.x][i] = (uint16_t)h[i];
         }
         __syncthreads();
-        uint32_t* out = d.h1 + (size_t)q0 * n * rstride;
-        for (int w0 = 0; w0 < nwords; w0 += wc) {
-            const int upr = min(wc, nwords - w0) / U;   // units (of U words) per row
-            const int per = n * upr;                    // units per pair
-            for (int i = threadIdx.x; i < np * per; i += blockDim.x) {
-                const int j = i / per, rem = i - j * per;
-                const int z = rem / upr, u = rem - z * upr;
-                const uint32_t xy = s_xy[j];
-                const int x = (int)(xy & 0xFFFFu), y = (int)(xy >> 16);
-                int cc[K];
-                cc[0] = z < x ? z : x;
-                cc[1] = z < x ? x : (z < y ? z : y);
-                cc[2] = z < y ? y : z;
-                uint32_t s = rank_s<K>(cc, sB, np1);
+        if (mine) {
+            int j = 0, z = first;
+            for (int i = first; i < np * n; i += per_it, z += per_it) {
+                while (z >= n) {
+                    z -= n;
+                    ++j;
+                }
+                int pos = 0;
+#pragma unroll
+                for (int q = 0; q < M; ++q) pos += z >= (int)s_head[j][q];
+                uint32_t s = s_rank[j][pos] + sD[pos * np1 + z];
                 const bool bad = s >= d.C;
                 if (bad) {
                     err |= kErrRank;
                     s = 0;
                 }
-                const bool live = !bad && CR_LDG(&fflag_in[s]) != 0;
-                const uint32_t* src = fin + (size_t)s * rstride + w0 + u * U;
-                uint32_t* dst = stage + (j * n + z) * wc + u * U;
-                if (vec4) {
-                    uint4 v = CR_LDG(reinterpret_cast<const uint4*>(src));
-                    if (!live) v = make_uint4(0u, 0u, 0u, 0u);
-                    *reinterpret_cast<uint4*>(dst) = v;
-                } else {
-                    const uint32_t v = CR_LDG(src);
-                    dst[0] = live ? v : 0u;
+                const bool live = CR_LDG(&fflag_in[s]) != 0 && !bad;
+                const uint32_t* src = fin + (size_t)s * rs + w0;
+                uint32_t* dst = stage + (uint32_t)i * rs + w0;
+                Words<NW> x;
+                x.ldg(src);
+                if (!live) x.zero();
+                x.store(dst);
+                if (two) {
+                    x.ldg(src + rwp);
+                    if (!live) x.zero();
+                    x.store(dst + rwp);
                 }
             }
-            __syncthreads();
-            for (int i = threadIdx.x; i < np * per; i += blockDim.x) {
-                const int j = i / per, rem = i - j * per;
-                const int c = rem / upr, u = rem - c * upr;
+        }
+        __syncthreads();
+        if (mine) {
+            uint32_t* out = d.h1 + (size_t)q0 * n * rs + w0;
+            int j = 0, c = first;
+            for (int i = first; i < np * n; i += per_it, c += per_it) {
+                while (c >= n) {
+                    c -= n;
+                    ++j;
+                }
+                const uint32_t* sj = stage + (uint32_t)(j * n) * rs + w0;
+                Words<NW> a0, a1, x;
+                a0.zero();
+                a1.zero();
                 const uint32_t e1 = CR_LDG(&rp[c + 1]);
-                const uint32_t* sj = stage + j * n * wc + u * U;
-                uint32_t* o = out + ((size_t)j * n + c) * rstride + w0 + u * U;
-                if (vec4) {
-                    uint4 a = make_uint4(0u, 0u, 0u, 0u);
-                    for (uint32_t e = CR_LDG(&rp[c]); e < e1; ++e) {
-                        const uint4 v = *reinterpret_cast<const uint4*>(sj + CR_LDG(&adj[e]) * wc);
-                        a.x |= v.x; a.y |= v.y; a.z |= v.z; a.w |= v.w;
+                for (uint32_t e = CR_LDG(&rp[c]); e < e1; ++e) {
+                    const uint32_t* row = sj + CR_LDG(&adj[e]) * rs;
+                    x.load(row);
+                    a0.orr(x);
+                    if (two) {
+                        x.load(row + rwp);
+                        a1.orr(x);
                     }
-                    *reinterpret_cast<uint4*>(o) = a;
-                } else {
-                    uint32_t a = 0u;
-                    for (uint32_t e = CR_LDG(&rp[c]); e < e1; ++e) a |= sj[CR_LDG(&adj[e]) * wc];
-                    o[0] = a;
                 }
+                a0.store(out + (uint32_t)i * rs);
+                if (two) a1.store(out + (uint32_t)i * rs + rwp);
             }
-            __syncthreads();
         }
     }
     err = __reduce_or_sync(FULL_MASK, err);
     if ((threadIdx.x & 31) == 0 && err) atomicOr(d.err, err);
 }
 
-// Stage 2: a lane group per configuration, its lanes over the deg^2 pairs (x, y).
-template <int NWP, int G>
+// Stage 2: a warp per unit = (head c_1 .. c_{k-1}, tile of consecutive last cops c_k), LQ lanes of
+// NW words per row and R rows per lane: the configurations of a unit are consecutive, and so are
+// their rows H1[h'][c_k] for every head h' of successors, so each load of the warp is one
+// contiguous stretch, the successor heads are found once per unit (a lane each) and broadcast, and
+// the words a lane ORs are the words it marks: no reduction across lanes.  Units run tile by tile
+// of last cops, so that the H1 rows in use at a time (every head, one tile) stay in L2 where all
+// of them do not, and the warps take them from a counter: their costs (deg^(k-1) heads) differ by
+// an order of magnitude.  Bound: L2 latency and bandwidth (deg^(k-1) rows per configuration).
+// Per launch, against a lane per (configuration, successor pair) with a reduction: Delaunay n = 199
+// 500 -> 270 us (6.3 TB/s of row reads), n = 389 11.5 -> 3.7 ms; G(n, p) n = 61, k = 4, both sides
+// staying: 16 ms gathering tuples one by one, 0.8 ms so.
+template <int K, int RW>
 __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, unsigned wk, unsigned nwk) {
-    extern __shared__ __align__(16) uint32_t sm[];
-    constexpr int K = 3;
-    constexpr int CPW = 32 / G;
-    const int warp = threadIdx.x >> 5;
-    const Lanes<G> L(threadIdx.x & 31);
-    const int gl = L.glane;
-    const int n = d.g.n, rw = d.g.rw, rwp = d.g.rwp, S = d.S;
+    constexpr int M = K - 1, NW = lane_words(RW), LQ = row_lanes(RW);
+    constexpr int CH = 32 / LQ;                    // rows per load of the warp
+    constexpr int R = LQ == 1 ? 1 : 2;             // loads per tile
+    constexpr int TW = CH * R;                     // last cops per tile
+    const int lane = threadIdx.x & 31;
+    const int li = lane / LQ, w0 = (lane % LQ) * NW;
+    const int n = d.g.n, rwp = d.g.rwp, cols = d.cols;
     const ColMeta mi = d.meta[nx];
     if (!d.h1 || mi.hi < mi.lo || mi.seed || frontier_sparse(d, mi)) return;
-    const int base_in = mi.base;
-    const int s_used = min(mi.hi - base_in + 1, S);
-    const int nwords = s_used * rwp;
+    const bool two = mi.hi > mi.base;              // the frontier's second value slot is in use
     const int out_base = d.meta[col].base;
-    const int append = d.meta[col].append;
-    uint32_t* wacc = sm + (warp * CPW + L.grp) * (2 * S * rwp);
-    uint32_t* wnew = wacc + S * rwp;
+    const int v0 = mi.base + 1, v1 = mi.base + 2;  // values of the slots' marks
+    const uint32_t keep0 = v0 < kMaxRound ? FULL_MASK : 0u, keep1 = v1 < kMaxRound ? FULL_MASK : 0u;
+    const bool mine = w0 < rwp;                    // rows of 12 words: the last lane has none
+    Words<NW> vm;
+#pragma unroll
+    for (int i = 0; i < NW; ++i) vm.w[i] = valid_mask(n, w0 + i);
     const uint32_t* CR_RESTRICT rp = cop_rows(d.g);
     const uint16_t* CR_RESTRICT adj = cop_cols(d.g);
-    const uint32_t* CR_RESTRICT h1 = d.h1;
-    const bool vec4 = (rwp & 3) == 0;
-    const size_t rstride = (size_t)S * rwp;
+    const uint32_t* CR_RESTRICT h1 = d.h1 + w0;
+    const uint32_t rs = 2u * rwp;                  // words of a row (S = 2 slots wherever H1 exists)
+    const int np1 = n + 1;
     Tally t;
-    const size_t step = (size_t)nwk * (blockDim.x >> 5) * CPW;
-    for (size_t cb = ((size_t)wk * (blockDim.x >> 5) + warp) * CPW; cb < d.C; cb += step) {
-        const uint32_t cid = (uint32_t)(cb + L.grp);
-        const bool ok = cid < d.C;
-        const uint32_t vm = (ok && gl < rw) ? valid_mask(n, gl) : 0u;
-        const uint32_t m = (ok && gl < rw) ? d.marked[((size_t)col * d.C + cid) * rwp + gl] : 0u;
-        const bool full = L.all(m == vm);
-        const bool need = ok && !full;
-        if (!__any_sync(FULL_MASK, need)) continue;
-        int lo0 = 0, dg0 = 0, lo1 = 0, dg1 = 0, c3 = 0;
-        if (need) {
-            const uint16_t* cc = d.configs + (size_t)cid * K;
-            const int v0 = cc[0], v1 = cc[1];
-            c3 = cc[2];
-            lo0 = CR_LDG(&rp[v0]);
-            dg0 = CR_LDG(&rp[v0 + 1]) - lo0;
-            lo1 = CR_LDG(&rp[v1]);
-            dg1 = CR_LDG(&rp[v1 + 1]) - lo1;
+    uint32_t ticket = 0;                           // lane 0's; the next one is drawn a unit ahead
+    if (lane == 0) ticket = atomicAdd(&d.sync[2], 1u);
+    int c0 = 0;
+    uint32_t tile_first = 0, tile_units = heads_below<M>(min(n, TW));
+    for (;;) {
+        const uint32_t u = __shfl_sync(FULL_MASK, ticket, 0);
+        while (u - tile_first >= tile_units && c0 < n) {
+            tile_first += tile_units;
+            c0 += TW;
+            tile_units = heads_below<M>(min(n, c0 + TW));
         }
-        const int T = dg0 * dg1;
-        uint32_t acc[NWP];
+        if (c0 >= n) break;
+        if (lane == 0) ticket = atomicAdd(&d.sync[2], 1u);
+        int h[M];
+        head_of<M>(u - tile_first, h);
+        uint32_t first;                            // rank of (h, h[M-1]): the head's first configuration
+        {
+            int cc[K];
 #pragma unroll
-        for (int i = 0; i < NWP; ++i) acc[i] = 0u;
-        // odometer over N(c1) x N(c2): this lane starts at pair gl and steps by G
-        int i0 = 0, i1 = 0;
-        if (T > 0) {
-            i0 = gl / dg1;
-            i1 = gl - i0 * dg1;
+            for (int i = 0; i < M; ++i) cc[i] = h[i];
+            cc[M] = h[M - 1];
+            first = rank_g<K>(cc, d.binom, np1);
         }
-#pragma unroll 2
-        for (int tt = gl; tt < T; tt += G) {
-            const int xa = CR_LDG(&adj[lo0 + i0]), yb = CR_LDG(&adj[lo1 + i1]);
-            const uint32_t q = xa <= yb ? pair_index(xa, yb, n) : pair_index(yb, xa, n);
-            const uint32_t* hr = h1 + ((size_t)q * n + c3) * rstride;
-            if (vec4) {
+        const int dc = c0 - h[M - 1];              // the tile's first configuration, from that one
+        uint32_t* const mcol = d.marked + ((size_t)col * d.C + first) * rwp + w0;
+        bool open[R];
+        bool some = false;
 #pragma unroll
-                for (int w = 0; w < NWP; w += 4) {
-                    if (w < nwords) {
-                        const uint4 v = CR_LDG(reinterpret_cast<const uint4*>(hr + w));
-                        acc[w] |= v.x; acc[w + 1] |= v.y; acc[w + 2] |= v.z; acc[w + 3] |= v.w;
+        for (int r = 0; r < R; ++r) {
+            const int at = dc + r * CH + li;       // this lane's configuration, from the head's first
+            open[r] = false;
+            if (mine && at >= 0 && c0 + r * CH + li < n) {
+                Words<NW> m;
+                m.load(mcol + (size_t)at * rwp);
+#pragma unroll
+                for (int i = 0; i < NW; ++i) open[r] |= m.w[i] != vm.w[i];
+            }
+            some |= open[r];
+        }
+        if (!__any_sync(FULL_MASK, some)) continue;
+        uint32_t lo[M], dg[M], T = 1;
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+            lo[i] = CR_LDG(&rp[h[i]]);
+            dg[i] = CR_LDG(&rp[h[i] + 1]) - lo[i];
+            T *= dg[i];
+        }
+        Words<NW> a0[R], a1[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            a0[r].zero();
+            a1[r].zero();
+        }
+        const uint32_t row0 = (uint32_t)(c0 + li);
+        for (uint32_t t0 = 0; t0 < T; t0 += 32) {
+            uint32_t q = 0;                        // this lane's successor head
+            if (t0 + lane < T) {
+                uint32_t rem = t0 + lane;
+                int x[M];
+#pragma unroll
+                for (int i = M - 1; i >= 0; --i) {
+                    const uint32_t r = i ? rem / dg[i] : 0u;
+                    x[i] = CR_LDG(&adj[lo[i] + rem - r * dg[i]]);
+                    rem = r;
+                }
+                sort_small<M>(x);
+                q = head_index<M>(x) * (uint32_t)n;
+            }
+            const int cnt = (int)min(32u, T - t0);
+#pragma unroll 4
+            for (int j = 0; j < cnt; ++j) {
+                const uint32_t* p = h1 + (uint64_t)(__shfl_sync(FULL_MASK, q, j) + row0) * rs;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (open[r]) {                 // (a lane whose words are all marked reads none)
+                        Words<NW> x;
+                        x.ldg(p + r * CH * rs);
+                        a0[r].orr(x);
+                        if (two) {
+                            x.ldg(p + r * CH * rs + rwp);
+                            a1[r].orr(x);
+                        }
                     }
                 }
-            } else {
-#pragma unroll
-                for (int w = 0; w < NWP; ++w)
-                    if (w < nwords) acc[w] |= CR_LDG(hr + w);
-            }
-            i1 += G;
-            while (i1 >= dg1 && i0 < dg0) {
-                i1 -= dg1;
-                ++i0;
             }
         }
-        group_or<NWP, G>(acc, gl, wacc, need ? nwords : 0);
-        __syncwarp();
-        emit_row<G>(d, cid, need, col, m, wacc, wnew, base_in, s_used, out_base, append, L, t);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            // the lane's new marks: the lower slot's value wins
+            const int at = dc + r * CH + li;
+            uint32_t* mrow = mcol + (size_t)at * rwp;
+            uint32_t any0 = 0u, any1 = 0u;
+            Words<NW> m;
+            if (open[r]) {
+                m.load(mrow);
+#pragma unroll
+                for (int i = 0; i < NW; ++i) {
+                    a0[r].w[i] &= ~m.w[i] & vm.w[i] & keep0;
+                    a1[r].w[i] &= ~(m.w[i] | a0[r].w[i]) & vm.w[i] & keep1;
+                }
+                any0 = a0[r].any();
+                any1 = a1[r].any();
+            }
+            // (the words of a lane that is not open are zero: it has read nothing)
+            bool newrow = (any0 | any1) != 0u;
+            if (!__any_sync(FULL_MASK, newrow)) continue;
+#pragma unroll
+            for (int o = 1; o < LQ; o <<= 1) newrow |= __shfl_xor_sync(FULL_MASK, (int)newrow, o) != 0;
+            const uint32_t cid = first + (uint32_t)at;
+            int marks = 0, words = 0;
+#pragma unroll
+            for (int i = 0; i < NW; ++i) {
+                marks += __popc(a0[r].w[i] | a1[r].w[i]);
+                words += (a0[r].w[i] | a1[r].w[i]) != 0u;
+            }
+            t.cnt += marks;
+            if (newrow && mine) {
+                if (any0) {
+                    t.lo = min(t.lo, v0);
+                    t.hi = max(t.hi, v0);
+                    if (v0 < out_base || v0 > out_base + 1) t.err |= kErrSlot;
+                }
+                if (any1) {
+                    t.lo = min(t.lo, v1);
+                    t.hi = max(t.hi, v1);
+                    if (v1 < out_base || v1 > out_base + 1) t.err |= kErrSlot;
+                }
+                uint32_t* frow = d.front + ((size_t)col * d.C + cid) * rs + w0;
+                Words<NW> z;
+                z.zero();
+                (v0 == out_base ? a0[r] : (v1 == out_base ? a1[r] : z)).store(frow);
+                (v0 == out_base + 1 ? a0[r] : (v1 == out_base + 1 ? a1[r] : z)).store(frow + rwp);
+                if (any0 | any1) {
+                    m.orr(a0[r]);
+                    m.orr(a1[r]);
+                    m.store(mrow);
+                }
+                if (w0 == 0) {
+                    d.fflag[(size_t)col * d.C + cid] = 1;
+                    t.rows++;
+                }
+            }
+            // table bytes (first + dc may lie before the head's first configuration: only lanes
+            // with marks, which lie behind it, are written for)
+            if (by_words(marks, words)) {
+                uint8_t* base = d.table + (size_t)first * n * cols + col;
+#pragma unroll
+                for (int i = 0; i < NW; ++i) {
+                    unsigned lanes = __ballot_sync(FULL_MASK, (a0[r].w[i] | a1[r].w[i]) != 0u);
+                    while (lanes) {
+                        const int l = __ffs(lanes) - 1;
+                        lanes &= lanes - 1;
+                        const uint32_t x0 = __shfl_sync(FULL_MASK, a0[r].w[i], l), x1 = __shfl_sync(FULL_MASK, a1[r].w[i], l);
+                        const uint32_t off = ((uint32_t)(dc + r * CH + l / LQ) * n + ((l % LQ) * NW + i) * 32) * cols;
+                        store_word(base + off, x1, x0, v1, v0, cols, lane);
+                    }
+                }
+            } else if (any0 | any1) {
+                uint8_t* trow = d.table + ((size_t)cid * n + w0 * 32) * cols + col;
+#pragma unroll
+                for (int i = 0; i < NW; ++i) {
+                    uint32_t b = a0[r].w[i] | a1[r].w[i];
+                    while (b) {
+                        const int j = __ffs(b) - 1;
+                        b &= b - 1;
+                        trow[(size_t)(i * 32 + j) * cols] = (uint8_t)(1 | (((a0[r].w[i] >> j) & 1u ? v0 : v1) << 1));
+                    }
+                }
+            }
+            // list the new rows: one atomic per R rows' load
+            const bool put = newrow && mine && w0 == 0;
+            const unsigned nb = __ballot_sync(FULL_MASK, put);
+            int list_at = 0;
+            if (lane == 0) list_at = atomicAdd(&d.meta[col].len, __popc(nb));
+            list_at = __shfl_sync(FULL_MASK, list_at, 0);
+            if (put) d.list[(size_t)col * d.C + list_at + __popc(nb & ((1u << lane) - 1u))] = cid;
+        }
     }
-    t.flush(d, col, L.lane);
+    t.flush(d, col, lane);
 }
 
 // Cop turn from the capture seeds (column 1 before pass 1): OR over T(C) of the seed rows
@@ -1905,24 +2140,6 @@ __device__ CR_BODY_INLINE void and_body(const V1Dev& d, int col, unsigned wk, un
         }
     }
     t.flush(d, col, L.lane);
-}
-
-// The table bytes of one row word's new marks, a lane per robber: n1 / n0 = the marks of the
-// higher and the lower value, at = the byte of the word's first robber.  The warp's stores fall
-// in one stretch of 32 * cols bytes, where a loop over one lane's bits is a transaction per byte.
-__device__ __forceinline__ void store_word(uint8_t* at, uint32_t n1, uint32_t n0, int v1, int v0, int cols, int lane) {
-    if (((n1 | n0) >> lane) & 1u) at[lane * cols] = (uint8_t)(1 | (((n1 >> lane) & 1u ? v1 : v0) << 1));
-}
-
-// Whether a warp writes its new marks word by word (store_word) or each lane the bits of its own
-// words, from the lane's marks and non-empty words.  By words costs about 15 instructions and a
-// transaction and a half per word; by lanes about 10 instructions per mark of the fullest lane and
-// a scattered transaction per mark, the transactions being the SM's and the instructions a
-// quarter's: by words where 8 words < 5 fullest + 2 marks.  (At n = 128 the two meet near two marks
-// per word: 80 against 90 us for a last column of 1.8 marks per word, 181 against 101 us at 3.8.)
-__device__ __forceinline__ bool by_words(int marks, int words) {
-    return 8 * __reduce_add_sync(FULL_MASK, words) <
-           5 * __reduce_max_sync(FULL_MASK, marks) + 2 * __reduce_add_sync(FULL_MASK, marks);
 }
 
 // 32 x 32 bit transpose across a warp: lane i holds row i and gets column i back (bit j of lane i

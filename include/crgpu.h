@@ -191,7 +191,7 @@ int cr_solver_set_v2_hash_capacity(cr_solver* s, uint64_t slots);
 #define CR_FORM_FUSED_FIRST 0x01u  /* initializeCaptures and pass 1 in one kernel (p = 1) */
 #define CR_FORM_PUSH        0x02u  /* cop turns of sparse frontiers: scatter to predecessors */
 #define CR_FORM_PULL        0x04u  /* cop turns of dense frontiers: gather from successors */
-#define CR_FORM_SEPARABLE   0x08u  /* the dense cop turn through pair rows (k = 3) */
+#define CR_FORM_SEPARABLE   0x08u  /* the dense cop turn through head rows (k = 2, 3, 4) */
 #define CR_FORM_FRESH_LAST  0x10u  /* the last column from this pass's column-0 marks */
 #define CR_FORMS_ALL        0x1Fu
 int cr_solver_set_forms(cr_solver* s, uint32_t mask);
@@ -321,7 +321,7 @@ int cr_server_destroy(cr_server* srv);
  *     primary context) it is stale, so do not call this entry point again in that process.
  *   - It runs the general forms only -- initializeCaptures unfused from pass 1 and the
  *     tuple-gathering cop turn -- because the fused first pass's tables and the separable
- *     turn's pair rows need memory beyond the area; it is slower than cr_solve.
+ *     turn's head rows need memory beyond the area; it is slower than cr_solve.
  *   - All calls share the array and leave their contents in it; each call clears what must
  *     start at zero.  Calls whose GPU work overlaps (other streams or host threads) race.
  * stream: cudaStream_t or NULL.  pass_counts[0 .. *passes) receive the per-pass counts;
