@@ -9,35 +9,43 @@
 //     robber ply d leaves no robber alive         -> 2d            (v2:312-319)
 //     d = p, cloud inside the marked set of C_p   -> 2p + max round (v2:321-334)
 // Branch-and-bound order and the two skip filters (v2:450-523) change only the work, not
-// that minimum, so these kernels compute it directly, level by level:
+// that minimum, so these kernels compute it directly, level by level.
 //
-//   val1[C1][r] = value of the depth-1 node (C1, N(r) \ C1): a warp per (C1, r), lanes over
-//                 the successors C2 of C1, each lane running the rest of the trajectory tree
-//                 depth first (clouds as multi-word vertex bitmasks, expanded by OR over
-//                 neighbour masks held in shared memory);
-//   root[C0][r] = min over C1 in T(C0) of (1 if r in C1, 2 if N(r) within C1, else val1).
+// Every pass needs only what the last one changed.  Terminal events do not depend on the table
+// and leaves need marks besides the captures (a cloud never holds a cop), so the first pass
+// evaluates terminal events only, and marks values in 1 .. 2p.  A leaf that becomes available in
+// a later pass t holds a state marked in pass t - 1; by induction the marks of pass s lie in
+// (2p(s-1), 2ps], so its cost lies in (2p(t-1), 2pt]: above everything found before, at any depth
+// (costs are absolute plies).  Hence a node's value is final in the pass that first finds one, and
+// a later pass evaluates open nodes only, from leaves at the configurations changed by the pass
+// before it.  lev[j] flags the configurations with a changed one exactly j cop steps away
+// (k_v2_dilate); a depth-d node has new leaves only within lev[p-d].
 //
-// Only leaves read the table, and a depth-1 node's leaves lie p-1 cop steps away, so after
-// the first pass val1 is recomputed only for configs within p-1 cop steps of a config that
-// gained marks ("dirty"); the others keep last pass's value, which is exact because the
-// snapshot they read has not changed there.
+// Clouds repeat heavily.  The robber moves first, so the depth-2 node below (C1, r) with cops C2
+// has the cloud N(N(r) \ C1 \ C2) \ C2: for every predecessor C1 of C2 that misses N(r) it is the
+// same plain node (C2, r).  So each pass goes
+//   k_v2_unsafe   per changed configuration C the vertices with a neighbour unmarked in row C: a
+//                 leaf at C is available when the cloud before the last robber ply misses them
+//                 (one AND, no expansion);
+//   k_v2_plain    plain[C2][r], the values of the plain depth-2 nodes;
+//   k_v2_val1     val1[C1][r], the values of the depth-1 nodes (C1, N(r) \ C1): for the robbers
+//                 with no cop in N(r), the minimum of the rows plain[C2] over the successors C2;
+//                 for the few touched ones, child by child;
+//   k_v2_root     root[C0][r] = min over C1 in T(C0) of (1 if r in C1, 2 if N(r) within C1, else
+//                 val1).
 //
-// For p >= 3 the depth-2 nodes (C2, V2) repeat heavily: V2 = N(N(r) \ C1 \ C2) \ C2 is the same
-// cloud for every predecessor C1 of C2 that misses N(r), so many depth-1 nodes share each
-// depth-2 subtree (on a Delaunay graph of 199 vertices with k = 2, one full pass visits 79.3 M
-// depth-2 children but only 4.69 M distinct ones).  Each pass therefore dedups the reachable
-// depth-2 clouds in a device hash table before any leaf is read:
-//   k_v2_hinsert  every dirty depth-1 node inserts its non-terminal children (C2, V2): key =
-//                 (rank of C2 + 1) << 32 | 32-bit fingerprint of V2, claimed by atomicCAS with
-//                 linear probing; the claiming thread writes the full cloud beside the key;
-//   k_v2_heval    one thread per occupied slot takes the exact subtree minimum of its node;
-//   k_v2_val1     looks every child up (key equal AND full cloud equal) and takes the stored
-//                 value; a child it does not find (probe limit, table full, or a fingerprint
-//                 shared by two clouds of the same C2, whose second cloud never got a slot) is
-//                 evaluated directly, so the result is exact whatever the table holds.
-// The subtree value of a node depends only on (depth, C2, V2) and the pass's snapshot, so the
-// table is rebuilt every pass.  When the depth-1 nodes outnumber half the table, they are
-// processed in chunks, each with a fresh table.
+// For p >= 3 the children of touched nodes that are not plain are deduplicated in a device hash
+// table: k_v2_hinsert inserts them (key = (rank of C2 + 1) << 32 | fingerprint of the cloud,
+// claimed by atomicCAS with linear probing; the claiming thread writes the full cloud beside the
+// key), k_v2_heval takes the subtree minimum of each slot's node, and k_v2_val1 looks every such
+// child up (key equal AND full cloud equal); a child it does not find (probe limit, table full,
+// or a fingerprint shared by two clouds of the same C2, whose second cloud never got a slot) is
+// evaluated directly, so the result is exact whatever the table holds.  The table is rebuilt
+// every pass; when the depth-1 nodes outnumber half the table, they are processed in chunks, each
+// with a fresh table.
+//
+// Measured (Delaunay n = 199, k = 2, p = 3, six passes): 94 ms with every dirty depth-1 node's
+// children in the hash table and every leaf's cloud expanded, 10 ms so.
 #include <algorithm>
 #include <string>
 #include <vector>
@@ -69,9 +77,14 @@ struct V2Solver {
     uint32_t* nbr = nullptr;
     uint8_t* val1 = nullptr;
     uint8_t* newval = nullptr;
-    uint8_t* changed = nullptr;
-    uint8_t* dirty = nullptr;
-    uint8_t* tmp = nullptr;
+    uint8_t* plain = nullptr;       // [C][n] plain depth-2 values
+    uint32_t* unsafe = nullptr;     // [C][rwp], rows of changed configurations only
+    uint8_t* changed = nullptr;     // configurations that gained marks
+    uint8_t* lev = nullptr;         // [p][C]: a changed configuration j cop steps away
+    uint8_t* fin1 = nullptr;        // configurations with a depth-1 / plain value found this pass
+    uint8_t* fin2 = nullptr;
+    uint32_t* rnbr = nullptr;       // [n][rwp]: in-neighbour masks
+    uint32_t* vsets = nullptr;      // [2][rwp]: vertices with at most k moves, with none
     unsigned long long* counters = nullptr;
     unsigned int* err = nullptr;
     unsigned long long* h_pinned = nullptr;
@@ -96,9 +109,17 @@ struct V2Dev {
     const uint8_t* table;
     const uint32_t* marked;
     const uint32_t* nbr;
+    const uint32_t* rnbr;          // [n][rwp]: in-neighbour masks
+    const uint32_t* small;         // [rwp]: vertices with at most k out-neighbours
+    const uint32_t* still;         // [rwp]: vertices with none
     uint8_t* val1;
     uint8_t* newval;
-    const uint8_t* dirty;
+    uint8_t* plain;
+    uint32_t* unsafe;
+    const uint8_t* lev;            // [p][C]
+    uint8_t* fin1;
+    uint8_t* fin2;
+    bool first;                    // the first pass: terminal events only
     unsigned long long* count;     // [0] marks found, [1] depth-2 child visits, [2] table entries
     unsigned long long* hkey;      // null = no cloud table (p < 3)
     uint32_t* hmask;
@@ -230,14 +251,9 @@ __device__ __forceinline__ uint32_t move_target(const Moves<K>& mv, int t, const
     return config_rank<K>(c, B, np1);
 }
 
-// Phase D boundary (v2:321-334): cloud within the marked set of config cid -> 2p + max round.
+// Largest round among the vertices of V in row cid of the table.
 template <int W>
-__device__ __forceinline__ int leaf_cost(const V2Dev& d, uint32_t cid, const Mask<W>& V) {
-    if (cid >= d.C) return kV2None;  // never taken for a well-formed rank table
-    const uint32_t* mrow = d.marked + (size_t)cid * d.rwp;
-#pragma unroll
-    for (int j = 0; j < W; ++j)
-        if (j < d.rwp && (V.w[j] & ~__ldg(&mrow[j]))) return kV2None;
+__device__ __forceinline__ int max_round(const V2Dev& d, uint32_t cid, const Mask<W>& V) {
     const uint8_t* trow = d.table + (size_t)cid * d.n;
     int mx = 0;
 #pragma unroll
@@ -249,7 +265,64 @@ __device__ __forceinline__ int leaf_cost(const V2Dev& d, uint32_t cid, const Mas
             mx = max(mx, (int)(__ldg(&trow[v]) >> 1));
         }
     }
-    return 2 * d.p + mx;
+    return mx;
+}
+
+// Phase D boundary (v2:321-334) for the cloud `mid` left before the last robber ply (cops c, rank
+// cid): 2p + max round when its expansion lies within the marked set, which is when no vertex of
+// mid has an unmarked neighbour (cops are marked in their own row), i.e. when mid misses the unsafe
+// row.  Clouds whose expansion is empty are terminal and never get here.
+template <int W, int K>
+__device__ __forceinline__ int leaf_cost(const V2Dev& d, uint32_t cid, const int (&c)[K], const Mask<W>& mid,
+                                         const uint32_t* snbr) {
+    const uint32_t* urow = d.unsafe + (size_t)cid * d.rwp;
+    uint32_t bad = 0u;
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+        if (j < d.rwp) bad |= mid.w[j] & __ldg(&urow[j]);
+    if (bad) return kV2None;
+    Mask<W> nx = expand<W>(mid, snbr, d.rwp);
+    mask_clear<W, K>(nx, c);
+    return 2 * d.p + max_round<W>(d, cid, nx);
+}
+
+// Whether some cop move below (c, V) can leave the robber nowhere: what a move leaves of V must
+// then be vertices with at most K neighbours, and a move takes at most K vertices away.
+template <int W, int K>
+__device__ __forceinline__ bool may_trap(const V2Dev& d, const Mask<W>& V) {
+    int big = 0;
+#pragma unroll
+    for (int j = 0; j < W; ++j)
+        if (j < d.rwp) big += __popc(V.w[j] & ~__ldg(&d.small[j]));
+    return big <= K;
+}
+
+// Minimum over the children of a depth p - 1 node (c, V).  In the first pass only the terminal
+// events count (no cloud lies within the captures alone), in a later one only the leaves at
+// configurations that gained marks in the last pass.
+template <int W, int K>
+__device__ int last_ply_min(const V2Dev& d, const int (&c)[K], const Mask<W>& V, const uint32_t* snbr, int best) {
+    if (d.first && !may_trap<W, K>(d, V)) return best;
+    Moves<K> mv;
+    moves_of<K>(mv, c, d.rp);
+    const int np1 = d.n + 1;
+    for (int t = 0; t < mv.T; ++t) {
+        int cp[K];
+        const uint32_t cid = next_target<K>(mv, d.col, d.binom, np1, cp);
+        if (cid >= d.C) continue;   // never taken for a well-formed rank table
+        if (!d.first && !__ldg(&d.lev[cid])) continue;
+        Mask<W> mid = V;
+        mask_clear<W, K>(mid, cp);
+        if (d.first) {
+            if (mask_empty<W>(mid)) return min(best, 2 * d.p - 1);   // the smallest value of such a node
+            Mask<W> nx = expand<W>(mid, snbr, d.rwp);
+            mask_clear<W, K>(nx, cp);
+            if (mask_empty<W>(nx)) best = min(best, 2 * d.p);
+        } else {
+            best = min(best, leaf_cost<W, K>(d, cid, cp, mid, snbr));
+        }
+    }
+    return best;
 }
 
 template <int W, int K>
@@ -259,11 +332,14 @@ struct Frame {
     int t;
 };
 
-// Minimum over the trajectory subtree below node (depth 2, cops c2, cloud V2), p >= 3.
+// Minimum over the trajectory subtree below node (depth 2, cops c2, cloud V2), p >= 3, of what this
+// pass can find: terminal events in the first pass, leaves at the changed configurations in the
+// others, where a child at depth dc is only entered when a changed configuration lies p - dc cop
+// steps away.
 template <int W, int K>
-__device__ int subtree_min(const V2Dev& d, const int (&c2)[K], const Mask<W>& V2,
-                           const uint32_t* snbr, int best) {
-    Frame<W, K> st[kV2MaxP - 2];
+__device__ int subtree_min(const V2Dev& d, const int (&c2)[K], const Mask<W>& V2, const uint32_t* snbr, int best) {
+    if (d.p == 3) return last_ply_min<W, K>(d, c2, V2, snbr, best);
+    Frame<W, K> st[kV2MaxP - 3];   // depths 2 .. p - 2
     int top = 0;
     st[0].V = V2;
     st[0].E = expand<W>(V2, snbr, d.rwp);
@@ -277,6 +353,8 @@ __device__ int subtree_min(const V2Dev& d, const int (&c2)[K], const Mask<W>& V2
         ++f.t;
         int c[K];
         const uint32_t cid = next_target<K>(f.mv, d.col, d.binom, np1, c);
+        if (cid >= d.C) continue;
+        if (!d.first && !__ldg(&d.lev[(size_t)(d.p - dc) * d.C + cid])) continue;
         Mask<W> nx;
         if (mask_hits<W, K>(f.V, c)) {
             Mask<W> mid = f.V;
@@ -288,41 +366,16 @@ __device__ int subtree_min(const V2Dev& d, const int (&c2)[K], const Mask<W>& V2
         }
         mask_clear<W, K>(nx, c);
         if (mask_empty<W>(nx)) { best = min(best, 2 * dc); continue; }
-        if (dc == d.p) { best = min(best, leaf_cost<W>(d, cid, nx)); continue; }
+        if (dc == d.p - 1) {
+            best = last_ply_min<W, K>(d, c, nx, snbr, best);
+            continue;
+        }
         Frame<W, K>& g = st[top + 1];
         g.V = nx;
         g.E = expand<W>(nx, snbr, d.rwp);
         moves_of<K>(g.mv, c, d.rp);
         g.t = 0;
         ++top;
-    }
-    return best;
-}
-
-// Minimum over the children of depth-2 node (c2, V2) when p = 3 (the children are leaves):
-// cop ply 3 empties the cloud -> 5, robber ply 3 leaves nobody -> 6, else the leaf cost.
-template <int W, int K>
-__device__ int node2_min_p3(const V2Dev& d, const int (&c2)[K], const Mask<W>& V2, const uint32_t* snbr) {
-    Moves<K> mv;
-    moves_of<K>(mv, c2, d.rp);
-    const Mask<W> E = expand<W>(V2, snbr, d.rwp);
-    const int np1 = d.n + 1;
-    int best = kV2None;
-    for (int t = 0; t < mv.T; ++t) {
-        int c[K];
-        const uint32_t cid = next_target<K>(mv, d.col, d.binom, np1, c);
-        Mask<W> nx;
-        if (mask_hits<W, K>(V2, c)) {
-            Mask<W> mid = V2;
-            mask_clear<W, K>(mid, c);
-            if (mask_empty<W>(mid)) return 5;   // the smallest value a depth-2 node can take
-            nx = expand<W>(mid, snbr, d.rwp);
-        } else {
-            nx = E;
-        }
-        mask_clear<W, K>(nx, c);
-        if (mask_empty<W>(nx)) { best = 6; continue; }
-        if (best > 6) best = min(best, leaf_cost<W>(d, cid, nx));
     }
     return best;
 }
@@ -350,8 +403,6 @@ __device__ __forceinline__ uint64_t cloud_slot(unsigned long long key, uint64_t 
     return (z ^ (z >> 31)) & (cap - 1);
 }
 
-// Insert (cid, V) unless its key is present; the thread that claims a slot writes the cloud.
-// Returns 1 when this call claimed a new slot.
 // Insert (cid, V) unless its key is present; the thread that claims a slot writes the cloud.
 // Returns 1 when this call claimed a new slot.
 template <int W>
@@ -394,54 +445,198 @@ __device__ __forceinline__ int cloud_lookup(const V2Dev& d, uint32_t cid, const 
     return -1;
 }
 
-// Depth-1 node (c1, r) of a chunk: its cops and cloud N(r) \ C1; false when the node is
-// decided without children (r on a cop, or no robber move left).
-template <int W, int K>
-__device__ __forceinline__ bool depth1_node(const V2Dev& d, uint32_t c1, int r, const uint32_t* snbr,
-                                            int (&cops1)[K], Mask<W>& V1) {
-    bool rin = false;
+template <int K>
+__device__ __forceinline__ void cops_of(const V2Dev& d, uint32_t cid, int (&c)[K]) {
 #pragma unroll
-    for (int i = 0; i < K; ++i) {
-        cops1[i] = d.configs[(size_t)c1 * K + i];
-        rin |= cops1[i] == r;
-    }
-    load_nbr<W>(V1, snbr, d.rwp, r);
-    mask_clear<W, K>(V1, cops1);
-    return !(rin || mask_empty<W>(V1));
+    for (int i = 0; i < K; ++i) c[i] = d.configs[(size_t)cid * K + i];
 }
 
-// Fill the cloud table with the distinct non-terminal depth-2 children of the chunk's dirty
-// depth-1 nodes: a warp per node, lanes over the cop moves.
+// The robbers r whose neighbourhood one of the cops stands in (N(r) meets C), cops left out: their
+// depth-1 clouds N(r) \ C are not N(r) itself.
+template <int W, int K>
+__device__ __forceinline__ Mask<W> touched_robbers(const V2Dev& d, const int (&c)[K]) {
+    Mask<W> e;
+#pragma unroll
+    for (int j = 0; j < W; ++j) {
+        e.w[j] = 0u;
+        if (j < d.rwp)
+#pragma unroll
+            for (int i = 0; i < K; ++i) e.w[j] |= __ldg(&d.rnbr[c[i] * d.rwp + j]);
+    }
+    mask_clear<W, K>(e, c);
+    return e;
+}
+
+// The child (C2, r) of a touched depth-1 node is the plain one of k_v2_plain when every cop of C1
+// in N(r) stands on a vertex of C2 too: C1 then takes nothing from N(r) that C2 does not.
+template <int W, int K>
+__device__ __forceinline__ bool plain_child(const Mask<W>& nr, const int (&c1)[K], const int (&c2)[K]) {
+    bool plain = true;
+#pragma unroll
+    for (int i = 0; i < K; ++i) {
+        bool in = false;
+#pragma unroll
+        for (int j = 0; j < K; ++j) in |= c1[i] == c2[j];
+        plain &= in || !((mask_word<W>(nr, c1[i] >> 5) >> (c1[i] & 31)) & 1u);
+    }
+    return plain;
+}
+
+__device__ __forceinline__ void load_graph(const V2Dev& d, uint32_t* snbr) {
+    for (int i = threadIdx.x; i < d.n * d.rwp; i += blockDim.x) snbr[i] = d.nbr[i];
+    __syncthreads();
+}
+
+// Unsafe rows of the configurations that gained marks: bit v of row C set iff v has a neighbour
+// unmarked in row C.  A warp per configuration, a lane per vertex.
+template <int W>
+__global__ void __launch_bounds__(256) k_v2_unsafe(V2Dev d) {
+    extern __shared__ uint32_t snbr[];
+    load_graph(d, snbr);
+    const int lane = threadIdx.x & 31;
+    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < d.C; c += nwarps) {
+        if (!d.lev[c]) continue;
+        Mask<W> m;
+#pragma unroll
+        for (int j = 0; j < W; ++j) m.w[j] = j < d.rwp ? __ldg(&d.marked[(size_t)c * d.rwp + j]) : 0u;
+        for (int w = 0; w < d.rwp; ++w) {
+            const int v = w * 32 + lane;
+            uint32_t out = 0u;
+            if (v < d.n) {
+#pragma unroll
+                for (int j = 0; j < W; ++j)
+                    if (j < d.rwp) out |= snbr[v * d.rwp + j] & ~m.w[j];
+            }
+            const unsigned u = __ballot_sync(0xFFFFFFFFu, out != 0u);
+            if (lane == 0) d.unsafe[(size_t)c * d.rwp + w] = u;
+        }
+    }
+}
+
+// Values of the plain depth-2 nodes plain[C2][r]: cloud N(N(r) \ C2) \ C2, the child of every
+// depth-1 node (C1, r) whose cops miss N(r).  3 / 4 = the cloud is empty after the cops' or the
+// robber's second ply; else p = 2: the leaf's cost; p >= 3: the subtree minimum.  A warp per
+// configuration C2, a lane per robber; for p = 3 the warp walks the moves in step (the changed
+// ones of 32 at a time), so a leaf test is one unsafe row, the same for all lanes, ANDed with each
+// lane's cloud.  Values are final once found (see the head of this file): later passes look at
+// the open nodes only.
+template <int K, int W>
+__global__ void __launch_bounds__(256) k_v2_plain(V2Dev d) {
+    extern __shared__ uint32_t snbr[];
+    load_graph(d, snbr);
+    const int lane = threadIdx.x & 31;
+    const int np1 = d.n + 1;
+    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
+    for (uint32_t c2 = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c2 < d.C; c2 += nwarps) {
+        if (!d.first && !d.lev[(size_t)(d.p - 2) * d.C + c2]) continue;
+        int cops[K];
+        cops_of<K>(d, c2, cops);
+        Moves<K> mv;
+        moves_of<K>(mv, cops, d.rp);
+        bool found = false;
+        for (int rb = 0; rb < d.n; rb += 32) {
+            const int r = rb + lane;
+            const size_t at = (size_t)c2 * d.n + r;
+            bool open = r < d.n && (d.first || d.plain[at] == kV2None);
+            if (!__any_sync(0xFFFFFFFFu, open)) continue;
+            int val = kV2None;
+            Mask<W> mid, V;
+            load_nbr<W>(mid, snbr, d.rwp, open ? r : 0);
+            mask_clear<W, K>(mid, cops);
+            V = expand<W>(mid, snbr, d.rwp);
+            mask_clear<W, K>(V, cops);
+            if (d.first) {
+                if (mask_empty<W>(mid)) val = 3;
+                else if (mask_empty<W>(V)) val = 4;
+            }
+            if (open && val == kV2None) {
+                if (d.p == 2) {
+                    if (!d.first) val = leaf_cost<W, K>(d, c2, cops, mid, snbr);
+                } else if (d.first || d.p > 3) {
+                    val = subtree_min<W, K>(d, cops, V, snbr, kV2None);
+                }
+            }
+            if (d.p == 3 && !d.first) {
+                for (int t0 = 0; t0 < mv.T; t0 += 32) {
+                    int c3[K];
+                    uint32_t cid = 0;
+                    bool go = false;
+                    if (t0 + lane < mv.T) {
+                        cid = move_target<K>(mv, t0 + lane, d.col, d.binom, np1, c3);
+                        go = cid < d.C && d.lev[cid];
+                    }
+                    unsigned todo = __ballot_sync(0xFFFFFFFFu, go);
+                    while (todo) {
+                        const int b = __ffs(todo) - 1;
+                        todo &= todo - 1;
+                        const uint32_t id = __shfl_sync(0xFFFFFFFFu, cid, b);
+                        int c[K];
+#pragma unroll
+                        for (int i = 0; i < K; ++i) c[i] = __shfl_sync(0xFFFFFFFFu, c3[i], b);
+                        if (open) {
+                            Mask<W> m = V;
+                            mask_clear<W, K>(m, c);
+                            val = min(val, leaf_cost<W, K>(d, id, c, m, snbr));
+                        }
+                    }
+                }
+            }
+            if (open && (d.first || val != kV2None)) {
+                d.plain[at] = (uint8_t)min(val, kV2None);
+                found |= val != kV2None;
+            }
+        }
+        if (__any_sync(0xFFFFFFFFu, found) && lane == 0) d.fin2[c2] = 1;
+    }
+}
+
+// Fill the cloud table with the distinct non-terminal depth-2 children of the chunk's touched
+// depth-1 nodes that are still open, plain ones (k_v2_plain) left out: a warp per configuration,
+// its touched robbers one by one, lanes over the cop moves.
 template <int K, int W>
 __global__ void __launch_bounds__(256) k_v2_hinsert(V2Dev d) {
     extern __shared__ uint32_t snbr[];
-    for (int i = threadIdx.x; i < d.n * d.rwp; i += blockDim.x) snbr[i] = d.nbr[i];
-    __syncthreads();
+    load_graph(d, snbr);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t nwarps = (size_t)gridDim.x * (blockDim.x >> 5);
+    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
     const int np1 = d.n + 1;
+    const uint32_t c_hi = (uint32_t)((d.node_hi + d.n - 1) / d.n);
     unsigned visits = 0, fresh = 0;
-    for (size_t idx = d.node_lo + (size_t)blockIdx.x * (blockDim.x >> 5) + warp; idx < d.node_hi; idx += nwarps) {
-        const uint32_t c1 = (uint32_t)(idx / d.n);
-        const int r = (int)(idx - (size_t)c1 * d.n);
-        if (!d.dirty[c1]) continue;
+    for (uint32_t c1 = (uint32_t)(d.node_lo / d.n) + blockIdx.x * (blockDim.x >> 5) + warp; c1 < c_hi; c1 += nwarps) {
+        if (!d.first && !d.lev[(size_t)(d.p - 1) * d.C + c1]) continue;
         int cops1[K];
-        Mask<W> V1;
-        if (!depth1_node<W, K>(d, c1, r, snbr, cops1, V1)) continue;
+        cops_of<K>(d, c1, cops1);
+        const Mask<W> touched = touched_robbers<W, K>(d, cops1);
         Moves<K> mv;
         moves_of<K>(mv, cops1, d.rp);
-        for (int t = lane; t < mv.T; t += 32) {
-            int c2[K];
-            const uint32_t cid2 = move_target<K>(mv, t, d.col, d.binom, np1, c2);
-            if (cid2 >= d.C) continue;
-            Mask<W> mid = V1;
-            mask_clear<W, K>(mid, c2);
-            if (mask_empty<W>(mid)) continue;
-            Mask<W> nx = expand<W>(mid, snbr, d.rwp);
-            mask_clear<W, K>(nx, c2);
-            if (mask_empty<W>(nx)) continue;
-            ++visits;
-            fresh += cloud_insert<W>(d, cid2, nx);
+        for (int j = 0; j < d.rwp; ++j) {
+            uint32_t bits = mask_word<W>(touched, j);
+            while (bits) {
+                const int r = j * 32 + __ffs(bits) - 1;
+                bits &= bits - 1;
+                const size_t idx = (size_t)c1 * d.n + r;
+                if (idx < d.node_lo || idx >= d.node_hi || (!d.first && d.val1[idx] != kV2None)) continue;
+                Mask<W> nr, V1;
+                load_nbr<W>(nr, snbr, d.rwp, r);
+                V1 = nr;
+                mask_clear<W, K>(V1, cops1);
+                if (mask_empty<W>(V1)) continue;
+                for (int t = lane; t < mv.T; t += 32) {
+                    int c2[K];
+                    const uint32_t cid2 = move_target<K>(mv, t, d.col, d.binom, np1, c2);
+                    if (cid2 >= d.C || (!d.first && !d.lev[(size_t)(d.p - 2) * d.C + cid2])) continue;
+                    if (plain_child<W, K>(nr, cops1, c2)) continue;
+                    Mask<W> mid = V1;
+                    mask_clear<W, K>(mid, c2);
+                    if (mask_empty<W>(mid)) continue;
+                    Mask<W> nx = expand<W>(mid, snbr, d.rwp);
+                    mask_clear<W, K>(nx, c2);
+                    if (mask_empty<W>(nx)) continue;
+                    ++visits;
+                    fresh += cloud_insert<W>(d, cid2, nx);
+                }
+            }
         }
     }
     visits = __reduce_add_sync(0xFFFFFFFFu, visits);
@@ -452,80 +647,185 @@ __global__ void __launch_bounds__(256) k_v2_hinsert(V2Dev d) {
     }
 }
 
-// Exact subtree minimum of every node in the cloud table: a thread per slot.
+// Subtree minimum of every node in the cloud table.  Few of the slots are taken (one in ten on a
+// Delaunay graph of 199 vertices), so each warp gathers the taken ones of its stretch in shared
+// memory and evaluates 32 at a time, a lane each: 1.70 ms a thread per slot, 0.61 ms so (largest pass of that solve).
 template <int K, int W>
 __global__ void __launch_bounds__(256) k_v2_heval(V2Dev d) {
     extern __shared__ uint32_t snbr[];
-    for (int i = threadIdx.x; i < d.n * d.rwp; i += blockDim.x) snbr[i] = d.nbr[i];
-    __syncthreads();
-    for (uint64_t h = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; h < d.hcap;
-         h += (uint64_t)gridDim.x * blockDim.x) {
-        const unsigned long long key = d.hkey[h];
-        if (key == 0ull) continue;
-        const uint32_t cid = (uint32_t)(key >> 32) - 1u;
-        int c2[K];
+    __shared__ uint64_t s_slots[8][64];
+    load_graph(d, snbr);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    uint64_t* slots = s_slots[warp];
+    int held = 0;   // warp-uniform
+    const uint64_t nwarps = (uint64_t)gridDim.x * 8;
+    const uint64_t per = (d.hcap / 32 + nwarps - 1) / nwarps * 32;   // (the capacity is a multiple of 1024)
+    const uint64_t lo = ((uint64_t)blockIdx.x * 8 + warp) * per, hi = lo + per < d.hcap ? lo + per : d.hcap;
+    for (uint64_t h0 = lo; h0 < hi || held > 0; h0 += 32) {
+        if (h0 < hi) {
+            const bool taken = d.hkey[h0 + lane] != 0ull;
+            const unsigned b = __ballot_sync(0xFFFFFFFFu, taken);
+            if (taken) slots[held + __popc(b & ((1u << lane) - 1u))] = h0 + lane;
+            held += __popc(b);
+            __syncwarp();
+            if (held < 32 && h0 + 32 < hi) continue;
+        }
+        const int take = min(held, 32);
+        if (lane < take) {
+            const uint64_t h = slots[lane];
+            const unsigned long long key = d.hkey[h];
+            const uint32_t cid = (uint32_t)(key >> 32) - 1u;
+            int c2[K];
+            cops_of<K>(d, cid, c2);
+            Mask<W> V;
 #pragma unroll
-        for (int i = 0; i < K; ++i) c2[i] = d.configs[(size_t)cid * K + i];
-        Mask<W> V;
-#pragma unroll
-        for (int j = 0; j < W; ++j) V.w[j] = j < d.rwp ? d.hmask[h * d.rwp + j] : 0u;
-        const int v = d.p == 3 ? node2_min_p3<W, K>(d, c2, V, snbr) : subtree_min<W, K>(d, c2, V, snbr, kV2None);
-        d.hkey[h] = key | (unsigned long long)min(v, kV2None);   // the value in the key word's low byte
+            for (int j = 0; j < W; ++j) V.w[j] = j < d.rwp ? d.hmask[h * d.rwp + j] : 0u;
+            const int v = subtree_min<W, K>(d, c2, V, snbr, kV2None);
+            d.hkey[h] = key | (unsigned long long)min(v, kV2None);   // the value in the key word's low byte
+        }
+        __syncwarp();
+        uint64_t rest = 0;
+        if (lane + 32 < held) rest = slots[lane + 32];
+        __syncwarp();
+        if (lane + 32 < held) slots[lane] = rest;
+        held -= take;
+        __syncwarp();
     }
 }
 
+// Depth-1 values: a warp per configuration C1 of the chunk.  The robbers whose neighbourhood no
+// cop of C1 stands in, a lane each: the minimum of plain[C2][r] over the successors C2 (whole rows
+// of bytes, the same C2 for all lanes; in later passes only the C2 that found something).  Then
+// the touched robbers one by one, lanes over the successors: a plain child's value, or the cloud
+// table's, or the node evaluated in place.
 template <int K, int W>
 __global__ void __launch_bounds__(256) k_v2_val1(V2Dev d) {
     extern __shared__ uint32_t snbr[];
-    for (int i = threadIdx.x; i < d.n * d.rwp; i += blockDim.x) snbr[i] = d.nbr[i];
-    __syncthreads();
+    load_graph(d, snbr);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t nwarps = (size_t)gridDim.x * (blockDim.x >> 5);
+    const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
     const int np1 = d.n + 1;
-    for (size_t idx = d.node_lo + (size_t)blockIdx.x * (blockDim.x >> 5) + warp; idx < d.node_hi; idx += nwarps) {
-        const uint32_t c1 = (uint32_t)(idx / d.n);
-        const int r = (int)(idx - (size_t)c1 * d.n);
-        if (!d.dirty[c1]) continue;
+    const uint32_t c_hi = (uint32_t)((d.node_hi + d.n - 1) / d.n);
+    unsigned visits = 0;
+    for (uint32_t c1 = (uint32_t)(d.node_lo / d.n) + blockIdx.x * (blockDim.x >> 5) + warp; c1 < c_hi; c1 += nwarps) {
+        if (!d.first && !d.lev[(size_t)(d.p - 1) * d.C + c1]) continue;
         int cops1[K];
-        Mask<W> V1;
-        if (!depth1_node<W, K>(d, c1, r, snbr, cops1, V1)) {
-            if (lane == 0) d.val1[idx] = kV2None;
+        cops_of<K>(d, c1, cops1);
+        bool found = false;
+        if (d.p == 1) {   // the depth-1 nodes are the leaves
+            if (!d.first) {
+                for (int r = lane; r < d.n; r += 32) {
+                    const size_t idx = (size_t)c1 * d.n + r;
+                    if (idx < d.node_lo || idx >= d.node_hi || d.val1[idx] != kV2None) continue;
+                    bool rin = false;
+#pragma unroll
+                    for (int i = 0; i < K; ++i) rin |= cops1[i] == r;
+                    if (rin || ((d.unsafe[(size_t)c1 * d.rwp + (r >> 5)] >> (r & 31)) & 1u)) continue;
+                    Mask<W> V1;
+                    load_nbr<W>(V1, snbr, d.rwp, r);
+                    mask_clear<W, K>(V1, cops1);
+                    if (mask_empty<W>(V1)) continue;
+                    d.val1[idx] = (uint8_t)(2 + max_round<W>(d, c1, V1));
+                    found = true;
+                }
+            }
+            if (__any_sync(0xFFFFFFFFu, found) && lane == 0) d.fin1[c1] = 1;
             continue;
         }
-        int best = kV2None;
-        if (d.p == 1) {
-            if (lane == 0) best = leaf_cost<W>(d, c1, V1);
-        } else {
-            Moves<K> mv;
-            moves_of<K>(mv, cops1, d.rp);
-            for (int t = lane; t < mv.T; t += 32) {
+        const Mask<W> touched = touched_robbers<W, K>(d, cops1);
+        Moves<K> mv;
+        moves_of<K>(mv, cops1, d.rp);
+        for (int rb = 0; rb < d.n; rb += 32) {
+            const int r = rb + lane;
+            const size_t idx = (size_t)c1 * d.n + r;
+            bool open = r < d.n && idx >= d.node_lo && idx < d.node_hi;
+            open = open && !((mask_word<W>(touched, r >> 5) >> (r & 31)) & 1u) && !((__ldg(&d.still[r >> 5]) >> (r & 31)) & 1u);
+#pragma unroll
+            for (int i = 0; i < K; ++i) open = open && cops1[i] != r;
+            if (open && !d.first) open = d.val1[idx] == kV2None;
+            if (!__any_sync(0xFFFFFFFFu, open)) continue;
+            int best = kV2None;
+            for (int t0 = 0; t0 < mv.T; t0 += 32) {
                 int c2[K];
-                const uint32_t cid2 = move_target<K>(mv, t, d.col, d.binom, np1, c2);
-                Mask<W> mid = V1;
-                mask_clear<W, K>(mid, c2);
-                if (mask_empty<W>(mid)) { best = 3; break; }
-                Mask<W> nx = expand<W>(mid, snbr, d.rwp);
-                mask_clear<W, K>(nx, c2);
-                if (mask_empty<W>(nx)) { best = min(best, 4); continue; }
-                if (d.p == 2) best = min(best, leaf_cost<W>(d, cid2, nx));
-                else if (best > 5) {
+                uint32_t cid = 0;
+                bool go = false;
+                if (t0 + lane < mv.T) {
+                    cid = move_target<K>(mv, t0 + lane, d.col, d.binom, np1, c2);
+                    go = cid < d.C && d.fin2[cid];
+                    if (d.first) go = cid < d.C;
+                }
+                unsigned todo = __ballot_sync(0xFFFFFFFFu, go);
+                while (todo) {
+                    const uint32_t id = __shfl_sync(0xFFFFFFFFu, cid, __ffs(todo) - 1);
+                    todo &= todo - 1;
+                    if (open) {
+                        const int v = d.plain[(size_t)id * d.n + r];
+                        best = min(best, v);
+                        visits += v > 4;
+                    }
+                }
+            }
+            if (open && best < kV2None) {
+                d.val1[idx] = (uint8_t)best;
+                found = true;
+            }
+        }
+        for (int j = 0; j < d.rwp; ++j) {
+            uint32_t bits = mask_word<W>(touched, j);
+            while (bits) {
+                const int r = j * 32 + __ffs(bits) - 1;
+                bits &= bits - 1;
+                const size_t idx = (size_t)c1 * d.n + r;
+                if (idx < d.node_lo || idx >= d.node_hi || (!d.first && d.val1[idx] != kV2None)) continue;
+                Mask<W> nr, V1;
+                load_nbr<W>(nr, snbr, d.rwp, r);
+                V1 = nr;
+                mask_clear<W, K>(V1, cops1);
+                if (mask_empty<W>(V1)) continue;
+                int best = kV2None;
+                for (int t = lane; t < mv.T; t += 32) {
+                    int c2[K];
+                    const uint32_t cid2 = move_target<K>(mv, t, d.col, d.binom, np1, c2);
+                    if (cid2 >= d.C || (!d.first && !d.lev[(size_t)(d.p - 2) * d.C + cid2])) continue;
+                    if (plain_child<W, K>(nr, cops1, c2)) {
+                        best = min(best, (int)d.plain[(size_t)cid2 * d.n + r]);
+                        continue;
+                    }
+                    Mask<W> mid = V1;
+                    mask_clear<W, K>(mid, c2);
+                    if (mask_empty<W>(mid)) { best = min(best, 3); continue; }
+                    if (d.p == 2 && !d.first) {
+                        best = min(best, leaf_cost<W, K>(d, cid2, c2, mid, snbr));
+                        continue;
+                    }
+                    Mask<W> nx = expand<W>(mid, snbr, d.rwp);
+                    mask_clear<W, K>(nx, c2);
+                    if (mask_empty<W>(nx)) { best = min(best, 4); continue; }
+                    if (d.p == 2 || best <= 5) continue;
                     // the cloud table holds the node unless an insert gave up on it
                     const int v = d.hkey ? cloud_lookup<W>(d, cid2, nx) : -1;
                     best = v >= 0 ? min(best, v) : subtree_min<W, K>(d, c2, nx, snbr, best);
                 }
+                best = __reduce_min_sync(0xFFFFFFFFu, best);
+                if (best < kV2None) {
+                    if (lane == 0) d.val1[idx] = (uint8_t)best;
+                    found = true;
+                }
             }
         }
-        best = __reduce_min_sync(0xFFFFFFFFu, best);
-        if (lane == 0) d.val1[idx] = (uint8_t)min(best, kV2None);
+        if (__any_sync(0xFFFFFFFFu, found) && lane == 0) d.fin1[c1] = 1;
     }
+    visits = __reduce_add_sync(0xFFFFFFFFu, visits);
+    if (lane == 0 && visits) atomicAdd(&d.count[1], (unsigned long long)visits);
 }
 
-// Root values of the unmarked states; buffered in newval (the snapshot stays intact).
+// Root values of the unmarked states; buffered in newval (the snapshot stays intact).  A warp per
+// configuration, a lane per robber, the successors 32 at a time; in later passes only the
+// successors that found something (a state unmarked so far has no older value).
 template <int K, int W>
 __global__ void __launch_bounds__(256) k_v2_root(V2Dev d) {
     extern __shared__ uint32_t snbr[];
-    for (int i = threadIdx.x; i < d.n * d.rwp; i += blockDim.x) snbr[i] = d.nbr[i];
-    __syncthreads();
+    if (d.first) load_graph(d, snbr);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
     const int np1 = d.n + 1;
@@ -533,36 +833,64 @@ __global__ void __launch_bounds__(256) k_v2_root(V2Dev d) {
     for (uint32_t c0 = blockIdx.x * (blockDim.x >> 5) + warp; c0 < d.C; c0 += nwarps) {
         const uint32_t* mrow = d.marked + (size_t)c0 * d.rwp;
         int cops0[K];
-#pragma unroll
-        for (int i = 0; i < K; ++i) cops0[i] = d.configs[(size_t)c0 * K + i];
+        cops_of<K>(d, c0, cops0);
         Moves<K> mv;
         moves_of<K>(mv, cops0, d.rp);
+        if (!d.first) {   // nothing found below: the common case
+            bool any = false;
+            for (int t = lane; t < mv.T; t += 32) {
+                int c1[K];
+                const uint32_t cid = move_target<K>(mv, t, d.col, d.binom, np1, c1);
+                any |= cid < d.C && d.fin1[cid];
+            }
+            if (!__any_sync(0xFFFFFFFFu, any)) continue;
+        }
         for (int rb = 0; rb < d.n; rb += 32) {
             const int r = rb + lane;
             const bool live = r < d.n && !((__ldg(&mrow[r >> 5]) >> (r & 31)) & 1u);
             if (!__any_sync(0xFFFFFFFFu, live)) continue;
             int best = kV2None;
             Mask<W> nr;
-            if (live) load_nbr<W>(nr, snbr, d.rwp, r);
+            // cop ply 1 catches r, or leaves it no move: only robbers with at most K moves
+            const bool few = d.first && live && ((__ldg(&d.small[r >> 5]) >> (r & 31)) & 1u);
+            if (few) load_nbr<W>(nr, snbr, d.rwp, r);
+            for (int t0 = 0; t0 < mv.T; t0 += 32) {
+                int own[K];
+                uint32_t cid = 0;
+                bool go = false;
 #pragma unroll
-            for (int i = 0; i < K; ++i) mv.idx[i] = 0;
-            for (int t = 0; t < mv.T; ++t) {
-                int c1[K];
-                const uint32_t cid1 = next_target<K>(mv, d.col, d.binom, np1, c1);
-                if (!live) continue;
-                bool rin = false;
+                for (int i = 0; i < K; ++i) own[i] = 0;
+                if (t0 + lane < mv.T) {
+                    cid = move_target<K>(mv, t0 + lane, d.col, d.binom, np1, own);
+                    go = cid < d.C && (d.first || d.fin1[cid]);
+                }
+                unsigned todo = __ballot_sync(0xFFFFFFFFu, go);
+                while (todo) {
+                    const int b = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const uint32_t id = __shfl_sync(0xFFFFFFFFu, cid, b);
+                    if (d.first) {
+                        int c1[K];
+                        bool rin = false;
 #pragma unroll
-                for (int i = 0; i < K; ++i) rin |= c1[i] == r;
-                if (rin) { best = 1; continue; }
-                Mask<W> v1 = nr;
-                mask_clear<W, K>(v1, c1);
-                if (mask_empty<W>(v1)) { best = min(best, 2); continue; }
-                if (cid1 < d.C) best = min(best, (int)d.val1[(size_t)cid1 * d.n + r]);
+                        for (int i = 0; i < K; ++i) {
+                            c1[i] = __shfl_sync(0xFFFFFFFFu, own[i], b);
+                            rin |= c1[i] == r;
+                        }
+                        if (rin) {
+                            best = 1;
+                        } else if (few) {
+                            Mask<W> v1 = nr;
+                            mask_clear<W, K>(v1, c1);
+                            if (mask_empty<W>(v1)) best = min(best, 2);
+                        }
+                    }
+                    if (live) best = min(best, (int)d.val1[(size_t)id * d.n + r]);
+                }
             }
-            if (live) {
-                const int v = best < kMaxRound ? best : kV2None;
-                d.newval[(size_t)c0 * d.n + r] = (uint8_t)v;
-                cnt += v != kV2None;
+            if (live && best < kMaxRound) {
+                d.newval[(size_t)c0 * d.n + r] = (uint8_t)best;
+                ++cnt;
             }
         }
     }
@@ -644,7 +972,7 @@ uint64_t v2_footprint(int n, int k, int p) {
     const uint64_t c = (uint64_t)C;
     const int rwp = round_words((n + 31) / 32);
     const uint64_t hcap = v2_hash_capacity(c * (uint64_t)n, p);
-    return c * n * 3 + c * (uint64_t)rwp * 4 + c * 3 + (uint64_t)n * rwp * 4 + c * (uint64_t)k * 2 +
+    return c * n * 4 + 2 * c * (uint64_t)rwp * 4 + c * (3 + kV2MaxP) + 2 * (uint64_t)n * rwp * 4 + c * (uint64_t)k * 2 +
            hcap * (8 + 4 * (uint64_t)rwp) + (1u << 16);
 }
 
@@ -655,7 +983,10 @@ static V2Dev v2_view(const V2Solver* s) {
     d.n = s->n; d.k = s->k; d.p = s->p; d.rwp = s->rwp; d.C = s->C;
     d.rp = s->rp; d.col = s->col; d.binom = s->binom; d.configs = s->configs;
     d.table = s->table; d.marked = s->marked; d.nbr = s->nbr;
-    d.val1 = s->val1; d.newval = s->newval; d.dirty = s->dirty; d.count = s->counters;
+    d.val1 = s->val1; d.newval = s->newval; d.count = s->counters;
+    d.plain = s->plain; d.unsafe = s->unsafe; d.lev = s->lev; d.fin1 = s->fin1; d.fin2 = s->fin2;
+    d.rnbr = s->rnbr; d.small = s->vsets; d.still = s->vsets + s->rwp;
+    d.first = s->first;
     d.hkey = s->hkey; d.hmask = s->hmask; d.hcap = s->hcap;
     d.node_lo = 0;
     d.node_hi = (uint64_t)s->C * s->n;
@@ -735,26 +1066,42 @@ int v2_create(V2Solver** out, cudaStream_t st, int num_sms, int n, int k, int p,
     V2_CUDA(cudaMalloc(&s->nbr, (size_t)n * s->rwp * 4));
     V2_CUDA(cudaMalloc(&s->val1, (size_t)C * n));
     V2_CUDA(cudaMalloc(&s->newval, (size_t)C * n));
+    V2_CUDA(cudaMalloc(&s->plain, (size_t)C * n));
+    V2_CUDA(cudaMalloc(&s->unsafe, (size_t)C * s->rwp * 4));
     V2_CUDA(cudaMalloc(&s->changed, C));
-    V2_CUDA(cudaMalloc(&s->dirty, C));
-    V2_CUDA(cudaMalloc(&s->tmp, C));
+    V2_CUDA(cudaMalloc(&s->lev, (size_t)C * p));
+    V2_CUDA(cudaMalloc(&s->fin1, C));
+    V2_CUDA(cudaMalloc(&s->fin2, C));
+    V2_CUDA(cudaMalloc(&s->rnbr, (size_t)n * s->rwp * 4));
+    V2_CUDA(cudaMalloc(&s->vsets, (size_t)2 * s->rwp * 4));
     V2_CUDA(cudaMalloc(&s->counters, 4 * sizeof(unsigned long long)));
     if (int rc = v2_set_hash_capacity(s, v2_hash_capacity((uint64_t)C * n, p), err)) return rc;
     V2_CUDA(cudaMallocHost(&s->h_pinned, 4 * sizeof(unsigned long long)));
     V2_CUDA(cudaEventCreate(&s->e0));
     V2_CUDA(cudaEventCreate(&s->e1));
     std::vector<uint32_t> nbr((size_t)n * s->rwp, 0);
-    for (int v = 0; v < n; ++v)
-        for (uint32_t e = h_rp[v]; e < h_rp[v + 1]; ++e) nbr[(size_t)v * s->rwp + (h_col[e] >> 5)] |= 1u << (h_col[e] & 31);
+    std::vector<uint32_t> rnbr((size_t)n * s->rwp, 0), vsets((size_t)2 * s->rwp, 0);
+    for (int v = 0; v < n; ++v) {
+        for (uint32_t e = h_rp[v]; e < h_rp[v + 1]; ++e) {
+            const int u = h_col[e];
+            nbr[(size_t)v * s->rwp + (u >> 5)] |= 1u << (u & 31);
+            rnbr[(size_t)u * s->rwp + (v >> 5)] |= 1u << (v & 31);
+        }
+        const uint32_t deg = h_rp[v + 1] - h_rp[v];
+        if (deg <= (uint32_t)k) vsets[v >> 5] |= 1u << (v & 31);
+        if (deg == 0) vsets[s->rwp + (v >> 5)] |= 1u << (v & 31);
+    }
     V2_CUDA(cudaMemcpyAsync(s->nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice, st));
+    V2_CUDA(cudaMemcpyAsync(s->rnbr, rnbr.data(), rnbr.size() * 4, cudaMemcpyHostToDevice, st));
+    V2_CUDA(cudaMemcpyAsync(s->vsets, vsets.data(), vsets.size() * 4, cudaMemcpyHostToDevice, st));
     V2_CUDA(cudaStreamSynchronize(st));
     return CR_OK;
 }
 
 void v2_destroy(V2Solver* s) {
     if (!s) return;
-    void* ptrs[] = {s->table, s->marked, s->nbr, s->val1, s->newval, s->changed, s->dirty, s->tmp, s->counters,
-                    s->hkey, s->hmask};
+    void* ptrs[] = {s->table, s->marked, s->nbr, s->val1, s->newval, s->plain, s->unsafe, s->changed, s->lev,
+                    s->fin1, s->fin2, s->rnbr, s->vsets, s->counters, s->hkey, s->hmask};
     for (void* q : ptrs)
         if (q) cudaFree(q);
     if (s->h_pinned) cudaFreeHost(s->h_pinned);
@@ -770,7 +1117,8 @@ int v2_init(V2Solver* s, uint64_t* caps, cr_solve_stats* stats, std::string* err
     V2_CUDA(cudaMemsetAsync(s->marked, 0, (size_t)s->C * s->rwp * 4, st));
     V2_CUDA(cudaMemsetAsync(s->newval, kV2None, (size_t)s->C * s->n, st));
     V2_CUDA(cudaMemsetAsync(s->val1, kV2None, (size_t)s->C * s->n, st));
-    V2_CUDA(cudaMemsetAsync(s->changed, 1, s->C, st));
+    V2_CUDA(cudaMemsetAsync(s->plain, kV2None, (size_t)s->C * s->n, st));
+    V2_CUDA(cudaMemsetAsync(s->changed, 0, s->C, st));
     V2_CUDA(cudaMemsetAsync(s->counters, 0, 4 * sizeof(unsigned long long), st));
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 255) / 256, (uint64_t)s->num_sms * 4));
     k_v2_init<<<grid, 256, 0, st>>>(s->table, s->marked, s->configs, s->C, s->n, s->k, s->rwp, s->counters);
@@ -792,7 +1140,7 @@ int v2_init(V2Solver* s, uint64_t* caps, cr_solve_stats* stats, std::string* err
 // Depth-1 values of the nodes [lo, hi): with a cloud table, fill it and evaluate its nodes
 // first.  Returns the kernels launched.
 template <int K, int W>
-static int launch_v2_val1(V2Solver* s, V2Dev d, uint64_t lo, uint64_t hi, int grid_pairs, size_t sm) {
+static int launch_v2_val1(V2Solver* s, V2Dev d, uint64_t lo, uint64_t hi, int grid_cfg, size_t sm) {
     cudaStream_t st = s->st;
     raise_smem_limit((const void*)k_v2_val1<K, W>, sm);
     d.node_lo = lo;
@@ -802,36 +1150,46 @@ static int launch_v2_val1(V2Solver* s, V2Dev d, uint64_t lo, uint64_t hi, int gr
         raise_smem_limit((const void*)k_v2_hinsert<K, W>, sm);
         raise_smem_limit((const void*)k_v2_heval<K, W>, sm);
         cudaMemsetAsync(d.hkey, 0, d.hcap * sizeof(unsigned long long), st);
-        k_v2_hinsert<K, W><<<grid_pairs, 256, sm, st>>>(d);
+        k_v2_hinsert<K, W><<<grid_cfg, 256, sm, st>>>(d);
         const int grid_h = (int)std::max<uint64_t>(1, std::min<uint64_t>((d.hcap + 255) / 256, (uint64_t)s->num_sms * 8));
         k_v2_heval<K, W><<<grid_h, 256, sm, st>>>(d);
         launches += 2;
         ++s->hstats.fills;
     }
-    k_v2_val1<K, W><<<grid_pairs, 256, sm, st>>>(d);
+    k_v2_val1<K, W><<<grid_cfg, 256, sm, st>>>(d);
     return launches + 1;
 }
 
 template <int K, int W>
-static int launch_v2_kernels(V2Solver* s, const V2Dev& d, int grid_pairs, int grid_cfg, size_t sm) {
+static int launch_v2_kernels(V2Solver* s, const V2Dev& d, int grid_cfg, size_t sm) {
     int launches = 0;
+    if (!d.first) {
+        raise_smem_limit((const void*)k_v2_unsafe<W>, sm);
+        k_v2_unsafe<W><<<grid_cfg, 256, sm, s->st>>>(d);
+        ++launches;
+    }
+    if (d.p >= 2) {
+        raise_smem_limit((const void*)k_v2_plain<K, W>, sm);
+        k_v2_plain<K, W><<<grid_cfg, 256, sm, s->st>>>(d);
+        ++launches;
+    }
     const uint64_t nodes = (uint64_t)s->C * s->n;
     const uint64_t chunk = d.hkey ? std::max<uint64_t>(1, s->chunk_nodes) : nodes;
     for (uint64_t lo = 0; lo < nodes; lo += chunk)
-        launches += launch_v2_val1<K, W>(s, d, lo, std::min(nodes, lo + chunk), grid_pairs, sm);
+        launches += launch_v2_val1<K, W>(s, d, lo, std::min(nodes, lo + chunk), grid_cfg, sm);
     raise_smem_limit((const void*)k_v2_root<K, W>, sm);
     k_v2_root<K, W><<<grid_cfg, 256, sm, s->st>>>(d);
     return launches + 1;
 }
 
 template <int K>
-static int launch_v2_k(V2Solver* s, const V2Dev& d, int W, int grid_pairs, int grid_cfg, size_t sm) {
+static int launch_v2_k(V2Solver* s, const V2Dev& d, int W, int grid_cfg, size_t sm) {
     switch (W) {
-        case 1: return launch_v2_kernels<K, 1>(s, d, grid_pairs, grid_cfg, sm);
-        case 2: return launch_v2_kernels<K, 2>(s, d, grid_pairs, grid_cfg, sm);
-        case 4: return launch_v2_kernels<K, 4>(s, d, grid_pairs, grid_cfg, sm);
-        case 8: return launch_v2_kernels<K, 8>(s, d, grid_pairs, grid_cfg, sm);
-        default: return launch_v2_kernels<K, 16>(s, d, grid_pairs, grid_cfg, sm);
+        case 1: return launch_v2_kernels<K, 1>(s, d, grid_cfg, sm);
+        case 2: return launch_v2_kernels<K, 2>(s, d, grid_cfg, sm);
+        case 4: return launch_v2_kernels<K, 4>(s, d, grid_cfg, sm);
+        case 8: return launch_v2_kernels<K, 8>(s, d, grid_cfg, sm);
+        default: return launch_v2_kernels<K, 16>(s, d, grid_cfg, sm);
     }
 }
 
@@ -846,18 +1204,11 @@ int v2_pass(V2Solver* s, uint64_t* found, cr_solve_stats* stats, std::string* er
     V2_CUDA(cudaMemsetAsync(s->counters, 0, 3 * sizeof(unsigned long long), st));
     const int grid_cfg_small = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 255) / 256, (uint64_t)s->num_sms * 4));
     int launches = 0;
-    if (s->first || s->p == 1) {
-        // first pass: every depth-1 node is evaluated; p = 1: dirty = changed
-        V2_CUDA(cudaMemcpyAsync(s->dirty, s->changed, s->C, cudaMemcpyDeviceToDevice, st));
-        if (s->first) V2_CUDA(cudaMemsetAsync(s->dirty, 1, s->C, st));
-    } else {
-        const uint8_t* in = s->changed;
-        uint8_t* bufs[2] = {s->dirty, s->tmp};
-        // p-1 steps; make the last one land in dirty
-        int steps = s->p - 1;
-        int cur = (steps % 2 == 1) ? 0 : 1;
-        for (int i = 0; i < steps; ++i) {
-            uint8_t* out = bufs[cur];
+    if (!s->first) {
+        V2_CUDA(cudaMemcpyAsync(s->lev, s->changed, s->C, cudaMemcpyDeviceToDevice, st));
+        for (int j = 1; j < s->p; ++j) {
+            const uint8_t* in = s->lev + (size_t)(j - 1) * s->C;
+            uint8_t* out = s->lev + (size_t)j * s->C;
             switch (s->k) {
                 case 1: launch_dilate<1>(s, in, out, grid_cfg_small); break;
                 case 2: launch_dilate<2>(s, in, out, grid_cfg_small); break;
@@ -865,22 +1216,21 @@ int v2_pass(V2Solver* s, uint64_t* found, cr_solve_stats* stats, std::string* er
                 default: launch_dilate<4>(s, in, out, grid_cfg_small); break;
             }
             ++launches;
-            in = out;
-            cur ^= 1;
         }
     }
-    s->first = false;
     V2_CUDA(cudaMemsetAsync(s->changed, 0, s->C, st));
-    V2Dev d = v2_view(s);
+    V2_CUDA(cudaMemsetAsync(s->fin1, 0, s->C, st));
+    V2_CUDA(cudaMemsetAsync(s->fin2, 0, s->C, st));
+    const V2Dev d = v2_view(s);
+    s->first = false;
     const size_t sm = (size_t)s->n * s->rwp * 4;
     const uint64_t pairs = (uint64_t)s->C * s->n;
-    const int grid_pairs = (int)std::max<uint64_t>(1, std::min<uint64_t>((pairs + 7) / 8, (uint64_t)s->num_sms * 8));
     const int grid_cfg = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 7) / 8, (uint64_t)s->num_sms * 8));
     switch (s->k) {
-        case 1: launches += launch_v2_k<1>(s, d, s->W, grid_pairs, grid_cfg, sm); break;
-        case 2: launches += launch_v2_k<2>(s, d, s->W, grid_pairs, grid_cfg, sm); break;
-        case 3: launches += launch_v2_k<3>(s, d, s->W, grid_pairs, grid_cfg, sm); break;
-        default: launches += launch_v2_k<4>(s, d, s->W, grid_pairs, grid_cfg, sm); break;
+        case 1: launches += launch_v2_k<1>(s, d, s->W, grid_cfg, sm); break;
+        case 2: launches += launch_v2_k<2>(s, d, s->W, grid_cfg, sm); break;
+        case 3: launches += launch_v2_k<3>(s, d, s->W, grid_cfg, sm); break;
+        default: launches += launch_v2_k<4>(s, d, s->W, grid_cfg, sm); break;
     }
     const int grid_apply = (int)std::max<uint64_t>(1, std::min<uint64_t>((pairs + 255) / 256, (uint64_t)s->num_sms * 8));
     k_v2_apply<<<grid_apply, 256, 0, st>>>(s->table, s->marked, s->newval, s->changed, s->C, s->n, s->rwp);
