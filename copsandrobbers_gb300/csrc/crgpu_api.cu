@@ -8,6 +8,7 @@
 #include <cstring>
 #include <new>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/crgpu.h"
@@ -17,18 +18,16 @@
 
 namespace crgpu {
 void launch_cop(const V1Dev& d, int col, int nx, int direct, int grid, cudaStream_t st, bool end = false);
-void launch_and(const V1Dev& d, int col, bool p1, int grid, cudaStream_t st, const LoopCtl* loop = nullptr);
-void launch_prep(const V1Dev& d, int col, int nx, int grid, cudaStream_t st);
+void launch_and(const V1Dev& d, int col, bool p1, int grid, cudaStream_t st, const LoopCtl& loop);
 void launch_init(const V1Dev& d, int grid, cudaStream_t st);
 void launch_init_pass1(const V1Dev& d, int num_sms, cudaStream_t st);
-void launch_list_compact(const V1Dev& d, int col, int num_sms, cudaStream_t st);
 void launch_marks_from_table(const uint8_t* table, uint32_t C, int n, int cols, int rwp, uint32_t* marked,
                              int grid, cudaStream_t st);
 void launch_game(const uint8_t* table, const uint16_t* configs, const unsigned long long* heads,
                  const unsigned long long* trans, const uint32_t* rp, const uint16_t* adj, int n, int k,
                  long long best, int cap, long long* out_c, int* out_r, int* count, int* captured,
                  cudaStream_t st);
-void launch_loop_enter(const V1Dev& d, const LoopCtl& c, int grid, cudaStream_t st);
+void launch_loop_enter(const V1Dev& d, const LoopCtl& c, int first, int grid, cudaStream_t st);
 void launch_verdict(const V1Dev& d, int cols, unsigned long long* best, int grid, cudaStream_t st);
 void launch_popcount(const uint32_t* plane, size_t words, unsigned long long* out, int grid,
                      cudaStream_t st);
@@ -49,6 +48,42 @@ void launch_digest(const uint8_t* table, size_t bytes, unsigned long long* out, 
 }  // namespace crgpu
 
 using namespace crgpu;
+
+// A solve's counters on the device, written whole before each initializeCaptures.
+struct SolveCtl {
+    unsigned long long counters[4];    // [0] pass_new, [1] verdict key, [2] scratch
+    unsigned err;
+    unsigned sync[kSyncWords];         // V1Dev::sync
+    int hist_n;                        // passes recorded since the last k_loop_enter
+    unsigned done;                     // V1Dev::done
+    int pad[2];
+    ColMeta* meta() { return reinterpret_cast<ColMeta*>(this + 1); }
+};
+// The pass counts go straight to the kit's pinned words, a ring that the host reads as they come;
+// the two words behind it take the verdict's and the digest's results.
+constexpr int kHistRing = 64;
+static_assert(sizeof(SolveCtl) % 16 == 0 && kHistRing + 2 <= cr_solver_kit::kWords, "control block");
+
+// Host images of a solver's small device arrays, laid out one after the other (256-byte aligned)
+// and uploaded with one copy.
+struct SmallArrays {
+    std::vector<uint8_t> bytes;
+    std::vector<std::pair<void**, size_t>> at;
+    template <typename T, typename D>
+    void add(D** slot, const std::vector<T>& v) {
+        const size_t off = (bytes.size() + 255) & ~size_t(255);
+        bytes.resize(off + std::max<size_t>(v.size() * sizeof(T), 1));
+        if (!v.empty()) memcpy(bytes.data() + off, v.data(), v.size() * sizeof(T));
+        at.push_back({(void**)slot, off});
+    }
+    // (the pageable source is staged before the copy call returns)
+    cudaError_t upload(cr_block_cache& cache, unsigned char** base, cudaStream_t st) {
+        cudaError_t e = cache.get((void**)base, bytes.size());
+        if (e == cudaSuccess) e = cudaMemcpyAsync(*base, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, st);
+        for (auto& a : at) *a.first = *base + a.second;
+        return e;
+    }
+};
 
 // Per-solve state.  Host copies of the graph are kept for the hop masks and file output.
 struct cr_solver {
@@ -82,7 +117,6 @@ struct cr_solver {
     uint32_t* d_cbits = nullptr;      // push-mode candidate bitmap
     uint32_t* d_list = nullptr;       // [cols][C] row lists of the frontiers
     uint32_t* d_clist = nullptr;      // [C] push-mode candidate list
-    unsigned* d_sync = nullptr;       // [kSyncWords] prep's block count, candidate count, units
     uint32_t* d_rrp = nullptr;
     uint16_t* d_rcol = nullptr;
     uint32_t* d_nbr = nullptr;
@@ -92,22 +126,16 @@ struct cr_solver {
     uint32_t* d_ell_off = nullptr;
     uint8_t* d_cover = nullptr;   // first-pass neighbour-slot masks (p = 1, max degree <= 32)
     int cover_w = 0, npad = 0;
-    ColMeta* d_meta = nullptr;
-    unsigned long long* d_counters = nullptr;  // [0] pass_new, [1] verdict key, [2] scratch
-    unsigned int* d_err = nullptr;
+    // the small arrays above (graph, rank table, masks) share one block, uploaded at once
+    unsigned char* d_small = nullptr;
+    // control block: SolveCtl, then the columns' ColMeta
+    SolveCtl* d_ctl = nullptr;
     unsigned long long* d_heads = nullptr;
     unsigned long long* d_trans = nullptr;
     uint64_t n_trans = 0;
-    // pinned read-back slots: [0..3] counters, [4..4+kPinHist) the pass history, then its
-    // length and the error bits
-    unsigned long long* h_pinned = nullptr;
-    cudaGraphExec_t pass_graph = nullptr;
-    // mainLoop on the device: a graph whose WHILE node replays one pass until a pass finds
-    // nothing; the pass counts land in d_hist, their number in d_hist_n
-    cudaGraphExec_t run_graph = nullptr;
-    unsigned long long* d_hist = nullptr;
-    int* d_hist_n = nullptr;
-    cudaEvent_t ev0 = nullptr, ev1 = nullptr, evc0 = nullptr, evc1 = nullptr;
+    cr_solver_kit kit;                // pinned: the ring of pass counts, then two words of results
+    bool init_timing = false;         // kit.ev[2], ev[3] bracket an initializeCaptures in flight
+    bool unsynced = false;            // the table may still be being written
     // phase state
     bool initialized = false;
     bool finished = false;
@@ -115,10 +143,6 @@ struct cr_solver {
     // set between cr_solver_init and that pass, and undone by materialize_init() when the
     // post-initializeCaptures state is read first
     bool init_pending = false;
-    // small solves launch each pass's kernels directly: capturing and instantiating a graph
-    // costs more than it saves over a handful of short passes, and contends for the CUDA driver
-    // when many solves run side by side (the solve server)
-    bool small = false;
     uint64_t base_caps = 0;
     std::vector<uint64_t> pass_counts;
     cr_solve_stats stats{};
@@ -144,8 +168,6 @@ static int fail(cr_context* ctx, int code, const char* fmt, ...) {
         if (e_ != cudaSuccess)                                                              \
             return fail((ctx), CR_ERR_CUDA, "%s failed: %s", #call, cudaGetErrorString(e_)); \
     } while (0)
-
-static constexpr int kPinHist = 64;   // pass counts read back with the pass loop's end
 
 static uint64_t binom_u64(int64_t n, int64_t k) {
     if (k < 0 || n < 0 || k > n) return 0;
@@ -189,6 +211,7 @@ int cr_context_destroy(cr_context* ctx) {
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     cudaSetDevice(ctx->device);
     ctx->cache.clear();
+    for (cr_solver_kit& k : ctx->kits) k.release();
     delete ctx;
     return CR_OK;
 }
@@ -286,45 +309,20 @@ uint64_t cr_solver_footprint(int32_t n, int32_t k, int32_t p, int32_t rules) {
     b += (uint64_t)cols * C * rwp * 4;                   // marked
     b += (uint64_t)cols * C * S * rwp * 4;               // frontiers
     b += C * S * rwp * 4 + cand_bits_bytes(C) + C * 4;   // push-mode candidate rows, bitmap, list
-    b += (uint64_t)cols * C * 4 + kSyncWords * sizeof(unsigned);  // frontier row lists, prep/list counters
+    b += (uint64_t)cols * C * 4;                         // frontier row lists
     b += h1_bytes(n, k, S, rwp);                         // separable dense cop turn
     b += (uint64_t)cols * C;                             // flags
     b += C * (uint64_t)k * 2;                            // configs
     b += (uint64_t)n * rwp * 4 * 3 + (uint64_t)k * (n + 1) * 4 + (1u << 16);
     if (cols == 2) b += 2ull * n * (uint64_t)((n + 7) & ~7) * 4;   // first-pass cover masks
-    b += (1u << 16) * 8ull + 256;                                 // device pass-loop history
     return b;
 }
 
 static void free_v1(cr_solver* s) {
-    if (s->pass_graph) cudaGraphExecDestroy(s->pass_graph);
-    s->pass_graph = nullptr;
-    if (s->run_graph) cudaGraphExecDestroy(s->run_graph);
-    s->run_graph = nullptr;
-    if (s->d_hist) cudaFree(s->d_hist);
-    if (s->d_hist_n) cudaFree(s->d_hist_n);
-    s->d_hist = nullptr;
-    s->d_hist_n = nullptr;
-    void* ptrs[] = {s->d_rp, s->d_col, s->d_binom, s->d_configs, s->d_hop, s->d_table,
-                    s->d_marked, s->d_front, s->d_fflag, s->d_meta, s->d_counters, s->d_err,
-                    s->d_heads, s->d_trans, s->d_cand, s->d_cbits, s->d_list, s->d_clist, s->d_sync,
-                    s->d_rrp, s->d_rcol, s->d_nbr, s->d_iso, s->d_rhop, s->d_cover, s->d_ell, s->d_ell_off,
-                    s->d_crp, s->d_ccol, s->d_ciso, s->d_h1};
-    for (void* q : ptrs) s->ctx->cache.put(q);   // the context keeps large blocks for reuse
-    s->d_rp = nullptr; s->d_col = nullptr; s->d_binom = nullptr; s->d_configs = nullptr;
-    s->d_hop = nullptr; s->d_table = nullptr; s->d_marked = nullptr; s->d_front = nullptr;
-    s->d_fflag = nullptr; s->d_meta = nullptr; s->d_counters = nullptr; s->d_err = nullptr;
-    s->d_heads = nullptr; s->d_trans = nullptr; s->d_cand = nullptr; s->d_cbits = nullptr;
-    s->d_list = nullptr; s->d_clist = nullptr; s->d_sync = nullptr;
-    s->d_rrp = nullptr; s->d_rcol = nullptr; s->d_nbr = nullptr; s->d_iso = nullptr; s->d_rhop = nullptr;
-    s->d_cover = nullptr; s->d_ell = nullptr; s->d_ell_off = nullptr;
-    s->d_crp = nullptr; s->d_ccol = nullptr; s->d_ciso = nullptr; s->d_h1 = nullptr;
-    if (s->h_pinned) cudaFreeHost(s->h_pinned);
-    s->h_pinned = nullptr;
-    cudaEvent_t evs[] = {s->ev0, s->ev1, s->evc0, s->evc1};
-    for (cudaEvent_t e : evs)
-        if (e) cudaEventDestroy(e);
-    s->ev0 = s->ev1 = s->evc0 = s->evc1 = nullptr;
+    void* ptrs[] = {s->d_small, s->d_ctl, s->d_configs, s->d_table, s->d_marked, s->d_front, s->d_fflag, s->d_heads,
+                    s->d_trans, s->d_cand, s->d_cbits, s->d_list, s->d_clist, s->d_h1};
+    for (void* q : ptrs) s->ctx->cache.put(q);   // the context keeps them for the next solver
+    s->ctx->put_kit(s->kit);
 }
 
 static V1Dev dev_view(const cr_solver* s) {
@@ -371,10 +369,11 @@ static V1Dev dev_view(const cr_solver* s) {
     d.fresh_last = (s->forms & CR_FORM_FRESH_LAST) ? 1 : 0;
     d.list = s->d_list;
     d.clist = s->d_clist;
-    d.sync = s->d_sync;
-    d.meta = s->d_meta;
-    d.pass_new = s->d_counters;
-    d.err = s->d_err;
+    d.sync = s->d_ctl->sync;      // (addresses only)
+    d.meta = s->d_ctl->meta();
+    d.pass_new = s->d_ctl->counters;
+    d.err = &s->d_ctl->err;
+    d.done = &s->d_ctl->done;
     return d;
 }
 
@@ -398,54 +397,48 @@ static std::vector<uint32_t> hop_masks(const cr_solver* s) {
     return hop;
 }
 
-static int alloc_v1(cr_solver* s) {
+static int alloc_v1(cr_solver* s, SmallArrays& small) {
     cr_context* ctx = s->ctx;
     const size_t C = s->C;
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_table, C * s->n * s->cols));
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_marked, (size_t)s->cols * C * s->rwp * 4));
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_front, (size_t)s->cols * C * s->S * s->rwp * 4));
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_fflag, (size_t)s->cols * C));
-    CR_CUDA(ctx, cudaMalloc(&s->d_meta, sizeof(ColMeta) * s->cols));
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_cand, C * s->S * s->rwp * 4));
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_cbits, cand_bits_bytes(C)));
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_list, (size_t)s->cols * C * 4));
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_clist, C * 4));
-    CR_CUDA(ctx, cudaMalloc(&s->d_sync, kSyncWords * sizeof(unsigned)));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_cand, 0, C * s->S * s->rwp * 4, ctx->stream));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_cbits, 0, cand_bits_bytes(C), ctx->stream));
     CR_CUDA(ctx, alloc_h1(s));
-    CR_CUDA(ctx, cudaMalloc(&s->d_hop, (size_t)s->n * s->rwp * 4));
     std::vector<uint32_t> hop = hop_masks(s);
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_hop, hop.data(), hop.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    // transposed hop masks: bit r of row u iff u in hop(r)
-    std::vector<uint32_t> rhop(hop.size(), 0);
-    for (int r = 0; r < s->n; ++r)
-        for (int u = 0; u < s->n; ++u)
-            if ((hop[(size_t)r * s->rwp + (u >> 5)] >> (u & 31)) & 1u)
+    small.add(&s->d_hop, hop);
+    // transposed hop masks (bit r of row u iff u in hop(r)), and hop(r) as lists
+    std::vector<uint32_t> rhop(hop.size(), 0), list_at(s->n + 1, 0);
+    std::vector<uint16_t> lists;
+    for (int r = 0; r < s->n; ++r) {
+        for (int w = 0; w < s->rw; ++w)
+            for (uint32_t b = hop[(size_t)r * s->rwp + w]; b; b &= b - 1) {
+                const int u = w * 32 + __builtin_ctz(b);
                 rhop[(size_t)u * s->rwp + (r >> 5)] |= 1u << (r & 31);
-    CR_CUDA(ctx, cudaMalloc(&s->d_rhop, rhop.size() * 4));
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_rhop, rhop.data(), rhop.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    // hop(r) as padded lists, 32 vertices side by side (the last column's tile form)
-    std::vector<uint32_t> ell_off(s->rw + 1, 0);
-    std::vector<uint16_t> ell;
-    for (int w = 0; w < s->rw; ++w) {
-        size_t longest = 0;
-        std::vector<uint16_t> of[32];
-        for (int j = 0; j < 32 && w * 32 + j < s->n; ++j) {
-            const uint32_t* h = hop.data() + (size_t)(w * 32 + j) * s->rwp;
-            for (int u = 0; u < s->n; ++u)
-                if ((h[u >> 5] >> (u & 31)) & 1u) of[j].push_back((uint16_t)u);
-            longest = std::max(longest, of[j].size());
-        }
-        for (size_t e = 0; e < longest; ++e)
-            for (int j = 0; j < 32; ++j) ell.push_back(e < of[j].size() ? of[j][e] : (uint16_t)(s->rw * 32));
-        ell_off[w + 1] = (uint32_t)(ell.size() / 32);
+                lists.push_back((uint16_t)u);
+            }
+        list_at[r + 1] = (uint32_t)lists.size();
     }
-    if (ell.empty()) ell.push_back(0);
-    CR_CUDA(ctx, cudaMalloc(&s->d_ell, ell.size() * 2));
-    CR_CUDA(ctx, cudaMalloc(&s->d_ell_off, ell_off.size() * 4));
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_ell, ell.data(), ell.size() * 2, cudaMemcpyHostToDevice, ctx->stream));
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_ell_off, ell_off.data(), ell_off.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    small.add(&s->d_rhop, rhop);
+    // the lists padded and 32 vertices side by side (the last column's tile form)
+    std::vector<uint32_t> ell_off(s->rw + 1, 0);
+    for (int w = 0; w < s->rw; ++w) {
+        uint32_t longest = 0;
+        for (int r = w * 32; r < std::min(w * 32 + 32, s->n); ++r) longest = std::max(longest, list_at[r + 1] - list_at[r]);
+        ell_off[w + 1] = ell_off[w] + longest;
+    }
+    std::vector<uint16_t> ell((size_t)ell_off[s->rw] * 32, (uint16_t)(s->rw * 32));
+    for (int r = 0; r < s->n; ++r)
+        for (uint32_t e = list_at[r]; e < list_at[r + 1]; ++e)
+            ell[(size_t)(ell_off[r >> 5] + e - list_at[r]) * 32 + (r & 31)] = lists[e];
+    small.add(&s->d_ell, ell);
+    small.add(&s->d_ell_off, ell_off);
     // the cops' out-neighbour masks (capture-seed closed form) and their in-neighbour CSR
     // (push mode), both of the cops' move graph
     const std::vector<uint32_t>& crp = s->h_crp;
@@ -469,22 +462,14 @@ static int alloc_v1(cr_solver* s) {
         if (crp[v + 1] == crp[v]) ciso[v >> 5] |= 1u << (v & 31);
     }
     if (s->cop_stay != s->robber_stay) {
-        CR_CUDA(ctx, cudaMalloc(&s->d_crp, crp.size() * 4));
-        CR_CUDA(ctx, cudaMalloc(&s->d_ccol, std::max<size_t>(ccol.size(), 1) * 2));
-        CR_CUDA(ctx, cudaMalloc(&s->d_ciso, ciso.size() * 4));
-        CR_CUDA(ctx, cudaMemcpyAsync(s->d_crp, crp.data(), crp.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-        if (!ccol.empty())
-            CR_CUDA(ctx, cudaMemcpyAsync(s->d_ccol, ccol.data(), ccol.size() * 2, cudaMemcpyHostToDevice, ctx->stream));
-        CR_CUDA(ctx, cudaMemcpyAsync(s->d_ciso, ciso.data(), ciso.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+        small.add(&s->d_crp, crp);
+        small.add(&s->d_ccol, ccol);
+        small.add(&s->d_ciso, ciso);
     }
-    CR_CUDA(ctx, cudaMalloc(&s->d_iso, iso.size() * 4));
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_iso, iso.data(), iso.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CR_CUDA(ctx, cudaMalloc(&s->d_nbr, nbr.size() * 4));
-    CR_CUDA(ctx, cudaMalloc(&s->d_rrp, rrp.size() * 4));
-    CR_CUDA(ctx, cudaMalloc(&s->d_rcol, rcol.size() * 2));
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_rrp, rrp.data(), rrp.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_rcol, rcol.data(), rcol.size() * 2, cudaMemcpyHostToDevice, ctx->stream));
+    small.add(&s->d_iso, iso);
+    small.add(&s->d_nbr, nbr);
+    small.add(&s->d_rrp, rrp);
+    small.add(&s->d_rcol, rcol);
     // uncovered-slot masks of the folded first pass (two columns, out-degrees <= 32), bit j
     // for the j-th out-neighbour of r: plane 0 [c][r] slots of r outside {c} + N(c), plane 1
     // [c][r] slots of r other than c; masks of cover_w bytes, rows padded to npad robbers
@@ -519,12 +504,10 @@ static int alloc_v1(cr_solver* s) {
         std::vector<uint8_t> bytes(m.size() * W);
         for (size_t i = 0; i < m.size(); ++i)
             for (int b = 0; b < W; ++b) bytes[i * W + b] = (uint8_t)(m[i] >> (8 * b));
-        CR_CUDA(ctx, cudaMalloc(&s->d_cover, bytes.size()));
-        CR_CUDA(ctx, cudaMemcpyAsync(s->d_cover, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, ctx->stream));
+        small.add(&s->d_cover, bytes);
         s->cover_w = W;
         s->npad = npad;
     }
-    CR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     return CR_OK;
 }
 
@@ -559,7 +542,6 @@ int cr_solver_create(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, i
     s->robber_stay = (stay & CR_ROBBER_STAY) != 0;
     s->S = slots_for(g->n);
     layout(s->n, k, p, rules, s->S, &s->C, &s->cols, &s->rw, &s->rwp);
-    s->small = s->C * (uint64_t)s->n * s->cols < (1ull << 24);
     if (s->C == 0 || s->C >= (1ull << 32)) {
         delete s;
         return fail(ctx, CR_ERR_LIMIT, "config count C(%d,%d) outside 1..2^32-1", g->n + k - 1, k);
@@ -608,44 +590,35 @@ int cr_solver_create(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, i
             return bail(e_ == cudaErrorMemoryAllocation ? CR_ERR_NOMEM : CR_ERR_CUDA);       \
         }                                                                                    \
     } while (0)
-    CR_TRY(cudaMalloc(&s->d_rp, s->h_rp.size() * 4));
-    CR_TRY(cudaMalloc(&s->d_col, std::max<size_t>(s->h_col.size(), 1) * 2));
-    CR_TRY(cudaMalloc(&s->d_binom, s->h_binom.size() * 4));
+    SmallArrays small;
+    small.add(&s->d_rp, s->h_rp);
+    small.add(&s->d_col, s->h_col);
+    small.add(&s->d_binom, s->h_binom);
+    CR_TRY(ctx->get_kit(&s->kit));
     CR_TRY(ctx->cache.get((void**)&s->d_configs, s->C * k * 2));
-    CR_TRY(cudaMalloc(&s->d_counters, 4 * sizeof(unsigned long long)));
-    CR_TRY(cudaMalloc(&s->d_err, sizeof(unsigned int)));
-    CR_TRY(cudaMallocHost(&s->h_pinned, (4 + kPinHist + 1) * sizeof(unsigned long long)));
-    CR_TRY(cudaEventCreate(&s->ev0));
-    CR_TRY(cudaEventCreate(&s->ev1));
-    CR_TRY(cudaEventCreate(&s->evc0));
-    CR_TRY(cudaEventCreate(&s->evc1));
-    CR_TRY(cudaMemcpyAsync(s->d_rp, s->h_rp.data(), s->h_rp.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    if (!s->h_col.empty())
-        CR_TRY(cudaMemcpyAsync(s->d_col, s->h_col.data(), s->h_col.size() * 2, cudaMemcpyHostToDevice, ctx->stream));
-    CR_TRY(cudaMemcpyAsync(s->d_binom, s->h_binom.data(), s->h_binom.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CR_TRY(cudaMemsetAsync(s->d_err, 0, sizeof(unsigned int), ctx->stream));
-    {
-        const int grid = (int)std::min<uint64_t>((s->C + 255) / 256, (uint64_t)ctx->num_sms * 8);
-        launch_unrank(s->d_binom, s->n, k, (uint32_t)s->C, s->d_configs, std::max(grid, 1), ctx->stream);
-        CR_TRY(cudaGetLastError());
-    }
+    CR_TRY(ctx->cache.get((void**)&s->d_ctl, sizeof(SolveCtl) + sizeof(ColMeta) * s->cols));
+    CR_TRY(cudaMemsetAsync(s->d_ctl, 0, sizeof(SolveCtl), ctx->stream));
     if (rules == CR_RULES_V1) {
         if (!pull_supported(s->S, s->rwp))
             return (fail(ctx, CR_ERR_LIMIT, "v1 rules: rows of %d vertices exceed the warp layout (n <= 512)", s->n), bail(CR_ERR_LIMIT));
-        int rc = alloc_v1(s);
+        int rc = alloc_v1(s, small);
         if (rc) return bail(rc);
+        CR_TRY(small.upload(ctx->cache, &s->d_small, ctx->stream));
         const int per_sm = max_cop_blocks_per_sm(k, s->rwp, s->S);
         s->grid_cop = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 7) / 8, (uint64_t)ctx->num_sms * per_sm));
         s->grid_small = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 255) / 256, (uint64_t)ctx->num_sms * 4));
         if (and_smem_bytes(s->S, s->rwp, s->n) > 48 * 1024 || cop_smem_bytes(s->S, s->rwp) > 48 * 1024)
             return (fail(ctx, CR_ERR_LIMIT, "shared memory layout too large"), bail(CR_ERR_LIMIT));
     } else {
-        int rc = crgpu::v2_create(&s->v2, ctx->stream, ctx->num_sms, s->n, k, p, s->d_rp, s->d_col,
+        CR_TRY(small.upload(ctx->cache, &s->d_small, ctx->stream));
+        int rc = crgpu::v2_create(&s->v2, &ctx->cache, s->kit, ctx->stream, ctx->num_sms, s->n, k, p, s->d_rp, s->d_col,
                                   s->h_rp.data(), s->h_col.data(), s->d_binom, s->d_configs,
                                   (uint32_t)s->C, &ctx->err);
         if (rc) return bail(rc);
     }
-    CR_TRY(cudaStreamSynchronize(ctx->stream));
+    const int grid = (int)std::min<uint64_t>((s->C + 255) / 256, (uint64_t)ctx->num_sms * 8);
+    launch_unrank(s->d_binom, s->n, k, (uint32_t)s->C, s->d_configs, std::max(grid, 1), ctx->stream);
+    CR_TRY(cudaGetLastError());
 #undef CR_TRY
     s->stats.slots = s->S;
     *out = s;
@@ -664,41 +637,60 @@ int cr_solver_destroy(cr_solver* s) {
 static int check_err(cr_solver* s, unsigned* bits) {
     cr_context* ctx = s->ctx;
     unsigned e = 0;
-    CR_CUDA(ctx, cudaMemcpyAsync(&e, s->d_err, sizeof(e), cudaMemcpyDeviceToHost, ctx->stream));
+    CR_CUDA(ctx, cudaMemcpyAsync(&e, &s->d_ctl->err, sizeof(e), cudaMemcpyDeviceToHost, ctx->stream));
     CR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     *bits = e;
     return CR_OK;
 }
 
-// v1 initializeCaptures on the device.
-static int v1_init(cr_solver* s, uint64_t* caps) {
+// The control block of a fresh solve: zeros and the columns' states.
+static int reset_ctl(cr_solver* s, const std::vector<ColMeta>& meta) {
+    cr_context* ctx = s->ctx;
+    std::vector<unsigned char> h(sizeof(SolveCtl) + sizeof(ColMeta) * meta.size(), 0);
+    memcpy(h.data() + sizeof(SolveCtl), meta.data(), sizeof(ColMeta) * meta.size());
+    CR_CUDA(ctx, cudaMemcpyAsync(s->d_ctl, h.data(), h.size(), cudaMemcpyHostToDevice, ctx->stream));
+    return CR_OK;
+}
+
+// Takes up the time of an initializeCaptures whose events have been recorded (they have completed,
+// or are waited for).
+static void settle_init_time(cr_solver* s) {
+    if (!s->init_timing) return;
+    s->init_timing = false;
+    float ms = 0;
+    if (cudaEventSynchronize(s->kit.ev[3]) == cudaSuccess) cudaEventElapsedTime(&ms, s->kit.ev[2], s->kit.ev[3]);
+    s->stats.init_ms = ms;
+}
+
+// Every configuration contributes its distinct cop vertices, and n * (multisets containing a given
+// vertex) = n * (C(n+k-1, k) - C(n+k-2, k)).
+static uint64_t base_capture_count(const cr_solver* s) {
+    return (uint64_t)s->n * (binom_u64(s->n + s->k - 1, s->k) - binom_u64(s->n + s->k - 2, s->k));
+}
+
+// v1 initializeCaptures on the device (enqueued).
+static int v1_init(cr_solver* s) {
     cr_context* ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     const size_t C = s->C;
-    CR_CUDA(ctx, cudaEventRecord(s->ev0, st));
+    settle_init_time(s);
+    CR_CUDA(ctx, cudaEventRecord(s->kit.ev[2], st));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_table, kUnmarked, C * s->n * s->cols, st));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_marked, 0, (size_t)s->cols * C * s->rwp * 4, st));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_fflag, 0, (size_t)s->cols * C, st));
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_counters, 0, 4 * sizeof(unsigned long long), st));
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_err, 0, sizeof(unsigned), st));
     std::vector<ColMeta> meta(s->cols);
     for (int c = 0; c < s->cols; ++c) meta[c] = ColMeta{0, kEmptyLo, -1, 0, 0, 0, 0, 0};
     // capture seeds in columns 0 and 1 (every row: the implicit list); pass 1's column-0
     // producer appends to column 0's
     meta[0] = ColMeta{0, 0, 0, 1, (int)std::min<uint64_t>(C, INT32_MAX), 0, -1, 0};
     meta[1] = ColMeta{0, 0, 0, 0, (int)std::min<uint64_t>(C, INT32_MAX), 1, -1, 0};
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_sync, 0, kSyncWords * sizeof(unsigned), st));
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_meta, meta.data(), sizeof(ColMeta) * s->cols, cudaMemcpyHostToDevice, st));
+    if (int rc = reset_ctl(s, meta)) return rc;
     V1Dev d = dev_view(s);
     launch_init(d, s->grid_small, st);
     CR_CUDA(ctx, cudaGetLastError());
-    CR_CUDA(ctx, cudaEventRecord(s->ev1, st));
-    CR_CUDA(ctx, cudaMemcpyAsync(s->h_pinned, s->d_counters, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    CR_CUDA(ctx, cudaStreamSynchronize(st));
-    *caps = s->h_pinned[0];
-    float ms = 0;
-    cudaEventElapsedTime(&ms, s->ev0, s->ev1);
-    s->stats.init_ms = ms;
+    CR_CUDA(ctx, cudaEventRecord(s->kit.ev[3], st));
+    s->init_timing = true;
+    s->unsynced = true;
     s->stats.kernel_launches = 1;
     return CR_OK;
 }
@@ -706,121 +698,138 @@ static int v1_init(cr_solver* s, uint64_t* caps) {
 // initializeCaptures and pass 1 of a p = 1 solve in one kernel (init_pass1_single /
 // init_pass1_body): every table byte, both marked planes and both flag planes are written whole
 // (column 1's frontier rows where they gained marks), so nothing is cleared first.
-static int v1_init_pass1_enqueue(cr_solver* s, bool defer_list = false) {
+static int v1_init_pass1(cr_solver* s) {
     cr_context* ctx = s->ctx;
     cudaStream_t st = ctx->stream;
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_counters, 0, 4 * sizeof(unsigned long long), st));
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_err, 0, sizeof(unsigned), st));
+    settle_init_time(s);
     // column 0's frontier after pass 1 is every row (the implicit list), already consumed by
     // the fused last column, which leaves its flags clear; column 1's list is built from its
-    // flags after the kernel, by k_list_compact or (defer_list) by the pass loop's entry
-    ColMeta meta[2] = {ColMeta{0, 0, 0, 0, (int)std::min<uint64_t>(s->C, INT32_MAX), 0, -1, 1},
-                       ColMeta{1, kEmptyLo, -1, 0, 0, 0, 0, 0, 0, defer_list ? 1 : 0}};
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_sync, 0, kSyncWords * sizeof(unsigned), st));
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_meta, meta, sizeof(meta), cudaMemcpyHostToDevice, st));
+    // flags after the kernel (k_loop_enter)
+    const std::vector<ColMeta> meta = {ColMeta{0, 0, 0, 0, (int)std::min<uint64_t>(s->C, INT32_MAX), 0, -1, 1},
+                                       ColMeta{1, kEmptyLo, -1, 0, 0, 0, 0, 0, 0, 1}};
+    if (int rc = reset_ctl(s, meta)) return rc;
     V1Dev d = dev_view(s);
-    CR_CUDA(ctx, cudaEventRecord(s->evc0, st));
+    CR_CUDA(ctx, cudaEventRecord(s->kit.ev[2], st));
     launch_init_pass1(d, ctx->num_sms, st);
     CR_CUDA(ctx, cudaGetLastError());
-    CR_CUDA(ctx, cudaEventRecord(s->evc1, st));
-    if (!defer_list) {
-        launch_list_compact(d, 1, ctx->num_sms, st);   // column 1's row list, from its flags
-        CR_CUDA(ctx, cudaGetLastError());
-    }
+    CR_CUDA(ctx, cudaEventRecord(s->kit.ev[3], st));
+    s->init_timing = true;
     s->init_pending = false;
-    s->stats.kernel_launches += defer_list ? 1 : 2;
-    return CR_OK;
-}
-
-static void v1_init_pass1_time(cr_solver* s) {
-    float ms = 0;
-    cudaEventElapsedTime(&ms, s->evc0, s->evc1);
-    s->stats.init_ms = ms;
-}
-
-static int v1_init_pass1(cr_solver* s, uint64_t* found) {
-    cr_context* ctx = s->ctx;
-    cudaStream_t st = ctx->stream;
-    if (int rc = v1_init_pass1_enqueue(s)) return rc;
-    CR_CUDA(ctx, cudaMemcpyAsync(s->h_pinned, s->d_counters, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    CR_CUDA(ctx, cudaStreamSynchronize(st));
-    v1_init_pass1_time(s);
-    *found = s->h_pinned[0];
+    s->unsynced = true;
+    s->stats.kernel_launches += 1;
     return CR_OK;
 }
 
 // The exact post-initializeCaptures state, for a caller that reads the table before pass 1.
 static int materialize_init(cr_solver* s) {
     if (!s->init_pending) return CR_OK;
-    uint64_t caps = 0;
-    int rc = v1_init(s, &caps);
-    if (rc) return rc;
+    if (int rc = v1_init(s)) return rc;
     s->init_pending = false;
     return CR_OK;
 }
 
-// Enqueue one pass: per column a prep kernel and its producer, then the pass counter copy.
-// Inside the device-side pass loop (loop set) the last column also ends the pass and runs
-// column 0's prep for the next one, so the pass starts with column 0's producer; with p = 1
-// the last column's prep rides on the cop turn's second launch and the last column itself.
-static int v1_enqueue_pass(cr_solver* s, bool profile, bool readback = true, const LoopCtl* loop = nullptr) {
+// Enqueue one pass.  Each column's prep rides on the launches of the column before it (column 0's
+// ran in k_loop_enter or in the previous pass's last column, which also records the pass's count):
+// three launches per cop turn and robber turn.  Profiling: each cop turn is timed with events.
+static int v1_enqueue_pass(cr_solver* s, const LoopCtl& loop) {
     cr_context* ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     V1Dev d = dev_view(s);
-    const bool fuse1 = loop && loop->fused_prep1;
     for (int col = 0; col < s->cols; ++col) {
         const int nx = (col + 1) % s->cols;
-        if (!(loop && col == 0) && !(fuse1 && col == 1)) launch_prep(d, col, nx, s->grid_small, st);
         if (col % 2 == 0) {
-            if (profile) CR_CUDA(ctx, cudaEventRecord(s->evc0, st));
-            launch_cop(d, col, nx, 0, s->grid_cop, st, fuse1 && col == 0);
-            if (profile) CR_CUDA(ctx, cudaEventRecord(s->evc1, st));
+            if (ctx->profiling) {
+                settle_init_time(s);
+                CR_CUDA(ctx, cudaEventRecord(s->kit.ev[2], st));
+            }
+            launch_cop(d, col, nx, 0, s->grid_cop, st, true);
+            if (ctx->profiling) CR_CUDA(ctx, cudaEventRecord(s->kit.ev[3], st));
         } else if (col < s->cols - 1) {
-            launch_cop(d, col, nx, 1, s->grid_cop, st);
+            launch_cop(d, col, nx, 1, s->grid_cop, st, true);
         } else {
             launch_and(d, col, s->p == 1, s->grid_cop, st, loop);
         }
         CR_CUDA(ctx, cudaGetLastError());
-        if (profile && col % 2 == 0) {
-            // per-launch timing of the cop turn (the dominant kernel)
-            CR_CUDA(ctx, cudaEventSynchronize(s->evc1));
+        if (ctx->profiling && col % 2 == 0) {
+            CR_CUDA(ctx, cudaEventSynchronize(s->kit.ev[3]));
             float ms = 0;
-            cudaEventElapsedTime(&ms, s->evc0, s->evc1);
+            cudaEventElapsedTime(&ms, s->kit.ev[2], s->kit.ev[3]);
             s->stats.cop_step_ms += ms;
             s->stats.cop_step_launches += 1;
         }
     }
-    if (readback)
-        CR_CUDA(ctx, cudaMemcpyAsync(s->h_pinned, s->d_counters, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     return CR_OK;
 }
 
-static int v1_pass(cr_solver* s, uint64_t* found) {
+// Waits until a pass has written its word of the ring: the word changes, or the stream runs empty
+// or fails without that.
+static int await_count(cr_solver* s, int slot, unsigned long long* value) {
+    cr_context* ctx = s->ctx;
+    volatile unsigned long long* word = s->kit.pinned + slot;
+    for (unsigned spin = 1; *word == kHistEmpty; ++spin) {
+        if (spin % 1024) continue;
+        std::this_thread::yield();
+        const cudaError_t e = cudaStreamQuery(ctx->stream);
+        if (e != cudaErrorNotReady && *word == kHistEmpty)
+            return fail(ctx, CR_ERR_CUDA, "a pass recorded nothing: %s", cudaGetErrorString(e));
+    }
+    *value = *word;
+    return CR_OK;
+}
+
+static int grow_slots_and_replay(cr_solver* s);
+
+constexpr unsigned long long kFewMarks = 1u << 15;   // the passes of the sparse ends of the solves measured
+
+// Up to `passes` passes, the fused first pass among them when it is pending, until one finds
+// nothing.  The host enqueues `ahead` passes beyond the one whose count it waits for, so that the
+// device does not idle while the count travels (about 10 us to the host and back); passes behind
+// the fixed point return at once, but cost their 3p launches.  So it goes ahead by one pass at
+// first, then by `ahead`, and no more once a pass finds little: the end is then near.  Appends the counts to pass_counts, sets finished; widens the value slots and
+// replays when a pass overflowed them (that pass is not counted).
+static int v1_advance(cr_solver* s, size_t passes, size_t ahead) {
     cr_context* ctx = s->ctx;
     cudaStream_t st = ctx->stream;
-    if (ctx->profiling || s->small) {
-        int rc = v1_enqueue_pass(s, ctx->profiling);
-        if (rc) return rc;
-    } else {
-        if (!s->pass_graph) {
-            cudaGraph_t graph;
-            CR_CUDA(ctx, cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-            int rc = v1_enqueue_pass(s, false);
-            cudaError_t e = cudaStreamEndCapture(st, &graph);
-            if (rc) return rc;
-            if (e != cudaSuccess) return fail(ctx, CR_ERR_CUDA, "pass capture: %s", cudaGetErrorString(e));
-            e = cudaGraphInstantiate(&s->pass_graph, graph, 0);
-            cudaGraphDestroy(graph);
-            if (e != cudaSuccess) return fail(ctx, CR_ERR_CUDA, "pass graph: %s", cudaGetErrorString(e));
-        }
-        CR_CUDA(ctx, cudaGraphLaunch(s->pass_graph, st));
+    CR_CUDA(ctx, cudaEventRecord(s->kit.ev[0], st));
+    const bool first = s->init_pending;
+    s->kit.pinned[0] = kHistEmpty;
+    if (first) {
+        if (int rc = v1_init_pass1(s)) return rc;
     }
-    CR_CUDA(ctx, cudaStreamSynchronize(st));
-    int per_pass = s->cols;  // prep kernels
+    const LoopCtl loop{s->kit.pinned, &s->d_ctl->hist_n, kHistRing};
+    launch_loop_enter(dev_view(s), loop, first ? 1 : 0, s->grid_small, st);
+    CR_CUDA(ctx, cudaGetLastError());
+    size_t sent = first ? 1 : 0, got = 0, lead = ahead ? 1 : 0;
+    unsigned long long f = 0;
+    while (got < passes && !s->finished) {
+        for (; sent < passes && sent < got + 1 + lead; ++sent) {
+            s->kit.pinned[sent % kHistRing] = kHistEmpty;
+            if (int rc = v1_enqueue_pass(s, loop)) return rc;
+        }
+        if (int rc = await_count(s, (int)(got % kHistRing), &f)) return rc;
+        if (f & kHistError) break;
+        ++got;
+        s->pass_counts.push_back(f);
+        s->finished = f == 0;
+        lead = f < kFewMarks ? 0 : ahead;
+    }
+    CR_CUDA(ctx, cudaEventRecord(s->kit.ev[1], st));
+    CR_CUDA(ctx, cudaStreamSynchronize(st));   // (the passes sent ahead; the ring is free again)
+    s->unsynced = false;
+    float ms = 0;
+    cudaEventElapsedTime(&ms, s->kit.ev[0], s->kit.ev[1]);
+    s->stats.main_ms += ms;
+    settle_init_time(s);
+    int per_pass = 0;
     for (int col = 0; col < s->cols; ++col)
         per_pass += col % 2 == 0 ? cop_launches_k(0, s->d_h1 != nullptr && (s->forms & CR_FORM_SEPARABLE)) : (col < s->cols - 1 ? cop_launches(1) : 1);
-    s->stats.kernel_launches += per_pass;
-    *found = s->h_pinned[0];
+    s->stats.kernel_launches += (int64_t)per_pass * (int64_t)(sent - (first ? 1 : 0)) + 1;   // and k_loop_enter
+    s->stats.passes = (int)s->pass_counts.size();
+    if (f & kHistError) {
+        if (f & kErrRank) return fail(ctx, CR_ERR_INTERNAL, "successor rank out of range");
+        if (f & kErrSlot) return grow_slots_and_replay(s);
+        return fail(ctx, CR_ERR_INTERNAL, "device error bits 0x%x", (unsigned)f);
+    }
     return CR_OK;
 }
 
@@ -832,15 +841,15 @@ int cr_solver_init(cr_solver* s, uint64_t* base_captures) {
     s->init_pending = false;
     int rc = CR_OK;
     if (s->rules == CR_RULES_V1 && s->cols == 2 && s->S >= 2 && s->cover_w > 0 && (s->forms & CR_FORM_FUSED_FIRST)) {
-        // folded into pass 1; the capture count has a closed form: every configuration
-        // contributes its distinct cop vertices, and n * (multisets containing a given vertex)
-        // = n * (C(n+k-1, k) - C(n+k-2, k))
-        caps = (uint64_t)s->n * (binom_u64(s->n + s->k - 1, s->k) - binom_u64(s->n + s->k - 2, s->k));
+        // folded into pass 1
+        caps = base_capture_count(s);
         s->init_pending = true;
+        s->init_timing = false;
         s->stats.init_ms = 0;
         s->stats.kernel_launches = 0;
     } else {
-        rc = s->rules == CR_RULES_V1 ? v1_init(s, &caps) : crgpu::v2_init(s->v2, &caps, &s->stats, &ctx->err);
+        caps = base_capture_count(s);
+        rc = s->rules == CR_RULES_V1 ? v1_init(s) : crgpu::v2_init(s->v2, &s->stats, &ctx->err);
     }
     if (rc) return rc;
     s->base_caps = caps;
@@ -859,17 +868,13 @@ static int grow_slots_and_replay(cr_solver* s) {
     // A frontier needed more value slots than allocated: widen and replay from the start.
     cr_context* ctx = s->ctx;
     if (s->S >= 8) return fail(ctx, CR_ERR_INTERNAL, "frontier value range exceeds 8 slots");
-    std::vector<uint64_t> done = s->pass_counts;
+    const std::vector<uint64_t> done = s->pass_counts;
     ctx->cache.put(s->d_front);
     s->d_front = nullptr;
     ctx->cache.put(s->d_cand);
     s->d_cand = nullptr;
     ctx->cache.put(s->d_h1);
     s->d_h1 = nullptr;
-    if (s->pass_graph) cudaGraphExecDestroy(s->pass_graph);
-    s->pass_graph = nullptr;
-    if (s->run_graph) cudaGraphExecDestroy(s->run_graph);
-    s->run_graph = nullptr;
     s->S *= 2;
     if (!pull_supported(s->S, s->rwp))
         return fail(ctx, CR_ERR_LIMIT, "row too wide for %d value slots", s->S);
@@ -880,16 +885,14 @@ static int grow_slots_and_replay(cr_solver* s) {
     CR_CUDA(ctx, alloc_h1(s));
     const int per_sm = max_cop_blocks_per_sm(s->k, s->rwp, s->S);
     s->grid_cop = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 7) / 8, (uint64_t)ctx->num_sms * per_sm));
-    uint64_t caps;
-    int rc = v1_init(s, &caps);
-    if (rc) return rc;
+    if (int rc = v1_init(s)) return rc;
     s->stats.slots = s->S;
-    for (size_t i = 0; i < done.size(); ++i) {
-        uint64_t f;
-        rc = v1_pass(s, &f);
-        if (rc) return rc;
-        if (f != done[i]) return fail(ctx, CR_ERR_INTERNAL, "replay diverged at pass %zu", i + 1);
+    s->pass_counts.clear();
+    while (s->pass_counts.size() < done.size()) {
+        if (int rc = v1_advance(s, done.size() - s->pass_counts.size(), 2)) return rc;
+        if (s->finished) break;
     }
+    if (s->pass_counts != done) return fail(ctx, CR_ERR_INTERNAL, "replay diverged within %zu passes", done.size());
     return CR_OK;
 }
 
@@ -904,24 +907,15 @@ int cr_solver_pass(cr_solver* s, uint64_t* new_wins) {
         int rc = crgpu::v2_pass(s->v2, &f, &s->stats, &ctx->err);
         if (rc) return rc;
     } else {
-        for (int attempt = 0;; ++attempt) {
-            CR_CUDA(ctx, cudaEventRecord(s->ev0, ctx->stream));
-            int rc = s->init_pending ? v1_init_pass1(s, &f) : v1_pass(s, &f);
-            if (rc) return rc;
-            CR_CUDA(ctx, cudaEventRecord(s->ev1, ctx->stream));
-            CR_CUDA(ctx, cudaEventSynchronize(s->ev1));
-            float ms = 0;
-            cudaEventElapsedTime(&ms, s->ev0, s->ev1);
-            s->stats.main_ms += ms;
-            unsigned bits = 0;
-            rc = check_err(s, &bits);
-            if (rc) return rc;
-            if (bits & kErrRank) return fail(ctx, CR_ERR_INTERNAL, "successor rank out of range");
-            if (!(bits & kErrSlot)) break;
-            if (attempt > 3) return fail(ctx, CR_ERR_INTERNAL, "value slots kept overflowing");
-            rc = grow_slots_and_replay(s);
-            if (rc) return rc;
+        // (a pass that overflows its value slots is not counted: the slots are widened, and it runs
+        // again)
+        const size_t before = s->pass_counts.size();
+        for (int attempt = 0; s->pass_counts.size() == before; ++attempt) {
+            if (attempt > 4) return fail(ctx, CR_ERR_INTERNAL, "value slots kept overflowing");
+            if (int rc = v1_advance(s, 1, 0)) return rc;
         }
+        *new_wins = s->pass_counts.back();
+        return CR_OK;
     }
     s->pass_counts.push_back(f);
     s->stats.passes = (int)s->pass_counts.size();
@@ -930,127 +924,19 @@ int cr_solver_pass(cr_solver* s, uint64_t* new_wins) {
     return CR_OK;
 }
 
-static constexpr int kHistCap = 1 << 16;   // passes one device-side loop may run
-
-// The pass loop graph: k_loop_enter; WHILE (flag) { one pass, ending in k_and_end }, the flag
-// set by k_loop_enter and then by each pass's last column.
-static int build_run_graph(cr_solver* s) {
-    cr_context* ctx = s->ctx;
-    cudaStream_t st = ctx->stream;
-    if (!s->d_hist) {
-        CR_CUDA(ctx, cudaMalloc(&s->d_hist, sizeof(unsigned long long) * kHistCap));
-        CR_CUDA(ctx, cudaMalloc(&s->d_hist_n, sizeof(int)));
-    }
-    cudaGraph_t g = nullptr;
-    CR_CUDA(ctx, cudaGraphCreate(&g, 0));
-    cudaGraphConditionalHandle loop;
-    cudaError_t e = cudaGraphConditionalHandleCreate(&loop, g, 0, cudaGraphCondAssignDefault);
-    const LoopCtl ctl{s->d_hist, s->d_hist_n, kHistCap, loop, s->cols == 2 ? 1 : 0};
-    const V1Dev d = dev_view(s);
-    // the start node sets the loop condition (and records a first pass run just before)
-    cudaGraphNode_t start = nullptr;
-    if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(st, g, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        launch_loop_enter(d, ctl, s->grid_small, st);
-        cudaGraph_t same = nullptr;
-        e = cudaStreamEndCapture(st, &same);
-    }
-    size_t nodes = 1;
-    if (e == cudaSuccess) e = cudaGraphGetNodes(g, &start, &nodes);
-    if (e == cudaSuccess && nodes != 1) e = cudaErrorInvalidValue;
-    cudaGraphNodeParams cp = {};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = loop;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    if (e == cudaSuccess) e = cudaGraphAddNode(&node, g, &start, nullptr, 1, &cp);
-    if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(st, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
-                                                            cudaStreamCaptureModeThreadLocal);
-    if (e == cudaSuccess) {
-        int rc = v1_enqueue_pass(s, false, false, &ctl);
-        cudaGraph_t body = nullptr;
-        e = cudaStreamEndCapture(st, &body);
-        if (rc) {
-            cudaGraphDestroy(g);
-            return rc;
-        }
-    }
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&s->run_graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) {
-        s->run_graph = nullptr;
-        return fail(ctx, CR_ERR_CUDA, "pass loop graph: %s", cudaGetErrorString(e));
-    }
-    return CR_OK;
-}
-
-// Passes until the fixed point in one graph launch (v1, not profiling).  Returns CR_OK with
-// the counts appended to pass_counts, or leaves the state for the caller's pass-by-pass loop
-// when the loop stopped on an error bit or a full history.
-static int v1_run_on_device(cr_solver* s) {
-    cr_context* ctx = s->ctx;
-    cudaStream_t st = ctx->stream;
-    if (!s->run_graph) {
-        int rc = build_run_graph(s);
-        if (rc) return rc;
-    }
-    // p = 1: the fused first pass is enqueued right before the loop, whose start node records
-    // its count, so the whole solve costs one host synchronisation
-    const bool first = s->init_pending;
-    CR_CUDA(ctx, cudaEventRecord(s->ev0, st));
-    if (first) {
-        if (int rc = v1_init_pass1_enqueue(s, true)) return rc;
-    }
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_hist_n, 0, sizeof(int), st));
-    if (first) CR_CUDA(ctx, cudaMemsetAsync(s->d_hist_n, 1, 1, st));   // the length 1 (low byte)
-    CR_CUDA(ctx, cudaGraphLaunch(s->run_graph, st));
-    CR_CUDA(ctx, cudaEventRecord(s->ev1, st));
-    unsigned long long* hist_pin = s->h_pinned + 4;
-    unsigned* tail = reinterpret_cast<unsigned*>(s->h_pinned + 4 + kPinHist);   // [0] length, [1] error bits
-    CR_CUDA(ctx, cudaMemcpyAsync(hist_pin, s->d_hist, sizeof(unsigned long long) * kPinHist, cudaMemcpyDeviceToHost, st));
-    CR_CUDA(ctx, cudaMemcpyAsync(&tail[0], s->d_hist_n, sizeof(int), cudaMemcpyDeviceToHost, st));
-    CR_CUDA(ctx, cudaMemcpyAsync(&tail[1], s->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    CR_CUDA(ctx, cudaStreamSynchronize(st));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, s->ev0, s->ev1);
-    s->stats.main_ms += ms;
-    if (first) v1_init_pass1_time(s);
-    const int n = (int)tail[0];
-    const unsigned bits = tail[1];
-    if (n <= 0 || n > kHistCap) return fail(ctx, CR_ERR_INTERNAL, "pass loop ran %d passes", n);
-    std::vector<unsigned long long> h(hist_pin, hist_pin + std::min(n, kPinHist));
-    if (n > kPinHist) {
-        h.resize(n);
-        CR_CUDA(ctx, cudaMemcpy(h.data() + kPinHist, s->d_hist + kPinHist, sizeof(unsigned long long) * (n - kPinHist),
-                                cudaMemcpyDeviceToHost));
-    }
-    const int loop_passes = first ? n - 1 : n;
-    // prep kernels: column 0's runs in the previous pass's last column, and with p = 1 the last
-    // column's in the cop turn and the last column
-    int per_pass = s->cols == 2 ? 0 : s->cols - 1;
-    for (int col = 0; col < s->cols; ++col)
-        per_pass += col % 2 == 0 ? cop_launches_k(0, s->d_h1 != nullptr && (s->forms & CR_FORM_SEPARABLE)) : (col < s->cols - 1 ? cop_launches(1) : 1);
-    s->stats.kernel_launches += (int64_t)per_pass * loop_passes + 1;   // and the loop's entry
-    if (bits & kErrRank) return fail(ctx, CR_ERR_INTERNAL, "successor rank out of range");
-    if (bits & kErrSlot) {
-        // the last pass overflowed its value slots: keep the passes before it, widen the slots
-        // and replay them; the caller continues pass by pass
-        for (int i = 0; i + 1 < n; ++i) s->pass_counts.push_back(h[i]);
-        return grow_slots_and_replay(s);
-    }
-    for (int i = 0; i < n; ++i) s->pass_counts.push_back(h[i]);
-    s->stats.passes = (int)s->pass_counts.size();
-    if (h[n - 1] == 0) s->finished = true;
-    return CR_OK;
-}
-
 int cr_solver_run(cr_solver* s, uint64_t* pass_counts, int32_t cap, int32_t* passes) {
     if (!s) return CR_ERR_INVALID;
-    if (s->initialized && !s->finished && s->rules == CR_RULES_V1 && !s->ctx->profiling && !s->small) {
+    if (s->initialized && s->rules == CR_RULES_V1) {
+        // two passes ahead with p = 1, whose passes are three launches; one with p > 1
         CR_CUDA(s->ctx, cudaSetDevice(s->ctx->device));
-        int rc = v1_run_on_device(s);   // with the fused first pass when it is still pending
-        if (rc) return rc;
+        const size_t ahead = s->ctx->profiling ? 0 : (s->p == 1 ? 2 : 1);
+        size_t stuck = 0;
+        while (!s->finished && s->pass_counts.size() < (1 << 16)) {
+            const size_t before = s->pass_counts.size();
+            if (int rc = v1_advance(s, (1 << 16) - before, ahead)) return rc;
+            stuck = s->pass_counts.size() == before ? stuck + 1 : 0;
+            if (stuck > 4) return fail(s->ctx, CR_ERR_INTERNAL, "value slots kept overflowing");
+        }
     }
     for (int i = 0; i < 1 << 16 && !s->finished; ++i) {
         uint64_t f;
@@ -1071,18 +957,20 @@ int cr_solver_verdict(cr_solver* s, cr_verdict* out) {
     CR_CUDA(ctx, cudaSetDevice(ctx->device));
     if (int rc = materialize_init(s)) return rc;
     cudaStream_t st = ctx->stream;
-    const unsigned long long init = ~0ull;
-    CR_CUDA(ctx, cudaMemcpyAsync(s->d_counters + 1, &init, sizeof(init), cudaMemcpyHostToDevice, st));
+    unsigned long long* const d_key = s->d_ctl->counters + 1;
+    unsigned long long* const h_key = s->kit.pinned + kHistRing;
+    CR_CUDA(ctx, cudaMemsetAsync(d_key, 0xFF, sizeof(*d_key), st));
     if (s->rules == CR_RULES_V1) {
         V1Dev d = dev_view(s);
-        launch_verdict(d, s->cols, s->d_counters + 1, s->grid_cop, st);
+        launch_verdict(d, s->cols, d_key, s->grid_cop, st);
     } else {
-        crgpu::v2_verdict(s->v2, s->d_counters + 1);
+        crgpu::v2_verdict(s->v2, d_key);
     }
     CR_CUDA(ctx, cudaGetLastError());
-    CR_CUDA(ctx, cudaMemcpyAsync(s->h_pinned + 1, s->d_counters + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    CR_CUDA(ctx, cudaMemcpyAsync(h_key, d_key, sizeof(*h_key), cudaMemcpyDeviceToHost, st));
     CR_CUDA(ctx, cudaStreamSynchronize(st));
-    const unsigned long long key = s->h_pinned[1];
+    s->unsynced = false;
+    const unsigned long long key = *h_key;
     memset(out, 0, sizeof(*out));
     if (key == ~0ull || (int)(key >> 32) >= kMaxRound) {
         out->win = 0;
@@ -1093,10 +981,18 @@ int cr_solver_verdict(cr_solver* s, cr_verdict* out) {
     out->win = 1;
     out->best_config = (int64_t)(key & 0xFFFFFFFFull);
     out->capture_plies = (int32_t)(key >> 32);
-    uint16_t pos[CR_MAX_K];
-    CR_CUDA(ctx, cudaMemcpyAsync(pos, s->d_configs + (size_t)out->best_config * s->k, s->k * 2, cudaMemcpyDeviceToHost, st));
-    CR_CUDA(ctx, cudaStreamSynchronize(st));
-    for (int i = 0; i < s->k; ++i) out->positions[i] = pos[i];
+    // the configuration from its rank (as k_unrank): per position the largest vertex whose block of
+    // configurations starts at or before it
+    uint32_t rem = (uint32_t)out->best_config;
+    int prev = 0;
+    for (int i = 0; i < s->k; ++i) {
+        const uint32_t* B = s->h_binom.data() + (size_t)i * (s->n + 1);
+        int x = prev;
+        while (x + 1 < s->n && B[x + 1] >= B[prev] - rem) ++x;
+        rem -= B[prev] - B[x];
+        out->positions[i] = (uint16_t)x;
+        prev = x;
+    }
     return CR_OK;
 }
 
@@ -1114,6 +1010,7 @@ int cr_solver_sizes(cr_solver* s, cr_table_sizes* out) {
 
 int cr_solver_stats(cr_solver* s, cr_solve_stats* out) {
     if (!s || !out) return CR_ERR_INVALID;
+    settle_init_time(s);
     *out = s->stats;
     uint64_t res = s->base_caps * (s->rules == CR_RULES_V1 ? 2 : 1);
     for (uint64_t c : s->pass_counts) res += c;
@@ -1135,11 +1032,6 @@ int cr_solver_set_forms(cr_solver* s, uint32_t mask) {
         return fail(s->ctx, CR_ERR_INVALID, "forms: v2 solves have one form");
     if (mask == s->forms) return CR_OK;
     s->forms = mask;
-    // the captured pass graphs hold the old device view
-    if (s->pass_graph) cudaGraphExecDestroy(s->pass_graph);
-    s->pass_graph = nullptr;
-    if (s->run_graph) cudaGraphExecDestroy(s->run_graph);
-    s->run_graph = nullptr;
     return CR_OK;
 }
 
@@ -1159,12 +1051,14 @@ int cr_solver_digest(cr_solver* s, uint64_t* digest) {
     CR_CUDA(ctx, cudaSetDevice(ctx->device));
     if (int rc = materialize_init(s)) return rc;
     cudaStream_t st = ctx->stream;
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_counters + 2, 0, sizeof(unsigned long long), st));
-    launch_digest(table_ptr(s), s->C * (size_t)s->n * s->cols, s->d_counters + 2, ctx->num_sms * 4, st);
+    unsigned long long* const d_sum = s->d_ctl->counters + 2;
+    unsigned long long* const h_sum = s->kit.pinned + kHistRing + 1;
+    CR_CUDA(ctx, cudaMemsetAsync(d_sum, 0, sizeof(*d_sum), st));
+    launch_digest(table_ptr(s), s->C * (size_t)s->n * s->cols, d_sum, ctx->num_sms * 4, st);
     CR_CUDA(ctx, cudaGetLastError());
-    CR_CUDA(ctx, cudaMemcpyAsync(s->h_pinned + 2, s->d_counters + 2, 8, cudaMemcpyDeviceToHost, st));
+    CR_CUDA(ctx, cudaMemcpyAsync(h_sum, d_sum, sizeof(*h_sum), cudaMemcpyDeviceToHost, st));
     CR_CUDA(ctx, cudaStreamSynchronize(st));
-    *digest = s->h_pinned[2];
+    *digest = *h_sum;
     return CR_OK;
 }
 
@@ -1172,6 +1066,10 @@ int cr_solver_device_states(cr_solver* s, void** dev_ptr, size_t* bytes) {
     if (!s || !dev_ptr || !bytes) return CR_ERR_INVALID;
     CR_CUDA(s->ctx, cudaSetDevice(s->ctx->device));
     if (int rc = materialize_init(s)) return rc;
+    if (s->unsynced) {   // the caller may read the table from another stream
+        CR_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
+        s->unsynced = false;
+    }
     *dev_ptr = (void*)table_ptr(s);
     *bytes = s->C * (size_t)s->n * s->cols;
     return CR_OK;
@@ -1211,24 +1109,24 @@ int cr_solver_build_transitions(cr_solver* s, uint64_t* total) {
         const int cap = trans_cap(s->k, s->cop_maxdeg);
         if (cap > 8192) return fail(ctx, CR_ERR_LIMIT, "successor fan-out %d too large for the CSR builder", cap);
         unsigned long long* counts = nullptr;
-        CR_CUDA(ctx, cudaMalloc(&counts, s->C * 8));
-        CR_CUDA(ctx, cudaMalloc(&s->d_heads, (s->C + 1) * 8));
-        CR_CUDA(ctx, cudaMemsetAsync(s->d_err, 0, sizeof(unsigned), st));
+        CR_CUDA(ctx, ctx->cache.get((void**)&counts, s->C * 8));
+        CR_CUDA(ctx, ctx->cache.get((void**)&s->d_heads, (s->C + 1) * 8));
+        CR_CUDA(ctx, cudaMemsetAsync(&s->d_ctl->err, 0, sizeof(unsigned), st));
         const int grid = ctx->num_sms * 8;
         const uint32_t* trp = s->d_crp ? s->d_crp : s->d_rp;
         const uint16_t* tcol = s->d_ccol ? s->d_ccol : s->d_col;
         launch_trans(s->k, s->d_configs, (uint32_t)s->C, s->n, trp, tcol, s->d_binom, cap, counts,
-                     nullptr, nullptr, s->d_err, grid, st);
+                     nullptr, nullptr, &s->d_ctl->err, grid, st);
         launch_scan(counts, s->d_heads, (uint32_t)s->C, st);
         CR_CUDA(ctx, cudaGetLastError());
         unsigned long long tot = 0;
         CR_CUDA(ctx, cudaMemcpyAsync(&tot, s->d_heads + s->C, 8, cudaMemcpyDeviceToHost, st));
         CR_CUDA(ctx, cudaStreamSynchronize(st));
-        cudaFree(counts);
+        ctx->cache.put(counts);
         s->n_trans = tot;
-        CR_CUDA(ctx, cudaMalloc(&s->d_trans, std::max<uint64_t>(tot, 1) * 8));
+        CR_CUDA(ctx, ctx->cache.get((void**)&s->d_trans, std::max<uint64_t>(tot, 1) * 8));
         launch_trans(s->k, s->d_configs, (uint32_t)s->C, s->n, trp, tcol, s->d_binom, cap, nullptr,
-                     s->d_heads, s->d_trans, s->d_err, grid, st);
+                     s->d_heads, s->d_trans, &s->d_ctl->err, grid, st);
         CR_CUDA(ctx, cudaGetLastError());
         unsigned bits = 0;
         int rc = check_err(s, &bits);
@@ -1363,12 +1261,12 @@ int cr_solver_load_table_file(cr_solver* s, const char* path) {
     CR_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     const uint64_t ntrans = (h[11] - h[10]) / 8;
-    if (!s->d_heads) CR_CUDA(ctx, cudaMalloc(&s->d_heads, heads));
+    if (!s->d_heads) CR_CUDA(ctx, ctx->cache.get((void**)&s->d_heads, heads));
     if (s->d_trans && ntrans > s->n_trans) {
-        cudaFree(s->d_trans);
+        ctx->cache.put(s->d_trans);
         s->d_trans = nullptr;
     }
-    if (!s->d_trans) CR_CUDA(ctx, cudaMalloc(&s->d_trans, std::max<uint64_t>(ntrans, 1) * 8));
+    if (!s->d_trans) CR_CUDA(ctx, ctx->cache.get((void**)&s->d_trans, std::max<uint64_t>(ntrans, 1) * 8));
     s->n_trans = ntrans;
     CR_CUDA(ctx, cudaMemcpyAsync(s->d_heads, blob.data() + h[9], heads, cudaMemcpyHostToDevice, st));
     if (ntrans) CR_CUDA(ctx, cudaMemcpyAsync(s->d_trans, blob.data() + h[10], ntrans * 8, cudaMemcpyHostToDevice, st));

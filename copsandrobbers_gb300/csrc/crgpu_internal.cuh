@@ -126,21 +126,21 @@ struct V1Dev {
     // turn handed out
     unsigned* sync;
     ColMeta* meta;            // [cols]
+    unsigned* done = nullptr; // set by the pass that found nothing: the passes behind it return at once
     unsigned long long* pass_new;
     unsigned int* err;
 };
 
-// Bookkeeping of a device-side pass loop: the history of pass counts, its length and capacity,
-// and the WHILE node's condition.
+// Bookkeeping of the passes: a ring of their counts in pinned host memory (its size a power of
+// two), which the host sets to kHistEmpty before it enqueues the pass, and the number recorded.  A
+// pass that ends with error bits set writes kHistError | bits instead and is not counted.
 struct LoopCtl {
-    unsigned long long* hist;
+    unsigned long long* hist;   // null = the caller reads each pass's count itself and runs the preps
     int* idx;
-    int cap;
-    cudaGraphConditionalHandle loop;
-    // p = 1: the last column's prep is split between the cop turn's second launch (column 1's
-    // flags and state) and the last column itself (the push form's candidate rows)
-    int fused_prep1;
+    int ring;
 };
+constexpr unsigned long long kHistEmpty = ~0ull;
+constexpr unsigned long long kHistError = 1ull << 62;
 
 __host__ __device__ inline int round_words(int rw) { return rw <= 2 ? rw : (rw + 3) & ~3; }
 

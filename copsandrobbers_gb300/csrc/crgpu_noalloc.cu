@@ -35,7 +35,7 @@
 
 namespace crgpu {
 void launch_cop(const V1Dev& d, int col, int nx, int direct, int grid, cudaStream_t st, bool end = false);
-void launch_and(const V1Dev& d, int col, bool p1, int grid, cudaStream_t st, const LoopCtl* loop = nullptr);
+void launch_and(const V1Dev& d, int col, bool p1, int grid, cudaStream_t st, const LoopCtl& loop);
 void launch_prep(const V1Dev& d, int col, int nx, int grid, cudaStream_t st);
 void launch_init(const V1Dev& d, int grid, cudaStream_t st);
 void launch_unrank(const uint32_t* B, int n, int k, uint32_t C, uint16_t* out, int grid, cudaStream_t st);
@@ -344,7 +344,7 @@ extern "C" int cr_solve_v1_noalloc(const cr_graph* g, int32_t k, int32_t p, void
                 launch_prep(d, col, nx, gsmall > 0 ? gsmall : 1, st);
                 if (col % 2 == 0) launch_cop(d, col, nx, 0, gcop > 0 ? gcop : 1, st);
                 else if (col < cols - 1) launch_cop(d, col, nx, 1, gcop > 0 ? gcop : 1, st);
-                else launch_and(d, col, p == 1, gcop > 0 ? gcop : 1, st);
+                else launch_and(d, col, p == 1, gcop > 0 ? gcop : 1, st, LoopCtl{});   // no history
             }
             NA_CUDA(cudaGetLastError());
             unsigned long long found = 0;

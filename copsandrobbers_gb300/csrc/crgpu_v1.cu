@@ -49,6 +49,15 @@ using namespace grid;
 
 __device__ void list_compact_body(const V1Dev& d, int col);
 
+// The kernels of a pass are short and each waits for the one before it, so they are launched with
+// programmatic stream serialisation: a kernel's blocks are placed while its predecessor drains, and
+// wait here before they touch memory.  False = nothing to do (behind the fixed point).
+__device__ __forceinline__ bool pass_kernel_begin(const V1Dev& d) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    return !d.done || *d.done == 0u;
+}
+
 __global__ void k_prep(V1Dev d, int col, int nx) { prep_body(d, col, nx, blockIdx.x, gridDim.x); }
 __global__ void k_init(V1Dev d, int K) { init_body(d, K, blockIdx.x, gridDim.x); }
 // The first pass in two instances: rows of one 256-robber block split into whole lane pieces
@@ -66,6 +75,7 @@ __global__ void __launch_bounds__(256, SINGLE ? 3 : 4) k_init_pass1(V1Dev d) {
 
 template <int K, int NWP, int G>
 __global__ void __launch_bounds__(256) k_cop_pull(V1Dev d, int col, int nx) {
+    if (!pass_kernel_begin(d)) return;
     cop_pull_body<K, NWP, G>(d, col, nx, blockIdx.x, gridDim.x);
 }
 // The other cop-turn forms share two launches, each body returning at once unless its form
@@ -76,70 +86,82 @@ __global__ void __launch_bounds__(256) k_cop_pull(V1Dev d, int col, int nx) {
 // registers, the bodies here at most 64 (80 with 32-word rows), being latency-bound.
 template <int K, int NWP, int G>
 __global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_a(V1Dev d, int col, int nx) {
+    if (!pass_kernel_begin(d)) return;
     cop_seed_body<K, G>(d, col, nx, blockIdx.x, gridDim.x);
     cop_push_body<K>(d, col, nx, blockIdx.x, gridDim.x);
     if constexpr (K >= 2) head_rows_body<K, NWP / 2>(d, nx, blockIdx.x, gridDim.x);
 }
 template <int K, int NWP, int G>
 __global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_b(V1Dev d, int col, int nx) {
+    if (!pass_kernel_begin(d)) return;
     if constexpr (K >= 2) sep_pull_body<K, NWP / 2>(d, col, nx, blockIdx.x, gridDim.x);
     cop_apply_body<G>(d, col, nx, blockIdx.x, gridDim.x);
 }
-// k_cop_b inside the device-side pass loop of a p = 1 solve, followed by the last column's prep
-// (column nx = 1): the flags a dense turn left in column 1 (no body of this launch reads them),
-// and in the last block the column's state reset.  The candidate rows wait for the last column.
+// k_cop_b followed by the prep of the column it consumed (nx): the flags a dense turn left there
+// (no body of this launch reads them), and in the last block the column's state reset.  The
+// candidate rows wait for that column's producer.
 template <int K, int NWP, int G>
 __global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_b_end(V1Dev d, int col, int nx) {
+    if (!pass_kernel_begin(d)) return;
     if constexpr (K >= 2) sep_pull_body<K, NWP / 2>(d, col, nx, blockIdx.x, gridDim.x);
     cop_apply_body<G>(d, col, nx, blockIdx.x, gridDim.x);
     prep_clear_flags(d, nx, blockIdx.x, gridDim.x);
     __syncthreads();
-    if (threadIdx.x == 0 && grid_last_block(d, gridDim.x)) prep_reset(d, nx, col);
+    if (threadIdx.x == 0 && grid_last_block(d, gridDim.x)) prep_reset(d, nx, (nx + 1) % d.cols);
 }
+// The deferred robber turn; with `end` also the rest of its own prep (the candidate rows) and, in
+// the last block, the prep of column nx, whose frontier it consumed (every listed flag cleared).
 template <int G>
-__global__ void __launch_bounds__(256) k_direct(V1Dev d, int col, int nx) {
+__global__ void __launch_bounds__(256) k_direct(V1Dev d, int col, int nx, bool end) {
+    if (!pass_kernel_begin(d)) return;
+    if (end) prep_clear_cand(d, blockIdx.x, gridDim.x);
     direct_body<G>(d, col, nx, blockIdx.x, gridDim.x);
+    if (!end) return;
+    __syncthreads();
+    if (threadIdx.x == 0 && grid_last_block(d, gridDim.x)) prep_reset(d, nx, (nx + 1) % d.cols);
 }
-// at most 64 registers: the grid runs 4 blocks of 256 per SM (more registers cost occupancy
-// that this latency-bound body needs more)
-template <bool P1, int G>
-__global__ void __launch_bounds__(256, 4) k_and(V1Dev d, int col) {
-    last_column_body<P1, G>(d, col, blockIdx.x, gridDim.x);
-}
-// The last column inside the device-side pass loop, with the loop's bookkeeping in its last
-// block: the pass's count joins the history, the loop goes on while the pass found something
-// (no error bit, history not full), and column 0's prep for the next pass runs (this column
-// cleared every flag of column 0's list, so that prep is a reset of the column's state).
+// The last column, with the end of the pass in its last block: the pass's count goes to the host's
+// ring, and column 0's prep for the next pass runs (this column cleared every flag of column 0's
+// list, so that prep is a reset of the column's state).
+// At most 64 registers: the grid runs 4 blocks of 256 per SM (more registers cost occupancy
+// that the latency-bound row forms need more).
 template <bool P1, int G>
 __global__ void __launch_bounds__(256, 4) k_and_end(V1Dev d, int col, LoopCtl c) {
-    if (c.fused_prep1) prep_clear_cand(d, blockIdx.x, gridDim.x);   // this column's prep, the rest
+    if (!pass_kernel_begin(d)) return;
+    if (c.hist) prep_clear_cand(d, blockIdx.x, gridDim.x);   // this column's prep, the rest
     last_column_body<P1, G>(d, col, blockIdx.x, gridDim.x);
+    if (!c.hist) return;
     __syncthreads();
     if (threadIdx.x == 0 && grid_last_block(d, gridDim.x)) {
         const int i = *c.idx;
-        const unsigned long long f = *d.pass_new;
-        c.hist[i] = f;
-        *c.idx = i + 1;
-        cudaGraphSetConditional(c.loop, (f != 0ull && *d.err == 0u && i + 1 < c.cap) ? 1u : 0u);
+        const unsigned err = *d.err;
+        volatile unsigned long long* word = c.hist + (i & (c.ring - 1));
+        if (err) {
+            *word = kHistError | err;
+        } else {
+            const unsigned long long found = *d.pass_new;
+            *word = found;
+            *c.idx = i + 1;
+            if (!found) *d.done = 1u;
+        }
         prep_reset(d, 0, 1);
     }
 }
 
-// Entry of the device-side pass loop: column 0's prep for the first pass of the loop; its last
-// block records a first pass run just before the loop (*idx = 1, set by the host) as the
-// history's first entry and starts the loop if the last pass found something and no error bit
-// is set.
-__global__ void __launch_bounds__(256) k_loop_enter(V1Dev d, LoopCtl c) {
-    // column 1's row list after a fused first pass (every block reads the marker before the
-    // last block clears it)
+// Before the first of the passes of a call: column 1's row list after a fused first pass (every block
+// reads the marker before the last block clears it), column 0's prep (again, harmlessly, when an
+// earlier call's last pass ran it), and in the last block the history, which a first pass run
+// just before opens with its count.
+__global__ void __launch_bounds__(256) k_loop_enter(V1Dev d, LoopCtl c, int first) {
     if (d.meta[1].compact) list_compact_body(d, 1);
     prep_clear(d, 0, blockIdx.x, gridDim.x);
     __syncthreads();
     if (threadIdx.x == 0 && grid_last_block(d, gridDim.x)) {
         d.meta[1].compact = 0;
-        const unsigned long long f = *d.pass_new;
-        if (*c.idx == 1) c.hist[0] = f;
-        cudaGraphSetConditional(c.loop, (f != 0ull && *d.err == 0u) ? 1u : 0u);
+        const unsigned err = *d.err;
+        if (first) *(volatile unsigned long long*)c.hist = err ? kHistError | err : *d.pass_new;
+        *c.idx = first;
+        *d.done = first && !*d.pass_new ? 1u : 0u;
         prep_reset(d, 0, 1);
     }
 }
@@ -178,16 +200,30 @@ static int pull_words(int S, int rwp) {
 
 bool pull_supported(int S, int rwp) { return pull_words(S, rwp) <= 32 && group_lanes(rwp) <= 32; }
 
+template <typename... P, typename... A>
+static void launch_pass_kernel(void (*kernel)(P...), int grid, size_t sm, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = sm;
+    cfg.stream = st;
+    cudaLaunchAttribute serial = {};
+    serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serial.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &serial;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 template <int K, int NWP, int G>
 static void launch_cop_ng(const V1Dev& d, int col, int nx, int grid, cudaStream_t st, bool end) {
     const size_t sm = cop_smem_bytes(d.S, d.g.rwp);
     const size_t smr = sm + (size_t)rank_table_words(K, d.g.n) * 4;
     const size_t sma = d.h1 ? std::max(smr, (size_t)head_smem_words(256, K, d.g.n, d.g.rwp) * 4) : smr;
     if (sma > 40 * 1024) raise_smem_limit((const void*)k_cop_a<K, NWP, G>, sma);   // (plus the static part)
-    k_cop_a<K, NWP, G><<<grid, 256, sma, st>>>(d, col, nx);
-    if (!d.h1) k_cop_pull<K, NWP, G><<<grid, 256, smr, st>>>(d, col, nx);
-    if (end) k_cop_b_end<K, NWP, G><<<grid, 256, sm, st>>>(d, col, nx);
-    else k_cop_b<K, NWP, G><<<grid, 256, sm, st>>>(d, col, nx);
+    launch_pass_kernel(k_cop_a<K, NWP, G>, grid, sma, st, d, col, nx);
+    if (!d.h1) launch_pass_kernel(k_cop_pull<K, NWP, G>, grid, smr, st, d, col, nx);
+    launch_pass_kernel(end ? k_cop_b_end<K, NWP, G> : k_cop_b<K, NWP, G>, grid, sm, st, d, col, nx);
 }
 
 // Accumulator words and lanes per configuration, as the pull and the separable turn use them.
@@ -211,8 +247,8 @@ static void launch_cop_k(const V1Dev& d, int col, int nx, int grid, cudaStream_t
 }
 
 template <int G>
-static void launch_direct_g(const V1Dev& d, int col, int nx, int grid, cudaStream_t st) {
-    k_direct<G><<<grid, 256, cop_smem_bytes(d.S, d.g.rwp), st>>>(d, col, nx);
+static void launch_direct_g(const V1Dev& d, int col, int nx, int grid, cudaStream_t st, bool end) {
+    launch_pass_kernel(k_direct<G>, grid, cop_smem_bytes(d.S, d.g.rwp), st, d, col, nx, end);
 }
 
 // Cop turn into column col (or, direct = 1, a deferred robber turn): every form that may apply
@@ -221,10 +257,10 @@ static void launch_direct_g(const V1Dev& d, int col, int nx, int grid, cudaStrea
 void launch_cop(const V1Dev& d, int col, int nx, int direct, int grid, cudaStream_t st, bool end) {
     if (direct) {
         switch (group_lanes(d.g.rwp)) {
-            case 4: launch_direct_g<4>(d, col, nx, grid, st); break;
-            case 8: launch_direct_g<8>(d, col, nx, grid, st); break;
-            case 16: launch_direct_g<16>(d, col, nx, grid, st); break;
-            default: launch_direct_g<32>(d, col, nx, grid, st); break;
+            case 4: launch_direct_g<4>(d, col, nx, grid, st, end); break;
+            case 8: launch_direct_g<8>(d, col, nx, grid, st, end); break;
+            case 16: launch_direct_g<16>(d, col, nx, grid, st, end); break;
+            default: launch_direct_g<32>(d, col, nx, grid, st, end); break;
         }
         return;
     }
@@ -246,15 +282,13 @@ size_t and_stage_words(int n, int rwp, int nnz) {
 }
 
 template <bool P1, int G>
-static void launch_and_g(const V1Dev& d, int col, int grid, size_t sm, cudaStream_t st, const LoopCtl* loop) {
-    const void* kern = loop ? (const void*)k_and_end<P1, G> : (const void*)k_and<P1, G>;
-    if (sm > 40 * 1024) raise_smem_limit(kern, sm);   // (the kernel has static shared memory too)
-    if (loop) k_and_end<P1, G><<<grid, 256, sm, st>>>(d, col, *loop);
-    else k_and<P1, G><<<grid, 256, sm, st>>>(d, col);
+static void launch_and_g(const V1Dev& d, int col, int grid, size_t sm, cudaStream_t st, const LoopCtl& loop) {
+    if (sm > 40 * 1024) raise_smem_limit((const void*)k_and_end<P1, G>, sm);   // (plus the static part)
+    launch_pass_kernel(k_and_end<P1, G>, grid, sm, st, d, col, loop);
 }
 
 template <bool P1>
-static void launch_and_p(const V1Dev& d0, int col, int grid, cudaStream_t st, const LoopCtl* loop) {
+static void launch_and_p(const V1Dev& d0, int col, int grid, cudaStream_t st, const LoopCtl& loop) {
     V1Dev d = d0;
     size_t sm = and_smem_bytes(d.S, d.g.rwp, d.g.n);
     d.and_stage_words = 0;
@@ -274,13 +308,13 @@ static void launch_and_p(const V1Dev& d0, int col, int grid, cudaStream_t st, co
     }
 }
 
-void launch_and(const V1Dev& d, int col, bool p1, int grid, cudaStream_t st, const LoopCtl* loop) {
+void launch_and(const V1Dev& d, int col, bool p1, int grid, cudaStream_t st, const LoopCtl& loop) {
     if (p1) launch_and_p<true>(d, col, grid, st, loop);
     else launch_and_p<false>(d, col, grid, st, loop);
 }
 
-void launch_loop_enter(const V1Dev& d, const LoopCtl& c, int grid, cudaStream_t st) {
-    k_loop_enter<<<grid, 256, 0, st>>>(d, c);
+void launch_loop_enter(const V1Dev& d, const LoopCtl& c, int first, int grid, cudaStream_t st) {
+    k_loop_enter<<<grid, 256, 0, st>>>(d, c, first);
 }
 
 void launch_prep(const V1Dev& d, int col, int nx, int grid, cudaStream_t st) {
@@ -362,14 +396,6 @@ __device__ void list_compact_body(const V1Dev& d, int col) {
         __syncthreads();
     }
 }
-__global__ void __launch_bounds__(256) k_list_compact(V1Dev d, int col) { list_compact_body(d, col); }
-
-void launch_list_compact(const V1Dev& d, int col, int num_sms, cudaStream_t st) {
-    const uint64_t segs = ((uint64_t)d.C + 256 * 16 - 1) / (256 * 16);
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(segs, (uint64_t)num_sms * 4));
-    k_list_compact<<<grid, 256, 0, st>>>(d, col);
-}
-
 void launch_verdict(const V1Dev& d, int cols, unsigned long long* best, int grid, cudaStream_t st) {
     k_verdict<<<grid, 256, 0, st>>>(d.table, d.marked, d.C, d.g.n, d.g.rw, d.g.rwp, cols, best);
 }

@@ -64,6 +64,7 @@ constexpr int kV2MaxP = 8;     // visibility periods handled by the device searc
 constexpr int kV2None = 255;   // "no winning trajectory"
 
 struct V2Solver {
+    cr_block_cache* cache = nullptr;
     cudaStream_t st = nullptr;
     int num_sms = 1;
     int n = 0, k = 0, p = 0, rw = 0, rwp = 0, W = 0;
@@ -96,7 +97,7 @@ struct V2Solver {
     uint64_t chunk_nodes = 0;   // depth-1 nodes per table fill
     cr_v2_hash_stats hstats{};
     bool first = true;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
+    cudaEvent_t e0 = nullptr, e1 = nullptr;   // (the solver's kit's)
 };
 
 struct V2Dev {
@@ -1016,7 +1017,7 @@ int v2_set_hash_capacity(V2Solver* s, uint64_t slots, std::string* err) {
     V2_CUDA(cudaStreamSynchronize(s->st));
     void* old[] = {s->hkey, s->hmask};
     for (void* q : old)
-        if (q) cudaFree(q);
+        s->cache->put(q);
     s->hkey = nullptr;
     s->hmask = nullptr;
     s->hcap = 0;
@@ -1025,12 +1026,12 @@ int v2_set_hash_capacity(V2Solver* s, uint64_t slots, std::string* err) {
     if (!cap) return CR_OK;
     // a solver whose table could not be allocated keeps working without one (every depth-2
     // node evaluated where it is reached)
-    cudaError_t e = cudaMalloc(&s->hkey, cap * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMalloc(&s->hmask, cap * s->rwp * sizeof(uint32_t));
+    cudaError_t e = s->cache->get((void**)&s->hkey, cap * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = s->cache->get((void**)&s->hmask, cap * s->rwp * sizeof(uint32_t));
     if (e != cudaSuccess) {
         void* got[] = {s->hkey, s->hmask};
         for (void* q : got)
-            if (q) cudaFree(q);
+            s->cache->put(q);
         s->hkey = nullptr;
         s->hmask = nullptr;
         if (err) *err = std::string("v2 cloud table: ") + cudaGetErrorString(e);
@@ -1042,7 +1043,7 @@ int v2_set_hash_capacity(V2Solver* s, uint64_t slots, std::string* err) {
     return CR_OK;
 }
 
-int v2_create(V2Solver** out, cudaStream_t st, int num_sms, int n, int k, int p,
+int v2_create(V2Solver** out, cr_block_cache* cache, const cr_solver_kit& kit, cudaStream_t st, int num_sms, int n, int k, int p,
               const uint32_t* d_rp, const uint16_t* d_col, const uint32_t* h_rp,
               const uint16_t* h_col, const uint32_t* d_binom, const uint16_t* d_configs,
               uint32_t C, std::string* err) {
@@ -1056,29 +1057,30 @@ int v2_create(V2Solver** out, cudaStream_t st, int num_sms, int n, int k, int p,
     }
     V2Solver* s = new V2Solver();
     *out = s;
+    s->cache = cache;
+    s->h_pinned = kit.pinned;
+    s->e0 = kit.ev[0];
+    s->e1 = kit.ev[1];
     s->st = st; s->num_sms = num_sms; s->n = n; s->k = k; s->p = p; s->C = C;
     s->rw = (n + 31) / 32;
     s->rwp = round_words(s->rw);
     s->W = v2_w(s->rwp);
     s->rp = d_rp; s->col = d_col; s->binom = d_binom; s->configs = d_configs;
-    V2_CUDA(cudaMalloc(&s->table, (size_t)C * n));
-    V2_CUDA(cudaMalloc(&s->marked, (size_t)C * s->rwp * 4));
-    V2_CUDA(cudaMalloc(&s->nbr, (size_t)n * s->rwp * 4));
-    V2_CUDA(cudaMalloc(&s->val1, (size_t)C * n));
-    V2_CUDA(cudaMalloc(&s->newval, (size_t)C * n));
-    V2_CUDA(cudaMalloc(&s->plain, (size_t)C * n));
-    V2_CUDA(cudaMalloc(&s->unsafe, (size_t)C * s->rwp * 4));
-    V2_CUDA(cudaMalloc(&s->changed, C));
-    V2_CUDA(cudaMalloc(&s->lev, (size_t)C * p));
-    V2_CUDA(cudaMalloc(&s->fin1, C));
-    V2_CUDA(cudaMalloc(&s->fin2, C));
-    V2_CUDA(cudaMalloc(&s->rnbr, (size_t)n * s->rwp * 4));
-    V2_CUDA(cudaMalloc(&s->vsets, (size_t)2 * s->rwp * 4));
-    V2_CUDA(cudaMalloc(&s->counters, 4 * sizeof(unsigned long long)));
+    V2_CUDA(s->cache->get((void**)&s->table, (size_t)C * n));
+    V2_CUDA(s->cache->get((void**)&s->marked, (size_t)C * s->rwp * 4));
+    V2_CUDA(s->cache->get((void**)&s->nbr, (size_t)n * s->rwp * 4));
+    V2_CUDA(s->cache->get((void**)&s->val1, (size_t)C * n));
+    V2_CUDA(s->cache->get((void**)&s->newval, (size_t)C * n));
+    V2_CUDA(s->cache->get((void**)&s->plain, (size_t)C * n));
+    V2_CUDA(s->cache->get((void**)&s->unsafe, (size_t)C * s->rwp * 4));
+    V2_CUDA(s->cache->get((void**)&s->changed, C));
+    V2_CUDA(s->cache->get((void**)&s->lev, (size_t)C * p));
+    V2_CUDA(s->cache->get((void**)&s->fin1, C));
+    V2_CUDA(s->cache->get((void**)&s->fin2, C));
+    V2_CUDA(s->cache->get((void**)&s->rnbr, (size_t)n * s->rwp * 4));
+    V2_CUDA(s->cache->get((void**)&s->vsets, (size_t)2 * s->rwp * 4));
+    V2_CUDA(s->cache->get((void**)&s->counters, 4 * sizeof(unsigned long long)));
     if (int rc = v2_set_hash_capacity(s, v2_hash_capacity((uint64_t)C * n, p), err)) return rc;
-    V2_CUDA(cudaMallocHost(&s->h_pinned, 4 * sizeof(unsigned long long)));
-    V2_CUDA(cudaEventCreate(&s->e0));
-    V2_CUDA(cudaEventCreate(&s->e1));
     std::vector<uint32_t> nbr((size_t)n * s->rwp, 0);
     std::vector<uint32_t> rnbr((size_t)n * s->rwp, 0), vsets((size_t)2 * s->rwp, 0);
     for (int v = 0; v < n; ++v) {
@@ -1094,7 +1096,6 @@ int v2_create(V2Solver** out, cudaStream_t st, int num_sms, int n, int k, int p,
     V2_CUDA(cudaMemcpyAsync(s->nbr, nbr.data(), nbr.size() * 4, cudaMemcpyHostToDevice, st));
     V2_CUDA(cudaMemcpyAsync(s->rnbr, rnbr.data(), rnbr.size() * 4, cudaMemcpyHostToDevice, st));
     V2_CUDA(cudaMemcpyAsync(s->vsets, vsets.data(), vsets.size() * 4, cudaMemcpyHostToDevice, st));
-    V2_CUDA(cudaStreamSynchronize(st));
     return CR_OK;
 }
 
@@ -1103,14 +1104,11 @@ void v2_destroy(V2Solver* s) {
     void* ptrs[] = {s->table, s->marked, s->nbr, s->val1, s->newval, s->plain, s->unsafe, s->changed, s->lev,
                     s->fin1, s->fin2, s->rnbr, s->vsets, s->counters, s->hkey, s->hmask};
     for (void* q : ptrs)
-        if (q) cudaFree(q);
-    if (s->h_pinned) cudaFreeHost(s->h_pinned);
-    if (s->e0) cudaEventDestroy(s->e0);
-    if (s->e1) cudaEventDestroy(s->e1);
+        s->cache->put(q);
     delete s;
 }
 
-int v2_init(V2Solver* s, uint64_t* caps, cr_solve_stats* stats, std::string* err) {
+int v2_init(V2Solver* s, cr_solve_stats* stats, std::string* err) {
     cudaStream_t st = s->st;
     V2_CUDA(cudaEventRecord(s->e0, st));
     V2_CUDA(cudaMemsetAsync(s->table, kUnmarked, (size_t)s->C * s->n, st));
@@ -1124,9 +1122,7 @@ int v2_init(V2Solver* s, uint64_t* caps, cr_solve_stats* stats, std::string* err
     k_v2_init<<<grid, 256, 0, st>>>(s->table, s->marked, s->configs, s->C, s->n, s->k, s->rwp, s->counters);
     V2_CUDA(cudaGetLastError());
     V2_CUDA(cudaEventRecord(s->e1, st));
-    V2_CUDA(cudaMemcpyAsync(s->h_pinned, s->counters, 8, cudaMemcpyDeviceToHost, st));
     V2_CUDA(cudaStreamSynchronize(st));
-    *caps = s->h_pinned[0];
     float ms = 0;
     cudaEventElapsedTime(&ms, s->e0, s->e1);
     stats->init_ms = ms;
