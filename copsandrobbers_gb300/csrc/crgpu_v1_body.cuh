@@ -2159,9 +2159,9 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
     return x;
 }
 
-// Shared-memory quads (16 bytes) of one warp of the tile form: an entry per vertex, the neutral
-// entry, and two words per (row word, lane).
-__host__ __device__ inline int and_tile_quads(int rw) { return rw * 48 + 1; }
+// Shared-memory quads (16 bytes) of one warp of the tile form: an entry of two words per vertex,
+// the neutral entry, and two words per (row word, lane).
+__host__ __device__ inline int and_tile_quads(int rw) { return rw * 32 + 1; }
 
 // Last column over long row lists, fresh form (see and_body): a warp takes 32 listed rows and
 // turns its words of column 0's marks and of the fresh marks of the (at most two) value slots
@@ -2169,12 +2169,15 @@ __host__ __device__ inline int and_tile_quads(int rw) { return rw * 48 + 1; }
 // robber r and decides it for all 32 rows at once: over v in hop(r), the AND of v's marked words
 // says in which rows r is complete, the OR of v's fresh words of a slot in which rows it meets a
 // fresh mark of that slot.  hop(r) comes from the ELL lists (d.g.ell), padded with the neutral
-// entry (all marked, nothing fresh), so a warp walks the 32 lists of a word in step.  The results
+// entry (all marked, nothing fresh), so a warp walks the 32 lists of a word in step.  A vertex is
+// unmarked, marked before, or freshly marked in one slot or the other: two bits per (vertex, row)
+// (00, 01, 10, 11), two planes to turn and 8 bytes to read per neighbour.  The results
 // are turned back to row words, masked with the open states and written by the row's lane.
 // Bound: issue and shared-memory wavefronts, about 25 warp instructions per row at n = 128 where
 // the row-by-row form takes several hundred (its bit loops diverge over the rows of a warp), and
 // in the densest passes the table bytes.  Last columns of a whole solve: G(n, p) n = 128 1016 us
-// row by row, 531 us in tiles; Delaunay n = 199 9.0 and 3.5 ms; n = 389 195 and 70 ms.
+// row by row, 540 us in tiles; Delaunay n = 199 9.0 and 3.5 ms; n = 389 195 and 58 ms (70 with three
+// words per vertex and half the warps per SM).
 __device__ CR_BODY_INLINE void and_tile_body(const V1Dev& d, int col, unsigned wk, unsigned nwk) {
     extern __shared__ __align__(16) uint32_t sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -2187,14 +2190,14 @@ __device__ CR_BODY_INLINE void and_tile_body(const V1Dev& d, int col, unsigned w
     const int v1 = mi.hi + 1, v0 = mi.lo + 1;
     const int so1 = v1 - out_base, so0 = v0 - out_base;
     const uint32_t keep1 = v1 < kMaxRound ? FULL_MASK : 0u, keep0 = two && v0 < kMaxRound ? FULL_MASK : 0u;
-    uint4* sx = reinterpret_cast<uint4*>(sm) + warp * and_tile_quads(rw);
-    uint32_t* sn1 = reinterpret_cast<uint32_t*>(sx + rw * 32 + 1) + lane;
+    uint2* sx = reinterpret_cast<uint2*>(reinterpret_cast<uint4*>(sm) + warp * and_tile_quads(rw));
+    uint32_t* sn1 = reinterpret_cast<uint32_t*>(sx + rw * 32 + 2) + lane;
     uint32_t* sn0 = sn1 + rw * 32;
     const uint16_t* CR_RESTRICT ell = d.g.ell + lane;
     const uint32_t* CR_RESTRICT ell_off = d.g.ell_off;
     const RowList rl(d, 0, mi);
     const bool vec4 = (rwp & 3) == 0;
-    if (lane == 0) sx[rw * 32] = make_uint4(FULL_MASK, 0u, 0u, 0u);
+    if (lane == 0) sx[rw * 32] = make_uint2(0u, FULL_MASK);
     Tally t;
     const uint32_t tiles = (rl.n + 31) / 32, step = nwk * (blockDim.x >> 5);
     for (uint32_t tile = wk * (blockDim.x >> 5) + warp; tile < tiles; tile += step) {
@@ -2226,12 +2229,9 @@ __device__ CR_BODY_INLINE void and_tile_body(const V1Dev& d, int col, unsigned w
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 if (w0 + j >= rw) break;
-                uint4 e;
-                e.x = warp_transpose(av[j], lane);
-                e.y = warp_transpose(hv[j], lane);
-                e.z = two ? warp_transpose(lv[j], lane) : 0u;
-                e.w = 0u;
-                sx[(w0 + j) * 32 + lane] = e;
+                // (fresh marks are marked: x = fresh, y = marked and not fresh in the lower slot)
+                sx[(w0 + j) * 32 + lane] = make_uint2(warp_transpose(hv[j] | lv[j], lane),
+                                                      warp_transpose(av[j] & ~lv[j], lane));
             }
         }
         __syncwarp();
@@ -2241,10 +2241,10 @@ __device__ CR_BODY_INLINE void and_tile_body(const V1Dev& d, int col, unsigned w
             const uint32_t e1 = CR_LDG(&ell_off[w + 1]);
 #pragma unroll 4
             for (uint32_t e = CR_LDG(&ell_off[w]); e < e1; ++e) {
-                const uint4 x = sx[CR_LDG(&ell[e * 32])];
-                all &= x.x;
-                t1 |= x.y;
-                t0 |= x.z;
+                const uint2 x = sx[CR_LDG(&ell[e * 32])];
+                all &= x.x | x.y;
+                t1 |= x.x & x.y;
+                t0 |= x.x & ~x.y;
             }
             uint32_t n1 = all & t1 & keep1, n0 = all & t0 & ~t1 & keep0;
             if (__any_sync(FULL_MASK, (n1 | n0) != 0u)) {
