@@ -90,7 +90,7 @@ struct cr_solver {
     cr_context* ctx = nullptr;
     int n = 0, k = 0, p = 0, rules = CR_RULES_V1, cols = 0, rw = 0, rwp = 0, S = 2;
     uint64_t C = 0;
-    int maxdeg = 0;
+    int maxdeg = 0, mindeg = CR_MAX_N;
     std::vector<uint32_t> h_rp;       // the robber's moves (with self-loops under CR_ROBBER_STAY)
     std::vector<uint16_t> h_col;
     std::vector<uint32_t> h_crp;      // the cops' moves (with self-loops under CR_COP_STAY)
@@ -124,6 +124,7 @@ struct cr_solver {
     uint32_t* d_rhop = nullptr;
     uint16_t* d_ell = nullptr;        // hop lists of the last column's tile form
     uint32_t* d_ell_off = nullptr;
+    uint32_t* d_cin = nullptr;        // closed in-neighbour words of the first pass's tiles
     uint8_t* d_cover = nullptr;   // first-pass neighbour-slot masks (p = 1, max degree <= 32)
     int cover_w = 0, npad = 0;
     // the small arrays above (graph, rank table, masks) share one block, uploaded at once
@@ -339,7 +340,9 @@ static V1Dev dev_view(const cr_solver* s) {
     d.g.rhop = s->d_rhop;
     d.g.ell = s->d_ell;
     d.g.ell_off = s->d_ell_off;
+    d.g.cin = s->d_cin;
     d.g.maxdeg = s->maxdeg;
+    d.g.mindeg = s->mindeg;
     d.g.cover = s->d_cover;
     d.g.cover_w = s->cover_w;
     d.g.npad = s->npad;
@@ -466,6 +469,18 @@ static int alloc_v1(cr_solver* s, SmallArrays& small) {
         small.add(&s->d_ccol, ccol);
         small.add(&s->d_ciso, ciso);
     }
+    bool all_move = true;
+    for (uint32_t w : ciso) all_move &= w == 0;
+    if (s->cols == 2 && s->n >= 16 && all_move) {
+        std::vector<uint32_t> cin((size_t)s->rw * s->rw * 32, 0);
+        for (int c = 0; c < s->n; ++c) {
+            uint32_t* row = cin.data() + (size_t)(c >> 5) * s->rw * 32;
+            const uint32_t bit = 1u << (c & 31);
+            row[c] |= bit;
+            for (uint32_t e = crp[c]; e < crp[c + 1]; ++e) row[ccol[e]] |= bit;
+        }
+        small.add(&s->d_cin, cin);
+    }
     small.add(&s->d_iso, iso);
     small.add(&s->d_nbr, nbr);
     small.add(&s->d_rrp, rrp);
@@ -567,6 +582,7 @@ int cr_solver_create(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, i
     move_graph(s->cop_stay, s->h_crp, s->h_ccol);
     for (int v = 0; v < s->n; ++v) {
         s->maxdeg = std::max<int>(s->maxdeg, s->h_rp[v + 1] - s->h_rp[v]);
+        s->mindeg = std::min<int>(s->mindeg, s->h_rp[v + 1] - s->h_rp[v]);
         s->cop_maxdeg = std::max<int>(s->cop_maxdeg, s->h_crp[v + 1] - s->h_crp[v]);
     }
     // B[i][x] = C(n - x + k - 1 - i, k - i)

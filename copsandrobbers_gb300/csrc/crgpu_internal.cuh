@@ -83,6 +83,10 @@ struct DevGraph {
     // entries down its column, padded with rw * 32.  Null = the tile form is not used.
     const uint16_t* ell = nullptr;
     const uint32_t* ell_off = nullptr;
+    // [rw][rw * 32]: bit j of word (t, v) set iff v is cop 32t + j's vertex or a move of it.  Null =
+    // the first pass does not go by tiles (a cop without a move, or n < 16).
+    const uint32_t* cin = nullptr;
+    int mindeg = 0;           // smallest out-degree (the robber's), where the host knows it
     int nnz = -1;             // row_ptr[n] when the host knows it (sizes shared-memory staging)
     // The cops' move graph when it differs from the robber's (row_ptr / col above), i.e. under
     // the stay-allowed rules; null = the same graph.  rrow_ptr / rcol and nbr always describe

@@ -60,9 +60,10 @@ __device__ __forceinline__ bool pass_kernel_begin(const V1Dev& d) {
 
 __global__ void k_prep(V1Dev d, int col, int nx) { prep_body(d, col, nx, blockIdx.x, gridDim.x); }
 __global__ void k_init(V1Dev d, int K) { init_body(d, K, blockIdx.x, gridDim.x); }
-// The first pass in two instances: rows of one 256-robber block split into whole lane pieces
-// (the run form; at most 85 registers, 3 blocks of 256 per SM, which measured faster than 64
-// registers at 4 blocks and than 2 blocks), and every other row shape (64 registers).
+// The first pass in three forms (launch_init_pass1): the run form of rows of one 256-robber block
+// split into whole lane pieces with byte masks (at most 85 registers, 3 blocks of 256 per SM, which
+// measured faster than 64 registers at 4 blocks and than 2 blocks), the tiles, and the general sweep
+// (64 registers).
 template <int K, int W, bool SINGLE>
 __global__ void __launch_bounds__(256, SINGLE ? 3 : 4) k_init_pass1(V1Dev d) {
     if (SINGLE) {
@@ -71,6 +72,11 @@ __global__ void __launch_bounds__(256, SINGLE ? 3 : 4) k_init_pass1(V1Dev d) {
     } else {
         init_pass1_body<K, W>(d, blockIdx.x, gridDim.x);
     }
+}
+template <int K>
+__global__ void __launch_bounds__(256, 3) k_init_tiles(V1Dev d) {
+    if ((d.g.n & 15) == 0) init_pass1_tiles<K, true>(d, blockIdx.x, gridDim.x);
+    else init_pass1_tiles<K, false>(d, blockIdx.x, gridDim.x);
 }
 
 template <int K, int NWP, int G>
@@ -332,22 +338,42 @@ static void launch_init_pass1_w(const V1Dev& d, int grid, size_t sm, cudaStream_
         default: k_init_pass1<4, W, SINGLE><<<grid, 256, sm, st>>>(d); break;
     }
 }
-template <bool SINGLE>
-static void launch_init_pass1_s(const V1Dev& d, int grid, size_t sm, cudaStream_t st) {
-    if (d.g.cover_w == 1) launch_init_pass1_w<1, SINGLE>(d, grid, sm, st);
-    else if (d.g.cover_w == 2) launch_init_pass1_w<2, SINGLE>(d, grid, sm, st);
-    else launch_init_pass1_w<4, SINGLE>(d, grid, sm, st);
+// Requires d.g.cover (cover_w 1, 2 or 4) and two columns.  Three forms, one wave of resident blocks:
+//   run      rows of one 256-robber block split into whole lane pieces, at most 8 neighbours, at
+//            least 3: column 1 then hardly marks anything in this pass, and the run form's test of
+//            that is the cheapest (4-regular n = 256, k = 3: 300 us, tiles 490 us);
+//   tiles    every other graph of 16 vertices and more whose cops can all move: where robbers with
+//            one or two neighbours are caught in most configurations the run form leaves its fast
+//            loop for each of them (G(n, p) n = 128, k = 3: 159 us, tiles 80 us), and the general
+//            sweep writes rows that are not 16-byte aligned byte by byte (Delaunay n = 199 1760 us,
+//            tiles 340; n = 389 25.0 and 3.8 ms; G(n, p) n = 61, k = 4 519 and 105 us);
+//   general  the rest.
+template <int K>
+static void launch_init_tiles(const V1Dev& d, int num_sms, cudaStream_t st) {
+    const size_t sm = (size_t)pass1_tile_words(8, d.g.n, d.g.rw) * 4;
+    if (sm > 40 * 1024) raise_smem_limit((const void*)k_init_tiles<K>, sm);
+    const int per_sm = std::max(1, std::min(3, (int)(220 * 1024 / (sm + 1024))));
+    const uint64_t cap = ((uint64_t)d.C + 31) / 32;
+    k_init_tiles<K><<<(int)std::max<uint64_t>(1, std::min<uint64_t>(cap, (uint64_t)num_sms * per_sm)), 256, sm, st>>>(d);
 }
 
-// Requires d.g.cover (cover_w 1, 2 or 4) and two columns.  Rows of one 256-robber block
-// split into whole lane pieces take the run form, which needs its tables in shared memory.
-// One wave of resident blocks: each warp sweeps one contiguous range of configurations.
 void launch_init_pass1(const V1Dev& d, int num_sms, cudaStream_t st) {
-    const bool single = d.g.n <= 256 && (d.g.n & 7) == 0;
+    const bool run = d.g.n <= 256 && (d.g.n & 7) == 0 && d.g.cover_w == 1 && (d.g.mindeg >= 3 || !d.g.cin);
+    if (!run && d.g.cin && d.g.ell) {
+        switch (d.k) {
+            case 1: launch_init_tiles<1>(d, num_sms, st); break;
+            case 2: launch_init_tiles<2>(d, num_sms, st); break;
+            case 3: launch_init_tiles<3>(d, num_sms, st); break;
+            default: launch_init_tiles<4>(d, num_sms, st); break;
+        }
+        return;
+    }
     const uint64_t cap = ((uint64_t)d.C + 7) / 8;
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(cap, (uint64_t)num_sms * (single ? 3 : 4)));
-    if (single) launch_init_pass1_s<true>(d, grid, (size_t)init_pass1_smem_words(d.g.n, d.g.rwp) * 4, st);
-    else launch_init_pass1_s<false>(d, grid, 0, st);
+    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(cap, (uint64_t)num_sms * (run ? 3 : 4)));
+    if (run) launch_init_pass1_w<1, true>(d, grid, (size_t)init_pass1_smem_words(d.g.n, d.g.rwp) * 4, st);
+    else if (d.g.cover_w == 1) launch_init_pass1_w<1, false>(d, grid, 0, st);
+    else if (d.g.cover_w == 2) launch_init_pass1_w<2, false>(d, grid, 0, st);
+    else launch_init_pass1_w<4, false>(d, grid, 0, st);
 }
 
 // Builds column col's row list from its flag plane (after the first pass): each block takes

@@ -1150,6 +1150,23 @@ __device__ CR_BODY_INLINE void cop_pull_body(const V1Dev& d, int col, int nx, un
     t.flush(d, col, L.lane);
 }
 
+// 32 x 32 bit transpose across a warp: lane i holds row i and gets column i back (bit j of lane i
+// becomes bit i of lane j).  Each of the five steps swaps one bit of the lane index with the same
+// bit of the bit index: one shuffle, one rotate, one select.
+__device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
+    uint32_t keep = 0x0000FFFFu;
+#pragma unroll
+    for (int s = 16; s >= 1; s >>= 1) {
+        const uint32_t y = __shfl_xor_sync(FULL_MASK, x, s);
+        const bool up = (lane & s) != 0;
+        const uint32_t r = __funnelshift_l(y, y, up ? 32 - s : s);
+        const uint32_t k = up ? ~keep : keep;
+        x = (x & k) | (r & ~k);
+        keep ^= keep << (s >> 1);
+    }
+    return x;
+}
+
 // The table bytes of one row word's new marks, a lane per robber: n1 / n0 = the marks of the
 // higher and the lower value, at = the byte of the word's first robber.  The warp's stores fall
 // in one stretch of 32 * cols bytes, where a loop over one lane's bits is a transaction per byte.
@@ -1600,6 +1617,284 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
         }
     }
     t.flush(d, col, lane);
+}
+
+// Shared-memory words of the tile sweep of the first pass: the cops' closed neighbour rows, and
+// per warp the head's rows, a word per vertex, and two words per (row word, lane).
+__host__ __device__ inline int pass1_tile_rows(int n, int rw) { return (n * (rw | 1) + 1 + 3) & ~3; }
+__host__ __device__ inline int pass1_tile_warp(int rw) { return (2 * (rw + 1) + rw * 32 + 1 + 2 * rw * 32 + 3) & ~3; }
+__host__ __device__ inline int pass1_tile_words(int warps, int n, int rw) {
+    return pass1_tile_rows(n, rw) + warps * pass1_tile_warp(rw);
+}
+
+// initializeCaptures and the first pass of a p = 1 solve (see above) by tiles, for n >= 16 and
+// graphs whose cops can all move.  A warp takes a unit as the separable turn does: a head (the
+// leading cops) and up to 32 consecutive last cops c, whose configurations and table rows are
+// consecutive.  Column 0's marks of a configuration are P | N[c] with P = the head's closed
+// neighbourhood.  Column 1 is decided a lane per robber for all 32 configurations at once: over v
+// in N(r), the AND of (v in P ? all : the c with v in N[c]), a word of the d.g.cin table; hardly
+// any robber survives a few neighbours, so the walk usually ends early.  The table rows of the unit
+// are one stretch of states, written as 32-byte pieces of 16 states whatever n's alignment: a
+// piece's bits come from its row (and the next one where it crosses), the pieces at the two ends of
+// the stretch state by state.  Column 1's few marks are patched in afterwards.
+// Bound: issue and its latencies more than the table's bytes: Delaunay n = 389 8.9 GB in 3.8 ms,
+// 2.3 TB/s (25 ms with rows written byte by byte); G(n, p) n = 128 80 us.
+// The bytes of 16 states of the first pass's table from their bits: column 0 = 0x03 on a mark (x),
+// column 1 = 0xFE, both 0x01 on a cop (y; x excludes them).  Each output word picks its four bytes
+// out of { 0xFE, 0x03, 0x01 } by the nibbles of a selector: the bits of two states, a byte apart.
+__device__ __forceinline__ void first_pass_bytes(uint32_t x, uint32_t y, uint32_t (&o)[8]) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        uint32_t sel = (((x >> (4 * k)) & 0xFu) * 0x00204081u) & 0x01010101u;
+        if (y) sel |= ((((y >> (4 * k)) & 0xFu) * 0x00204081u) & 0x01010101u) * 0x22u;
+        o[2 * k] = __byte_perm(0x000103FEu, 0u, sel & 0xFFFFu);
+        o[2 * k + 1] = __byte_perm(0x000103FEu, 0u, sel >> 16);
+    }
+}
+
+// ALIGNED: n a multiple of 16, so that every piece is whole and lies in one row.
+template <int K, bool ALIGNED>
+__device__ CR_BODY_INLINE void init_pass1_tiles(const V1Dev& d, unsigned wk, unsigned nwk) {
+    extern __shared__ __align__(16) uint32_t sm[];
+    constexpr int M = K > 1 ? K - 1 : 1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int n = d.g.n, rw = d.g.rw, rwp = d.g.rwp, S = d.S, rws = rw | 1, np1 = n + 1;
+    uint32_t* sclos = sm;                                          // [n][rws]
+    uint32_t* sP = sm + pass1_tile_rows(n, rw) + warp * pass1_tile_warp(rw);   // [rw + 1]
+    uint32_t* sH = sP + rw + 1;                                    // [rw + 1]: the head's own bits
+    uint32_t* sM = sH + rw + 1;                                    // [rw * 32 + 1], the last one neutral
+    uint32_t* sA1 = sM + rw * 32 + 1 + lane;                       // [rw][32]: marks of round 1
+    uint32_t* sA2 = sA1 + rw * 32;                                 // and of round 2
+    for (int i = threadIdx.x; i < n * rw; i += blockDim.x) {
+        const int v = i / rw, w = i - v * rw;
+        sclos[v * rws + w] = CR_LDG(&d.g.nbr[v * rwp + w]) | ((v >> 5) == w ? 1u << (v & 31) : 0u);
+    }
+    if (lane == 0) {
+        sP[rw] = sH[rw] = 0u;
+        sM[rw * 32] = FULL_MASK;
+    }
+    __syncthreads();
+    const uint16_t* CR_RESTRICT ell = d.g.ell + lane;
+    const uint32_t* CR_RESTRICT ell_off = d.g.ell_off;
+    const uint32_t magic = 0xFFFFFFFFu / (uint32_t)n + 1u;         // s / n = umulhi(s, magic), s < 2^15
+    const bool vec4 = (rwp & 3) == 0;
+    unsigned cnt = 0, rows1 = 0, any1 = 0, any2 = 0;
+    bool seeds = false;
+    const uint32_t nwarps = nwk * (blockDim.x >> 5);
+    uint32_t u = wk * (blockDim.x >> 5) + warp;                    // unit, from the current tile's first
+    for (int c0 = 0, tile = 0; c0 < n; c0 += 32, ++tile) {
+        const uint32_t units = K > 1 ? heads_below<M>(min(n, c0 + 32)) : 1u;
+        for (; u < units; u += nwarps) {
+            int h[M];
+            if (K > 1) head_of<M>(u, h);
+            else h[0] = 0;
+            const int hmax = h[M - 1];
+            const int cf = max(c0, hmax), count = min(n, c0 + 32) - cf;   // the unit's last cops
+            uint32_t cid0;                                         // its first configuration
+            {
+                int cc[K];
+#pragma unroll
+                for (int i = 0; i < K - 1; ++i) cc[i] = h[i];
+                cc[K - 1] = cf;
+                cid0 = rank_g<K>(cc, d.binom, np1);
+            }
+            const uint32_t live = (count == 32 ? FULL_MASK : (1u << count) - 1u) << (cf - c0);   // bit = cop - c0
+            if (lane < rw) {
+                uint32_t p = 0u, b = 0u;
+                if (K > 1) {
+#pragma unroll
+                    for (int i = 0; i < M; ++i) {
+                        p |= sclos[h[i] * rws + lane];
+                        if ((h[i] >> 5) == lane) b |= 1u << (h[i] & 31);
+                    }
+                }
+                sP[lane] = p;
+                sH[lane] = b;
+            }
+            __syncwarp();
+            const uint32_t* cin = d.g.cin + (size_t)tile * rw * 32 + lane;
+            for (int w = 0; w < rw; ++w) sM[w * 32 + lane] = ((sP[w] >> lane) & 1u) ? FULL_MASK : CR_LDG(&cin[w * 32]);
+            __syncwarp();
+            // column 1, a lane per robber
+            bool some = false;
+            for (int w = 0; w < rw; ++w) {
+                uint32_t a = w * 32 + lane < n ? live : 0u;
+                const uint32_t e0 = CR_LDG(&ell_off[w]), e1 = CR_LDG(&ell_off[w + 1]);
+                for (uint32_t e = e0; e < e1; ++e) {
+                    a &= sM[CR_LDG(&ell[e * 32])];
+                    if (!__any_sync(FULL_MASK, a != 0u)) break;
+                }
+                uint32_t a1 = 0u, a2 = 0u;
+                if ((sH[w] >> lane) & 1u) a = 0u;                  // (a robber on a cop is a capture)
+                if (w == tile) a &= ~(1u << lane);
+                if (__any_sync(FULL_MASK, a != 0u)) {
+                    // round 1 where every neighbour is a cop, else round 2
+                    uint32_t only = FULL_MASK;
+                    for (uint32_t e = e0; e < e1; ++e) {
+                        const int v = CR_LDG(&ell[e * 32]);
+                        if (v < n && !((sH[v >> 5] >> (v & 31)) & 1u)) only &= (v >> 5) == tile ? 1u << (v & 31) : 0u;
+                    }
+                    a1 = a & only;
+                    a2 = a & ~only;
+                    cnt += __popc(a);
+                    any1 |= a1;
+                    any2 |= a2;
+                    some = true;
+                    a1 = warp_transpose(a1, lane);                 // now bit = robber, lane = cop - c0
+                    a2 = warp_transpose(a2, lane);
+                }
+                sA1[w * 32] = a1;
+                sA2[w * 32] = a2;
+            }
+            // the rows of this lane's configuration
+            const int c = c0 + lane;
+            const bool mine = (live >> lane) & 1u;
+            const uint32_t cid = cid0 + (uint32_t)(c - cf);
+            bool row1 = false;
+            if (mine) {
+                const uint32_t* clos = sclos + c * rws;
+                uint32_t* m0 = d.marked + (size_t)cid * rwp;
+                uint32_t* m1 = d.marked + ((size_t)d.C + cid) * rwp;
+                for (int w0 = 0; w0 < rwp; w0 += 4) {
+                    uint32_t x0[4], x1[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        x0[j] = x1[j] = 0u;
+                        const int w = w0 + j;
+                        if (w < rw) {
+                            const uint32_t cops = sH[w] | ((c >> 5) == w ? 1u << (c & 31) : 0u);
+                            const uint32_t a = some ? sA1[w * 32] | sA2[w * 32] : 0u;
+                            x0[j] = sP[w] | clos[w];
+                            x1[j] = cops | a;
+                            row1 |= a != 0u;
+                            const int s = __popc(x0[j] & ~cops);
+                            cnt += s;
+                            seeds |= s != 0;
+                        }
+                    }
+                    if (vec4) {
+                        *reinterpret_cast<uint4*>(m0 + w0) = make_uint4(x0[0], x0[1], x0[2], x0[3]);
+                        *reinterpret_cast<uint4*>(m1 + w0) = make_uint4(x1[0], x1[1], x1[2], x1[3]);
+                    } else {
+                        m0[0] = x0[0];
+                        m1[0] = x1[0];
+                        if (rwp > 1) {
+                            m0[1] = x0[1];
+                            m1[1] = x1[1];
+                        }
+                    }
+                }
+                // column 0's frontier is consumed by this sweep; column 1's row only where it marks
+                d.fflag[cid] = 0;
+                d.fflag[(size_t)d.C + cid] = row1 ? 1 : 0;
+                if (row1) {
+                    ++rows1;
+                    uint32_t* frow = d.front + ((size_t)d.C + cid) * (size_t)(S * rwp);
+                    for (int so = 0; so < S; ++so) {
+                        const uint32_t* src = so == 0 ? sA1 : (so == 1 ? sA2 : nullptr);
+                        if (vec4) {
+                            for (int w = 0; w < rwp; w += 4) {
+                                uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                                if (src) {
+                                    x.x = src[w * 32];
+                                    if (w + 1 < rw) x.y = src[(w + 1) * 32];
+                                    if (w + 2 < rw) x.z = src[(w + 2) * 32];
+                                    if (w + 3 < rw) x.w = src[(w + 3) * 32];
+                                }
+                                *reinterpret_cast<uint4*>(frow + so * rwp + w) = x;
+                            }
+                        } else {
+                            for (int w = 0; w < rwp; ++w) frow[so * rwp + w] = src && w < rw ? src[w * 32] : 0u;
+                        }
+                    }
+                }
+            }
+            // the table: states [0, count * n) of the unit, in pieces of 16 aligned to 32 bytes
+            const size_t g0 = (size_t)cid0 * n;
+            const int s0 = (int)(g0 & 15), total = count * n;
+            uint4* piece = reinterpret_cast<uint4*>(d.table + 2 * (g0 - s0)) + 2 * lane;
+            uint32_t o[8];
+            if (ALIGNED) {
+                for (int st = lane * 16; st < total; st += 32 * 16, piece += 64) {
+                    const int i = (int)__umulhi((uint32_t)st, magic), r0 = st - i * n, w = r0 >> 5, sh = r0 & 16;
+                    uint32_t x = ((sP[w] | sclos[(cf + i) * rws + w]) >> sh) & 0xFFFFu;
+                    uint32_t y = (sH[w] >> sh) & 0xFFFFu;
+                    const unsigned q = (unsigned)(cf + i - r0);
+                    if (q < 16u) y |= 1u << q;
+                    x &= ~y;
+                    first_pass_bytes(x, y, o);
+                    piece[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                    piece[1] = make_uint4(o[4], o[5], o[6], o[7]);
+                }
+            } else {
+                for (int st = lane * 16 - s0; st < total; st += 32 * 16, piece += 64) {
+                    const int a = max(st, 0);
+                    const int i = (int)__umulhi((uint32_t)a, magic), r0 = a - i * n;
+                    const int w = r0 >> 5, sh = r0 & 31, left = n - r0;    // states left in row i
+                    const uint32_t* clos = sclos + (cf + i) * rws;
+                    uint32_t x = __funnelshift_r(sP[w] | clos[w], sP[w + 1] | clos[w + 1], sh);
+                    uint32_t y = __funnelshift_r(sH[w], sH[w + 1], sh);
+                    const unsigned q = (unsigned)(cf + i - r0);
+                    if (q < 16u) y |= 1u << q;
+                    if (left < 16) {
+                        const uint32_t in = (1u << left) - 1u;
+                        x &= in;
+                        y &= in;
+                        if (i + 1 < count) {
+                            x |= (sP[0] | clos[rws]) << left;
+                            y |= sH[0] << left;
+                            const unsigned q2 = (unsigned)(cf + i + 1 + left);
+                            if (q2 < 16u) y |= 1u << q2;
+                        }
+                    }
+                    const int skip = a - st;                               // states before the unit's first
+                    x = (x << skip) & 0xFFFFu;
+                    y = (y << skip) & 0xFFFFu;
+                    x &= ~y;
+                    first_pass_bytes(x, y, o);
+                    const int hi = min(16, total - st);
+                    if (skip == 0 && hi == 16) {
+                        piece[0] = make_uint4(o[0], o[1], o[2], o[3]);
+                        piece[1] = make_uint4(o[4], o[5], o[6], o[7]);
+                    } else {                                               // the ends of the stretch
+                        uint16_t* at = reinterpret_cast<uint16_t*>(piece);
+#pragma unroll
+                        for (int k = 0; k < 16; ++k)
+                            if (k >= skip && k < hi) at[k] = (uint16_t)(o[k >> 1] >> (16 * (k & 1)));
+                    }
+                }
+            }
+            __syncwarp();   // (orders the patches behind the pieces)
+            if (row1) {
+                uint8_t* trow = d.table + (size_t)cid * n * 2 + 1;
+                for (int w = 0; w < rw; ++w) {
+                    const uint32_t a1 = sA1[w * 32];
+                    uint32_t b = a1 | sA2[w * 32];
+                    while (b) {
+                        const int j = __ffs(b) - 1;
+                        b &= b - 1;
+                        trow[(w * 32 + j) * 2] = ((a1 >> j) & 1u) ? 0x03 : 0x05;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+        u -= units;
+    }
+    cnt = __reduce_add_sync(FULL_MASK, cnt);
+    rows1 = __reduce_add_sync(FULL_MASK, rows1);
+    any1 = __reduce_or_sync(FULL_MASK, any1);
+    any2 = __reduce_or_sync(FULL_MASK, any2);
+    seeds = __any_sync(FULL_MASK, seeds);
+    if (lane == 0) {
+        if (cnt) atomicAdd(d.pass_new, (unsigned long long)cnt);
+        if (rows1) atomicAdd(&d.meta[1].rows, (int)rows1);
+        if (seeds) atomicMax(&d.meta[0].hi, 1);
+        if (any1 | any2) {
+            atomicMin(&d.meta[1].lo, any1 ? 1 : 2);
+            atomicMax(&d.meta[1].hi, any2 ? 2 : 1);
+        }
+    }
 }
 
 // Cop turn from the capture seeds (column 1 before pass 1): OR over T(C) of the seed rows
@@ -2140,23 +2435,6 @@ __device__ CR_BODY_INLINE void and_body(const V1Dev& d, int col, unsigned wk, un
         }
     }
     t.flush(d, col, L.lane);
-}
-
-// 32 x 32 bit transpose across a warp: lane i holds row i and gets column i back (bit j of lane i
-// becomes bit i of lane j).  Each of the five steps swaps one bit of the lane index with the same
-// bit of the bit index: one shuffle, one rotate, one select.
-__device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
-    uint32_t keep = 0x0000FFFFu;
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) {
-        const uint32_t y = __shfl_xor_sync(FULL_MASK, x, s);
-        const bool up = (lane & s) != 0;
-        const uint32_t r = __funnelshift_l(y, y, up ? 32 - s : s);
-        const uint32_t k = up ? ~keep : keep;
-        x = (x & k) | (r & ~k);
-        keep ^= keep << (s >> 1);
-    }
-    return x;
 }
 
 // Shared-memory quads (16 bytes) of one warp of the tile form: an entry of two words per vertex,
