@@ -2649,46 +2649,68 @@ __device__ CR_BODY_INLINE void last_column_body(const V1Dev& d, int col, unsigne
     }
 }
 
+// Largest byte at even offsets (column 0) of one 16-byte piece of a two-column row; bytes outside
+// [lo, hi) of the piece (even bounds) count as zero.
+__device__ __forceinline__ uint32_t piece_max(uint4 v, int lo, int hi) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    uint32_t m = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        uint32_t x = w[k] & 0x00FF00FFu;
+        if (lo > 4 * k) x &= lo >= 4 * k + 4 ? 0u : 0xFFFF0000u;
+        if (hi < 4 * k + 4) x &= hi <= 4 * k ? 0u : 0x0000FFFFu;
+        m = __vmaxu2(m, x);
+    }
+    return max(m & 0xFFFFu, m >> 16);
+}
+
 // findFinalResult (k_cops_visibility.cpp:301-331): over the configurations whose column-0 row
-// is all marked, the smallest (worst capture round, config id) key.  A warp takes 32
-// configurations at a time, each lane testing its own row's marks; the warp then reads each
-// full row (two columns: one 16-byte load per lane covers 8 robbers, 256 per step) and keeps a
-// per-lane running minimum, reduced once per warp into one atomic.
+// is all marked, the smallest (worst capture round, config id) key.  A lane per configuration; it
+// gives its row up as soon as its key is no smaller than the best found so far (read again with
+// each stretch of the row), which on a graph the cops win is nearly always in the first stretch, so
+// that most of the table is never read (the whole of it at one coalesced row per warp took 5.96 ms
+// at Delaunay n = 389, k = 3, and 64 us at G(n, p) n = 128; this takes 0.39 ms and 52 us).
+// Two-column tables are read in 16-byte pieces whatever the rows' alignment, others byte by byte.
 __device__ CR_BODY_INLINE void verdict_body(const uint8_t* table, const uint32_t* m0, uint32_t C,
                                              int n, int rw, int rwp, int cols,
                                              unsigned long long* best, unsigned wk, unsigned nwk) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const size_t stride = (size_t)nwk * blockDim.x;
-    const bool vec = cols == 2 && (n & 7) == 0 && ((uintptr_t)table & 15u) == 0;
-    unsigned long long mine = ~0ull;
-    for (size_t base = (size_t)wk * blockDim.x + warp * 32; base < C; base += stride) {
-        const size_t cid = base + lane;
-        bool full = cid < C;
+    const uint8_t* const end = table + (size_t)C * n * cols;
+    const bool vec = cols == 2 && ((uintptr_t)table & 15u) == 0;
+    for (size_t cid = (size_t)wk * blockDim.x + threadIdx.x; cid < C; cid += stride) {
+        bool full = true;
         for (int w = 0; w < rw && full; ++w) full = m0[cid * rwp + w] == valid_mask(n, w);
-        unsigned act = __ballot_sync(FULL_MASK, full);
-        while (act) {
-            const size_t c = base + __ffs(act) - 1;
-            act &= act - 1;
-            const uint8_t* row = table + c * n * cols;
-            uint32_t wc = 0;
-            if (vec) {
-                for (int r0 = lane * 8; r0 < n; r0 += 256) {
-                    const uint4 v = *reinterpret_cast<const uint4*>(row + r0 * 2);
-                    // column-0 bytes are the even bytes; round = byte >> 1
-                    const uint32_t e0 = __byte_perm(v.x, v.y, 0x6420), e1 = __byte_perm(v.z, v.w, 0x6420);
-                    const uint32_t m = __vmaxu4(e0 >> 1 & 0x7F7F7F7Fu, e1 >> 1 & 0x7F7F7F7Fu);
-                    wc = max(wc, max(max(m & 0xFFu, (m >> 8) & 0xFFu), max((m >> 16) & 0xFFu, m >> 24)));
+        if (!full) continue;
+        unsigned long long cur = *(volatile unsigned long long*)best;   // (no result yet: the largest key)
+        const uint8_t* row = table + cid * n * cols;
+        uint32_t wc = 0;
+        auto key = [&]() { return ((unsigned long long)wc << 32) | cid; };
+        if (vec) {
+            const int off = (int)((uintptr_t)row & 15u), bytes = off + 2 * n;   // the row in its pieces
+            const uint8_t* p = row - off;
+            // four pieces at a time (their loads in flight together) while they lie in the table
+            for (int at = 0; at < bytes && key() < cur; at += 64) {
+                uint4 v[4];
+                cur = *(volatile unsigned long long*)best;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    v[k] = make_uint4(0u, 0u, 0u, 0u);
+                    if (at + 16 * k < bytes && p + at + 16 * k + 16 <= end)
+                        v[k] = *reinterpret_cast<const uint4*>(p + at + 16 * k);
                 }
-            } else {
-                for (int r = lane; r < n; r += 32) wc = max(wc, (uint32_t)(row[(size_t)r * cols] >> 1));
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int b = at + 16 * k;
+                    wc = max(wc, piece_max(v[k], max(0, off - b), min(16, max(0, bytes - b))) >> 1);
+                }
             }
-            wc = __reduce_max_sync(FULL_MASK, wc);
-            const unsigned long long key = ((unsigned long long)wc << 32) | c;
-            mine = key < mine ? key : mine;
+            if (row + 2 * n == end)   // the last row: its end may lie in a piece that the table only begins
+                for (const uint8_t* q = row; q < end; q += 2) wc = max(wc, (uint32_t)(*q >> 1));
+        } else {
+            for (int r = 0; r < n && key() < cur; ++r) wc = max(wc, (uint32_t)(row[(size_t)r * cols] >> 1));
         }
+        if (key() < cur) atomicMin(best, key());
     }
-    // every lane holds the same running minimum (the keys are warp-uniform)
-    if (lane == 0 && mine != ~0ull) atomicMin(best, mine);
 }
 
 }  // namespace CR_BODY_NS
