@@ -8,8 +8,15 @@
 // largest first), solves its k = 1, 2, ... sequence itself in a private slot of device memory,
 // and writes a result per (graph, k): verdict, pass counts digest and a table digest.  The
 // block runs the same frontier bodies as the stand-alone kernels (crgpu_v1_body.cuh) with
-// (worker 0 of 1), separated by __syncthreads, so its tables are the same bytes.  No block
-// ever waits for another; the only shared state is the queue counter.
+// (worker 0 of 1), separated by __syncthreads, so its tables are the same bytes.
+//
+// A graph of 128 vertices keeps one block busy for a quarter of a second, so a batch that does not
+// hold many times more graphs than the GPU has blocks would wait for the last large ones.  The
+// batch is therefore split: its largest graphs are solved first by teams of 2, 4 or 8 blocks (a
+// thread-block cluster, the bodies running as workers 0 .. size-1 with cluster barriers between
+// them), then every block goes on alone through the smaller ones.  How many graphs the teams take
+// and how large the teams are comes from a model of the batch's run time (plan_teams).  No block
+// ever waits for one outside its cluster; the only state shared beyond it are the queue counters.
 //
 // The block size and blocks per SM are chosen by a small autotuner that times candidate
 // launch shapes on a calibration slice of the batch (cached per device and batch shape).
@@ -20,6 +27,7 @@
 #include <map>
 #include <mutex>
 #include <numeric>
+#include <queue>
 #include <tuple>
 #include <vector>
 
@@ -52,12 +60,31 @@ struct BatchDev {
     const uint32_t* rrp_all;
     const uint16_t* rcol_all;
     unsigned char* slots;
-    size_t slot_bytes;
-    int* next;
+    size_t team_bytes;             // a team's slot, and a block's share of it once it goes alone
+    size_t solo_bytes;
+    int team_count;                // order[0 .. team_count) are the teams'
+    int* next;                     // [0] the teams' queue, [1] the single blocks'
+    int* mail;                     // per team: the graph it took
     int32_t* cop;
     cr_batch_result* res;
     unsigned long long* cta_time;  // per block: globaltimer at start and after its last graph
     uint32_t smem_words;           // dynamic shared memory of the launch
+};
+
+// The blocks solving one graph together: one, or a thread-block cluster.
+struct Team {
+    unsigned rank, size;
+    // Every thread of the team, with the memory effects of __syncthreads over all of it (the cluster
+    // barrier's arrive releases and its wait acquires at cluster scope).
+    __device__ __forceinline__ void sync() const {
+        __syncthreads();
+        if (size > 1) {
+            asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        }
+    }
+    __device__ __forceinline__ unsigned thread() const { return rank * blockDim.x + threadIdx.x; }
+    __device__ __forceinline__ unsigned threads() const { return size * blockDim.x; }
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -143,26 +170,26 @@ __device__ inline uint64_t digest_word(const uint8_t* t, size_t bytes, size_t j)
     return mix64(w ^ (j * 0x9E3779B97F4A7C15ull));
 }
 
-__device__ void block_fill(unsigned char* p, unsigned char v, size_t bytes) {
+__device__ void team_fill(const Team& tm, unsigned char* p, unsigned char v, size_t bytes) {
     // p is 256-byte aligned (slot layout)
     const uint32_t v4 = 0x01010101u * v;
     const uint4 q = make_uint4(v4, v4, v4, v4);
     uint4* p16 = reinterpret_cast<uint4*>(p);
     const size_t n16 = bytes / 16;
-    for (size_t i = threadIdx.x; i < n16; i += blockDim.x) p16[i] = q;
-    for (size_t i = n16 * 16 + threadIdx.x; i < bytes; i += blockDim.x) p[i] = v;
+    for (size_t i = tm.thread(); i < n16; i += tm.threads()) p16[i] = q;
+    for (size_t i = n16 * 16 + tm.thread(); i < bytes; i += tm.threads()) p[i] = v;
 }
 
 // The uncovered-slot masks of the fused first pass, as the stand-alone solver builds them on the
 // host (cover[c][r] bit j: r's j-th neighbour v is neither c nor a neighbour of c; cover[n+c][r]:
 // v is not c; a cop's own entry all ones, the rows of a cop without a move zero), W = 1, 2 or 4
 // bytes per mask by the largest degree.  Sets d.g.cover, cover_w and npad.
-__device__ void build_cover(V1Dev& d, uint8_t* cov, int maxdeg) {
+__device__ void build_cover(const Team& tm, V1Dev& d, uint8_t* cov, int maxdeg) {
     const int n = d.g.n, rwp = d.g.rwp, npad = (n + 7) & ~7;
     const int W = maxdeg <= 8 ? 1 : (maxdeg <= 16 ? 2 : 4);
     const uint32_t ones = W == 4 ? 0xFFFFFFFFu : ((1u << (8 * W)) - 1u);
     const size_t plane = (size_t)n * npad * W;
-    for (int t = threadIdx.x; t < n * npad; t += blockDim.x) {
+    for (int t = tm.thread(); t < n * npad; t += tm.threads()) {
         const int c = t / npad, r = t - c * npad;
         uint32_t m0 = 0, m1 = 0;
         if (r < n) {
@@ -184,12 +211,19 @@ __device__ void build_cover(V1Dev& d, uint8_t* cov, int maxdeg) {
     d.g.cover = cov;
     d.g.cover_w = W;
     d.g.npad = npad;
-    __syncthreads();
+    tm.sync();
 }
 
 // The padded neighbour lists of the last column's tile form (d.g.ell): row word w's 32 lists
-// take as many rows as the longest of them.  The block has a warp for every word (n <= 128).
-__device__ void build_ell(V1Dev& d, uint16_t* ell, uint32_t* off) {
+// take as many rows as the longest of them.  The team's first block builds them, a warp for every
+// word (n <= 128).
+__device__ void build_ell(const Team& tm, V1Dev& d, uint16_t* ell, uint32_t* off) {
+    d.g.ell = ell;
+    d.g.ell_off = off;
+    if (tm.rank != 0) {
+        tm.sync();
+        return;
+    }
     const int n = d.g.n, rw = d.g.rw, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int r = warp * 32 + lane;
     uint32_t e0 = 0, deg = 0;
@@ -209,17 +243,15 @@ __device__ void build_ell(V1Dev& d, uint16_t* ell, uint32_t* off) {
         uint16_t* at = ell + (size_t)off[warp] * 32 + lane;
         for (uint32_t e = 0; e < longest; ++e) at[e * 32] = e < deg ? d.g.col[e0 + e] : (uint16_t)(rw * 32);
     }
-    d.g.ell = ell;
-    d.g.ell_off = off;
-    __syncthreads();
+    tm.sync();
 }
 
-// Column col's row list from its flag plane, by the whole block (after the fused first pass).
-__device__ void block_list_compact(const V1Dev& d, int col) {
+// Column col's row list from its flag plane, by the whole team (after the fused first pass).
+__device__ void team_list_compact(const Team& tm, const V1Dev& d, int col) {
     const uint8_t* f = d.fflag + (size_t)col * d.C;
     uint32_t* out = d.list + (size_t)col * d.C;
     const int lane = threadIdx.x & 31;
-    for (uint32_t base = threadIdx.x & ~31u; base < d.C; base += blockDim.x) {
+    for (uint32_t base = tm.thread() & ~31u; base < d.C; base += tm.threads()) {
         const uint32_t i = base + lane;
         const bool set = i < d.C && f[i];
         const unsigned b = __ballot_sync(0xFFFFFFFFu, set);
@@ -231,9 +263,9 @@ __device__ void block_list_compact(const V1Dev& d, int col) {
     }
 }
 
-// One (graph, k) solve by the whole block.  Returns 1 on WIN.
+// One (graph, k) solve by a team.  Returns 1 on WIN.
 template <int K, int RWP, bool P1>
-__device__ int solve_job(const BatchDev& b, unsigned char* slot, int gi, int jr, uint64_t* sh) {
+__device__ int solve_job(const BatchDev& b, const Team& tm, unsigned char* slot, int gi, int jr) {
     constexpr int G = RWP <= 4 ? 4 : RWP;
     constexpr int NWP = RWP * 2 <= 2 ? 2 : RWP * 2;  // S = 2 slots
     const int n = b.n[gi], p = b.p, cols = 2 * p, S = 2;
@@ -290,19 +322,19 @@ __device__ int solve_job(const BatchDev& b, unsigned char* slot, int gi, int jr,
     const int maxdeg = b.maxdeg[gi];
     const bool fused = P1 && maxdeg <= 32;
     // ---- buildAuxGraph: zeroed planes, rank table, neighbour masks, configurations
-    block_fill(slot + L.nbr, 0, L.ell - L.nbr);
+    team_fill(tm, slot + L.nbr, 0, L.ell - L.nbr);
     if (!fused) {
-        block_fill(slot + L.marked, 0, L.front - L.marked);
-        block_fill(d.table, kUnmarked, C * (size_t)n * cols);
+        team_fill(tm, slot + L.marked, 0, L.front - L.marked);
+        team_fill(tm, d.table, kUnmarked, C * (size_t)n * cols);
     }
-    block_fill(slot + L.fflag, 0, L.total - L.fflag);
+    team_fill(tm, slot + L.fflag, 0, L.total - L.fflag);
     const int np1 = n + 1;
-    for (int t = threadIdx.x; t < K * np1; t += blockDim.x) {
+    for (int t = tm.thread(); t < K * np1; t += tm.threads()) {
         const int i = t / np1, x = t - i * np1;
         binom[t] = (uint32_t)binom_dev((int64_t)n - x + K - 1 - i, K - i);
     }
-    __syncthreads();
-    for (int u = threadIdx.x; u < n; u += blockDim.x) {
+    tm.sync();
+    for (int u = tm.thread(); u < n; u += tm.threads()) {
         const uint32_t e0 = d.g.row_ptr[u], e1 = d.g.row_ptr[u + 1];
         if (e0 == e1) atomicOr(&iso[u >> 5], 1u << (u & 31));
         for (uint32_t e = e0; e < e1; ++e) {
@@ -316,7 +348,7 @@ __device__ int solve_job(const BatchDev& b, unsigned char* slot, int gi, int jr,
             rh[r >> 5] |= 1u << (r & 31);
         }
     }
-    for (uint32_t cid = threadIdx.x; cid < C; cid += blockDim.x) {
+    for (uint32_t cid = tm.thread(); cid < C; cid += tm.threads()) {
         uint32_t rem = cid;
         int prev = 0;
         for (int i = 0; i < K; ++i) {
@@ -331,10 +363,10 @@ __device__ int solve_job(const BatchDev& b, unsigned char* slot, int gi, int jr,
             prev = lo;
         }
     }
-    __syncthreads();
-    if (P1) build_ell(d, reinterpret_cast<uint16_t*>(slot + L.ell), reinterpret_cast<uint32_t*>(slot + L.ell_off));
+    tm.sync();
+    if (P1) build_ell(tm, d, reinterpret_cast<uint16_t*>(slot + L.ell), reinterpret_cast<uint32_t*>(slot + L.ell_off));
     if (!P1) {
-        for (int r = threadIdx.x; r < n; r += blockDim.x) {
+        for (int r = tm.thread(); r < n; r += tm.threads()) {
             uint32_t cur[kBatchMaxN / 32], nxt[kBatchMaxN / 32];
             for (int w = 0; w < rwp; ++w) cur[w] = 0u;
             cur[r >> 5] = 1u << (r & 31);
@@ -357,149 +389,163 @@ __device__ int solve_job(const BatchDev& b, unsigned char* slot, int gi, int jr,
     int passes = 0;
     bool more = true;
     if (fused) {
-        build_cover(d, slot + L.cover, maxdeg);
-        if (threadIdx.x == 0) {
+        build_cover(tm, d, slot + L.cover, maxdeg);
+        if (tm.thread() == 0) {
             for (int c = 0; c < cols; ++c) d.meta[c] = ColMeta{0, kEmptyLo, -1, 0, 0, 0, 0, 0};
             d.meta[0] = ColMeta{0, 0, 0, 0, (int)C, 0, -1, 1};   // consumed: flags left clear
             d.meta[1] = ColMeta{1, kEmptyLo, -1, 0, 0, 0, 0, 0};
         }
-        __syncthreads();
-        if (d.g.cover_w == 1) init_pass1_body<K, 1>(d, 0, 1);
-        else if (d.g.cover_w == 2) init_pass1_body<K, 2>(d, 0, 1);
-        else init_pass1_body<K, 4>(d, 0, 1);
-        __syncthreads();
-        block_list_compact(d, 1);
-        __syncthreads();
+        tm.sync();
+        if (d.g.cover_w == 1) init_pass1_body<K, 1>(d, tm.rank, tm.size);
+        else if (d.g.cover_w == 2) init_pass1_body<K, 2>(d, tm.rank, tm.size);
+        else init_pass1_body<K, 4>(d, tm.rank, tm.size);
+        tm.sync();
+        team_list_compact(tm, d, 1);
+        tm.sync();
         // every configuration's distinct cops: n times the multisets holding a given vertex
         caps = (uint64_t)n * (binom_dev((int64_t)n + K - 1, K) - binom_dev((int64_t)n + K - 2, K));
         const uint64_t found = *d.pass_new;
         const unsigned bits = *d.err;
-        __syncthreads();
+        tm.sync();
         passes = 1;
         phash = mix64(found ^ (1ull * 0xD1B54A32D192ED03ull));
         more = found != 0 && !bits;
     } else {
         // ---- initializeCaptures
-        if (threadIdx.x == 0) {
+        if (tm.thread() == 0) {
             for (int c = 0; c < cols; ++c) d.meta[c] = ColMeta{0, kEmptyLo, -1, 0, 0, 0, 0, 0};
             d.meta[0] = ColMeta{0, 0, 0, 1, (int)C, 0, -1, 0};
             d.meta[1] = ColMeta{0, 0, 0, 0, (int)C, 1, -1, 0};
         }
-        __syncthreads();
-        init_body(d, K, 0, 1);
-        __syncthreads();
+        tm.sync();
+        init_body(d, K, tm.rank, tm.size);
+        tm.sync();
         caps = *d.pass_new;
-        __syncthreads();
+        tm.sync();
     }
     // ---- mainLoop
     while (more) {
         for (int col = 0; col < cols; ++col) {
             const int nx = (col + 1) % cols;
-            prep_body(d, col, nx, 0, 1);
-            __syncthreads();
+            prep_body(d, col, nx, tm.rank, tm.size);
+            tm.sync();
             if (col % 2 == 0) {
-                cop_seed_body<K, G>(d, col, nx, 0, 1);
-                __syncthreads();
+                cop_seed_body<K, G>(d, col, nx, tm.rank, tm.size);
+                tm.sync();
                 if constexpr (K == 1) {
-                    cop_pull_body<K, NWP, G>(d, col, nx, 0, 1);
-                    __syncthreads();
+                    cop_pull_body<K, NWP, G>(d, col, nx, tm.rank, tm.size);
+                    tm.sync();
                 }
                 if constexpr (K >= 2) {
-                    head_rows_body<K, RWP>(d, nx, 0, 1);
-                    __syncthreads();
-                    sep_pull_body<K, RWP>(d, col, nx, 0, 1);
-                    __syncthreads();
+                    head_rows_body<K, RWP>(d, nx, tm.rank, tm.size);
+                    tm.sync();
+                    sep_pull_body<K, RWP>(d, col, nx, tm.rank, tm.size);
+                    tm.sync();
                 }
-                cop_push_body<K>(d, col, nx, 0, 1);
-                __syncthreads();
-                cop_apply_body<G>(d, col, nx, 0, 1);
+                cop_push_body<K>(d, col, nx, tm.rank, tm.size);
+                tm.sync();
+                cop_apply_body<G>(d, col, nx, tm.rank, tm.size);
             } else if (col < cols - 1) {
-                direct_body<G>(d, col, nx, 0, 1);
+                direct_body<G>(d, col, nx, tm.rank, tm.size);
             } else {
-                last_column_body<P1, G>(d, col, 0, 1);
+                last_column_body<P1, G>(d, col, tm.rank, tm.size);
             }
-            __syncthreads();
+            tm.sync();
         }
         const uint64_t found = *d.pass_new;
         const unsigned bits = *d.err;
-        __syncthreads();
+        tm.sync();
         ++passes;
         phash += mix64(found ^ ((uint64_t)passes * 0xD1B54A32D192ED03ull));
         if (bits || found == 0 || passes >= 4096) break;
     }
     // ---- findFinalResult
-    unsigned long long* best = d.pass_new + 1;
-    if (threadIdx.x == 0) *best = ~0ull;
-    __syncthreads();
-    verdict_body(d.table, d.marked, d.C, n, rw, rwp, cols, best, 0, 1);
+    unsigned long long* best = d.pass_new + 1;   // then the digest, and whether the cops win
+    if (tm.thread() == 0) *best = ~0ull;
+    tm.sync();
+    verdict_body(d.table, d.marked, d.C, n, rw, rwp, cols, best, tm.rank, tm.size);
     // ---- table digest
     const size_t bytes = C * (size_t)n * cols;
     uint64_t part = 0;
-    for (size_t j = threadIdx.x; j < (bytes + 7) / 8; j += blockDim.x) part += digest_word(d.table, bytes, j);
+    for (size_t j = tm.thread(); j < (bytes + 7) / 8; j += tm.threads()) part += digest_word(d.table, bytes, j);
     for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xFFFFFFFFu, part, off);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = part;
-    __syncthreads();
-    int win = 0;
-    if (threadIdx.x == 0) {
-        uint64_t dg = 0;
-        for (unsigned w = 0; w < (blockDim.x >> 5); ++w) dg += sh[w];
+    if ((threadIdx.x & 31) == 0) atomicAdd(d.pass_new + 2, (unsigned long long)part);
+    tm.sync();
+    if (tm.thread() == 0) {
         const unsigned long long key = *best;
         cr_batch_result& r = b.res[jr];
         r.solved = 1;
         r.status = *d.err ? CR_ERR_INTERNAL : (passes >= 4096 ? CR_ERR_BUDGET : CR_OK);
-        win = (key != ~0ull && (int)(key >> 32) < kMaxRound) ? 1 : 0;
-        r.win = win;
-        r.capture_plies = win ? (int32_t)(key >> 32) : kMaxRound;
-        r.best_config = win ? (int64_t)(key & 0xFFFFFFFFull) : -1;
+        const int won = (key != ~0ull && (int)(key >> 32) < kMaxRound) ? 1 : 0;
+        r.win = won;
+        r.capture_plies = won ? (int32_t)(key >> 32) : kMaxRound;
+        r.best_config = won ? (int64_t)(key & 0xFFFFFFFFull) : -1;
         r.passes = passes;
         r.base_captures = caps;
         r.states = C * (uint64_t)n * cols;
-        r.digest = dg;
+        r.digest = d.pass_new[2];
         r.pass_hash = phash;
-        sh[0] = (uint64_t)win;
+        d.pass_new[3] = (unsigned long long)won;
     }
-    __syncthreads();
-    win = (int)sh[0];
-    __syncthreads();
+    tm.sync();
+    const int win = (int)*(volatile unsigned long long*)(d.pass_new + 3);
+    tm.sync();
     return win;
 }
 
 template <int K, bool P1>
-__device__ int solve_job_k(const BatchDev& b, unsigned char* slot, int gi, int jr, uint64_t* sh) {
+__device__ int solve_job_k(const BatchDev& b, const Team& tm, unsigned char* slot, int gi, int jr) {
     const int rwp = round_words((b.n[gi] + 31) / 32);
-    if (rwp <= 1) return solve_job<K, 1, P1>(b, slot, gi, jr, sh);
-    if (rwp <= 2) return solve_job<K, 2, P1>(b, slot, gi, jr, sh);
-    return solve_job<K, 4, P1>(b, slot, gi, jr, sh);
+    if (rwp <= 1) return solve_job<K, 1, P1>(b, tm, slot, gi, jr);
+    if (rwp <= 2) return solve_job<K, 2, P1>(b, tm, slot, gi, jr);
+    return solve_job<K, 4, P1>(b, tm, slot, gi, jr);
 }
 
 // Two builds: up to 512 threads per block with up to 128 registers (no spills in the bodies),
 // and 1024 threads with 64 (a few spills, twice the threads on each graph).
+template <bool P1>
+__device__ void solve_graph(const BatchDev& b, const Team& tm, unsigned char* slot, int gi) {
+    int cop = 0;
+    for (int k = 1; k <= b.kmax; ++k) {
+        const int jr = gi * b.kmax + (k - 1);
+        int win;
+        if (k == 1) win = solve_job_k<1, P1>(b, tm, slot, gi, jr);
+        else if (k == 2) win = solve_job_k<2, P1>(b, tm, slot, gi, jr);
+        else win = solve_job_k<3, P1>(b, tm, slot, gi, jr);
+        if (win) { cop = k; break; }
+    }
+    if (tm.thread() == 0) b.cop[gi] = cop;
+    if (threadIdx.x == 0) b.cta_time[2 * blockIdx.x + 1] = global_ns();
+}
+
 template <bool P1, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) k_batch(BatchDev b) {
-    __shared__ uint64_t sh[32];
     __shared__ int s_job;
-    unsigned char* slot = b.slots + (size_t)blockIdx.x * b.slot_bytes;
+    Team tm;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(tm.rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(tm.size));
+    const unsigned team = blockIdx.x / tm.size;
+    unsigned char* slot = b.slots + (size_t)team * b.team_bytes;
     if (threadIdx.x == 0) b.cta_time[2 * blockIdx.x] = b.cta_time[2 * blockIdx.x + 1] = global_ns();
+    // the teams' graphs
     for (;;) {
-        if (threadIdx.x == 0) s_job = atomicAdd(b.next, 1);
+        if (tm.thread() == 0) b.mail[team] = atomicAdd(&b.next[0], 1);
+        tm.sync();
+        const int jj = *(volatile int*)(b.mail + team);
+        tm.sync();
+        if (jj >= b.team_count) break;
+        solve_graph<P1>(b, tm, slot, b.order[jj]);
+    }
+    // the others, a block each, in its share of the team's slot
+    slot += tm.rank * b.solo_bytes;
+    const Team solo{0u, 1u};
+    for (;;) {
+        if (threadIdx.x == 0) s_job = atomicAdd(&b.next[1], 1);
         __syncthreads();
-        const int jj = s_job;
+        const int jj = b.team_count + s_job;
         __syncthreads();
         if (jj >= b.count) break;
-        const int gi = b.order[jj];
-        int cop = 0;
-        for (int k = 1; k <= b.kmax; ++k) {
-            const int jr = gi * b.kmax + (k - 1);
-            int win;
-            if (k == 1) win = solve_job_k<1, P1>(b, slot, gi, jr, sh);
-            else if (k == 2) win = solve_job_k<2, P1>(b, slot, gi, jr, sh);
-            else win = solve_job_k<3, P1>(b, slot, gi, jr, sh);
-            if (win) { cop = k; break; }
-        }
-        if (threadIdx.x == 0) {
-            b.cop[gi] = cop;
-            b.cta_time[2 * blockIdx.x + 1] = global_ns();
-        }
+        solve_graph<P1>(b, solo, slot, b.order[jj]);
     }
 }
 
@@ -545,6 +591,11 @@ struct Shape {
     int threads, per_sm;
 };
 
+// How a batch is split: order[0 .. count) goes to teams of `size` blocks, `teams` of them resident.
+struct TeamPlan {
+    int size = 1, teams = 0, count = 0;
+};
+
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int>, Shape> g_tuned;
 
@@ -576,28 +627,122 @@ struct BatchInputs {
     size_t max_stage_words = 0;   // the largest graph staging of the last-column body
 };
 
+using BatchKernel = void (*)(BatchDev);
+BatchKernel batch_kernel(Shape shape) { return shape.threads > 512 ? k_batch<true, 1024> : k_batch<true, 512>; }
+
+size_t launch_smem(const BatchInputs& in, Shape shape) {
+    return batch_smem(shape.threads, in.max_n) + in.max_stage_words * 4;
+}
+
+// The launch of `blocks` blocks in clusters of `size`.
+struct BatchLaunch {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr = {};
+    BatchLaunch(Shape shape, int blocks, int size, size_t sm, cudaStream_t st) {
+        cfg.gridDim = dim3((unsigned)blocks);
+        cfg.blockDim = dim3((unsigned)shape.threads);
+        cfg.dynamicSmemBytes = sm;
+        cfg.stream = st;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)size;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+    }
+};
+
+// Clusters of `size` blocks that are resident at a time.
+int resident_teams(Shape shape, int size, size_t sm, int num_sms) {
+    if (size == 1) return num_sms * shape.per_sm;
+    BatchLaunch l(shape, size, size, sm, nullptr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, (const void*)batch_kernel(shape), &l.cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
+}
+
+// Splits the batch between teams and single blocks.  Run time of a graph on one block: proportional
+// to its configurations times vertices at the largest k, plus a constant for its launches' worth of
+// barriers; a team of s blocks is worth a little less than s blocks (measured on 256 graphs of
+// n = 128: 0.95, 0.88 and 0.78 of them for 2, 4 and 8).  Each split is played through the two
+// queues, largest graph first, and the shortest run wins; a batch of more than 64 graphs per block
+// needs no teams (the longest graph is then a small part of the run).
+TeamPlan plan_teams(const std::vector<double>& cost, Shape shape, size_t sm, int num_sms) {
+    const int count = (int)cost.size();   // in descending order
+    const int blocks1 = num_sms * shape.per_sm;
+    TeamPlan best;
+    best.teams = std::min(count, blocks1);
+    if (count > 64 * blocks1) return best;
+    const double fixed = 2.5e4;   // in the cost's unit
+    double total = 0;
+    for (double c : cost) total += c + fixed;
+    auto play = [&](int size, int teams, double eff, int by_teams) {
+        std::priority_queue<double, std::vector<double>, std::greater<double>> q;
+        for (int t = 0; t < teams; ++t) q.push(0.0);
+        double end = 0;
+        for (int i = 0; i < by_teams; ++i) {
+            const double t = q.top() + cost[i] / (size * eff) + 1.5 * fixed;
+            q.pop();
+            q.push(t);
+            end = std::max(end, t);
+        }
+        std::vector<double> at;
+        for (; !q.empty(); q.pop())
+            for (int k = 0; k < size; ++k) at.push_back(q.top());
+        std::priority_queue<double, std::vector<double>, std::greater<double>> r(std::greater<double>(), std::move(at));
+        for (int i = by_teams; i < count; ++i) {
+            const double t = r.top() + cost[i] + fixed;
+            r.pop();
+            r.push(t);
+            end = std::max(end, t);
+        }
+        return end;
+    };
+    double shortest = play(1, blocks1, 1.0, 0);
+    const struct { int size; double eff; } kinds[] = {{2, 0.95}, {4, 0.88}, {8, 0.78}};
+    for (const auto& k : kinds) {
+        const int teams = resident_teams(shape, k.size, sm, num_sms);
+        if (teams <= 0) continue;
+        int last = -1;
+        for (double f = 2.0; f > 0.01; f /= 1.6) {
+            // the graphs longer than a share f of the ideal run
+            int m = 0;
+            while (m < count && cost[m] > f * total / blocks1) ++m;
+            if (m == last || m == 0) continue;
+            last = m;
+            const double t = play(k.size, teams, k.eff, m);
+            if (t < 0.98 * shortest) {
+                shortest = t;
+                best = TeamPlan{k.size, teams, m};
+            }
+        }
+    }
+    return best;
+}
+
 int launch_batch(cr_context* ctx, const BatchInputs& in, const std::vector<int32_t>& order, int kmax,
-                 int p, Shape shape, size_t slot_bytes, std::vector<int32_t>* cop,
+                 int p, Shape shape, TeamPlan plan, size_t team_bytes, size_t solo_bytes, std::vector<int32_t>* cop,
                  std::vector<cr_batch_result>* res, float* ms,
                  std::vector<unsigned long long>* times = nullptr) {
     const int count = (int)order.size();
-    const int nblocks = std::max(1, std::min(count, ctx->num_sms * shape.per_sm));
-    void* bufs[13] = {};
+    const int nteams = std::max(1, std::min(count, plan.teams)), nblocks = nteams * plan.size;
+    void* bufs[14] = {};
     auto cleanup = [&]() {
-        for (void* q : bufs)
-            if (q) cudaFree(q);
+        for (void* q : bufs) ctx->cache.put(q);
     };
     BatchDev b;
     b.count = count;
     b.kmax = kmax;
     b.p = p;
-    size_t sizes[13] = {order.size() * 4, in.n.size() * 4, in.maxdeg.size() * 4, in.rp_off.size() * 8,
+    size_t sizes[14] = {order.size() * 4, in.n.size() * 4, in.maxdeg.size() * 4, in.rp_off.size() * 8,
                         in.col_off.size() * 8, in.rp.size() * 4, std::max<size_t>(in.col.size(), 1) * 2,
                         in.rrp.size() * 4, std::max<size_t>(in.rcol.size(), 1) * 2,
-                        (size_t)nblocks * slot_bytes, sizeof(int) + in.n.size() * 4,
-                        in.n.size() * kmax * sizeof(cr_batch_result), (size_t)nblocks * 16};
-    for (int i = 0; i < 13; ++i) {
-        cudaError_t e = cudaMalloc(&bufs[i], sizes[i]);
+                        (size_t)nteams * team_bytes, 2 * sizeof(int) + in.n.size() * 4,
+                        in.n.size() * kmax * sizeof(cr_batch_result), (size_t)nblocks * 16, (size_t)nteams * sizeof(int)};
+    for (int i = 0; i < 14; ++i) {
+        cudaError_t e = ctx->cache.get(&bufs[i], sizes[i]);
         if (e != cudaSuccess) {
             cleanup();
             ctx->err = std::string("batch allocation: ") + cudaGetErrorString(e);
@@ -622,27 +767,31 @@ int launch_batch(cr_context* ctx, const BatchInputs& in, const std::vector<int32
     b.rrp_all = (const uint32_t*)bufs[7];
     b.rcol_all = (const uint16_t*)bufs[8];
     b.slots = (unsigned char*)bufs[9];
-    b.slot_bytes = slot_bytes;
+    b.team_bytes = team_bytes;
+    b.solo_bytes = solo_bytes;
+    b.team_count = plan.count;
     b.next = (int*)bufs[10];
-    b.cop = (int32_t*)((char*)bufs[10] + sizeof(int));
+    b.cop = (int32_t*)((char*)bufs[10] + 2 * sizeof(int));
     b.res = (cr_batch_result*)bufs[11];
     b.cta_time = (unsigned long long*)bufs[12];
-    b.smem_words = (uint32_t)((batch_smem(shape.threads, in.max_n) + in.max_stage_words * 4) / 4);
+    b.mail = (int*)bufs[13];
+    const size_t sm = launch_smem(in, shape);
+    b.smem_words = (uint32_t)(sm / 4);
     cudaMemsetAsync(bufs[10], 0, sizes[10], st);
     cudaMemsetAsync(bufs[11], 0, sizes[11], st);
-    const size_t sm = batch_smem(shape.threads, in.max_n) + in.max_stage_words * 4;
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     // the batch launch is captured once as a CUDA graph and replayed
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    void (*kern)(BatchDev) = shape.threads > 512 ? k_batch<true, 1024> : k_batch<true, 512>;
-    raise_smem_limit((const void*)kern, sm);
+    raise_smem_limit((const void*)batch_kernel(shape), sm);
     cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
     if (e == cudaSuccess) {
-        kern<<<nblocks, shape.threads, sm, st>>>(b);
+        const BatchLaunch l(shape, nblocks, plan.size, sm, st);
+        const cudaError_t launched = cudaLaunchKernelEx(&l.cfg, batch_kernel(shape), b);
         e = cudaStreamEndCapture(st, &graph);
+        if (e == cudaSuccess) e = launched;
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
     if (e == cudaSuccess) {
@@ -759,7 +908,8 @@ int cr_batch_solve(cr_context* ctx, const cr_graph* graphs, int32_t count, int32
                 std::vector<int32_t> cp;
                 std::vector<cr_batch_result> rs;
                 float ms = 0;
-                if (launch_batch(ctx, in, calib, kmax, p, c, slot_bytes, &cp, &rs, &ms) != CR_OK) continue;
+                const TeamPlan alone{1, ctx->num_sms * c.per_sm, 0};
+                if (launch_batch(ctx, in, calib, kmax, p, c, alone, slot_bytes, slot_bytes, &cp, &rs, &ms) != CR_OK) continue;
                 if (ms < best) {
                     best = ms;
                     shape = c;
@@ -774,7 +924,20 @@ int cr_batch_solve(cr_context* ctx, const cr_graph* graphs, int32_t count, int32
     std::vector<cr_batch_result> res;
     float ms = 0;
     std::vector<unsigned long long> times;
-    int rc = launch_batch(ctx, in, order, kmax, p, shape, slot_bytes, &cop, &res, &ms, &times);
+    // the teams' share of the batch (a block's share of a team's slot holds the largest graph that
+    // is solved alone)
+    raise_smem_limit((const void*)batch_kernel(shape), launch_smem(in, shape));
+    std::vector<double> sorted(count);
+    for (int i = 0; i < count; ++i) sorted[i] = cost[order[i]];
+    const TeamPlan plan = plan_teams(sorted, shape, launch_smem(in, shape), ctx->num_sms);
+    size_t solo_bytes = slot_bytes;
+    if (plan.count > 0) {
+        int solo_n = 1;
+        for (int i = plan.count; i < count; ++i) solo_n = std::max(solo_n, (int)in.n[order[i]]);
+        solo_bytes = job_layout(solo_n, kmax, p, 2).total;
+    }
+    const size_t team_bytes = std::max(slot_bytes, plan.size * solo_bytes);
+    int rc = launch_batch(ctx, in, order, kmax, p, shape, plan, team_bytes, solo_bytes, &cop, &res, &ms, &times);
     if (rc) return rc;
     memcpy(cop_number, cop.data(), count * sizeof(int32_t));
     memcpy(results, res.data(), res.size() * sizeof(cr_batch_result));
@@ -783,8 +946,8 @@ int cr_batch_solve(cr_context* ctx, const cr_graph* graphs, int32_t count, int32
         stats->ms = ms;
         for (const auto& r : res) stats->states += r.solved ? r.states : 0;
         stats->threads = shape.threads;
-        stats->ctas = std::min(count, ctx->num_sms * shape.per_sm);
-        stats->slot_bytes = (int64_t)slot_bytes;
+        stats->ctas = std::max(1, std::min(count, plan.teams)) * plan.size;
+        stats->slot_bytes = (int64_t)(plan.count > 0 ? team_bytes / plan.size : slot_bytes);
         // how evenly the blocks were kept busy: mean busy span over the whole span, and the
         // time from the median block's last graph to the last block's
         const size_t nb = times.size() / 2;

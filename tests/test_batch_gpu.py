@@ -96,3 +96,16 @@ def test_batch_limits(gpu_ctx):
         batch_solve(gpu_ctx, small_batch(2, 1), kmax=4)
     with pytest.raises(N.CrGpuError):
         batch_solve(gpu_ctx, small_batch(2, 1), kmax=2, p=2)
+
+
+@pytest.mark.parametrize("count, lo, hi", [(1, 40, 40), (3, 30, 66), (9, 8, 97), (200, 8, 44)])
+def test_batches_split_between_teams_and_blocks(gpu_ctx, count, lo, hi):
+    """Few and large graphs go to clusters of blocks, the others to single blocks: every split
+    gives the tables of single solves."""
+    graphs = small_batch(count, 100 + count, lo, hi)
+    out = batch_solve(gpu_ctx, graphs, kmax=3, p=1, threads=1024)
+    for gi, g in enumerate(graphs):
+        for k in range(1, (out.cop_numbers[gi] or 3) + 1):
+            s = single(gpu_ctx, g, k)
+            r = out.results[gi][k - 1]
+            assert (r["digest"], r["pass_hash"], r["best_config"]) == (s["digest"], s["pass_hash"], s["best_config"])
