@@ -367,6 +367,7 @@ static V1Dev dev_view(const cr_solver* s) {
     // forms switched off: no head rows (the tuple pull), a push ratio that always or never
     // pushes, the last column's general form
     if (!(s->forms & CR_FORM_SEPARABLE)) d.h1 = nullptr;
+    if (d.h1) d.push_ratio = kPushRatioSeparable;
     if (!(s->forms & CR_FORM_PULL)) d.push_ratio = 0u;
     else if (!(s->forms & CR_FORM_PUSH)) d.push_ratio = 0xFFFFFFFFu;
     d.fresh_last = (s->forms & CR_FORM_FRESH_LAST) ? 1 : 0;

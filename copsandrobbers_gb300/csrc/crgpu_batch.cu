@@ -297,6 +297,7 @@ __device__ int solve_job(const BatchDev& b, const Team& tm, unsigned char* slot,
     d.fflag = slot + L.fflag;
     d.cand = reinterpret_cast<uint32_t*>(slot + L.cand);
     d.h1 = K >= 2 ? reinterpret_cast<uint32_t*>(slot + L.h1) : nullptr;
+    if (d.h1) d.push_ratio = kPushRatioSeparable;
     d.cbits = reinterpret_cast<uint32_t*>(slot + L.cbits);
     d.list = reinterpret_cast<uint32_t*>(slot + L.list);
     d.clist = reinterpret_cast<uint32_t*>(slot + L.clist);

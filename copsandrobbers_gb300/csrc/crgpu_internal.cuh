@@ -33,6 +33,10 @@ constexpr unsigned kErrBudget = 4u;  // a bounded device loop ran out
 // A frontier with fewer non-empty rows than C / kPushRatio is pushed to its predecessors
 // (scatter with atomic ORs); a denser one is pulled by every configuration (gather).
 constexpr int kPushRatio = 16;
+// Where the pull is the separable one it is the cheaper earlier (last pushes of solves at just under
+// C / 16 rows against separable turns: Delaunay n = 199 418 and 290 us, G(n, p) n = 61, k = 4 376 and
+// 200 us).
+constexpr int kPushRatioSeparable = 32;
 
 constexpr int kSyncWords = 3;   // counters of V1Dev::sync
 

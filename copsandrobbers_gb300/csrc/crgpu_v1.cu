@@ -89,7 +89,8 @@ __global__ void __launch_bounds__(256) k_cop_pull(V1Dev d, int col, int nx) {
 //   k_cop_a  the capture-seed form, the push scatter, or the separable turn's head rows;
 //   k_cop_b  the separable turn's configurations or the push form's marking.
 // The tuple-gathering pull (k = 1, or no head rows) keeps its own launch: it wants up to 127
-// registers, the bodies here at most 64 (80 with 32-word rows), being latency-bound.
+// registers; k_cop_a at most 64 (80 with 32-word rows), k_cop_b up to 85, which keep the rows of four
+// successor heads in flight (Delaunay n = 199: 5.5 ms of cop turns, 5.7 at 64 registers with spills).
 template <int K, int NWP, int G>
 __global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_a(V1Dev d, int col, int nx) {
     if (!pass_kernel_begin(d)) return;
@@ -98,7 +99,7 @@ __global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_a(V1Dev d, int c
     if constexpr (K >= 2) head_rows_body<K, NWP / 2>(d, nx, blockIdx.x, gridDim.x);
 }
 template <int K, int NWP, int G>
-__global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_b(V1Dev d, int col, int nx) {
+__global__ void __launch_bounds__(256, 3) k_cop_b(V1Dev d, int col, int nx) {
     if (!pass_kernel_begin(d)) return;
     if constexpr (K >= 2) sep_pull_body<K, NWP / 2>(d, col, nx, blockIdx.x, gridDim.x);
     cop_apply_body<G>(d, col, nx, blockIdx.x, gridDim.x);
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_b(V1Dev d, int c
 // (no body of this launch reads them), and in the last block the column's state reset.  The
 // candidate rows wait for that column's producer.
 template <int K, int NWP, int G>
-__global__ void __launch_bounds__(256, NWP >= 32 ? 3 : 4) k_cop_b_end(V1Dev d, int col, int nx) {
+__global__ void __launch_bounds__(256, 3) k_cop_b_end(V1Dev d, int col, int nx) {
     if (!pass_kernel_begin(d)) return;
     if constexpr (K >= 2) sep_pull_body<K, NWP / 2>(d, col, nx, blockIdx.x, gridDim.x);
     cop_apply_body<G>(d, col, nx, blockIdx.x, gridDim.x);

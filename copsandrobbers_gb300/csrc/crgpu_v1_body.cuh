@@ -1167,22 +1167,21 @@ __device__ __forceinline__ uint32_t warp_transpose(uint32_t x, int lane) {
     return x;
 }
 
-// The table bytes of one row word's new marks, a lane per robber: n1 / n0 = the marks of the
-// higher and the lower value, at = the byte of the word's first robber.  The warp's stores fall
-// in one stretch of 32 * cols bytes, where a loop over one lane's bits is a transaction per byte.
-__device__ __forceinline__ void store_word(uint8_t* at, uint32_t n1, uint32_t n0, int v1, int v0, int cols, int lane) {
-    if (((n1 | n0) >> lane) & 1u) at[lane * cols] = (uint8_t)(1 | (((n1 >> lane) & 1u ? v1 : v0) << 1));
+// The table byte of one row word's new marks, a lane per robber (lm = the lane's bit): n1 / n0 = the
+// marks of the higher and the lower value, b1 / b0 = their bytes, at = the byte of the lane's robber.
+// The warp's stores fall in one stretch of 32 * cols bytes, where a loop over one lane's bits is a
+// transaction per byte.
+__device__ __forceinline__ void store_word(uint8_t* at, uint32_t n1, uint32_t n0, uint32_t lm, uint8_t b1, uint8_t b0) {
+    if ((n1 | n0) & lm) *at = (n1 & lm) ? b1 : b0;
 }
 
-// Whether a warp writes its new marks word by word (store_word) or each lane the bits of its own
-// words, from the lane's marks and non-empty words.  By words costs about 15 instructions and a
-// transaction and a half per word; by lanes about 10 instructions per mark of the fullest lane and
-// a scattered transaction per mark, the transactions being the SM's and the instructions a
-// quarter's: by words where 8 words < 5 fullest + 2 marks.  (At n = 128 the two meet near two marks
-// per word: 80 against 90 us for a last column of 1.8 marks per word, 181 against 101 us at 3.8.)
-__device__ __forceinline__ bool by_words(int marks, int words) {
-    return 8 * __reduce_add_sync(FULL_MASK, words) <
-           5 * __reduce_max_sync(FULL_MASK, marks) + 2 * __reduce_add_sync(FULL_MASK, marks);
+// Whether a warp writes its new marks row by row (store_word over all `width` words of each row that
+// has any) or each lane the bits of its own row.  By rows costs about 4 + 3 width SM cycles per row
+// (4 instructions a word), by lanes about 5.4 per mark (measured at n = 128, 7 marks a row: the
+// lanes' stores scatter, and the lanes of a warp wait for the fullest).
+__device__ __forceinline__ bool by_rows(int marks, int width) {
+    return 2 * __reduce_add_sync(FULL_MASK, marks) >=
+           (width + 2) * __popc(__ballot_sync(FULL_MASK, marks != 0));
 }
 
 // Heads: sorted multisets h[0] <= .. <= h[M-1] of M = k - 1 vertices, numbered in colexicographic
@@ -1317,6 +1316,9 @@ __device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned w
     const bool mine = w0 < rwp;                // rows of 12 words: the last of 4 lanes has none
     const uint32_t P = heads_below<M>(n);
     const int PR = heads_per_round(blockDim.x, n, rwp);
+    // the staged rows, slot by slot (rows of one slot lie a row apart, so that the scattered reads of
+    // a warp spread over all the banks)
+    const uint32_t plane = (uint32_t)(PR * n) * rwp;
     unsigned err = 0;
     for (uint32_t q0 = wk * PR; q0 < P; q0 += nwk * PR) {
         const int np = (int)min((uint32_t)PR, P - q0);
@@ -1358,7 +1360,7 @@ __device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned w
                 }
                 const bool live = CR_LDG(&fflag_in[s]) != 0 && !bad;
                 const uint32_t* src = fin + (size_t)s * rs + w0;
-                uint32_t* dst = stage + (uint32_t)i * rs + w0;
+                uint32_t* dst = stage + (uint32_t)i * rwp + w0;
                 Words<NW> x;
                 x.ldg(src);
                 if (!live) x.zero();
@@ -1366,7 +1368,7 @@ __device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned w
                 if (two) {
                     x.ldg(src + rwp);
                     if (!live) x.zero();
-                    x.store(dst + rwp);
+                    x.store(dst + plane);
                 }
             }
         }
@@ -1379,17 +1381,17 @@ __device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned w
                     c -= n;
                     ++j;
                 }
-                const uint32_t* sj = stage + (uint32_t)(j * n) * rs + w0;
+                const uint32_t* sj = stage + (uint32_t)(j * n) * rwp + w0;
                 Words<NW> a0, a1, x;
                 a0.zero();
                 a1.zero();
                 const uint32_t e1 = CR_LDG(&rp[c + 1]);
                 for (uint32_t e = CR_LDG(&rp[c]); e < e1; ++e) {
-                    const uint32_t* row = sj + CR_LDG(&adj[e]) * rs;
+                    const uint32_t* row = sj + (uint32_t)CR_LDG(&adj[e]) * rwp;
                     x.load(row);
                     a0.orr(x);
                     if (two) {
-                        x.load(row + rwp);
+                        x.load(row + plane);
                         a1.orr(x);
                     }
                 }
@@ -1403,22 +1405,22 @@ __device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned w
 }
 
 // Stage 2: a warp per unit = (head c_1 .. c_{k-1}, tile of consecutive last cops c_k), LQ lanes of
-// NW words per row and R rows per lane: the configurations of a unit are consecutive, and so are
+// NW words per row: the configurations of a unit are consecutive, and so are
 // their rows H1[h'][c_k] for every head h' of successors, so each load of the warp is one
 // contiguous stretch, the successor heads are found once per unit (a lane each) and broadcast, and
 // the words a lane ORs are the words it marks: no reduction across lanes.  Units run tile by tile
 // of last cops, so that the H1 rows in use at a time (every head, one tile) stay in L2 where all
 // of them do not, and the warps take them from a counter: their costs (deg^(k-1) heads) differ by
 // an order of magnitude.  Bound: L2 latency and bandwidth (deg^(k-1) rows per configuration).
-// Per launch, against a lane per (configuration, successor pair) with a reduction: Delaunay n = 199
-// 500 -> 270 us (6.3 TB/s of row reads), n = 389 11.5 -> 3.7 ms; G(n, p) n = 61, k = 4, both sides
-// staying: 16 ms gathering tuples one by one, 0.8 ms so.
+// Cop turns of a whole solve (both stages) with two rows per lane and a branch around the loads of
+// lanes that are not open, and so: G(n, p) n = 128 1.13 and 0.85 ms, Delaunay n = 199 6.5 and 5.5 ms.
+// A lane per (configuration, successor pair) with a reduction took 500 us a launch at n = 199 where
+// this takes 250; gathering tuples one by one 16 ms at n = 61, k = 4, both sides staying, this 0.8.
 template <int K, int RW>
 __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, unsigned wk, unsigned nwk) {
     constexpr int M = K - 1, NW = lane_words(RW), LQ = row_lanes(RW);
-    constexpr int CH = 32 / LQ;                    // rows per load of the warp
-    constexpr int R = LQ == 1 ? 1 : 2;             // loads per tile
-    constexpr int TW = CH * R;                     // last cops per tile
+    constexpr int TW = 32 / LQ;                    // last cops per tile
+    constexpr int U = 4;                           // successor heads whose rows are in flight together
     const int lane = threadIdx.x & 31;
     const int li = lane / LQ, w0 = (lane % LQ) * NW;
     const int n = d.g.n, rwp = d.g.rwp, cols = d.cols;
@@ -1428,6 +1430,8 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
     const int out_base = d.meta[col].base;
     const int v0 = mi.base + 1, v1 = mi.base + 2;  // values of the slots' marks
     const uint32_t keep0 = v0 < kMaxRound ? FULL_MASK : 0u, keep1 = v1 < kMaxRound ? FULL_MASK : 0u;
+    const uint32_t lm = 1u << lane;
+    const uint8_t b1 = (uint8_t)(1 | (v1 << 1)), b0 = (uint8_t)(1 | (v0 << 1));
     const bool mine = w0 < rwp;                    // rows of 12 words: the last lane has none
     Words<NW> vm;
 #pragma unroll
@@ -1463,21 +1467,14 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
         }
         const int dc = c0 - h[M - 1];              // the tile's first configuration, from that one
         uint32_t* const mcol = d.marked + ((size_t)col * d.C + first) * rwp + w0;
-        bool open[R];
-        bool some = false;
+        const int at = dc + li;                    // this lane's configuration, from the head's first
+        uint32_t* const mrow = mcol + (size_t)at * rwp;
+        Words<NW> m = vm;
+        if (mine && at >= 0 && c0 + li < n) m.load(mrow);
+        bool open = false;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int at = dc + r * CH + li;       // this lane's configuration, from the head's first
-            open[r] = false;
-            if (mine && at >= 0 && c0 + r * CH + li < n) {
-                Words<NW> m;
-                m.load(mcol + (size_t)at * rwp);
-#pragma unroll
-                for (int i = 0; i < NW; ++i) open[r] |= m.w[i] != vm.w[i];
-            }
-            some |= open[r];
-        }
-        if (!__any_sync(FULL_MASK, some)) continue;
+        for (int i = 0; i < NW; ++i) open |= m.w[i] != vm.w[i];
+        if (!__any_sync(FULL_MASK, open)) continue;
         uint32_t lo[M], dg[M], T = 1;
 #pragma unroll
         for (int i = 0; i < M; ++i) {
@@ -1485,13 +1482,13 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
             dg[i] = CR_LDG(&rp[h[i] + 1]) - lo[i];
             T *= dg[i];
         }
-        Words<NW> a0[R], a1[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            a0[r].zero();
-            a1[r].zero();
-        }
-        const uint32_t row0 = (uint32_t)(c0 + li);
+        Words<NW> a0, a1;
+        a0.zero();
+        a1.zero();
+        // a lane whose words are all marked reads the buffer's first words, the same as every other
+        // such lane: the loads need no branch and stay in flight together
+        const uint32_t* const mybase = open ? h1 + (size_t)(c0 + li) * rs : h1;
+        const uint32_t stride = open ? rs : 0u;
         for (uint32_t t0 = 0; t0 < T; t0 += 32) {
             uint32_t q = 0;                        // this lane's successor head
             if (t0 + lane < T) {
@@ -1506,53 +1503,50 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
                 sort_small<M>(x);
                 q = head_index<M>(x) * (uint32_t)n;
             }
-            const int cnt = (int)min(32u, T - t0);
-#pragma unroll 4
-            for (int j = 0; j < cnt; ++j) {
-                const uint32_t* p = h1 + (uint64_t)(__shfl_sync(FULL_MASK, q, j) + row0) * rs;
+            const int last = (int)min(32u, T - t0) - 1;
+            if (two) {
+                for (int j = 0; j <= last; j += U) {   // (the last head again and again past the end)
+                    Words<NW> x[U], y[U];
 #pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    if (open[r]) {                 // (a lane whose words are all marked reads none)
-                        Words<NW> x;
-                        x.ldg(p + r * CH * rs);
-                        a0[r].orr(x);
-                        if (two) {
-                            x.ldg(p + r * CH * rs + rwp);
-                            a1[r].orr(x);
-                        }
+                    for (int k = 0; k < U; ++k) {
+                        const uint32_t* p = mybase + (uint64_t)__shfl_sync(FULL_MASK, q, min(j + k, last)) * stride;
+                        x[k].ldg(p);
+                        y[k].ldg(p + rwp);
                     }
+#pragma unroll
+                    for (int k = 0; k < U; ++k) {
+                        a0.orr(x[k]);
+                        a1.orr(y[k]);
+                    }
+                }
+            } else {
+                for (int j = 0; j <= last; j += U) {
+                    Words<NW> x[U];
+#pragma unroll
+                    for (int k = 0; k < U; ++k)
+                        x[k].ldg(mybase + (uint64_t)__shfl_sync(FULL_MASK, q, min(j + k, last)) * stride);
+#pragma unroll
+                    for (int k = 0; k < U; ++k) a0.orr(x[k]);
                 }
             }
         }
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
+        {
             // the lane's new marks: the lower slot's value wins
-            const int at = dc + r * CH + li;
-            uint32_t* mrow = mcol + (size_t)at * rwp;
-            uint32_t any0 = 0u, any1 = 0u;
-            Words<NW> m;
-            if (open[r]) {
-                m.load(mrow);
 #pragma unroll
-                for (int i = 0; i < NW; ++i) {
-                    a0[r].w[i] &= ~m.w[i] & vm.w[i] & keep0;
-                    a1[r].w[i] &= ~(m.w[i] | a0[r].w[i]) & vm.w[i] & keep1;
-                }
-                any0 = a0[r].any();
-                any1 = a1[r].any();
+            for (int i = 0; i < NW; ++i) {
+                a0.w[i] &= ~m.w[i] & vm.w[i] & keep0;
+                a1.w[i] &= ~(m.w[i] | a0.w[i]) & vm.w[i] & keep1;
             }
-            // (the words of a lane that is not open are zero: it has read nothing)
+            // (a lane that is not open has every valid word marked)
+            const uint32_t any0 = a0.any(), any1 = a1.any();
             bool newrow = (any0 | any1) != 0u;
             if (!__any_sync(FULL_MASK, newrow)) continue;
 #pragma unroll
             for (int o = 1; o < LQ; o <<= 1) newrow |= __shfl_xor_sync(FULL_MASK, (int)newrow, o) != 0;
             const uint32_t cid = first + (uint32_t)at;
-            int marks = 0, words = 0;
+            int marks = 0;
 #pragma unroll
-            for (int i = 0; i < NW; ++i) {
-                marks += __popc(a0[r].w[i] | a1[r].w[i]);
-                words += (a0[r].w[i] | a1[r].w[i]) != 0u;
-            }
+            for (int i = 0; i < NW; ++i) marks += __popc(a0.w[i] | a1.w[i]);
             t.cnt += marks;
             if (newrow && mine) {
                 if (any0) {
@@ -1568,11 +1562,11 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
                 uint32_t* frow = d.front + ((size_t)col * d.C + cid) * rs + w0;
                 Words<NW> z;
                 z.zero();
-                (v0 == out_base ? a0[r] : (v1 == out_base ? a1[r] : z)).store(frow);
-                (v0 == out_base + 1 ? a0[r] : (v1 == out_base + 1 ? a1[r] : z)).store(frow + rwp);
+                (v0 == out_base ? a0 : (v1 == out_base ? a1 : z)).store(frow);
+                (v0 == out_base + 1 ? a0 : (v1 == out_base + 1 ? a1 : z)).store(frow + rwp);
                 if (any0 | any1) {
-                    m.orr(a0[r]);
-                    m.orr(a1[r]);
+                    m.orr(a0);
+                    m.orr(a1);
                     m.store(mrow);
                 }
                 if (w0 == 0) {
@@ -1582,32 +1576,31 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
             }
             // table bytes (first + dc may lie before the head's first configuration: only lanes
             // with marks, which lie behind it, are written for)
-            if (by_words(marks, words)) {
-                uint8_t* base = d.table + (size_t)first * n * cols + col;
+            if (by_rows(marks, 2 * NW)) {   // (the words come by shuffle)
+                uint8_t* base = d.table + ((size_t)first * n + lane) * cols + col;
+                unsigned lanes = __ballot_sync(FULL_MASK, marks != 0);
+                while (lanes) {
+                    const int l = __ffs(lanes) - 1;
+                    lanes &= lanes - 1;
+                    uint8_t* to = base + ((uint32_t)(dc + l / LQ) * n + (l % LQ) * NW * 32) * cols;
 #pragma unroll
-                for (int i = 0; i < NW; ++i) {
-                    unsigned lanes = __ballot_sync(FULL_MASK, (a0[r].w[i] | a1[r].w[i]) != 0u);
-                    while (lanes) {
-                        const int l = __ffs(lanes) - 1;
-                        lanes &= lanes - 1;
-                        const uint32_t x0 = __shfl_sync(FULL_MASK, a0[r].w[i], l), x1 = __shfl_sync(FULL_MASK, a1[r].w[i], l);
-                        const uint32_t off = ((uint32_t)(dc + r * CH + l / LQ) * n + ((l % LQ) * NW + i) * 32) * cols;
-                        store_word(base + off, x1, x0, v1, v0, cols, lane);
-                    }
+                    for (int i = 0; i < NW; ++i)
+                        store_word(to + i * 32 * cols, __shfl_sync(FULL_MASK, a1.w[i], l),
+                                   __shfl_sync(FULL_MASK, a0.w[i], l), lm, b1, b0);
                 }
             } else if (any0 | any1) {
                 uint8_t* trow = d.table + ((size_t)cid * n + w0 * 32) * cols + col;
 #pragma unroll
                 for (int i = 0; i < NW; ++i) {
-                    uint32_t b = a0[r].w[i] | a1[r].w[i];
+                    uint32_t b = a0.w[i] | a1.w[i];
                     while (b) {
                         const int j = __ffs(b) - 1;
                         b &= b - 1;
-                        trow[(size_t)(i * 32 + j) * cols] = (uint8_t)(1 | (((a0[r].w[i] >> j) & 1u ? v0 : v1) << 1));
+                        trow[(size_t)(i * 32 + j) * cols] = ((a0.w[i] >> j) & 1u) ? b0 : b1;
                     }
                 }
             }
-            // list the new rows: one atomic per R rows' load
+            // list the new rows: one atomic per unit
             const bool put = newrow && mine && w0 == 0;
             const unsigned nb = __ballot_sync(FULL_MASK, put);
             int list_at = 0;
@@ -2469,8 +2462,9 @@ __device__ CR_BODY_INLINE void and_tile_body(const V1Dev& d, int col, unsigned w
     const int so1 = v1 - out_base, so0 = v0 - out_base;
     const uint32_t keep1 = v1 < kMaxRound ? FULL_MASK : 0u, keep0 = two && v0 < kMaxRound ? FULL_MASK : 0u;
     uint2* sx = reinterpret_cast<uint2*>(reinterpret_cast<uint4*>(sm) + warp * and_tile_quads(rw));
-    uint32_t* sn1 = reinterpret_cast<uint32_t*>(sx + rw * 32 + 2) + lane;
-    uint32_t* sn0 = sn1 + rw * 32;
+    uint2* sn = sx + rw * 32 + 2 + lane;    // per (word, lane): marks of the higher and the lower slot
+    const uint32_t lm = 1u << lane;
+    const uint8_t b1 = (uint8_t)(1 | (v1 << 1)), b0 = (uint8_t)(1 | (v0 << 1));
     const uint16_t* CR_RESTRICT ell = d.g.ell + lane;
     const uint32_t* CR_RESTRICT ell_off = d.g.ell_off;
     const RowList rl(d, 0, mi);
@@ -2530,25 +2524,25 @@ __device__ CR_BODY_INLINE void and_tile_body(const V1Dev& d, int col, unsigned w
                 n1 = warp_transpose(n1, lane);
                 if (two) n0 = warp_transpose(n0, lane);
             }
-            sn1[w * 32] = n1;
-            sn0[w * 32] = n0;
+            sn[w * 32] = make_uint2(n1, n0);
         }
         if (!found) continue;
         // the row's lane again: mask with the open states
         uint32_t* mrow = d.marked + ((size_t)col * d.C + cid) * rwp;
         uint32_t any1 = 0u, any0 = 0u;
-        int marks = 0, words = 0;
+        int marks = 0;
         if (valid) {
             for (int w = 0; w < rw; ++w) {
-                const uint32_t mc = mrow[w], n1 = sn1[w * 32] & ~mc, n0 = sn0[w * 32] & ~mc;
-                sn1[w * 32] = n1;
-                sn0[w * 32] = n0;
-                any1 |= n1;
-                any0 |= n0;
-                if (n1 | n0) {
-                    mrow[w] = mc | n1 | n0;
-                    marks += __popc(n1 | n0);
-                    ++words;
+                const uint32_t mc = mrow[w];
+                uint2 x = sn[w * 32];
+                x.x &= ~mc;
+                x.y &= ~mc;
+                sn[w * 32] = x;
+                any1 |= x.x;
+                any0 |= x.y;
+                if (x.x | x.y) {
+                    mrow[w] = mc | x.x | x.y;
+                    marks += __popc(x.x | x.y);
                 }
             }
         }
@@ -2567,47 +2561,46 @@ __device__ CR_BODY_INLINE void and_tile_body(const V1Dev& d, int col, unsigned w
             }
             uint32_t* frow = d.front + ((size_t)col * d.C + cid) * S * rwp;
             for (int so = 0; so < S; ++so) {
-                const uint32_t* src = so == so1 ? sn1 : (two && so == so0 ? sn0 : nullptr);
+                const uint32_t* src = so == so1 ? &sn->x : (two && so == so0 ? &sn->y : nullptr);   // (stride 64)
                 if (vec4) {
                     for (int w = 0; w < rwp; w += 4) {
                         uint4 x = make_uint4(0u, 0u, 0u, 0u);
                         if (src) {
-                            x.x = src[w * 32];
-                            if (w + 1 < rw) x.y = src[(w + 1) * 32];
-                            if (w + 2 < rw) x.z = src[(w + 2) * 32];
-                            if (w + 3 < rw) x.w = src[(w + 3) * 32];
+                            x.x = src[w * 64];
+                            if (w + 1 < rw) x.y = src[(w + 1) * 64];
+                            if (w + 2 < rw) x.z = src[(w + 2) * 64];
+                            if (w + 3 < rw) x.w = src[(w + 3) * 64];
                         }
                         *reinterpret_cast<uint4*>(frow + so * rwp + w) = x;
                     }
                 } else {
-                    for (int w = 0; w < rwp; ++w) frow[so * rwp + w] = src && w < rw ? src[w * 32] : 0u;
+                    for (int w = 0; w < rwp; ++w) frow[so * rwp + w] = src && w < rw ? src[w * 64] : 0u;
                 }
             }
             d.fflag[(size_t)col * d.C + cid] = 1;
             t.rows++;
         }
-        if (by_words(marks, words)) {
+        if (by_rows(marks, rw)) {
             __syncwarp();
-            for (int w = 0; w < rw; ++w) {
-                const uint32_t* row1 = sn1 - lane + w * 32;
-                unsigned rows = __ballot_sync(FULL_MASK, valid && (sn1[w * 32] | sn0[w * 32]) != 0u);
-                while (rows) {
-                    const int i = __ffs(rows) - 1;
-                    rows &= rows - 1;
-                    const uint32_t id = __shfl_sync(FULL_MASK, cid, i);
-                    store_word(d.table + ((size_t)id * n + w * 32) * cols + col, row1[i], row1[rw * 32 + i], v1, v0, cols, lane);
-                }
+            unsigned rows = __ballot_sync(FULL_MASK, newrow);
+            while (rows) {
+                const int i = __ffs(rows) - 1;
+                rows &= rows - 1;
+                uint8_t* at = d.table + ((size_t)__shfl_sync(FULL_MASK, cid, i) * n + lane) * cols + col;
+                const uint2* row = sn - lane + i;
+#pragma unroll 4
+                for (int w = 0; w < rw; ++w, at += 32 * cols) store_word(at, row[w * 32].x, row[w * 32].y, lm, b1, b0);
             }
             __syncwarp();
         } else if (newrow) {
             uint8_t* trow = d.table + (size_t)cid * n * cols + col;
             for (int w = 0; w < rw; ++w) {
-                const uint32_t n1 = sn1[w * 32];
-                uint32_t b = n1 | sn0[w * 32];
+                const uint2 x = sn[w * 32];
+                uint32_t b = x.x | x.y;
                 while (b) {
                     const int j = __ffs(b) - 1;
                     b &= b - 1;
-                    trow[(size_t)(w * 32 + j) * cols] = (uint8_t)(1 | (((n1 >> j) & 1u ? v1 : v0) << 1));
+                    trow[(size_t)(w * 32 + j) * cols] = ((x.x >> j) & 1u) ? b1 : b0;
                 }
             }
         }
