@@ -1276,9 +1276,11 @@ struct Words {
 // clear counts as empty), then every H1 row of the head is the OR of the staged rows of N(c), and
 // the head's rows are written as one contiguous stretch.  A thread handles NW words of a row in
 // both value slots.  Inserting z at position i of a head splits the rank into a constant of
-// (head, i) and a term of (i, z), so a row's rank is one table entry and one add.
+// (head, i) and a term of (i, z), so a row's rank is one table entry and one add.  The next round's
+// rows are copied to a second buffer (cp.async) while this round's are combined: one barrier a round.
 // Bound: issue and shared-memory reads; both planes stay in L2 up to n of about 128.  Per launch:
-// G(n, p) n = 128 42 us with a rank per unit, 35 us so; Delaunay n = 389 4.9 and 3.4 ms.
+// G(n, p) n = 128 42 us with a rank per unit, 29 us so; Delaunay n = 199 224 and 142 us, n = 389 4.9
+// and 2.35 ms (167 us and 3.2 ms with the rows staged through registers between two barriers).
 __host__ __device__ constexpr int lane_words(int RW) { return RW < 4 ? RW : 4; }
 __host__ __device__ constexpr int row_lanes(int RW) { return RW <= 4 ? 1 : (RW <= 8 ? 2 : 4); }
 // Heads per round of a block, and the body's words of shared memory.
@@ -1288,15 +1290,28 @@ __host__ __device__ inline int heads_per_round(int threads, int n, int rwp) {
     return h < 1 ? 1 : (h > 32 ? 32 : h);
 }
 __host__ __device__ inline int head_smem_words(int threads, int k, int n, int rwp) {
-    return rank_table_words(k, n) + heads_per_round(threads, n, rwp) * n * 2 * rwp;
+    return rank_table_words(k, n) + 2 * heads_per_round(threads, n, rwp) * n * 2 * rwp;
+}
+
+// Copies NW words (4, 8 or 16 bytes, aligned so) from global to shared memory without registers, or
+// clears them when `live` is false; complete after copies_done().
+template <int NW>
+__device__ __forceinline__ void copy_words(uint32_t* dst, const uint32_t* src, bool live) {
+    const unsigned to = (unsigned)__cvta_generic_to_shared(dst);
+    const int bytes = live ? NW * 4 : 0;
+    if (NW == 4) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(src), "r"(bytes) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(to), "l"(src), "n"(NW * 4), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copies_done() {
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
 }
 
 template <int K, int RW>
 __device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned wk, unsigned nwk) {
     extern __shared__ __align__(16) uint32_t sm[];
     constexpr int M = K - 1, NW = lane_words(RW), LQ = row_lanes(RW);
-    __shared__ uint16_t s_head[32][M];
-    __shared__ uint32_t s_rank[32][K];
+    __shared__ uint16_t s_head[2][32][M];
+    __shared__ uint32_t s_rank[2][32][K];
     const int n = d.g.n, rwp = d.g.rwp, np1 = n + 1;
     const ColMeta mi = d.meta[nx];
     if (!d.h1 || mi.hi < mi.lo || mi.seed || frontier_sparse(d, mi)) return;
@@ -1320,68 +1335,88 @@ __device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned w
     // a warp spread over all the banks)
     const uint32_t plane = (uint32_t)(PR * n) * rwp;
     unsigned err = 0;
-    for (uint32_t q0 = wk * PR; q0 < P; q0 += nwk * PR) {
-        const int np = (int)min((uint32_t)PR, P - q0);
-        if ((int)threadIdx.x < np) {
-            int h[M];
-            head_of<M>(q0 + threadIdx.x, h);
-            // position i: sum over j < i of B[j][h_{j-1}] - B[j][h_j], then B[i][h_{i-1}], then
-            // -B[i+1][h_i], then sum over j > i of B[j+1][h_{j-1}] - B[j+1][h_j]
+    // the constants of a round's heads
+    auto open_round = [&](uint32_t q0, int buf) {
+        if (q0 >= P || threadIdx.x >= min((uint32_t)PR, P - q0)) return;
+        int h[M];
+        head_of<M>(q0 + threadIdx.x, h);
+        // position i: sum over j < i of B[j][h_{j-1}] - B[j][h_j], then B[i][h_{i-1}], then
+        // -B[i+1][h_i], then sum over j > i of B[j+1][h_{j-1}] - B[j+1][h_j]
 #pragma unroll
-            for (int i = 0; i < K; ++i) {
-                uint32_t r = CR_LDG(&d.binom[i * np1 + (i ? h[i ? i - 1 : 0] : 0)]);
+        for (int i = 0; i < K; ++i) {
+            uint32_t r = CR_LDG(&d.binom[i * np1 + (i ? h[i ? i - 1 : 0] : 0)]);
 #pragma unroll
-                for (int j = 0; j < M; ++j) {
-                    if (j < i) r += CR_LDG(&d.binom[j * np1 + (j ? h[j ? j - 1 : 0] : 0)]) - CR_LDG(&d.binom[j * np1 + h[j]]);
-                    else if (j == i) r -= CR_LDG(&d.binom[(j + 1) * np1 + h[j]]);
-                    else r += CR_LDG(&d.binom[(j + 1) * np1 + h[j - 1 < 0 ? 0 : j - 1]]) - CR_LDG(&d.binom[(j + 1) * np1 + h[j]]);
-                }
-                s_rank[threadIdx.x][i] = r;
+            for (int j = 0; j < M; ++j) {
+                if (j < i) r += CR_LDG(&d.binom[j * np1 + (j ? h[j ? j - 1 : 0] : 0)]) - CR_LDG(&d.binom[j * np1 + h[j]]);
+                else if (j == i) r -= CR_LDG(&d.binom[(j + 1) * np1 + h[j]]);
+                else r += CR_LDG(&d.binom[(j + 1) * np1 + h[j - 1 < 0 ? 0 : j - 1]]) - CR_LDG(&d.binom[(j + 1) * np1 + h[j]]);
             }
-#pragma unroll
-            for (int i = 0; i < M; ++i) s_head[threadIdx.x][i] = (uint16_t)h[i];
+            s_rank[buf][threadIdx.x][i] = r;
         }
-        __syncthreads();
-        if (mine) {
-            int j = 0, z = first;
-            for (int i = first; i < np * n; i += per_it, z += per_it) {
+#pragma unroll
+        for (int i = 0; i < M; ++i) s_head[buf][threadIdx.x][i] = (uint16_t)h[i];
+    };
+    // the copies of a round's frontier rows, four rows' flags in flight at a time
+    auto stage_round = [&](uint32_t q0, int buf) {
+        if (q0 >= P || !mine) return;
+        const int rows = (int)min((uint32_t)PR, P - q0) * n;
+        uint32_t* to = stage + (uint32_t)buf * 2u * plane;
+        int j = 0, z = first;
+        for (int i0 = first; i0 < rows; i0 += 4 * per_it) {
+            uint32_t id[4];
+            bool live[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                id[u] = 0;
+                live[u] = false;
+                if (i0 + u * per_it >= rows) continue;
                 while (z >= n) {
                     z -= n;
                     ++j;
                 }
                 int pos = 0;
 #pragma unroll
-                for (int q = 0; q < M; ++q) pos += z >= (int)s_head[j][q];
-                uint32_t s = s_rank[j][pos] + sD[pos * np1 + z];
-                const bool bad = s >= d.C;
-                if (bad) {
+                for (int q = 0; q < M; ++q) pos += z >= (int)s_head[buf][j][q];
+                id[u] = s_rank[buf][j][pos] + sD[pos * np1 + z];
+                if (id[u] >= d.C) {
                     err |= kErrRank;
-                    s = 0;
+                    id[u] = 0;
+                } else {
+                    live[u] = CR_LDG(&fflag_in[id[u]]) != 0;
                 }
-                const bool live = CR_LDG(&fflag_in[s]) != 0 && !bad;
-                const uint32_t* src = fin + (size_t)s * rs + w0;
-                uint32_t* dst = stage + (uint32_t)i * rwp + w0;
-                Words<NW> x;
-                x.ldg(src);
-                if (!live) x.zero();
-                x.store(dst);
-                if (two) {
-                    x.ldg(src + rwp);
-                    if (!live) x.zero();
-                    x.store(dst + plane);
-                }
+                z += per_it;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int i = i0 + u * per_it;
+                if (i >= rows) break;
+                const uint32_t* src = fin + (size_t)id[u] * rs + w0;
+                uint32_t* dst = to + (uint32_t)i * rwp + w0;
+                copy_words<NW>(dst, src, live[u]);
+                if (two) copy_words<NW>(dst + plane, src + rwp, live[u]);
             }
         }
-        __syncthreads();
+    };
+    open_round(wk * PR, 0);
+    __syncthreads();
+    stage_round(wk * PR, 0);
+    int buf = 0;
+    for (uint32_t q0 = wk * PR; q0 < P; q0 += nwk * PR, buf ^= 1) {
+        const int np = (int)min((uint32_t)PR, P - q0);
+        open_round(q0 + nwk * PR, buf ^ 1);
+        copies_done();
+        __syncthreads();   // this round's rows and the next one's constants are there, and the other rows are free
+        stage_round(q0 + nwk * PR, buf ^ 1);
         if (mine) {
             uint32_t* out = d.h1 + (size_t)q0 * n * rs + w0;
+            const uint32_t* from = stage + (uint32_t)buf * 2u * plane + w0;
             int j = 0, c = first;
             for (int i = first; i < np * n; i += per_it, c += per_it) {
                 while (c >= n) {
                     c -= n;
                     ++j;
                 }
-                const uint32_t* sj = stage + (uint32_t)(j * n) * rwp + w0;
+                const uint32_t* sj = from + (uint32_t)(j * n) * rwp;
                 Words<NW> a0, a1, x;
                 a0.zero();
                 a1.zero();
@@ -1400,6 +1435,8 @@ __device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned w
             }
         }
     }
+    copies_done();
+    __syncthreads();
     err = __reduce_or_sync(FULL_MASK, err);
     if ((threadIdx.x & 31) == 0 && err) atomicOr(d.err, err);
 }
