@@ -45,7 +45,8 @@
 // with a fresh table.
 //
 // Measured (Delaunay n = 199, k = 2, p = 3, six passes): 94 ms with every dirty depth-1 node's
-// children in the hash table and every leaf's cloud expanded, 10 ms so.
+// children in the hash table and every leaf's cloud expanded, 8.7 ms so (10.0 ms without the limit of
+// 64 registers, 9.5 ms at 48).
 #include <algorithm>
 #include <string>
 #include <vector>
@@ -523,7 +524,7 @@ __global__ void __launch_bounds__(256) k_v2_unsafe(V2Dev d) {
 // lane's cloud.  Values are final once found (see the head of this file): later passes look at
 // the open nodes only.
 template <int K, int W>
-__global__ void __launch_bounds__(256) k_v2_plain(V2Dev d) {
+__global__ void __launch_bounds__(256, 4) k_v2_plain(V2Dev d) {
     extern __shared__ uint32_t snbr[];
     load_graph(d, snbr);
     const int lane = threadIdx.x & 31;
@@ -596,7 +597,7 @@ __global__ void __launch_bounds__(256) k_v2_plain(V2Dev d) {
 // depth-1 nodes that are still open, plain ones (k_v2_plain) left out: a warp per configuration,
 // its touched robbers one by one, lanes over the cop moves.
 template <int K, int W>
-__global__ void __launch_bounds__(256) k_v2_hinsert(V2Dev d) {
+__global__ void __launch_bounds__(256, 4) k_v2_hinsert(V2Dev d) {
     extern __shared__ uint32_t snbr[];
     load_graph(d, snbr);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -652,7 +653,7 @@ __global__ void __launch_bounds__(256) k_v2_hinsert(V2Dev d) {
 // Delaunay graph of 199 vertices), so each warp gathers the taken ones of its stretch in shared
 // memory and evaluates 32 at a time, a lane each: 1.70 ms a thread per slot, 0.61 ms so (largest pass of that solve).
 template <int K, int W>
-__global__ void __launch_bounds__(256) k_v2_heval(V2Dev d) {
+__global__ void __launch_bounds__(256, 4) k_v2_heval(V2Dev d) {
     extern __shared__ uint32_t snbr[];
     __shared__ uint64_t s_slots[8][64];
     load_graph(d, snbr);
@@ -700,7 +701,7 @@ __global__ void __launch_bounds__(256) k_v2_heval(V2Dev d) {
 // the touched robbers one by one, lanes over the successors: a plain child's value, or the cloud
 // table's, or the node evaluated in place.
 template <int K, int W>
-__global__ void __launch_bounds__(256) k_v2_val1(V2Dev d) {
+__global__ void __launch_bounds__(256, 4) k_v2_val1(V2Dev d) {
     extern __shared__ uint32_t snbr[];
     load_graph(d, snbr);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
