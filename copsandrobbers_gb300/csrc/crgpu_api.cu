@@ -33,6 +33,8 @@ void launch_popcount(const uint32_t* plane, size_t words, unsigned long long* ou
                      cudaStream_t st);
 int max_cop_blocks_per_sm(int k, int rwp, int S);
 bool pull_supported(int S, int rwp);
+int small_team(const V1Dev& d, double avg_deg);
+cudaError_t launch_small_run(const V1Dev& d, const LoopCtl& c, int first, int passes, bool p1, int team, cudaStream_t st);
 int cop_launches(int direct);
 int cop_launches_k(int direct, bool sep);
 size_t cop_smem_bytes(int S, int rwp);
@@ -809,16 +811,30 @@ static int v1_advance(cr_solver* s, size_t passes, size_t ahead) {
     cudaStream_t st = ctx->stream;
     CR_CUDA(ctx, cudaEventRecord(s->kit.ev[0], st));
     const bool first = s->init_pending;
-    s->kit.pinned[0] = kHistEmpty;
+    const int team = ctx->profiling ? 0 : small_team(dev_view(s), (double)s->h_ccol.size() / s->n);
+    if (team) passes = std::min<size_t>(passes, kHistRing);
+    for (size_t i = 0; i < (team ? passes : 1); ++i) s->kit.pinned[i] = kHistEmpty;
     if (first) {
         if (int rc = v1_init_pass1(s)) return rc;
     }
     const LoopCtl loop{s->kit.pinned, &s->d_ctl->hist_n, kHistRing};
-    launch_loop_enter(dev_view(s), loop, first ? 1 : 0, s->grid_small, st);
-    CR_CUDA(ctx, cudaGetLastError());
     size_t sent = first ? 1 : 0, got = 0, lead = ahead ? 1 : 0;
     unsigned long long f = 0;
-    while (got < passes && !s->finished) {
+    if (team) {   // all of them in one launch
+        CR_CUDA(ctx, launch_small_run(dev_view(s), loop, first ? 1 : 0, (int)passes, s->p == 1, team, st));
+        CR_CUDA(ctx, cudaStreamSynchronize(st));
+        for (; got < passes && !s->finished; ++got) {
+            f = s->kit.pinned[got];
+            if (f == kHistEmpty) return fail(ctx, CR_ERR_INTERNAL, "a pass recorded nothing");
+            if (f & kHistError) break;
+            s->pass_counts.push_back(f);
+            s->finished = f == 0;
+        }
+    } else {
+        launch_loop_enter(dev_view(s), loop, first ? 1 : 0, s->grid_small, st);
+        CR_CUDA(ctx, cudaGetLastError());
+    }
+    while (!team && got < passes && !s->finished) {
         for (; sent < passes && sent < got + 1 + lead; ++sent) {
             s->kit.pinned[sent % kHistRing] = kHistEmpty;
             if (int rc = v1_enqueue_pass(s, loop)) return rc;
@@ -840,7 +856,8 @@ static int v1_advance(cr_solver* s, size_t passes, size_t ahead) {
     int per_pass = 0;
     for (int col = 0; col < s->cols; ++col)
         per_pass += col % 2 == 0 ? cop_launches_k(0, s->d_h1 != nullptr && (s->forms & CR_FORM_SEPARABLE)) : (col < s->cols - 1 ? cop_launches(1) : 1);
-    s->stats.kernel_launches += (int64_t)per_pass * (int64_t)(sent - (first ? 1 : 0)) + 1;   // and k_loop_enter
+    // (and k_loop_enter, or the small solve's one launch)
+    s->stats.kernel_launches += (int64_t)per_pass * (int64_t)(sent - (first ? 1 : 0)) + 1;
     s->stats.passes = (int)s->pass_counts.size();
     if (f & kHistError) {
         if (f & kErrRank) return fail(ctx, CR_ERR_INTERNAL, "successor rank out of range");

@@ -38,6 +38,7 @@
 #include "../../include/crgpu.h"
 #include "crgpu_ctx.h"
 #include "crgpu_v1_body.cuh"
+#include "crgpu_team.cuh"
 
 namespace crgpu {
 
@@ -69,22 +70,6 @@ struct BatchDev {
     cr_batch_result* res;
     unsigned long long* cta_time;  // per block: globaltimer at start and after its last graph
     uint32_t smem_words;           // dynamic shared memory of the launch
-};
-
-// The blocks solving one graph together: one, or a thread-block cluster.
-struct Team {
-    unsigned rank, size;
-    // Every thread of the team, with the memory effects of __syncthreads over all of it (the cluster
-    // barrier's arrive releases and its wait acquires at cluster scope).
-    __device__ __forceinline__ void sync() const {
-        __syncthreads();
-        if (size > 1) {
-            asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
-            asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
-        }
-    }
-    __device__ __forceinline__ unsigned thread() const { return rank * blockDim.x + threadIdx.x; }
-    __device__ __forceinline__ unsigned threads() const { return size * blockDim.x; }
 };
 
 __device__ __forceinline__ unsigned long long global_ns() {
@@ -523,8 +508,7 @@ template <bool P1, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) k_batch(BatchDev b) {
     __shared__ int s_job;
     Team tm;
-    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(tm.rank));
-    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(tm.size));
+    tm.of_cluster();
     const unsigned team = blockIdx.x / tm.size;
     unsigned char* slot = b.slots + (size_t)team * b.team_bytes;
     if (threadIdx.x == 0) b.cta_time[2 * blockIdx.x] = b.cta_time[2 * blockIdx.x + 1] = global_ns();
