@@ -230,7 +230,9 @@ static void launch_cop_ng(const V1Dev& d, int col, int nx, int grid, cudaStream_
     if (sma > 40 * 1024) raise_smem_limit((const void*)k_cop_a<K, NWP, G>, sma);   // (plus the static part)
     launch_pass_kernel(k_cop_a<K, NWP, G>, grid, sma, st, d, col, nx);
     if (!d.h1) launch_pass_kernel(k_cop_pull<K, NWP, G>, grid, smr, st, d, col, nx);
-    launch_pass_kernel(end ? k_cop_b_end<K, NWP, G> : k_cop_b<K, NWP, G>, grid, sm, st, d, col, nx);
+    // (three blocks of k_cop_b per SM are resident, four of the other kernels)
+    const int grid_b = grid - grid / 4;
+    launch_pass_kernel(end ? k_cop_b_end<K, NWP, G> : k_cop_b<K, NWP, G>, grid_b, sm, st, d, col, nx);
 }
 
 // Accumulator words and lanes per configuration, as the pull and the separable turn use them.
