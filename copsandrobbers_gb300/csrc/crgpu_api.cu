@@ -321,6 +321,23 @@ uint64_t cr_solver_footprint(int32_t n, int32_t k, int32_t p, int32_t rules) {
     return b;
 }
 
+}  // extern "C"
+
+namespace crgpu {
+// Bytes of cr_solver_footprint that a solve may lack and still run, or that the budget's head room
+// covers: the head rows of k = 2 and 4 (the solver does without where the device has no room), and
+// the plain values and unsafe rows of the v2 rules.  A server admits by the rest.
+uint64_t footprint_slack(int n, int k, int p, int rules) {
+    uint64_t C;
+    int cols, rw, rwp;
+    layout(n, k, p, rules, slots_for(n), &C, &cols, &rw, &rwp);
+    if (rules == CR_RULES_V2) return C * ((uint64_t)n + 4 * (uint64_t)rwp + 8);
+    return k == 3 ? 0 : h1_bytes(n, k, slots_for(n), rwp);
+}
+}  // namespace crgpu
+
+extern "C" {
+
 static void free_v1(cr_solver* s) {
     void* ptrs[] = {s->d_small, s->d_ctl, s->d_configs, s->d_table, s->d_marked, s->d_front, s->d_fflag, s->d_heads,
                     s->d_trans, s->d_cand, s->d_cbits, s->d_list, s->d_clist, s->d_h1};

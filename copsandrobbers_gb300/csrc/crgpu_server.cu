@@ -28,6 +28,10 @@
 
 #include "../../include/crgpu.h"
 
+namespace crgpu {
+uint64_t footprint_slack(int n, int k, int p, int rules);
+}  // namespace crgpu
+
 namespace {
 
 using Clock = std::chrono::steady_clock;
@@ -236,6 +240,9 @@ int cr_server_submit(cr_server* srv, const cr_graph* g, int32_t k, int32_t p, in
     r->footprint = cr_solver_footprint(g->n, k, p, rules);
     if (r->footprint == 0) return CR_ERR_INVALID;
     std::lock_guard<std::mutex> lock(srv->mu);
+    if (r->footprint > srv->budget &&
+        r->footprint - crgpu::footprint_slack(g->n, k, p, rules & ~(CR_COP_STAY | CR_ROBBER_STAY)) <= srv->budget)
+        r->footprint = srv->budget;
     if (r->footprint > srv->budget) {
         srv->err = "request footprint exceeds the server's memory budget";
         return CR_ERR_NOMEM;
