@@ -24,9 +24,9 @@
 // Clouds repeat heavily.  The robber moves first, so the depth-2 node below (C1, r) with cops C2
 // has the cloud N(N(r) \ C1 \ C2) \ C2: for every predecessor C1 of C2 that misses N(r) it is the
 // same plain node (C2, r).  So each pass goes
-//   k_v2_unsafe   per changed configuration C the vertices with a neighbour unmarked in row C: a
-//                 leaf at C is available when the cloud before the last robber ply misses them
-//                 (one AND, no expansion);
+//   k_v2_begin    per changed configuration C the vertices with a neighbour unmarked in row C (its
+//                 unsafe row): a leaf at C is available when the cloud before the last robber ply
+//                 misses them (one AND, no expansion);
 //   k_v2_plain    plain[C2][r], the values of the plain depth-2 nodes;
 //   k_v2_val1     val1[C1][r], the values of the depth-1 nodes (C1, N(r) \ C1): for the robbers
 //                 with no cop in N(r), the minimum of the rows plain[C2] over the successors C2;
@@ -489,16 +489,26 @@ __device__ __forceinline__ void load_graph(const V2Dev& d, uint32_t* snbr) {
     __syncthreads();
 }
 
-// Unsafe rows of the configurations that gained marks: bit v of row C set iff v has a neighbour
-// unmarked in row C.  A warp per configuration, a lane per vertex.
+// The begin of a pass, a warp per configuration: the counters and the flags of what this pass finds
+// are cleared, the last pass's changes become lev[0], and a changed configuration gets its unsafe
+// row (a lane per vertex): bit v of row C set iff v has a neighbour unmarked in row C.
 template <int W>
-__global__ void __launch_bounds__(256) k_v2_unsafe(V2Dev d) {
+__global__ void __launch_bounds__(256) k_v2_begin(V2Dev d, uint8_t* lev0, uint8_t* changed) {
     extern __shared__ uint32_t snbr[];
-    load_graph(d, snbr);
+    if (!d.first) load_graph(d, snbr);
+    if (blockIdx.x == 0 && threadIdx.x < 3) d.count[threadIdx.x] = 0ull;
     const int lane = threadIdx.x & 31;
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
     for (uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < d.C; c += nwarps) {
-        if (!d.lev[c]) continue;
+        const uint8_t ch = changed[c];
+        __syncwarp();
+        if (lane == 0) {
+            lev0[c] = ch;
+            changed[c] = 0;
+            d.fin1[c] = 0;
+            d.fin2[c] = 0;
+        }
+        if (d.first || !ch) continue;
         Mask<W> m;
 #pragma unroll
         for (int j = 0; j < W; ++j) m.w[j] = j < d.rwp ? __ldg(&d.marked[(size_t)c * d.rwp + j]) : 0u;
@@ -1116,7 +1126,6 @@ int v2_init(V2Solver* s, cr_solve_stats* stats, std::string* err) {
     V2_CUDA(cudaMemsetAsync(s->marked, 0, (size_t)s->C * s->rwp * 4, st));
     V2_CUDA(cudaMemsetAsync(s->newval, kV2None, (size_t)s->C * s->n, st));
     V2_CUDA(cudaMemsetAsync(s->val1, kV2None, (size_t)s->C * s->n, st));
-    V2_CUDA(cudaMemsetAsync(s->plain, kV2None, (size_t)s->C * s->n, st));
     V2_CUDA(cudaMemsetAsync(s->changed, 0, s->C, st));
     V2_CUDA(cudaMemsetAsync(s->counters, 0, 4 * sizeof(unsigned long long), st));
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 255) / 256, (uint64_t)s->num_sms * 4));
@@ -1160,11 +1169,6 @@ static int launch_v2_val1(V2Solver* s, V2Dev d, uint64_t lo, uint64_t hi, int gr
 template <int K, int W>
 static int launch_v2_kernels(V2Solver* s, const V2Dev& d, int grid_cfg, size_t sm) {
     int launches = 0;
-    if (!d.first) {
-        raise_smem_limit((const void*)k_v2_unsafe<W>, sm);
-        k_v2_unsafe<W><<<grid_cfg, 256, sm, s->st>>>(d);
-        ++launches;
-    }
     if (d.p >= 2) {
         raise_smem_limit((const void*)k_v2_plain<K, W>, sm);
         k_v2_plain<K, W><<<grid_cfg, 256, sm, s->st>>>(d);
@@ -1190,6 +1194,12 @@ static int launch_v2_k(V2Solver* s, const V2Dev& d, int W, int grid_cfg, size_t 
     }
 }
 
+template <int W>
+static void launch_v2_begin(const V2Solver* s, const V2Dev& d, int grid, size_t sm) {
+    raise_smem_limit((const void*)k_v2_begin<W>, sm);
+    k_v2_begin<W><<<grid, 256, sm, s->st>>>(d, s->lev, s->changed);
+}
+
 template <int K>
 static void launch_dilate(const V2Solver* s, const uint8_t* in, uint8_t* out, int grid) {
     k_v2_dilate<K><<<grid, 256, 0, s->st>>>(in, out, s->configs, s->C, s->n, s->rp, s->col, s->binom);
@@ -1198,11 +1208,20 @@ static void launch_dilate(const V2Solver* s, const uint8_t* in, uint8_t* out, in
 int v2_pass(V2Solver* s, uint64_t* found, cr_solve_stats* stats, std::string* err) {
     cudaStream_t st = s->st;
     V2_CUDA(cudaEventRecord(s->e0, st));
-    V2_CUDA(cudaMemsetAsync(s->counters, 0, 3 * sizeof(unsigned long long), st));
+    const V2Dev d = v2_view(s);
+    const size_t sm = (size_t)s->n * s->rwp * 4;
+    const uint64_t pairs = (uint64_t)s->C * s->n;
+    const int grid_cfg = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 7) / 8, (uint64_t)s->num_sms * 8));
     const int grid_cfg_small = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 255) / 256, (uint64_t)s->num_sms * 4));
-    int launches = 0;
+    int launches = 1;
+    switch (s->W) {
+        case 1: launch_v2_begin<1>(s, d, grid_cfg, sm); break;
+        case 2: launch_v2_begin<2>(s, d, grid_cfg, sm); break;
+        case 4: launch_v2_begin<4>(s, d, grid_cfg, sm); break;
+        case 8: launch_v2_begin<8>(s, d, grid_cfg, sm); break;
+        default: launch_v2_begin<16>(s, d, grid_cfg, sm); break;
+    }
     if (!s->first) {
-        V2_CUDA(cudaMemcpyAsync(s->lev, s->changed, s->C, cudaMemcpyDeviceToDevice, st));
         for (int j = 1; j < s->p; ++j) {
             const uint8_t* in = s->lev + (size_t)(j - 1) * s->C;
             uint8_t* out = s->lev + (size_t)j * s->C;
@@ -1215,14 +1234,7 @@ int v2_pass(V2Solver* s, uint64_t* found, cr_solve_stats* stats, std::string* er
             ++launches;
         }
     }
-    V2_CUDA(cudaMemsetAsync(s->changed, 0, s->C, st));
-    V2_CUDA(cudaMemsetAsync(s->fin1, 0, s->C, st));
-    V2_CUDA(cudaMemsetAsync(s->fin2, 0, s->C, st));
-    const V2Dev d = v2_view(s);
     s->first = false;
-    const size_t sm = (size_t)s->n * s->rwp * 4;
-    const uint64_t pairs = (uint64_t)s->C * s->n;
-    const int grid_cfg = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 7) / 8, (uint64_t)s->num_sms * 8));
     switch (s->k) {
         case 1: launches += launch_v2_k<1>(s, d, s->W, grid_cfg, sm); break;
         case 2: launches += launch_v2_k<2>(s, d, s->W, grid_cfg, sm); break;
