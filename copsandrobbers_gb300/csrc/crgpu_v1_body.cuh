@@ -2700,12 +2700,14 @@ __device__ __forceinline__ uint32_t piece_max(uint4 v, int lo, int hi) {
 // each stretch of the row), which on a graph the cops win is nearly always in the first stretch, so
 // that most of the table is never read (the whole of it at one coalesced row per warp took 5.96 ms
 // at Delaunay n = 389, k = 3, and 64 us at G(n, p) n = 128; this takes 0.39 ms and 52 us).
-// Two-column tables are read in 16-byte pieces whatever the rows' alignment, others byte by byte.
+// Two-column tables are read in 16-byte pieces whatever the rows' alignment, others byte by byte.  A
+// piece that the table only begins is not loaded: the states in it, which with rows shorter than a
+// piece belong to several of the last rows, are read one by one.
 __device__ CR_BODY_INLINE void verdict_body(const uint8_t* table, const uint32_t* m0, uint32_t C,
                                              int n, int rw, int rwp, int cols,
                                              unsigned long long* best, unsigned wk, unsigned nwk) {
     const size_t stride = (size_t)nwk * blockDim.x;
-    const uint8_t* const end = table + (size_t)C * n * cols;
+    const uint8_t* const whole = table + ((size_t)C * n * cols & ~(size_t)15);   // the end of the whole pieces
     const bool vec = cols == 2 && ((uintptr_t)table & 15u) == 0;
     for (size_t cid = (size_t)wk * blockDim.x + threadIdx.x; cid < C; cid += stride) {
         bool full = true;
@@ -2718,14 +2720,14 @@ __device__ CR_BODY_INLINE void verdict_body(const uint8_t* table, const uint32_t
         if (vec) {
             const int off = (int)((uintptr_t)row & 15u), bytes = off + 2 * n;   // the row in its pieces
             const uint8_t* p = row - off;
-            // four pieces at a time (their loads in flight together) while they lie in the table
+            // four pieces at a time (their loads in flight together)
             for (int at = 0; at < bytes && key() < cur; at += 64) {
                 uint4 v[4];
                 cur = *(volatile unsigned long long*)best;
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     v[k] = make_uint4(0u, 0u, 0u, 0u);
-                    if (at + 16 * k < bytes && p + at + 16 * k + 16 <= end)
+                    if (at + 16 * k < bytes && p + at + 16 * k < whole)
                         v[k] = *reinterpret_cast<const uint4*>(p + at + 16 * k);
                 }
 #pragma unroll
@@ -2734,8 +2736,7 @@ __device__ CR_BODY_INLINE void verdict_body(const uint8_t* table, const uint32_t
                     wc = max(wc, piece_max(v[k], max(0, off - b), min(16, max(0, bytes - b))) >> 1);
                 }
             }
-            if (row + 2 * n == end)   // the last row: its end may lie in a piece that the table only begins
-                for (const uint8_t* q = row; q < end; q += 2) wc = max(wc, (uint32_t)(*q >> 1));
+            for (const uint8_t* q = row < whole ? whole : row; q < row + 2 * n; q += 2) wc = max(wc, (uint32_t)(*q >> 1));
         } else {
             for (int r = 0; r < n && key() < cur; ++r) wc = max(wc, (uint32_t)(row[(size_t)r * cols] >> 1));
         }
