@@ -3,10 +3,14 @@
 // the stand-alone kernels pass (blockIdx.x, gridDim.x); the persistent batch kernel, where one
 // block owns a whole solve, passes (0, 1) and separates the bodies with __syncthreads.
 //
-// The including file defines CR_BODY_NS (the namespace of this instance), CR_LDG (a load of
-// data that does not change while the kernel runs), CR_RESTRICT and CR_BODY_INLINE.  Inside the persistent
-// batch kernel a block writes the very buffers it later reads (and reuses them job after job),
-// so there both are plain coherent loads; the stand-alone kernels use the read-only path.
+// The including file defines CR_BODY_NS (the namespace of this instance), CR_LDG (a load of what a
+// solve does not change: the graph, its masks and lists, the rank table, the configurations),
+// CR_RESTRICT and CR_BODY_INLINE.  In the stand-alone kernels CR_LDG is the read-only path.  What the
+// kernels of a pass write for one another (frontier rows and flags, row lists, head rows, candidate
+// and marked rows, the table) never goes through it or a restricted pointer: a kernel of a pass is
+// resident, and so alive, while the one before it still writes.  Inside the persistent batch kernel a
+// block writes the very buffers it later reads (and reuses them job after job), so there both are
+// plain coherent loads.
 #pragma once
 #include "crgpu_internal.cuh"
 
@@ -217,7 +221,7 @@ struct RowList {
     bool all;
     __device__ RowList(const V1Dev& d, int col, const ColMeta& m)
         : ids(d.list + (size_t)col * d.C), n(m.len < 0 ? d.C : (uint32_t)m.len), all(m.len < 0) {}
-    __device__ __forceinline__ uint32_t id(uint32_t i) const { return all ? i : CR_LDG(&ids[i]); }
+    __device__ __forceinline__ uint32_t id(uint32_t i) const { return all ? i : ids[i]; }
 };
 
 // initializeCaptures (k_cops_visibility.cpp:85-127): the table was memset to 0xFE; a robber
@@ -1019,8 +1023,8 @@ __device__ CR_BODY_INLINE void cop_pull_body(const V1Dev& d, int col, int nx, un
     __syncthreads();
     uint32_t* wacc = sm + rank_table_words(K, n) + (warp * CPW + L.grp) * (2 * S * rwp);
     uint32_t* wnew = wacc + S * rwp;
-    const uint32_t* CR_RESTRICT fin = d.front + (size_t)nx * d.C * S * rwp;
-    const uint8_t* CR_RESTRICT fflag_in = d.fflag + (size_t)nx * d.C;
+    const uint32_t* fin = d.front + (size_t)nx * d.C * S * rwp;
+    const uint8_t* fflag_in = d.fflag + (size_t)nx * d.C;
     const uint32_t* CR_RESTRICT rp = cop_rows(d.g);     // the cops' moves
     const uint16_t* CR_RESTRICT adj = cop_cols(d.g);
     const bool vec4 = (rwp & 3) == 0;
@@ -1100,13 +1104,13 @@ __device__ CR_BODY_INLINE void cop_pull_body(const V1Dev& d, int col, int nx, un
 #pragma unroll
                     for (int u = 0; u < U; ++u) {
                         if (!((ok >> u) & 1u)) continue;
-                        const uint32_t keep = CR_LDG(&fflag_in[s[u]]) ? 0xFFFFFFFFu : 0u;
+                        const uint32_t keep = fflag_in[s[u]] ? 0xFFFFFFFFu : 0u;
                         const uint32_t* row = fin + (size_t)s[u] * S * rwp;
                         if (vec4) {
 #pragma unroll
                             for (int w = 0; w < NWP; w += 4) {
                                 if (w < nwords) {
-                                    const uint4 x = CR_LDG(reinterpret_cast<const uint4*>(row + w));
+                                    const uint4 x = *reinterpret_cast<const uint4*>(row + w);
                                     acc[w] |= x.x & keep; acc[w + 1] |= x.y & keep;
                                     acc[w + 2] |= x.z & keep; acc[w + 3] |= x.w & keep;
                                 }
@@ -1114,7 +1118,7 @@ __device__ CR_BODY_INLINE void cop_pull_body(const V1Dev& d, int col, int nx, un
                         } else {
 #pragma unroll
                             for (int w = 0; w < NWP; ++w)
-                                if (w < nwords) acc[w] |= CR_LDG(row + w) & keep;
+                                if (w < nwords) acc[w] |= row[w] & keep;
                         }
                     }
                     continue;
@@ -1122,7 +1126,7 @@ __device__ CR_BODY_INLINE void cop_pull_body(const V1Dev& d, int col, int nx, un
                 unsigned live = 0;
 #pragma unroll
                 for (int u = 0; u < U; ++u)
-                    if (((ok >> u) & 1u) && CR_LDG(&fflag_in[s[u]])) live |= 1u << u;
+                    if (((ok >> u) & 1u) && fflag_in[s[u]]) live |= 1u << u;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                     if (!((live >> u) & 1u)) continue;
@@ -1131,14 +1135,14 @@ __device__ CR_BODY_INLINE void cop_pull_body(const V1Dev& d, int col, int nx, un
 #pragma unroll
                         for (int w = 0; w < NWP; w += 4) {
                             if (w < nwords) {
-                                const uint4 x = CR_LDG(reinterpret_cast<const uint4*>(row + w));
+                                const uint4 x = *reinterpret_cast<const uint4*>(row + w);
                                 acc[w] |= x.x; acc[w + 1] |= x.y; acc[w + 2] |= x.z; acc[w + 3] |= x.w;
                             }
                         }
                     } else {
 #pragma unroll
                         for (int w = 0; w < NWP; ++w)
-                            if (w < nwords) acc[w] |= CR_LDG(row + w);
+                            if (w < nwords) acc[w] |= row[w];
                     }
                 }
             }
@@ -1253,17 +1257,6 @@ struct Words {
             w[0] = p[0];
         }
     }
-    __device__ __forceinline__ void ldg(const uint32_t* p) {
-        if (NW == 4) {
-            const uint4 v = CR_LDG(reinterpret_cast<const uint4*>(p));
-            w[0] = v.x; w[NW > 1 ? 1 : 0] = v.y; w[NW > 2 ? 2 : 0] = v.z; w[NW > 3 ? 3 : 0] = v.w;
-        } else if (NW == 2) {
-            const uint2 v = CR_LDG(reinterpret_cast<const uint2*>(p));
-            w[0] = v.x; w[NW > 1 ? 1 : 0] = v.y;
-        } else {
-            w[0] = CR_LDG(p);
-        }
-    }
     __device__ __forceinline__ void store(uint32_t* p) const {
         if (NW == 4) *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[NW > 1 ? 1 : 0], w[NW > 2 ? 2 : 0], w[NW > 3 ? 3 : 0]);
         else if (NW == 2) *reinterpret_cast<uint2*>(p) = make_uint2(w[0], w[NW > 1 ? 1 : 0]);
@@ -1322,8 +1315,8 @@ __device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned w
         const uint32_t next = i + np1 < K * np1 ? CR_LDG(&d.binom[i + np1]) : 0u;
         sD[i] = next - CR_LDG(&d.binom[i]);
     }
-    const uint32_t* CR_RESTRICT fin = d.front + (size_t)nx * d.C * 2 * rwp;
-    const uint8_t* CR_RESTRICT fflag_in = d.fflag + (size_t)nx * d.C;
+    const uint32_t* fin = d.front + (size_t)nx * d.C * 2 * rwp;
+    const uint8_t* fflag_in = d.fflag + (size_t)nx * d.C;
     const uint32_t* CR_RESTRICT rp = cop_rows(d.g);
     const uint16_t* CR_RESTRICT adj = cop_cols(d.g);
     const uint32_t rs = 2u * rwp;              // words of a row (S = 2 slots wherever H1 exists)
@@ -1382,7 +1375,7 @@ __device__ CR_BODY_INLINE void head_rows_body(const V1Dev& d, int nx, unsigned w
                     err |= kErrRank;
                     id[u] = 0;
                 } else {
-                    live[u] = CR_LDG(&fflag_in[id[u]]) != 0;
+                    live[u] = fflag_in[id[u]] != 0;
                 }
                 z += per_it;
             }
@@ -1475,7 +1468,7 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
     for (int i = 0; i < NW; ++i) vm.w[i] = valid_mask(n, w0 + i);
     const uint32_t* CR_RESTRICT rp = cop_rows(d.g);
     const uint16_t* CR_RESTRICT adj = cop_cols(d.g);
-    const uint32_t* CR_RESTRICT h1 = d.h1 + w0;
+    const uint32_t* h1 = d.h1 + w0;
     const uint32_t rs = 2u * rwp;                  // words of a row (S = 2 slots wherever H1 exists)
     const int np1 = n + 1;
     Tally t;
@@ -1547,8 +1540,8 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
 #pragma unroll
                     for (int k = 0; k < U; ++k) {
                         const uint32_t* p = mybase + (uint64_t)__shfl_sync(FULL_MASK, q, min(j + k, last)) * stride;
-                        x[k].ldg(p);
-                        y[k].ldg(p + rwp);
+                        x[k].load(p);
+                        y[k].load(p + rwp);
                     }
 #pragma unroll
                     for (int k = 0; k < U; ++k) {
@@ -1561,7 +1554,7 @@ __device__ CR_BODY_INLINE void sep_pull_body(const V1Dev& d, int col, int nx, un
                     Words<NW> x[U];
 #pragma unroll
                     for (int k = 0; k < U; ++k)
-                        x[k].ldg(mybase + (uint64_t)__shfl_sync(FULL_MASK, q, min(j + k, last)) * stride);
+                        x[k].load(mybase + (uint64_t)__shfl_sync(FULL_MASK, q, min(j + k, last)) * stride);
 #pragma unroll
                     for (int k = 0; k < U; ++k) a0.orr(x[k]);
                 }
@@ -1991,7 +1984,7 @@ __device__ CR_BODY_INLINE void cop_push_body(const V1Dev& d, int col, int nx, un
     const int s_used = min(mi.hi - mi.base + 1, S);
     const int nwords = s_used * rwp;
     uint32_t* wrow = sm + warp * (S * rwp);
-    const uint32_t* CR_RESTRICT fin = d.front + (size_t)nx * d.C * S * rwp;
+    const uint32_t* fin = d.front + (size_t)nx * d.C * S * rwp;
     uint8_t* fflag_in = d.fflag + (size_t)nx * d.C;
     const uint32_t* CR_RESTRICT rrp = d.g.rrow_ptr;
     const uint16_t* CR_RESTRICT radj = d.g.rcol;
