@@ -33,6 +33,7 @@ void launch_popcount(const uint32_t* plane, size_t words, unsigned long long* ou
                      cudaStream_t st);
 int max_cop_blocks_per_sm(int k, int rwp, int S);
 bool pull_supported(int S, int rwp);
+int create_solver(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, int32_t rules, bool lean, cr_solver** out);
 int small_team(const V1Dev& d, double avg_deg);
 cudaError_t launch_small_run(const V1Dev& d, const LoopCtl& c, int first, int passes, bool p1, int team, cudaStream_t st);
 int cop_launches(int direct);
@@ -98,6 +99,7 @@ struct cr_solver {
     std::vector<uint32_t> h_crp;      // the cops' moves (with self-loops under CR_COP_STAY)
     std::vector<uint16_t> h_ccol;
     bool cop_stay = false, robber_stay = false;
+    bool lean = false;                // without what lean_footprint leaves out
     int cop_maxdeg = 0;
     uint32_t forms = CR_FORMS_ALL;    // cr_solver_set_forms
     uint32_t* d_crp = nullptr;        // set only when the two move graphs differ
@@ -282,10 +284,10 @@ static uint64_t h1_bytes(int n, int k, int S, int rwp) {
 }
 
 // The head rows of a solver.  k = 2 and 4 do without them (in the tuple-gathering form) where
-// the device has no room.
+// the device or the solver's footprint has no room.
 static cudaError_t alloc_h1(cr_solver* s) {
     const uint64_t hb = h1_bytes(s->n, s->k, s->S, s->rwp);
-    if (!hb) return cudaSuccess;
+    if (!hb || (s->lean && s->k != 3)) return cudaSuccess;
     const cudaError_t e = s->ctx->cache.get((void**)&s->d_h1, hb);
     if (e != cudaErrorMemoryAllocation || s->k == 3) return e;
     cudaGetLastError();
@@ -317,6 +319,7 @@ uint64_t cr_solver_footprint(int32_t n, int32_t k, int32_t p, int32_t rules) {
     b += (uint64_t)cols * C;                             // flags
     b += C * (uint64_t)k * 2;                            // configs
     b += (uint64_t)n * rwp * 4 * 3 + (uint64_t)k * (n + 1) * 4 + (1u << 16);
+    b += (uint64_t)n * rw * 64;                          // hop lists of the last column's tiles (at most)
     if (cols == 2) b += 2ull * n * (uint64_t)((n + 7) & ~7) * 4;   // first-pass cover masks
     return b;
 }
@@ -324,15 +327,15 @@ uint64_t cr_solver_footprint(int32_t n, int32_t k, int32_t p, int32_t rules) {
 }  // extern "C"
 
 namespace crgpu {
-// Bytes of cr_solver_footprint that a solve may lack and still run, or that the budget's head room
-// covers: the head rows of k = 2 and 4 (the solver does without where the device has no room), and
-// the plain values and unsafe rows of the v2 rules.  A server admits by the rest.
-uint64_t footprint_slack(int n, int k, int p, int rules) {
+// Bytes of a lean solve: without the head rows of k = 2 and 4 (the solver then gathers tuples), or the
+// plain values of the v2 rules (which are looked up where they are reached).  A server admits by it
+// what its budget cannot hold whole.
+uint64_t lean_footprint(int n, int k, int p, int rules) {
+    if (rules == CR_RULES_V2) return v2_lean_footprint(n, k, p);
     uint64_t C;
     int cols, rw, rwp;
     layout(n, k, p, rules, slots_for(n), &C, &cols, &rw, &rwp);
-    if (rules == CR_RULES_V2) return C * ((uint64_t)n + 4 * (uint64_t)rwp + 8);
-    return k == 3 ? 0 : h1_bytes(n, k, slots_for(n), rwp);
+    return cr_solver_footprint(n, k, p, rules) - (k == 3 ? 0 : h1_bytes(n, k, slots_for(n), rwp));
 }
 }  // namespace crgpu
 
@@ -546,8 +549,11 @@ static int alloc_v1(cr_solver* s, SmallArrays& small) {
     return CR_OK;
 }
 
-int cr_solver_create(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, int32_t rules,
-                     cr_solver** out) {
+}  // extern "C"
+
+// A solver for (g, k, p, rules); lean = one that holds lean_footprint bytes.
+int crgpu::create_solver(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, int32_t rules, bool lean,
+                         cr_solver** out) {
     if (!ctx || !g || !out) return CR_ERR_INVALID;
     *out = nullptr;
     if (g->n <= 0) return fail(ctx, CR_ERR_INVALID, "Graph is empty or failed to load.");
@@ -573,6 +579,7 @@ int cr_solver_create(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, i
     s->p = p;
     s->rules = base_rules;
     rules = base_rules;
+    s->lean = lean;
     s->cop_stay = (stay & CR_COP_STAY) != 0;
     s->robber_stay = (stay & CR_ROBBER_STAY) != 0;
     s->S = slots_for(g->n);
@@ -649,7 +656,7 @@ int cr_solver_create(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, i
         CR_TRY(small.upload(ctx->cache, &s->d_small, ctx->stream));
         int rc = crgpu::v2_create(&s->v2, &ctx->cache, s->kit, ctx->stream, ctx->num_sms, s->n, k, p, s->d_rp, s->d_col,
                                   s->h_rp.data(), s->h_col.data(), s->d_binom, s->d_configs,
-                                  (uint32_t)s->C, &ctx->err);
+                                  (uint32_t)s->C, lean, &ctx->err);
         if (rc) return bail(rc);
     }
     const int grid = (int)std::min<uint64_t>((s->C + 255) / 256, (uint64_t)ctx->num_sms * 8);
@@ -659,6 +666,13 @@ int cr_solver_create(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, i
     s->stats.slots = s->S;
     *out = s;
     return CR_OK;
+}
+
+extern "C" {
+
+int cr_solver_create(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, int32_t rules,
+                     cr_solver** out) {
+    return crgpu::create_solver(ctx, g, k, p, rules, false, out);
 }
 
 int cr_solver_destroy(cr_solver* s) {

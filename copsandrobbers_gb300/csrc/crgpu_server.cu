@@ -29,7 +29,8 @@
 #include "../../include/crgpu.h"
 
 namespace crgpu {
-uint64_t footprint_slack(int n, int k, int p, int rules);
+uint64_t lean_footprint(int n, int k, int p, int rules);
+int create_solver(cr_context* ctx, const cr_graph* g, int32_t k, int32_t p, int32_t rules, bool lean, cr_solver** out);
 }  // namespace crgpu
 
 namespace {
@@ -56,6 +57,7 @@ struct Request {
     std::vector<uint32_t> row_ptr;
     std::vector<uint16_t> col;
     uint64_t footprint = 0;
+    bool lean = false;            // footprint is lean_footprint: the whole one exceeds the budget
     State state = State::Queued;
     Clock::time_point t_submit, t_start, t_done;
     cr_request_result res{};
@@ -96,7 +98,7 @@ namespace {
 void run_request(cr_server* srv, cr_context* ctx, Request* r) {
     cr_graph g{r->n, r->row_ptr.data(), r->col.data()};
     cr_solver* s = nullptr;
-    int rc = cr_solver_create(ctx, &g, r->k, r->p, r->rules, &s);
+    int rc = crgpu::create_solver(ctx, &g, r->k, r->p, r->rules, r->lean, &s);
     uint64_t caps = 0;
     std::vector<uint64_t> counts(1 << 12);
     int32_t passes = 0;
@@ -240,9 +242,10 @@ int cr_server_submit(cr_server* srv, const cr_graph* g, int32_t k, int32_t p, in
     r->footprint = cr_solver_footprint(g->n, k, p, rules);
     if (r->footprint == 0) return CR_ERR_INVALID;
     std::lock_guard<std::mutex> lock(srv->mu);
-    if (r->footprint > srv->budget &&
-        r->footprint - crgpu::footprint_slack(g->n, k, p, rules & ~(CR_COP_STAY | CR_ROBBER_STAY)) <= srv->budget)
-        r->footprint = srv->budget;
+    if (r->footprint > srv->budget) {
+        r->lean = true;
+        r->footprint = crgpu::lean_footprint(g->n, k, p, rules & ~(CR_COP_STAY | CR_ROBBER_STAY));
+    }
     if (r->footprint > srv->budget) {
         srv->err = "request footprint exceeds the server's memory budget";
         return CR_ERR_NOMEM;

@@ -44,6 +44,11 @@
 // every pass; when the depth-1 nodes outnumber half the table, they are processed in chunks, each
 // with a fresh table.
 //
+// A lean solver (V2Solver::lean) has no plain values: every child of a depth-1 node is then looked at
+// where it is reached, as a touched node's are, and three byte arrays share the memory of others
+// (v2_create).  It serves requests that a memory budget would refuse otherwise; Delaunay n = 199,
+// k = 2, p = 3 takes 166 ms so.
+//
 // Measured (Delaunay n = 199, k = 2, p = 3, six passes): 94 ms with every dirty depth-1 node's
 // children in the hash table and every leaf's cloud expanded, 8.7 ms so (10.0 ms without the limit of
 // 64 registers, 9.5 ms at 48).
@@ -79,7 +84,8 @@ struct V2Solver {
     uint32_t* nbr = nullptr;
     uint8_t* val1 = nullptr;
     uint8_t* newval = nullptr;
-    uint8_t* plain = nullptr;       // [C][n] plain depth-2 values
+    bool lean = false;              // without the plain values
+    uint8_t* plain = nullptr;       // [C][n] plain depth-2 values; null = lean
     uint32_t* unsafe = nullptr;     // [C][rwp], rows of changed configurations only
     uint8_t* changed = nullptr;     // configurations that gained marks
     uint8_t* lev = nullptr;         // [p][C]: a changed configuration j cop steps away
@@ -116,7 +122,7 @@ struct V2Dev {
     const uint32_t* still;         // [rwp]: vertices with none
     uint8_t* val1;
     uint8_t* newval;
-    uint8_t* plain;
+    uint8_t* plain;                // null = lean: every depth-1 node counts as touched
     uint32_t* unsafe;
     const uint8_t* lev;            // [p][C]
     uint8_t* fin1;
@@ -454,13 +460,13 @@ __device__ __forceinline__ void cops_of(const V2Dev& d, uint32_t cid, int (&c)[K
 }
 
 // The robbers r whose neighbourhood one of the cops stands in (N(r) meets C), cops left out: their
-// depth-1 clouds N(r) \ C are not N(r) itself.
+// depth-1 clouds N(r) \ C are not N(r) itself.  Without plain values: all but the cops.
 template <int W, int K>
 __device__ __forceinline__ Mask<W> touched_robbers(const V2Dev& d, const int (&c)[K]) {
     Mask<W> e;
 #pragma unroll
     for (int j = 0; j < W; ++j) {
-        e.w[j] = 0u;
+        e.w[j] = d.plain ? 0u : valid_mask(d.n, j);
         if (j < d.rwp)
 #pragma unroll
             for (int i = 0; i < K; ++i) e.w[j] |= __ldg(&d.rnbr[c[i] * d.rwp + j]);
@@ -503,8 +509,10 @@ __global__ void __launch_bounds__(256) k_v2_begin(V2Dev d, uint8_t* lev0, uint8_
         const uint8_t ch = changed[c];
         __syncwarp();
         if (lane == 0) {
-            lev0[c] = ch;
-            changed[c] = 0;
+            if (lev0 != changed) {
+                lev0[c] = ch;
+                changed[c] = 0;
+            }
             d.fin1[c] = 0;
             d.fin2[c] = 0;
         }
@@ -638,7 +646,7 @@ __global__ void __launch_bounds__(256, 4) k_v2_hinsert(V2Dev d) {
                     int c2[K];
                     const uint32_t cid2 = move_target<K>(mv, t, d.col, d.binom, np1, c2);
                     if (cid2 >= d.C || (!d.first && !d.lev[(size_t)(d.p - 2) * d.C + cid2])) continue;
-                    if (plain_child<W, K>(nr, cops1, c2)) continue;
+                    if (d.plain && plain_child<W, K>(nr, cops1, c2)) continue;
                     Mask<W> mid = V1;
                     mask_clear<W, K>(mid, c2);
                     if (mask_empty<W>(mid)) continue;
@@ -799,7 +807,7 @@ __global__ void __launch_bounds__(256, 4) k_v2_val1(V2Dev d) {
                     int c2[K];
                     const uint32_t cid2 = move_target<K>(mv, t, d.col, d.binom, np1, c2);
                     if (cid2 >= d.C || (!d.first && !d.lev[(size_t)(d.p - 2) * d.C + cid2])) continue;
-                    if (plain_child<W, K>(nr, cops1, c2)) {
+                    if (d.plain && plain_child<W, K>(nr, cops1, c2)) {
                         best = min(best, (int)d.plain[(size_t)cid2 * d.n + r]);
                         continue;
                     }
@@ -988,6 +996,27 @@ uint64_t v2_footprint(int n, int k, int p) {
            hcap * (8 + 4 * (uint64_t)rwp) + (1u << 16);
 }
 
+// Of a lean solver (see v2_create): at most half of that, so much less that the table makes room for the
+// levels beyond the second (0 = none; a table of the least size stays).  A lean solver then holds no
+// more than three bytes a state, three a configuration, the marks and a table of the usual size.
+static uint64_t v2_lean_hash_capacity(uint64_t C, int n, int p, int rwp) {
+    const uint64_t full = v2_hash_capacity(C * n, p), slot = 8 + 4 * (uint64_t)rwp;
+    if (full <= 1024) return full;
+    uint64_t cap = full / 2;
+    while (cap && (full - cap) * slot < C * (uint64_t)(p - 2)) cap = cap > 1024 ? cap / 2 : 0;
+    return cap;
+}
+
+uint64_t v2_lean_footprint(int n, int k, int p) {
+    long double C = 1;
+    for (int i = 1; i <= k; ++i) C = C * (n + k - i) / i;
+    const uint64_t c = (uint64_t)C;
+    const int rwp = round_words((n + 31) / 32);
+    const uint64_t hcap = v2_lean_hash_capacity(c, n, p, rwp);
+    return c * n * 3 + c * (uint64_t)rwp * 4 + c * (1 + (uint64_t)p) + (uint64_t)n * rwp * 4 + c * (uint64_t)k * 2 +
+           hcap * (8 + 4 * (uint64_t)rwp) + (60u << 10);
+}
+
 static int v2_w(int rwp) { return rwp <= 1 ? 1 : rwp <= 2 ? 2 : rwp <= 4 ? 4 : rwp <= 8 ? 8 : 16; }
 
 static V2Dev v2_view(const V2Solver* s) {
@@ -1057,7 +1086,7 @@ int v2_set_hash_capacity(V2Solver* s, uint64_t slots, std::string* err) {
 int v2_create(V2Solver** out, cr_block_cache* cache, const cr_solver_kit& kit, cudaStream_t st, int num_sms, int n, int k, int p,
               const uint32_t* d_rp, const uint16_t* d_col, const uint32_t* h_rp,
               const uint16_t* h_col, const uint32_t* d_binom, const uint16_t* d_configs,
-              uint32_t C, std::string* err) {
+              uint32_t C, bool lean, std::string* err) {
     if (n > 512) {
         if (err) *err = "v2 rules: clouds are limited to 512 vertices";
         return CR_ERR_LIMIT;
@@ -1077,21 +1106,33 @@ int v2_create(V2Solver** out, cr_block_cache* cache, const cr_solver_kit& kit, c
     s->rwp = round_words(s->rw);
     s->W = v2_w(s->rwp);
     s->rp = d_rp; s->col = d_col; s->binom = d_binom; s->configs = d_configs;
+    s->lean = lean;
     V2_CUDA(s->cache->get((void**)&s->table, (size_t)C * n));
     V2_CUDA(s->cache->get((void**)&s->marked, (size_t)C * s->rwp * 4));
     V2_CUDA(s->cache->get((void**)&s->nbr, (size_t)n * s->rwp * 4));
     V2_CUDA(s->cache->get((void**)&s->val1, (size_t)C * n));
     V2_CUDA(s->cache->get((void**)&s->newval, (size_t)C * n));
-    V2_CUDA(s->cache->get((void**)&s->plain, (size_t)C * n));
-    V2_CUDA(s->cache->get((void**)&s->unsafe, (size_t)C * s->rwp * 4));
-    V2_CUDA(s->cache->get((void**)&s->changed, C));
     V2_CUDA(s->cache->get((void**)&s->lev, (size_t)C * p));
     V2_CUDA(s->cache->get((void**)&s->fin1, C));
-    V2_CUDA(s->cache->get((void**)&s->fin2, C));
+    if (lean) {
+        // the unsafe rows, which k_v2_root does not need, lie in newval, which only it and k_v2_apply
+        // do; the changed flags are lev[0] itself, which nothing needs once k_v2_apply sets new ones
+        // (v2_pass clears both in between); no kernel sets or takes fin2
+        if ((size_t)s->rwp * 4 <= (size_t)n) s->unsafe = reinterpret_cast<uint32_t*>(s->newval);
+        else V2_CUDA(s->cache->get((void**)&s->unsafe, (size_t)C * s->rwp * 4));   // (below 4 vertices)
+        s->changed = s->lev;
+        s->fin2 = s->fin1;
+    } else {
+        V2_CUDA(s->cache->get((void**)&s->plain, (size_t)C * n));
+        V2_CUDA(s->cache->get((void**)&s->unsafe, (size_t)C * s->rwp * 4));
+        V2_CUDA(s->cache->get((void**)&s->changed, C));
+        V2_CUDA(s->cache->get((void**)&s->fin2, C));
+    }
     V2_CUDA(s->cache->get((void**)&s->rnbr, (size_t)n * s->rwp * 4));
     V2_CUDA(s->cache->get((void**)&s->vsets, (size_t)2 * s->rwp * 4));
     V2_CUDA(s->cache->get((void**)&s->counters, 4 * sizeof(unsigned long long)));
-    if (int rc = v2_set_hash_capacity(s, v2_hash_capacity((uint64_t)C * n, p), err)) return rc;
+    const uint64_t slots = lean ? v2_lean_hash_capacity(C, n, p, s->rwp) : v2_hash_capacity((uint64_t)C * n, p);
+    if (int rc = v2_set_hash_capacity(s, slots, err)) return rc;
     std::vector<uint32_t> nbr((size_t)n * s->rwp, 0);
     std::vector<uint32_t> rnbr((size_t)n * s->rwp, 0), vsets((size_t)2 * s->rwp, 0);
     for (int v = 0; v < n; ++v) {
@@ -1112,6 +1153,9 @@ int v2_create(V2Solver** out, cr_block_cache* cache, const cr_solver_kit& kit, c
 
 void v2_destroy(V2Solver* s) {
     if (!s) return;
+    if (s->unsafe == (void*)s->newval) s->unsafe = nullptr;   // (a lean solver's shared arrays)
+    if (s->changed == s->lev) s->changed = nullptr;
+    if (s->fin2 == s->fin1) s->fin2 = nullptr;
     void* ptrs[] = {s->table, s->marked, s->nbr, s->val1, s->newval, s->plain, s->unsafe, s->changed, s->lev,
                     s->fin1, s->fin2, s->rnbr, s->vsets, s->counters, s->hkey, s->hmask};
     for (void* q : ptrs)
@@ -1169,7 +1213,7 @@ static int launch_v2_val1(V2Solver* s, V2Dev d, uint64_t lo, uint64_t hi, int gr
 template <int K, int W>
 static int launch_v2_kernels(V2Solver* s, const V2Dev& d, int grid_cfg, size_t sm) {
     int launches = 0;
-    if (d.p >= 2) {
+    if (d.p >= 2 && d.plain) {
         raise_smem_limit((const void*)k_v2_plain<K, W>, sm);
         k_v2_plain<K, W><<<grid_cfg, 256, sm, s->st>>>(d);
         ++launches;
@@ -1178,6 +1222,7 @@ static int launch_v2_kernels(V2Solver* s, const V2Dev& d, int grid_cfg, size_t s
     const uint64_t chunk = d.hkey ? std::max<uint64_t>(1, s->chunk_nodes) : nodes;
     for (uint64_t lo = 0; lo < nodes; lo += chunk)
         launches += launch_v2_val1<K, W>(s, d, lo, std::min(nodes, lo + chunk), grid_cfg, sm);
+    if (s->lean) cudaMemsetAsync(s->newval, kV2None, nodes, s->st);   // (it held the unsafe rows)
     raise_smem_limit((const void*)k_v2_root<K, W>, sm);
     k_v2_root<K, W><<<grid_cfg, 256, sm, s->st>>>(d);
     return launches + 1;
@@ -1241,6 +1286,7 @@ int v2_pass(V2Solver* s, uint64_t* found, cr_solve_stats* stats, std::string* er
         case 3: launches += launch_v2_k<3>(s, d, s->W, grid_cfg, sm); break;
         default: launches += launch_v2_k<4>(s, d, s->W, grid_cfg, sm); break;
     }
+    if (s->lean) cudaMemsetAsync(s->changed, 0, s->C, st);
     const int grid_apply = (int)std::max<uint64_t>(1, std::min<uint64_t>((pairs + 255) / 256, (uint64_t)s->num_sms * 8));
     k_v2_apply<<<grid_apply, 256, 0, st>>>(s->table, s->marked, s->newval, s->changed, s->C, s->n, s->rwp);
     launches += 1;

@@ -13,10 +13,11 @@ namespace crgpu {
 struct V2Solver;
 
 uint64_t v2_footprint(int n, int k, int p);
+uint64_t v2_lean_footprint(int n, int k, int p);   // of a solver without the plain values
 int v2_create(V2Solver** out, cr_block_cache* cache, const cr_solver_kit& kit, cudaStream_t st, int num_sms, int n, int k, int p,
               const uint32_t* d_rp, const uint16_t* d_col, const uint32_t* h_rp,
               const uint16_t* h_col, const uint32_t* d_binom, const uint16_t* d_configs,
-              uint32_t C, std::string* err);
+              uint32_t C, bool lean, std::string* err);
 void v2_destroy(V2Solver* s);
 int v2_init(V2Solver* s, cr_solve_stats* stats, std::string* err);
 int v2_pass(V2Solver* s, uint64_t* found, cr_solve_stats* stats, std::string* err);

@@ -262,7 +262,9 @@ int cr_solver_digest(cr_solver* s, uint64_t* digest);
  * process run).  Requests queue as they arrive; worker threads, each with its own stream,
  * start the first queued request whose device footprint (cr_solver_footprint) fits in the
  * memory budget left, so requests arriving while others run are admitted as soon as a worker
- * and memory free up and their solves overlap on the GPU.  Finished tables stay resident
+ * and memory free up and their solves overlap on the GPU.  A request whose footprint exceeds the
+ * whole budget is solved with less memory where that fits (without the head rows of k = 2 and 4,
+ * or the plain values of the v2 rules; slower, the same results) and else refused.  Finished tables stay resident
  * until cr_server_release.  A queued request waiting more than 2 s is not overtaken. */
 typedef struct cr_server cr_server;
 
