@@ -26,7 +26,7 @@ EXE = os.path.join(BIN, "k_cops_gpu")
 CU_SOURCES = ["crgpu_api.cu", "crgpu_v1.cu", "crgpu_v2.cu", "crgpu_tables.cu", "crgpu_batch.cu", "crgpu_small.cu",
               "crgpu_small_1.cu", "crgpu_small_2.cu", "crgpu_small_3.cu", "crgpu_small_4.cu",
               "crgpu_noalloc.cu", "crgpu_server.cu"]
-HEADERS = ["crgpu_internal.cuh", "crgpu_smem.h", "crgpu_v1_body.cuh", "crgpu_team.cuh", "crgpu_small.cuh",
+HEADERS = ["crgpu_internal.cuh", "crgpu_smem.h", "crgpu_batch_plan.h", "crgpu_v1_body.cuh", "crgpu_team.cuh", "crgpu_small.cuh",
            "crgpu_small_run.cuh", "crgpu_ctx.h", "crgpu_v2.h",
            os.path.join("..", "..", "include", "crgpu.h")]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]

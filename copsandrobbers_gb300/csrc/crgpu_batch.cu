@@ -27,7 +27,6 @@
 #include <map>
 #include <mutex>
 #include <numeric>
-#include <queue>
 #include <tuple>
 #include <vector>
 
@@ -36,6 +35,7 @@
 #define CR_RESTRICT
 #define CR_BODY_INLINE __noinline__
 #include "../../include/crgpu.h"
+#include "crgpu_batch_plan.h"
 #include "crgpu_ctx.h"
 #include "crgpu_v1_body.cuh"
 #include "crgpu_team.cuh"
@@ -576,11 +576,6 @@ struct Shape {
     int threads, per_sm;
 };
 
-// How a batch is split: order[0 .. count) goes to teams of `size` blocks, `teams` of them resident.
-struct TeamPlan {
-    int size = 1, teams = 0, count = 0;
-};
-
 std::mutex g_tune_mu;
 std::map<std::tuple<int, int, int, int>, Shape> g_tuned;
 
@@ -648,71 +643,12 @@ int resident_teams(Shape shape, int size, size_t sm, int num_sms) {
     return n;
 }
 
-// Splits the batch between teams and single blocks.  Run time of a graph on one block: proportional
-// to its configurations times vertices at the largest k, plus a constant for its launches' worth of
-// barriers; a team of s blocks is worth a little less than s blocks (measured on 256 graphs of
-// n = 128: 0.95, 0.88 and 0.78 of them for 2, 4 and 8).  Each split is played through the two
-// queues, largest graph first, and the shortest run wins; a batch of more than 64 graphs per block
-// needs no teams (the longest graph is then a small part of the run).
-TeamPlan plan_teams(const std::vector<double>& cost, Shape shape, size_t sm, int num_sms) {
-    const int count = (int)cost.size();   // in descending order
-    const int blocks1 = num_sms * shape.per_sm;
-    TeamPlan best;
-    best.teams = std::min(count, blocks1);
-    if (count > 64 * blocks1) return best;
-    const double fixed = 2.5e4;   // in the cost's unit
-    double total = 0;
-    for (double c : cost) total += c + fixed;
-    auto play = [&](int size, int teams, double eff, int by_teams) {
-        std::priority_queue<double, std::vector<double>, std::greater<double>> q;
-        for (int t = 0; t < teams; ++t) q.push(0.0);
-        double end = 0;
-        for (int i = 0; i < by_teams; ++i) {
-            const double t = q.top() + cost[i] / (size * eff) + 1.5 * fixed;
-            q.pop();
-            q.push(t);
-            end = std::max(end, t);
-        }
-        std::vector<double> at;
-        for (; !q.empty(); q.pop())
-            for (int k = 0; k < size; ++k) at.push_back(q.top());
-        std::priority_queue<double, std::vector<double>, std::greater<double>> r(std::greater<double>(), std::move(at));
-        for (int i = by_teams; i < count; ++i) {
-            const double t = r.top() + cost[i] + fixed;
-            r.pop();
-            r.push(t);
-            end = std::max(end, t);
-        }
-        return end;
-    };
-    double shortest = play(1, blocks1, 1.0, 0);
-    const struct { int size; double eff; } kinds[] = {{2, 0.95}, {4, 0.88}, {8, 0.78}};
-    for (const auto& k : kinds) {
-        const int teams = resident_teams(shape, k.size, sm, num_sms);
-        if (teams <= 0) continue;
-        int last = -1;
-        for (double f = 2.0; f > 0.01; f /= 1.6) {
-            // the graphs longer than a share f of the ideal run
-            int m = 0;
-            while (m < count && cost[m] > f * total / blocks1) ++m;
-            if (m == last || m == 0) continue;
-            last = m;
-            const double t = play(k.size, teams, k.eff, m);
-            if (t < 0.98 * shortest) {
-                shortest = t;
-                best = TeamPlan{k.size, teams, m};
-            }
-        }
-    }
-    return best;
-}
-
 int launch_batch(cr_context* ctx, const BatchInputs& in, const std::vector<int32_t>& order, int kmax,
-                 int p, Shape shape, TeamPlan plan, size_t team_bytes, size_t solo_bytes, std::vector<int32_t>* cop,
+                 int p, Shape shape, const TeamPlan& plan, std::vector<int32_t>* cop,
                  std::vector<cr_batch_result>* res, float* ms,
                  std::vector<unsigned long long>* times = nullptr) {
     const int count = (int)order.size();
-    const int nteams = std::max(1, std::min(count, plan.teams)), nblocks = nteams * plan.size;
+    const int nteams = plan.resident(count), nblocks = nteams * plan.size;
     void* bufs[14] = {};
     auto cleanup = [&]() {
         for (void* q : bufs) ctx->cache.put(q);
@@ -724,7 +660,7 @@ int launch_batch(cr_context* ctx, const BatchInputs& in, const std::vector<int32
     size_t sizes[14] = {order.size() * 4, in.n.size() * 4, in.maxdeg.size() * 4, in.rp_off.size() * 8,
                         in.col_off.size() * 8, in.rp.size() * 4, std::max<size_t>(in.col.size(), 1) * 2,
                         in.rrp.size() * 4, std::max<size_t>(in.rcol.size(), 1) * 2,
-                        (size_t)nteams * team_bytes, 2 * sizeof(int) + in.n.size() * 4,
+                        (size_t)nteams * plan.team_bytes, 2 * sizeof(int) + in.n.size() * 4,
                         in.n.size() * kmax * sizeof(cr_batch_result), (size_t)nblocks * 16, (size_t)nteams * sizeof(int)};
     for (int i = 0; i < 14; ++i) {
         cudaError_t e = ctx->cache.get(&bufs[i], sizes[i]);
@@ -752,8 +688,8 @@ int launch_batch(cr_context* ctx, const BatchInputs& in, const std::vector<int32
     b.rrp_all = (const uint32_t*)bufs[7];
     b.rcol_all = (const uint16_t*)bufs[8];
     b.slots = (unsigned char*)bufs[9];
-    b.team_bytes = team_bytes;
-    b.solo_bytes = solo_bytes;
+    b.team_bytes = plan.team_bytes;
+    b.solo_bytes = plan.solo_bytes;
     b.team_count = plan.count;
     b.next = (int*)bufs[10];
     b.cop = (int32_t*)((char*)bufs[10] + 2 * sizeof(int));
@@ -867,11 +803,13 @@ int cr_batch_solve(cr_context* ctx, const cr_graph* graphs, int32_t count, int32
     std::stable_sort(order.begin(), order.end(), [&](int a, int c) { return cost[a] > cost[c]; });
     const size_t slot_bytes = job_layout(in.max_n, kmax, p, 2).total;
 
+    // half of what the device has free, the context's held blocks included (an allocation that does
+    // not fit otherwise gets them back)
     size_t free_b = 0, total_b = 0;
     cudaMemGetInfo(&free_b, &total_b);
-    auto fits = [&](Shape s) {
-        return (size_t)std::min(count, ctx->num_sms * s.per_sm) * slot_bytes < free_b / 2;
-    };
+    const size_t memory = (free_b + ctx->cache.free_bytes()) / 2;
+    auto alone = [&](Shape s) { return TeamPlan::alone(ctx->num_sms * s.per_sm, slot_bytes); };
+    auto fits = [&](Shape s) { return alone(s).bytes(count) < memory; };
     Shape shape{threads_per_cta ? threads_per_cta : 512, threads_per_cta == 256 ? 2 : 1};
     if (threads_per_cta == 0) {
         // autotune: time candidate launch shapes on a calibration slice (every 8th graph of
@@ -893,8 +831,7 @@ int cr_batch_solve(cr_context* ctx, const cr_graph* graphs, int32_t count, int32
                 std::vector<int32_t> cp;
                 std::vector<cr_batch_result> rs;
                 float ms = 0;
-                const TeamPlan alone{1, ctx->num_sms * c.per_sm, 0};
-                if (launch_batch(ctx, in, calib, kmax, p, c, alone, slot_bytes, slot_bytes, &cp, &rs, &ms) != CR_OK) continue;
+                if (launch_batch(ctx, in, calib, kmax, p, c, alone(c), &cp, &rs, &ms) != CR_OK) continue;
                 if (ms < best) {
                     best = ms;
                     shape = c;
@@ -909,20 +846,21 @@ int cr_batch_solve(cr_context* ctx, const cr_graph* graphs, int32_t count, int32
     std::vector<cr_batch_result> res;
     float ms = 0;
     std::vector<unsigned long long> times;
-    // the teams' share of the batch (a block's share of a team's slot holds the largest graph that
-    // is solved alone)
-    raise_smem_limit((const void*)batch_kernel(shape), launch_smem(in, shape));
+    // the teams' share of the batch
+    const size_t smem = launch_smem(in, shape);
+    raise_smem_limit((const void*)batch_kernel(shape), smem);
     std::vector<double> sorted(count);
     for (int i = 0; i < count; ++i) sorted[i] = cost[order[i]];
-    const TeamPlan plan = plan_teams(sorted, shape, launch_smem(in, shape), ctx->num_sms);
-    size_t solo_bytes = slot_bytes;
-    if (plan.count > 0) {
-        int solo_n = 1;
-        for (int i = plan.count; i < count; ++i) solo_n = std::max(solo_n, (int)in.n[order[i]]);
-        solo_bytes = job_layout(solo_n, kmax, p, 2).total;
+    TeamPlan plan = plan_teams(
+        sorted, ctx->num_sms * shape.per_sm, slot_bytes, memory,
+        [&](int size) { return resident_teams(shape, size, smem, ctx->num_sms); },
+        [&](int by_teams) { return job_layout(by_teams < count ? in.n[order[by_teams]] : 1, kmax, p, 2).total; });
+    int rc = launch_batch(ctx, in, order, kmax, p, shape, plan, &cop, &res, &ms, &times);
+    if (rc == CR_ERR_NOMEM && plan.size > 1) {   // (taken by others meanwhile)
+        cudaGetLastError();
+        plan = alone(shape);
+        rc = launch_batch(ctx, in, order, kmax, p, shape, plan, &cop, &res, &ms, &times);
     }
-    const size_t team_bytes = std::max(slot_bytes, plan.size * solo_bytes);
-    int rc = launch_batch(ctx, in, order, kmax, p, shape, plan, team_bytes, solo_bytes, &cop, &res, &ms, &times);
     if (rc) return rc;
     memcpy(cop_number, cop.data(), count * sizeof(int32_t));
     memcpy(results, res.data(), res.size() * sizeof(cr_batch_result));
@@ -931,8 +869,8 @@ int cr_batch_solve(cr_context* ctx, const cr_graph* graphs, int32_t count, int32
         stats->ms = ms;
         for (const auto& r : res) stats->states += r.solved ? r.states : 0;
         stats->threads = shape.threads;
-        stats->ctas = std::max(1, std::min(count, plan.teams)) * plan.size;
-        stats->slot_bytes = (int64_t)(plan.count > 0 ? team_bytes / plan.size : slot_bytes);
+        stats->ctas = plan.resident(count) * plan.size;
+        stats->slot_bytes = (int64_t)(plan.team_bytes / plan.size);
         // how evenly the blocks were kept busy: mean busy span over the whole span, and the
         // time from the median block's last graph to the last block's
         const size_t nb = times.size() / 2;

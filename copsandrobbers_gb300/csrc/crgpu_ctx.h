@@ -81,6 +81,10 @@ struct cr_block_cache {
         std::lock_guard<std::mutex> lock(mu);
         release_free();
     }
+    size_t free_bytes() {
+        std::lock_guard<std::mutex> lock(mu);
+        return held_bytes;
+    }
     // (the callers below hold the lock)
     void trim() {
         while (held_bytes > limit) {
