@@ -141,6 +141,7 @@ struct cr_solver {
     cr_solver_kit kit;                // pinned: the ring of pass counts, then two words of results
     bool init_timing = false;         // kit.ev[2], ev[3] bracket an initializeCaptures in flight
     bool unsynced = false;            // the table may still be being written
+    bool shared = false;              // the table's address has been given away
     // phase state
     bool initialized = false;
     bool finished = false;
@@ -898,6 +899,14 @@ static int v1_advance(cr_solver* s, size_t passes, size_t ahead) {
     return CR_OK;
 }
 
+// A caller that holds the table's address may read it from another stream.
+static int wait_for_table(cr_solver* s) {
+    if (!s->unsynced) return CR_OK;
+    CR_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
+    s->unsynced = false;
+    return CR_OK;
+}
+
 int cr_solver_init(cr_solver* s, uint64_t* base_captures) {
     if (!s) return CR_ERR_INVALID;
     cr_context* ctx = s->ctx;
@@ -915,6 +924,7 @@ int cr_solver_init(cr_solver* s, uint64_t* base_captures) {
     } else {
         caps = base_capture_count(s);
         rc = s->rules == CR_RULES_V1 ? v1_init(s) : crgpu::v2_init(s->v2, &s->stats, &ctx->err);
+        if (!rc && s->shared) rc = wait_for_table(s);
     }
     if (rc) return rc;
     s->base_caps = caps;
@@ -1131,10 +1141,8 @@ int cr_solver_device_states(cr_solver* s, void** dev_ptr, size_t* bytes) {
     if (!s || !dev_ptr || !bytes) return CR_ERR_INVALID;
     CR_CUDA(s->ctx, cudaSetDevice(s->ctx->device));
     if (int rc = materialize_init(s)) return rc;
-    if (s->unsynced) {   // the caller may read the table from another stream
-        CR_CUDA(s->ctx, cudaStreamSynchronize(s->ctx->stream));
-        s->unsynced = false;
-    }
+    s->shared = true;
+    if (int rc = wait_for_table(s)) return rc;
     *dev_ptr = (void*)table_ptr(s);
     *bytes = s->C * (size_t)s->n * s->cols;
     return CR_OK;

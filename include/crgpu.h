@@ -140,7 +140,10 @@ int cr_solver_sizes(cr_solver* s, cr_table_sizes* out);
 int cr_solver_stats(cr_solver* s, cr_solve_stats* out);
 /* The states section of the table file (CacheManager.h:67): byte = marked | round << 1. */
 int cr_solver_read_states(cr_solver* s, uint8_t* dst, size_t bytes);
-/* Device pointer to the same table (valid until cr_solver_destroy). */
+/* Device pointer to the same table (valid until cr_solver_destroy).  What the table holds when this,
+ * cr_solver_init, cr_solver_pass or cr_solver_run returns may be read on any stream -- except that an
+ * initializeCaptures folded into pass 1 (p = 1) is written when it is asked for: by this call again, a
+ * read or the pass. */
 int cr_solver_device_states(cr_solver* s, void** dev_ptr, size_t* bytes);
 /* The configs section (CacheManager.h:64): config_count * k bytes; n must be <= 256. */
 int cr_solver_read_configs(cr_solver* s, uint8_t* dst, size_t bytes);
