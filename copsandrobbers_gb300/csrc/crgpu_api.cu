@@ -231,6 +231,16 @@ int cr_context_set_cache_limit(cr_context* ctx, uint64_t bytes) {
     return CR_OK;
 }
 
+// For tests: the device is full once this context's blocks take `bytes`; *peak = the most that solvers
+// have taken of them so far.
+int cr_context_limit_blocks(cr_context* ctx, uint64_t bytes, uint64_t* peak) {
+    if (!ctx) return CR_ERR_INVALID;
+    std::lock_guard<std::mutex> lock(ctx->cache.mu);
+    ctx->cache.most = bytes;
+    if (peak) *peak = ctx->cache.peak_used;
+    return CR_OK;
+}
+
 int cr_context_set_profiling(cr_context* ctx, int32_t on) {
     if (!ctx) return CR_ERR_INVALID;
     ctx->profiling = on != 0;
@@ -290,10 +300,23 @@ static cudaError_t alloc_h1(cr_solver* s) {
     const uint64_t hb = h1_bytes(s->n, s->k, s->S, s->rwp);
     if (!hb || (s->lean && s->k != 3)) return cudaSuccess;
     const cudaError_t e = s->ctx->cache.get((void**)&s->d_h1, hb);
-    if (e != cudaErrorMemoryAllocation || s->k == 3) return e;
-    cudaGetLastError();
-    s->d_h1 = nullptr;
-    return cudaSuccess;
+    return e == cudaErrorMemoryAllocation && s->k != 3 ? cudaSuccess : e;
+}
+
+// A block that a solver needs later than its own, in place of what it can do without (head rows of
+// k = 2 and 4, the plain values of the v2 rules) where the device has no room for both.
+static cudaError_t get_or_shed(cr_solver* s, void** out, size_t bytes) {
+    cr_block_cache& cache = s->ctx->cache;
+    const cudaError_t e = cache.get(out, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    if (s->v2) {
+        if (!crgpu::v2_shed(s->v2)) return e;
+    } else {
+        if (!s->d_h1 || s->k == 3) return e;
+        cache.put(s->d_h1);
+        s->d_h1 = nullptr;
+    }
+    return cache.get(out, bytes);
 }
 
 static void layout(int n, int k, int p, int rules, int S, uint64_t* C, int* cols, int* rw, int* rwp) {
@@ -437,7 +460,6 @@ static int alloc_v1(cr_solver* s, SmallArrays& small) {
     CR_CUDA(ctx, ctx->cache.get((void**)&s->d_clist, C * 4));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_cand, 0, C * s->S * s->rwp * 4, ctx->stream));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_cbits, 0, cand_bits_bytes(C), ctx->stream));
-    CR_CUDA(ctx, alloc_h1(s));
     std::vector<uint32_t> hop = hop_masks(s);
     small.add(&s->d_hop, hop);
     // transposed hop masks (bit r of row u iff u in hop(r)), and hop(r) as lists
@@ -648,6 +670,7 @@ int crgpu::create_solver(cr_context* ctx, const cr_graph* g, int32_t k, int32_t 
         int rc = alloc_v1(s, small);
         if (rc) return bail(rc);
         CR_TRY(small.upload(ctx->cache, &s->d_small, ctx->stream));
+        CR_TRY(alloc_h1(s));   // (last: the rest has to fit without it)
         const int per_sm = max_cop_blocks_per_sm(k, s->rwp, s->S);
         s->grid_cop = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 7) / 8, (uint64_t)ctx->num_sms * per_sm));
         s->grid_small = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 255) / 256, (uint64_t)ctx->num_sms * 4));
@@ -1182,8 +1205,8 @@ int cr_solver_build_transitions(cr_solver* s, uint64_t* total) {
         const int cap = trans_cap(s->k, s->cop_maxdeg);
         if (cap > 8192) return fail(ctx, CR_ERR_LIMIT, "successor fan-out %d too large for the CSR builder", cap);
         unsigned long long* counts = nullptr;
-        CR_CUDA(ctx, ctx->cache.get((void**)&counts, s->C * 8));
-        CR_CUDA(ctx, ctx->cache.get((void**)&s->d_heads, (s->C + 1) * 8));
+        CR_CUDA(ctx, get_or_shed(s, (void**)&counts, s->C * 8));
+        CR_CUDA(ctx, get_or_shed(s, (void**)&s->d_heads, (s->C + 1) * 8));
         CR_CUDA(ctx, cudaMemsetAsync(&s->d_ctl->err, 0, sizeof(unsigned), st));
         const int grid = ctx->num_sms * 8;
         const uint32_t* trp = s->d_crp ? s->d_crp : s->d_rp;
@@ -1197,7 +1220,7 @@ int cr_solver_build_transitions(cr_solver* s, uint64_t* total) {
         CR_CUDA(ctx, cudaStreamSynchronize(st));
         ctx->cache.put(counts);
         s->n_trans = tot;
-        CR_CUDA(ctx, ctx->cache.get((void**)&s->d_trans, std::max<uint64_t>(tot, 1) * 8));
+        CR_CUDA(ctx, get_or_shed(s, (void**)&s->d_trans, std::max<uint64_t>(tot, 1) * 8));
         launch_trans(s->k, s->d_configs, (uint32_t)s->C, s->n, trp, tcol, s->d_binom, cap, nullptr,
                      s->d_heads, s->d_trans, &s->d_ctl->err, grid, st);
         CR_CUDA(ctx, cudaGetLastError());
@@ -1334,12 +1357,12 @@ int cr_solver_load_table_file(cr_solver* s, const char* path) {
     CR_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     const uint64_t ntrans = (h[11] - h[10]) / 8;
-    if (!s->d_heads) CR_CUDA(ctx, ctx->cache.get((void**)&s->d_heads, heads));
+    if (!s->d_heads) CR_CUDA(ctx, get_or_shed(s, (void**)&s->d_heads, heads));
     if (s->d_trans && ntrans > s->n_trans) {
         ctx->cache.put(s->d_trans);
         s->d_trans = nullptr;
     }
-    if (!s->d_trans) CR_CUDA(ctx, ctx->cache.get((void**)&s->d_trans, std::max<uint64_t>(ntrans, 1) * 8));
+    if (!s->d_trans) CR_CUDA(ctx, get_or_shed(s, (void**)&s->d_trans, std::max<uint64_t>(ntrans, 1) * 8));
     s->n_trans = ntrans;
     CR_CUDA(ctx, cudaMemcpyAsync(s->d_heads, blob.data() + h[9], heads, cudaMemcpyHostToDevice, st));
     if (ntrans) CR_CUDA(ctx, cudaMemcpyAsync(s->d_trans, blob.data() + h[10], ntrans * 8, cudaMemcpyHostToDevice, st));

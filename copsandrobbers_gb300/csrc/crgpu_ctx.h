@@ -25,8 +25,9 @@ struct cr_block_cache {
     };
     std::vector<Block> held;                     // free
     std::unordered_map<void*, size_t> used;
-    size_t held_bytes = 0;
+    size_t held_bytes = 0, used_bytes = 0, peak_used = 0;
     size_t limit = 4ull << 30;
+    size_t most = ~size_t(0);                    // of held and used blocks together (a full device, for tests)
     std::mutex mu;
 
     cudaError_t get(void** out, size_t bytes) {
@@ -46,18 +47,20 @@ struct cr_block_cache {
             *out = held[best].p;
             used[held[best].p] = held[best].bytes;
             held_bytes -= held[best].bytes;
+            add_used(held[best].bytes);
             held[best] = held.back();
             held.pop_back();
             return cudaSuccess;
         }
-        cudaError_t e = cudaMalloc(out, bytes);
+        cudaError_t e = allocate(out, bytes);
         if (e == cudaErrorMemoryAllocation) {   // give the held blocks back and try once more
-            cudaGetLastError();
             release_free();
-            e = cudaMalloc(out, bytes);
+            e = allocate(out, bytes);
         }
-        if (e == cudaSuccess) used[*out] = bytes;
-        return e;
+        if (e != cudaSuccess) return e;
+        used[*out] = bytes;
+        add_used(bytes);
+        return cudaSuccess;
     }
     void put(void* p) {
         if (!p) return;
@@ -69,6 +72,7 @@ struct cr_block_cache {
         }
         held.push_back(Block{p, it->second});
         held_bytes += it->second;
+        used_bytes -= it->second;
         used.erase(it);
         trim();
     }
@@ -86,6 +90,20 @@ struct cr_block_cache {
         return held_bytes;
     }
     // (the callers below hold the lock)
+    void add_used(size_t bytes) {
+        used_bytes += bytes;
+        if (used_bytes > peak_used) peak_used = used_bytes;
+    }
+    // An error is the caller's to report: none is left behind for the check of a later launch.
+    cudaError_t allocate(void** out, size_t bytes) {
+        if (bytes > most || held_bytes + used_bytes > most - bytes) return cudaErrorMemoryAllocation;
+        const cudaError_t e = cudaMalloc(out, bytes);
+        if (e != cudaSuccess) {
+            *out = nullptr;
+            cudaGetLastError();
+        }
+        return e;
+    }
     void trim() {
         while (held_bytes > limit) {
             size_t big = 0;

@@ -44,9 +44,9 @@
 // every pass; when the depth-1 nodes outnumber half the table, they are processed in chunks, each
 // with a fresh table.
 //
-// A lean solver (V2Solver::lean) has no plain values: every child of a depth-1 node is then looked at
+// A lean solver has no plain values: every child of a depth-1 node is then looked at
 // where it is reached, as a touched node's are, and three byte arrays share the memory of others
-// (v2_create).  It serves requests that a memory budget would refuse otherwise; Delaunay n = 199,
+// (v2_arrays).  It serves where a memory budget or the device has no room for more; Delaunay n = 199,
 // k = 2, p = 3 takes 166 ms so.
 //
 // Measured (Delaunay n = 199, k = 2, p = 3, six passes): 94 ms with every dirty depth-1 node's
@@ -84,8 +84,8 @@ struct V2Solver {
     uint32_t* nbr = nullptr;
     uint8_t* val1 = nullptr;
     uint8_t* newval = nullptr;
-    bool lean = false;              // without the plain values
-    uint8_t* plain = nullptr;       // [C][n] plain depth-2 values; null = lean
+    bool lean = false;              // without the plain values, and with shared arrays (v2_arrays)
+    uint8_t* plain = nullptr;       // [C][n] plain depth-2 values; null = lean, or given back (v2_shed)
     uint32_t* unsafe = nullptr;     // [C][rwp], rows of changed configurations only
     uint8_t* changed = nullptr;     // configurations that gained marks
     uint8_t* lev = nullptr;         // [p][C]: a changed configuration j cop steps away
@@ -122,7 +122,7 @@ struct V2Dev {
     const uint32_t* still;         // [rwp]: vertices with none
     uint8_t* val1;
     uint8_t* newval;
-    uint8_t* plain;                // null = lean: every depth-1 node counts as touched
+    uint8_t* plain;                // null = every depth-1 node counts as touched
     uint32_t* unsafe;
     const uint8_t* lev;            // [p][C]
     uint8_t* fin1;
@@ -996,7 +996,7 @@ uint64_t v2_footprint(int n, int k, int p) {
            hcap * (8 + 4 * (uint64_t)rwp) + (1u << 16);
 }
 
-// Of a lean solver (see v2_create): at most half of that, so much less that the table makes room for the
+// Of a lean solver (see v2_arrays): at most half of that, so much less that the table makes room for the
 // levels beyond the second (0 = none; a table of the least size stays).  A lean solver then holds no
 // more than three bytes a state, three a configuration, the marks and a table of the usual size.
 static uint64_t v2_lean_hash_capacity(uint64_t C, int n, int p, int rwp) {
@@ -1083,6 +1083,49 @@ int v2_set_hash_capacity(V2Solver* s, uint64_t slots, std::string* err) {
     return CR_OK;
 }
 
+static void v2_put_arrays(V2Solver* s) {
+    if (s->unsafe == (void*)s->newval) s->unsafe = nullptr;   // (a lean solver's shared arrays)
+    if (s->changed == s->lev) s->changed = nullptr;
+    if (s->fin2 == s->fin1) s->fin2 = nullptr;
+    void* ptrs[] = {s->plain, s->unsafe, s->changed, s->lev, s->fin1, s->fin2, s->hkey, s->hmask};
+    for (void* q : ptrs) s->cache->put(q);
+    s->plain = s->changed = s->lev = s->fin1 = s->fin2 = nullptr;
+    s->unsafe = s->hmask = nullptr;
+    s->hkey = nullptr;
+}
+
+// The arrays that a lean solver has fewer of.  There the unsafe rows, which k_v2_root does not need, lie
+// in newval, which only it and k_v2_apply do; the changed flags are lev[0] itself, which nothing needs
+// once k_v2_apply sets new ones (v2_pass clears both in between); no kernel sets or takes fin2.
+static int v2_arrays(V2Solver* s, bool lean, std::string* err) {
+    v2_put_arrays(s);
+    s->lean = lean;
+    const size_t C = s->C, n = s->n;
+    V2_CUDA(s->cache->get((void**)&s->lev, C * s->p));
+    V2_CUDA(s->cache->get((void**)&s->fin1, C));
+    if (lean && (size_t)s->rwp * 4 <= n) s->unsafe = reinterpret_cast<uint32_t*>(s->newval);
+    else V2_CUDA(s->cache->get((void**)&s->unsafe, C * s->rwp * 4));   // (lean: below 4 vertices)
+    if (lean) {
+        s->changed = s->lev;
+        s->fin2 = s->fin1;
+    } else {
+        V2_CUDA(s->cache->get((void**)&s->plain, C * n));
+        V2_CUDA(s->cache->get((void**)&s->changed, C));
+        V2_CUDA(s->cache->get((void**)&s->fin2, C));
+    }
+    const uint64_t slots = lean ? v2_lean_hash_capacity(C, s->n, s->p, s->rwp) : v2_hash_capacity(C * n, s->p);
+    return v2_set_hash_capacity(s, slots, err);
+}
+
+// Between passes: from here on every depth-1 node counts as touched, whose open children the passes look
+// at where they are reached (what the plain values had found has already reached the nodes above).
+bool v2_shed(V2Solver* s) {
+    if (!s->plain) return false;
+    s->cache->put(s->plain);
+    s->plain = nullptr;
+    return true;
+}
+
 int v2_create(V2Solver** out, cr_block_cache* cache, const cr_solver_kit& kit, cudaStream_t st, int num_sms, int n, int k, int p,
               const uint32_t* d_rp, const uint16_t* d_col, const uint32_t* h_rp,
               const uint16_t* h_col, const uint32_t* d_binom, const uint16_t* d_configs,
@@ -1106,33 +1149,17 @@ int v2_create(V2Solver** out, cr_block_cache* cache, const cr_solver_kit& kit, c
     s->rwp = round_words(s->rw);
     s->W = v2_w(s->rwp);
     s->rp = d_rp; s->col = d_col; s->binom = d_binom; s->configs = d_configs;
-    s->lean = lean;
     V2_CUDA(s->cache->get((void**)&s->table, (size_t)C * n));
     V2_CUDA(s->cache->get((void**)&s->marked, (size_t)C * s->rwp * 4));
     V2_CUDA(s->cache->get((void**)&s->nbr, (size_t)n * s->rwp * 4));
     V2_CUDA(s->cache->get((void**)&s->val1, (size_t)C * n));
     V2_CUDA(s->cache->get((void**)&s->newval, (size_t)C * n));
-    V2_CUDA(s->cache->get((void**)&s->lev, (size_t)C * p));
-    V2_CUDA(s->cache->get((void**)&s->fin1, C));
-    if (lean) {
-        // the unsafe rows, which k_v2_root does not need, lie in newval, which only it and k_v2_apply
-        // do; the changed flags are lev[0] itself, which nothing needs once k_v2_apply sets new ones
-        // (v2_pass clears both in between); no kernel sets or takes fin2
-        if ((size_t)s->rwp * 4 <= (size_t)n) s->unsafe = reinterpret_cast<uint32_t*>(s->newval);
-        else V2_CUDA(s->cache->get((void**)&s->unsafe, (size_t)C * s->rwp * 4));   // (below 4 vertices)
-        s->changed = s->lev;
-        s->fin2 = s->fin1;
-    } else {
-        V2_CUDA(s->cache->get((void**)&s->plain, (size_t)C * n));
-        V2_CUDA(s->cache->get((void**)&s->unsafe, (size_t)C * s->rwp * 4));
-        V2_CUDA(s->cache->get((void**)&s->changed, C));
-        V2_CUDA(s->cache->get((void**)&s->fin2, C));
-    }
     V2_CUDA(s->cache->get((void**)&s->rnbr, (size_t)n * s->rwp * 4));
     V2_CUDA(s->cache->get((void**)&s->vsets, (size_t)2 * s->rwp * 4));
     V2_CUDA(s->cache->get((void**)&s->counters, 4 * sizeof(unsigned long long)));
-    const uint64_t slots = lean ? v2_lean_hash_capacity(C, n, p, s->rwp) : v2_hash_capacity((uint64_t)C * n, p);
-    if (int rc = v2_set_hash_capacity(s, slots, err)) return rc;
+    int rc = v2_arrays(s, lean, err);
+    if (rc == CR_ERR_NOMEM && !lean) rc = v2_arrays(s, true, err);
+    if (rc) return rc;
     std::vector<uint32_t> nbr((size_t)n * s->rwp, 0);
     std::vector<uint32_t> rnbr((size_t)n * s->rwp, 0), vsets((size_t)2 * s->rwp, 0);
     for (int v = 0; v < n; ++v) {
@@ -1153,11 +1180,8 @@ int v2_create(V2Solver** out, cr_block_cache* cache, const cr_solver_kit& kit, c
 
 void v2_destroy(V2Solver* s) {
     if (!s) return;
-    if (s->unsafe == (void*)s->newval) s->unsafe = nullptr;   // (a lean solver's shared arrays)
-    if (s->changed == s->lev) s->changed = nullptr;
-    if (s->fin2 == s->fin1) s->fin2 = nullptr;
-    void* ptrs[] = {s->table, s->marked, s->nbr, s->val1, s->newval, s->plain, s->unsafe, s->changed, s->lev,
-                    s->fin1, s->fin2, s->rnbr, s->vsets, s->counters, s->hkey, s->hmask};
+    v2_put_arrays(s);
+    void* ptrs[] = {s->table, s->marked, s->nbr, s->val1, s->newval, s->rnbr, s->vsets, s->counters};
     for (void* q : ptrs)
         s->cache->put(q);
     delete s;
