@@ -946,7 +946,14 @@ int cr_solver_init(cr_solver* s, uint64_t* base_captures) {
         s->stats.kernel_launches = 0;
     } else {
         caps = base_capture_count(s);
-        rc = s->rules == CR_RULES_V1 ? v1_init(s) : crgpu::v2_init(s->v2, &s->stats, &ctx->err);
+        if (s->rules == CR_RULES_V1) {
+            rc = v1_init(s);
+        } else {
+            settle_init_time(s);
+            rc = crgpu::v2_init(s->v2, &ctx->err);
+            s->init_timing = s->unsynced = !rc;
+            s->stats.kernel_launches = 1;
+        }
         if (!rc && s->shared) rc = wait_for_table(s);
     }
     if (rc) return rc;
@@ -1004,6 +1011,8 @@ int cr_solver_pass(cr_solver* s, uint64_t* new_wins) {
     if (s->rules == CR_RULES_V2) {
         int rc = crgpu::v2_pass(s->v2, &f, &s->stats, &ctx->err);
         if (rc) return rc;
+        s->unsynced = false;
+        settle_init_time(s);
     } else {
         // (a pass that overflows its value slots is not counted: the slots are widened, and it runs
         // again)

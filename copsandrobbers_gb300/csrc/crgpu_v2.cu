@@ -104,7 +104,8 @@ struct V2Solver {
     uint64_t chunk_nodes = 0;   // depth-1 nodes per table fill
     cr_v2_hash_stats hstats{};
     bool first = true;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;   // (the solver's kit's)
+    cudaEvent_t e0 = nullptr, e1 = nullptr;   // around a pass (the solver's kit's)
+    cudaEvent_t i0 = nullptr, i1 = nullptr;   // around initializeCaptures
 };
 
 struct V2Dev {
@@ -495,13 +496,14 @@ __device__ __forceinline__ void load_graph(const V2Dev& d, uint32_t* snbr) {
     __syncthreads();
 }
 
-// The begin of a pass, a warp per configuration: the counters and the flags of what this pass finds
-// are cleared, the last pass's changes become lev[0], and a changed configuration gets its unsafe
-// row (a lane per vertex): bit v of row C set iff v has a neighbour unmarked in row C.
+// The begin of a pass after the first (whose clears are k_v2_init's), a warp per configuration: the
+// counters and the flags of what this pass finds are cleared, the last pass's changes become lev[0],
+// and a changed configuration gets its unsafe row (a lane per vertex): bit v of row C set iff v has a
+// neighbour unmarked in row C.
 template <int W>
 __global__ void __launch_bounds__(256) k_v2_begin(V2Dev d, uint8_t* lev0, uint8_t* changed) {
     extern __shared__ uint32_t snbr[];
-    if (!d.first) load_graph(d, snbr);
+    load_graph(d, snbr);
     if (blockIdx.x == 0 && threadIdx.x < 3) d.count[threadIdx.x] = 0ull;
     const int lane = threadIdx.x & 31;
     const uint32_t nwarps = gridDim.x * (blockDim.x >> 5);
@@ -516,7 +518,7 @@ __global__ void __launch_bounds__(256) k_v2_begin(V2Dev d, uint8_t* lev0, uint8_
             d.fin1[c] = 0;
             d.fin2[c] = 0;
         }
-        if (d.first || !ch) continue;
+        if (!ch) continue;
         Mask<W> m;
 #pragma unroll
         for (int j = 0; j < W; ++j) m.w[j] = j < d.rwp ? __ldg(&d.marked[(size_t)c * d.rwp + j]) : 0u;
@@ -918,9 +920,12 @@ __global__ void __launch_bounds__(256) k_v2_root(V2Dev d) {
     if (lane == 0 && cnt) atomicAdd(d.count, (unsigned long long)cnt);
 }
 
-// Apply the buffered marks (v2:541-557).
+// Apply the buffered marks (v2:541-557).  The pass's three counts, final by now, go to the host's pinned
+// words from here: a copy of its own cost a pass of the smallest solves 4 us.
 __global__ void k_v2_apply(uint8_t* table, uint32_t* marked, uint8_t* newval, uint8_t* changed,
-                           uint32_t C, int n, int rwp) {
+                           uint32_t C, int n, int rwp, const unsigned long long* count,
+                           volatile unsigned long long* out) {
+    if (blockIdx.x == 0 && threadIdx.x < 3) out[threadIdx.x] = count[threadIdx.x];
     const size_t total = (size_t)C * n;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
          i += (size_t)gridDim.x * blockDim.x) {
@@ -935,22 +940,26 @@ __global__ void k_v2_apply(uint8_t* table, uint32_t* marked, uint8_t* newval, ui
     }
 }
 
-__global__ void k_v2_init(uint8_t* table, uint32_t* marked, const uint16_t* configs, uint32_t C,
-                          int n, int k, int rwp, unsigned long long* caps_out) {
-    unsigned caps = 0;
+// initializeCaptures over a table of unmarked bytes: the captures' bytes and the marked rows, written
+// whole, and what the first pass begins with: counters and flags cleared (no configuration counts as
+// changed, leaves at captures alone are never available).
+__global__ void k_v2_init(uint8_t* table, uint32_t* marked, uint8_t* changed, uint8_t* fin1, uint8_t* fin2,
+                          unsigned long long* count, const uint16_t* configs, uint32_t C, int n, int k, int rwp) {
+    if (blockIdx.x == 0 && threadIdx.x < 3) count[threadIdx.x] = 0ull;
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x) {
+        changed[c] = 0;
+        fin1[c] = 0;
+        fin2[c] = 0;
+        for (int w = 0; w < rwp; ++w) marked[(size_t)c * rwp + w] = 0u;
         int prev = -1;
         for (int i = 0; i < k; ++i) {
             const int r = configs[(size_t)c * k + i];
             if (r == prev) continue;
             prev = r;
-            ++caps;
             table[(size_t)c * n + r] = 1;
             marked[(size_t)c * rwp + (r >> 5)] |= 1u << (r & 31);
         }
     }
-    caps = __reduce_add_sync(0xFFFFFFFFu, caps);
-    if ((threadIdx.x & 31) == 0 && caps) atomicAdd(caps_out, (unsigned long long)caps);
 }
 
 // out[C] = OR over C' in T(C) of in[C']  (one cop step of the dirty-region dilation).
@@ -1144,6 +1153,8 @@ int v2_create(V2Solver** out, cr_block_cache* cache, const cr_solver_kit& kit, c
     s->h_pinned = kit.pinned;
     s->e0 = kit.ev[0];
     s->e1 = kit.ev[1];
+    s->i0 = kit.ev[2];
+    s->i1 = kit.ev[3];
     s->st = st; s->num_sms = num_sms; s->n = n; s->k = k; s->p = p; s->C = C;
     s->rw = (n + 31) / 32;
     s->rwp = round_words(s->rw);
@@ -1187,24 +1198,17 @@ void v2_destroy(V2Solver* s) {
     delete s;
 }
 
-int v2_init(V2Solver* s, cr_solve_stats* stats, std::string* err) {
+int v2_init(V2Solver* s, std::string* err) {
     cudaStream_t st = s->st;
-    V2_CUDA(cudaEventRecord(s->e0, st));
+    V2_CUDA(cudaEventRecord(s->i0, st));
     V2_CUDA(cudaMemsetAsync(s->table, kUnmarked, (size_t)s->C * s->n, st));
-    V2_CUDA(cudaMemsetAsync(s->marked, 0, (size_t)s->C * s->rwp * 4, st));
     V2_CUDA(cudaMemsetAsync(s->newval, kV2None, (size_t)s->C * s->n, st));
     V2_CUDA(cudaMemsetAsync(s->val1, kV2None, (size_t)s->C * s->n, st));
-    V2_CUDA(cudaMemsetAsync(s->changed, 0, s->C, st));
-    V2_CUDA(cudaMemsetAsync(s->counters, 0, 4 * sizeof(unsigned long long), st));
     const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 255) / 256, (uint64_t)s->num_sms * 4));
-    k_v2_init<<<grid, 256, 0, st>>>(s->table, s->marked, s->configs, s->C, s->n, s->k, s->rwp, s->counters);
+    k_v2_init<<<grid, 256, 0, st>>>(s->table, s->marked, s->changed, s->fin1, s->fin2, s->counters, s->configs, s->C, s->n,
+                                    s->k, s->rwp);
     V2_CUDA(cudaGetLastError());
-    V2_CUDA(cudaEventRecord(s->e1, st));
-    V2_CUDA(cudaStreamSynchronize(st));
-    float ms = 0;
-    cudaEventElapsedTime(&ms, s->e0, s->e1);
-    stats->init_ms = ms;
-    stats->kernel_launches = 1;
+    V2_CUDA(cudaEventRecord(s->i1, st));
     s->first = true;
     s->hstats = cr_v2_hash_stats{};
     s->hstats.capacity = s->hcap;
@@ -1282,15 +1286,16 @@ int v2_pass(V2Solver* s, uint64_t* found, cr_solve_stats* stats, std::string* er
     const uint64_t pairs = (uint64_t)s->C * s->n;
     const int grid_cfg = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 7) / 8, (uint64_t)s->num_sms * 8));
     const int grid_cfg_small = (int)std::max<uint64_t>(1, std::min<uint64_t>((s->C + 255) / 256, (uint64_t)s->num_sms * 4));
-    int launches = 1;
-    switch (s->W) {
-        case 1: launch_v2_begin<1>(s, d, grid_cfg, sm); break;
-        case 2: launch_v2_begin<2>(s, d, grid_cfg, sm); break;
-        case 4: launch_v2_begin<4>(s, d, grid_cfg, sm); break;
-        case 8: launch_v2_begin<8>(s, d, grid_cfg, sm); break;
-        default: launch_v2_begin<16>(s, d, grid_cfg, sm); break;
-    }
+    int launches = 0;
     if (!s->first) {
+        switch (s->W) {
+            case 1: launch_v2_begin<1>(s, d, grid_cfg, sm); break;
+            case 2: launch_v2_begin<2>(s, d, grid_cfg, sm); break;
+            case 4: launch_v2_begin<4>(s, d, grid_cfg, sm); break;
+            case 8: launch_v2_begin<8>(s, d, grid_cfg, sm); break;
+            default: launch_v2_begin<16>(s, d, grid_cfg, sm); break;
+        }
+        ++launches;
         for (int j = 1; j < s->p; ++j) {
             const uint8_t* in = s->lev + (size_t)(j - 1) * s->C;
             uint8_t* out = s->lev + (size_t)j * s->C;
@@ -1312,11 +1317,11 @@ int v2_pass(V2Solver* s, uint64_t* found, cr_solve_stats* stats, std::string* er
     }
     if (s->lean) cudaMemsetAsync(s->changed, 0, s->C, st);
     const int grid_apply = (int)std::max<uint64_t>(1, std::min<uint64_t>((pairs + 255) / 256, (uint64_t)s->num_sms * 8));
-    k_v2_apply<<<grid_apply, 256, 0, st>>>(s->table, s->marked, s->newval, s->changed, s->C, s->n, s->rwp);
+    k_v2_apply<<<grid_apply, 256, 0, st>>>(s->table, s->marked, s->newval, s->changed, s->C, s->n, s->rwp, s->counters,
+                                           s->h_pinned);
     launches += 1;
     V2_CUDA(cudaGetLastError());
     V2_CUDA(cudaEventRecord(s->e1, st));
-    V2_CUDA(cudaMemcpyAsync(s->h_pinned, s->counters, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
     V2_CUDA(cudaStreamSynchronize(st));
     *found = s->h_pinned[0];
     s->hstats.child_visits += s->h_pinned[1];

@@ -20,7 +20,7 @@ int v2_create(V2Solver** out, cr_block_cache* cache, const cr_solver_kit& kit, c
               uint32_t C, bool lean, std::string* err);
 void v2_destroy(V2Solver* s);
 bool v2_shed(V2Solver* s);   // gives the plain values' memory back; false = it has none
-int v2_init(V2Solver* s, cr_solve_stats* stats, std::string* err);
+int v2_init(V2Solver* s, std::string* err);   // enqueued, between the kit's events 2 and 3
 int v2_pass(V2Solver* s, uint64_t* found, cr_solve_stats* stats, std::string* err);
 void v2_verdict(V2Solver* s, unsigned long long* best_key);
 const uint8_t* v2_table(const V2Solver* s);

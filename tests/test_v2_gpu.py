@@ -76,3 +76,18 @@ def test_v2_table_file_round_trip(gpu_ctx, tmp_path):
             with pytest.raises(N.CrGpuError) as e:
                 u.load_table_file(path)
             assert e.value.code in (1, 7)
+
+
+def test_v2_launches_of_a_pass(gpu_ctx):
+    """The smallest solves are launches and their gaps: initializeCaptures is one kernel and the first
+    pass begins where it ends (plain values, depth-1 values, roots, marks); a later pass adds the clears
+    and unsafe rows, and a dilation per further ply."""
+    for p, first, later in ((1, 3, 4), (2, 4, 6)):
+        with Solver(gpu_ctx, G.delaunay_thinned(13, 3), 2, p, N.CR_RULES_V2) as s:
+            s.init()
+            launches = [s.stats().kernel_launches]
+            while s.step():
+                launches.append(s.stats().kernel_launches)
+            launches.append(s.stats().kernel_launches)
+            assert len(launches) > 2
+            assert [b - a for a, b in zip([0, *launches], launches)] == [1, first] + [later] * (len(launches) - 2)
