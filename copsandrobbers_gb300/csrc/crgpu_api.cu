@@ -504,10 +504,10 @@ static int alloc_v1(cr_solver* s, SmallArrays& small) {
             nbr[(size_t)u * s->rwp + (v >> 5)] |= 1u << (v & 31);
             rcol[fill[v]++] = (uint16_t)u;  // in-neighbours of v, ascending u
         }
-    // robbers without a move (the last column's vacuous AND), cops without a move
+    // robbers without a walk of p moves (the last column's vacuous AND), cops without a move
     std::vector<uint32_t> iso(s->rwp, 0), ciso(s->rwp, 0);
     for (int v = 0; v < s->n; ++v) {
-        if (s->h_rp[v + 1] == s->h_rp[v]) iso[v >> 5] |= 1u << (v & 31);
+        if (list_at[v + 1] == list_at[v]) iso[v >> 5] |= 1u << (v & 31);
         if (crp[v + 1] == crp[v]) ciso[v >> 5] |= 1u << (v & 31);
     }
     if (s->cop_stay != s->robber_stay) {

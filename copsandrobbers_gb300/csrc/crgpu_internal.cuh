@@ -70,7 +70,9 @@ struct DevGraph {
     const uint32_t* rrow_ptr; // n + 1: in-neighbours (predecessor moves)
     const uint16_t* rcol;
     const uint32_t* nbr;      // [n][rwp]: out-neighbour masks
-    const uint32_t* isolated; // [rwp]: vertices without out-neighbours
+    // [rwp]: vertices whose hop set is empty (with p = 1, where the first pass reads it for the cops too:
+    // without out-neighbours)
+    const uint32_t* isolated;
     const uint32_t* rhop;     // [n][rwp]: bit r of row u set iff u is in hop(r) (transposed hop)
     // Uncovered-slot masks for the first pass's closed form (cover_w bytes per mask, 0 = not
     // built; npad = n rounded up to 8).  Bit j of a mask refers to r's j-th out-neighbour:

@@ -141,11 +141,9 @@ __global__ void k_na_binom(uint32_t* B, int n, int k) {
     }
 }
 
-// In-degree counts, out-neighbour masks and the isolated-vertex mask.
-__global__ void k_na_graph(const uint32_t* rp, const uint16_t* col, int n, int rwp, uint32_t* indeg,
-                           uint32_t* nbr, uint32_t* iso) {
+// In-degree counts and out-neighbour masks.
+__global__ void k_na_graph(const uint32_t* rp, const uint16_t* col, int n, int rwp, uint32_t* indeg, uint32_t* nbr) {
     for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n; u += gridDim.x * blockDim.x) {
-        if (rp[u + 1] == rp[u]) atomicOr(&iso[u >> 5], 1u << (u & 31));
         for (uint32_t e = rp[u]; e < rp[u + 1]; ++e) {
             const int v = col[e];
             atomicAdd(&indeg[v], 1u);
@@ -172,8 +170,9 @@ __global__ void k_na_fill(const uint32_t* rp, const uint16_t* col, int n, uint32
         for (uint32_t e = rp[u]; e < rp[u + 1]; ++e) rcol[atomicAdd(&cursor[col[e]], 1u)] = (uint16_t)u;
 }
 
-// Exact-p-hop vertex sets (k_cops_visibility.cpp:245-262, robber self-edges off).
-__global__ void k_na_hop(const uint32_t* nbr, int n, int rwp, int p, uint32_t* hop) {
+// Exact-p-hop vertex sets (k_cops_visibility.cpp:245-262, robber self-edges off), and the vertices whose
+// set is empty.
+__global__ void k_na_hop(const uint32_t* nbr, int n, int rwp, int p, uint32_t* hop, uint32_t* iso) {
     constexpr int W = kNoallocMaxN / 32;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         uint32_t cur[W], nxt[W];
@@ -191,7 +190,12 @@ __global__ void k_na_hop(const uint32_t* nbr, int n, int rwp, int p, uint32_t* h
             }
             for (int w = 0; w < W; ++w) cur[w] = nxt[w];
         }
-        for (int w = 0; w < rwp; ++w) hop[(size_t)r * rwp + w] = cur[w];
+        uint32_t any = 0u;
+        for (int w = 0; w < rwp; ++w) {
+            hop[(size_t)r * rwp + w] = cur[w];
+            any |= cur[w];
+        }
+        if (!any) atomicOr(&iso[r >> 5], 1u << (r & 31));
     }
 }
 
@@ -311,11 +315,11 @@ extern "C" int cr_solve_v1_noalloc(const cr_graph* g, int32_t k, int32_t p, void
         uint32_t* cursor = reinterpret_cast<uint32_t*>(base + L.cursor);
         k_na_binom<<<8, 256, 0, st>>>(reinterpret_cast<uint32_t*>(base + L.binom), n, k);
         k_na_graph<<<4, 256, 0, st>>>(d.g.row_ptr, d.g.col, n, rwp, cursor,
-                                      reinterpret_cast<uint32_t*>(base + L.nbr),
-                                      reinterpret_cast<uint32_t*>(base + L.iso));
+                                      reinterpret_cast<uint32_t*>(base + L.nbr));
         k_na_scan<<<1, 1, 0, st>>>(cursor, reinterpret_cast<uint32_t*>(base + L.rrp), n);
         k_na_fill<<<4, 256, 0, st>>>(d.g.row_ptr, d.g.col, n, cursor, reinterpret_cast<uint16_t*>(base + L.rcol));
-        k_na_hop<<<4, 128, 0, st>>>(d.g.nbr, n, rwp, p, reinterpret_cast<uint32_t*>(base + L.hop));
+        k_na_hop<<<4, 128, 0, st>>>(d.g.nbr, n, rwp, p, reinterpret_cast<uint32_t*>(base + L.hop),
+                                    reinterpret_cast<uint32_t*>(base + L.iso));
         k_na_rhop<<<4, 128, 0, st>>>(d.hop, n, rwp, reinterpret_cast<uint32_t*>(base + L.rhop));
         launch_unrank(d.binom, n, k, (uint32_t)C, reinterpret_cast<uint16_t*>(base + L.configs),
                       gsmall > 0 ? gsmall : 1, st);
