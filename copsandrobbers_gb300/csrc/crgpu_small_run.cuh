@@ -15,23 +15,6 @@
 namespace crgpu {
 namespace CR_BODY_NS {
 
-// Column col's row list from its flags, by the whole team.
-__device__ __noinline__ void flags_to_list(const Team& tm, const V1Dev& d, int col) {
-    const uint8_t* f = d.fflag + (size_t)col * d.C;
-    uint32_t* out = d.list + (size_t)col * d.C;
-    const int lane = threadIdx.x & 31;
-    for (uint32_t base = tm.thread() & ~31u; base < d.C; base += tm.threads()) {
-        const uint32_t i = base + lane;
-        const bool set = i < d.C && f[i];
-        const unsigned b = __ballot_sync(0xFFFFFFFFu, set);
-        if (!b) continue;
-        int at = 0;
-        if (lane == 0) at = atomicAdd(&d.meta[col].len, __popc(b));
-        at = __shfl_sync(0xFFFFFFFFu, at, 0);
-        if (set) out[at + __popc(b & ((1u << lane) - 1u))] = i;
-    }
-}
-
 // A pass's end: its count (or the error bits) to the ring, column 0's prep for the next one, and
 // whether there is one.  By one thread, between two barriers.
 __device__ __noinline__ void end_pass(const V1Dev& d, const LoopCtl& c, int i) {
@@ -49,7 +32,7 @@ __device__ void run_passes(const V1Dev& d, const LoopCtl& c, const Team& tm, int
     const unsigned wk = tm.rank, nwk = tm.size;
     const bool lead = tm.thread() == 0;
     // as k_loop_enter: column 1's list after a fused first pass, column 0's prep, the first count
-    if (d.meta[1].compact) flags_to_list(tm, d, 1);
+    if (d.meta[1].compact) team_list_compact(tm, d, 1);
     prep_clear(d, 0, wk, nwk);
     tm.sync();
     if (lead) {
