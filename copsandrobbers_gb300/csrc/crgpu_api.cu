@@ -19,7 +19,7 @@
 namespace crgpu {
 void launch_cop(const V1Dev& d, int col, int nx, int direct, int grid, cudaStream_t st, bool end = false);
 void launch_and(const V1Dev& d, int col, bool p1, int grid, cudaStream_t st, const LoopCtl& loop);
-void launch_init(const V1Dev& d, int grid, cudaStream_t st);
+void launch_init(const V1Dev& d, bool whole, int grid, cudaStream_t st);
 void launch_init_pass1(const V1Dev& d, int num_sms, cudaStream_t st);
 void launch_marks_from_table(const uint8_t* table, uint32_t C, int n, int cols, int rwp, uint32_t* marked,
                              int grid, cudaStream_t st);
@@ -750,17 +750,8 @@ static int v1_init(cr_solver* s) {
     settle_init_time(s);
     CR_CUDA(ctx, cudaEventRecord(s->kit.ev[2], st));
     CR_CUDA(ctx, cudaMemsetAsync(s->d_table, kUnmarked, C * s->n * s->cols, st));
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_marked, 0, (size_t)s->cols * C * s->rwp * 4, st));
-    CR_CUDA(ctx, cudaMemsetAsync(s->d_fflag, 0, (size_t)s->cols * C, st));
-    std::vector<ColMeta> meta(s->cols);
-    for (int c = 0; c < s->cols; ++c) meta[c] = ColMeta{0, kEmptyLo, -1, 0, 0, 0, 0, 0};
-    // capture seeds in columns 0 and 1 (every row: the implicit list); pass 1's column-0
-    // producer appends to column 0's
-    meta[0] = ColMeta{0, 0, 0, 1, (int)std::min<uint64_t>(C, INT32_MAX), 0, -1, 0};
-    meta[1] = ColMeta{0, 0, 0, 0, (int)std::min<uint64_t>(C, INT32_MAX), 1, -1, 0};
-    if (int rc = reset_ctl(s, meta)) return rc;
     V1Dev d = dev_view(s);
-    launch_init(d, s->grid_small, st);
+    launch_init(d, true, s->grid_small, st);
     CR_CUDA(ctx, cudaGetLastError());
     CR_CUDA(ctx, cudaEventRecord(s->kit.ev[3], st));
     s->init_timing = true;

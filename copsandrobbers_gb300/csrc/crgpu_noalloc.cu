@@ -37,7 +37,7 @@ namespace crgpu {
 void launch_cop(const V1Dev& d, int col, int nx, int direct, int grid, cudaStream_t st, bool end = false);
 void launch_and(const V1Dev& d, int col, bool p1, int grid, cudaStream_t st, const LoopCtl& loop);
 void launch_prep(const V1Dev& d, int col, int nx, int grid, cudaStream_t st);
-void launch_init(const V1Dev& d, int grid, cudaStream_t st);
+void launch_init(const V1Dev& d, bool whole, int grid, cudaStream_t st);
 void launch_unrank(const uint32_t* B, int n, int k, uint32_t C, uint16_t* out, int grid, cudaStream_t st);
 bool pull_supported(int S, int rwp);
 size_t cop_smem_bytes(int S, int rwp);
@@ -333,7 +333,7 @@ extern "C" int cr_solve_v1_noalloc(const cr_graph* g, int32_t k, int32_t p, void
         meta[1] = ColMeta{0, 0, 0, 0, rows, 1, -1, 0};
         NA_CUDA(cudaMemcpyAsync(d.meta, meta, sizeof(ColMeta) * cols, cudaMemcpyHostToDevice, st));
         NA_CUDA(cudaMemsetAsync(states_dev, kUnmarked, table_bytes, st));
-        launch_init(d, gsmall > 0 ? gsmall : 1, st);
+        launch_init(d, false, gsmall > 0 ? gsmall : 1, st);
         NA_CUDA(cudaGetLastError());
         unsigned long long caps = 0;
         NA_CUDA(cudaMemcpyAsync(&caps, d.pass_new, sizeof(caps), cudaMemcpyDeviceToHost, st));

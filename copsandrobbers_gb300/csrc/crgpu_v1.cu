@@ -59,7 +59,32 @@ __device__ __forceinline__ bool pass_kernel_begin(const V1Dev& d) {
 }
 
 __global__ void k_prep(V1Dev d, int col, int nx) { prep_body(d, col, nx, blockIdx.x, gridDim.x); }
-__global__ void k_init(V1Dev d, int K) { init_body(d, K, blockIdx.x, gridDim.x); }
+// initializeCaptures; with `whole` also the columns without captures (marked rows and flags cleared, so
+// that only the table's bytes are left to a clear) and the state of a fresh solve: capture seeds in
+// columns 0 and 1 (every row, the implicit list), pass 1's column-0 producer appending to column 0's.
+__global__ void k_init(V1Dev d, int K, bool whole) {
+    if (whole) {
+        if (blockIdx.x == 0) {
+            const int rows = d.C < 0x7FFFFFFFu ? (int)d.C : 0x7FFFFFFF;
+            for (int c = threadIdx.x; c < d.cols; c += blockDim.x)
+                d.meta[c] = c == 0   ? ColMeta{0, 0, 0, 1, rows, 0, -1, 0}
+                            : c == 1 ? ColMeta{0, 0, 0, 0, rows, 1, -1, 0}
+                                     : ColMeta{0, kEmptyLo, -1, 0, 0, 0, 0, 0};
+            if (threadIdx.x < kSyncWords) d.sync[threadIdx.x] = 0u;
+            if (threadIdx.x == 0) *d.err = 0u;
+        }
+        const size_t flags = (size_t)(d.cols - 2) * d.C, words = flags * d.g.rwp;
+        const size_t step = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+        for (size_t i = first; i < flags; i += step) d.fflag[2 * (size_t)d.C + i] = 0;
+        uint32_t* m = d.marked + 2 * (size_t)d.C * d.g.rwp;
+        if (d.g.rwp & 3) {
+            for (size_t i = first; i < words; i += step) m[i] = 0u;
+        } else {
+            for (size_t i = first; i < words / 4; i += step) reinterpret_cast<uint4*>(m)[i] = make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+    init_body(d, K, blockIdx.x, gridDim.x);
+}
 // The first pass in three forms (launch_init_pass1): the run form of rows of one 256-robber block
 // split into whole lane pieces with byte masks (at most 85 registers, 3 blocks of 256 per SM, which
 // measured faster than 64 registers at 4 blocks and than 2 blocks), the tiles, and the general sweep
@@ -330,7 +355,7 @@ void launch_prep(const V1Dev& d, int col, int nx, int grid, cudaStream_t st) {
     k_prep<<<grid, 256, 0, st>>>(d, col, nx);
 }
 
-void launch_init(const V1Dev& d, int grid, cudaStream_t st) { k_init<<<grid, 256, 0, st>>>(d, d.k); }
+void launch_init(const V1Dev& d, bool whole, int grid, cudaStream_t st) { k_init<<<grid, 256, 0, st>>>(d, d.k, whole); }
 
 template <int W, bool SINGLE>
 static void launch_init_pass1_w(const V1Dev& d, int grid, size_t sm, cudaStream_t st) {
