@@ -2477,8 +2477,8 @@ __host__ __device__ inline int and_tile_quads(int rw) { return rw * 32 + 1; }
 // Bound: issue and shared-memory wavefronts, about 25 warp instructions per row at n = 128 where
 // the row-by-row form takes several hundred (its bit loops diverge over the rows of a warp), and
 // in the densest passes the table bytes.  Last columns of a whole solve: G(n, p) n = 128 1016 us
-// row by row, 540 us in tiles; Delaunay n = 199 9.0 and 3.5 ms; n = 389 195 and 58 ms (70 with three
-// words per vertex and half the warps per SM).
+// row by row, 461 us in tiles; Delaunay n = 199 9.0 and 2.6 ms; n = 389 195 and 44 ms (70 with three
+// words per vertex, half the warps per SM and table bytes word by word).
 __device__ CR_BODY_INLINE void and_tile_body(const V1Dev& d, int col, unsigned wk, unsigned nwk) {
     extern __shared__ __align__(16) uint32_t sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -50,8 +50,8 @@
 // k = 2, p = 3 takes 166 ms so.
 //
 // Measured (Delaunay n = 199, k = 2, p = 3, six passes): 94 ms with every dirty depth-1 node's
-// children in the hash table and every leaf's cloud expanded, 8.7 ms so (10.0 ms without the limit of
-// 64 registers, 9.5 ms at 48).
+// children in the hash table and every leaf's cloud expanded, 8.3 ms so (limits of registers were
+// compared at 8.7 ms: 10.0 without one, 9.5 at 48).
 #include <algorithm>
 #include <string>
 #include <vector>

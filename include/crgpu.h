@@ -168,13 +168,13 @@ int cr_solver_load_table_file(cr_solver* s, const char* path);
 
 /* Deduplication of the robber clouds of a v2 solve with p >= 3.  The reference's
  * trajectoryDFS (solvers/k_cops_visibility_v2.cpp:243-341) walks every cop trajectory of every
- * state separately; the device inserts the depth-2 nodes (config, cloud) each pass reaches
- * into a hash table and evaluates each distinct node once.  Counts accumulate from
- * cr_solver_init. */
+ * state separately.  The device keeps the depth-2 nodes (config, robber) whose clouds no cop before
+ * them touched in an array, inserts the others (config, cloud) that a pass has to look at into a
+ * hash table, and evaluates each distinct node once.  Counts accumulate from cr_solver_init. */
 typedef struct cr_v2_hash_stats {
     uint64_t capacity;       /* slots of the table; 0 = no table (v1 rules or p < 3) */
-    uint64_t child_visits;   /* non-terminal depth-2 children generated */
-    uint64_t entries;        /* distinct (config, cloud) nodes stored, summed over fills */
+    uint64_t child_visits;   /* non-terminal depth-2 children looked at, in the array or inserted */
+    uint64_t entries;        /* distinct (config, cloud) nodes stored in the table, summed over fills */
     uint64_t fills;          /* table fills (one per pass, more when depth-1 nodes are chunked) */
 } cr_v2_hash_stats;
 int cr_solver_v2_hash_stats(cr_solver* s, cr_v2_hash_stats* out);
