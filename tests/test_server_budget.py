@@ -127,5 +127,5 @@ def test_a_named_budget_bounds_the_memory_taken(n, k, p, rules):
         free = torch.cuda.mem_get_info()[0]
         assert srv.poll(srv.submit(g, k, p, rules), wait_ms=-1)["status"] == 0
         taken = free - torch.cuda.mem_get_info()[0]
-    # the driver hands out 2 MiB pages: up to one more for each of some dozen blocks
+    # CUDA hands out 2 MiB pages: up to one more for each of some dozen blocks
     assert taken <= budget + 16 * (2 << 20), (taken, budget)
